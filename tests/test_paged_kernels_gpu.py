@@ -1,0 +1,126 @@
+"""The kernels behind b200_paged_attention in bfloat16, each over the sizes where its tiles end, against a plain float64 statement of
+the attention (one sequence at a time, every option of the call)."""
+import ctypes as C
+import math
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def S(pkg):
+    if not torch.cuda.is_available():
+        pytest.skip("needs a GPU")
+    return pkg.serve
+
+
+def seen(o, p):
+    """first key that position p sees"""
+    f = p // o["chunk"] * o["chunk"] if o.get("chunk") else 0
+    return max(f, p - o["window"] + 1) if o.get("window") else f
+
+
+def reference(q, k, v, pos, o):
+    """q [T, H, M, d] at positions pos of ONE sequence with keys k [n, G, M, d], values v [n, G, dv] -> [T, H, M, dv]"""
+    T, H, M, d = q.shape
+    G, n = k.shape[1], k.shape[0]
+    j, p = torch.arange(n), torch.tensor(pos)
+    first = torch.tensor([seen(o, x) for x in pos])
+    ok = (j[None, :] <= p[:, None]) & (j[None, :] >= first[:, None])
+    out = torch.zeros(T, H, M, v.shape[2], dtype=torch.float64)
+    for h in range(H):
+        for m in range(M):
+            s = q[:, h, m] @ k[:, h // (H // G), m].T * o["scale"]
+            if o.get("cap"):
+                s = o["cap"] * torch.tanh(s / o["cap"])
+            if o.get("bias") is not None:
+                s = s + o["bias"][h][(p[:, None] - j[None, :]).clamp(0, o["bias"].shape[1] - 1)]
+            if o.get("sigmoid"):
+                w = torch.sigmoid(s + o["head_bias"][h]) * ok
+            else:
+                s = s.masked_fill(~ok, float("-inf"))
+                sink = o["sink"][h] if o.get("sink") is not None else torch.tensor(math.log(o["denom"]) if o.get("denom") else float("-inf"), dtype=torch.float64)
+                top = torch.maximum(s.amax(1, keepdim=True), sink)
+                e = torch.exp(s - top)
+                w = e / (e.sum(1, keepdim=True) + torch.exp(sink - top))
+            out[:, h, m] = w @ v[:, h // (H // G)]
+    return out
+
+
+def run(S, q, keys, values, table, PR, slot, pos, o, longest, f32=True, workspace=True):
+    """one call over device tensors q [T, H, M, d] (bfloat16), pools [rows, G, M, d] / [rows, G, dv]"""
+    T, H, M, d = q.shape
+    G, dv = values.shape[1], values.shape[2]
+    out = torch.full((T, H, M, dv), float("nan"), dtype=torch.float32 if f32 else torch.bfloat16, device="cuda")
+    keep = [torch.tensor(slot, dtype=torch.int32, device="cuda"), torch.tensor(pos, dtype=torch.int32, device="cuda")]
+    a = S.PagedAttentionArgs()
+    a.q, a.out, a.k_pool, a.v_pool, a.pages, a.max_pages, a.page_rows = q.data_ptr(), out.data_ptr(), keys.data_ptr(), values.data_ptr(), table.data_ptr(), table.shape[1], PR
+    a.slot, a.pos, a.n_tokens, a.heads, a.kv_heads, a.dim, a.vdim = keep[0].data_ptr(), keep[1].data_ptr(), T, H, G, d, dv
+    a.scale, a.softcap, a.denom_bias, a.dtype, a.longest_entry, a.longest_context = o["scale"], o.get("cap", 0.0), o.get("denom", 0.0), S.BF16, longest, max(pos) + 1
+    a.chunk, a.maps, a.out_f32, a.window, a.sigmoid_weights = o.get("chunk", 0), M, int(f32), o.get("window", 0), int(bool(o.get("sigmoid")))
+    for name, key in (("sink", "sink"), ("dist_bias", "bias"), ("head_bias", "head_bias")):
+        if o.get(key) is not None:
+            keep.append(o[key].float().cuda().contiguous())
+            setattr(a, name, keep[-1].data_ptr())
+    if o.get("bias") is not None:
+        a.dist_n = o["bias"].shape[1]
+    need = S.lib().b200_paged_attention_workspace_bytes(T, H * M, dv) if workspace else 0
+    keep.append(torch.empty(max(need, 16), dtype=torch.uint8, device="cuda"))
+    a.workspace, a.workspace_bytes = keep[-1].data_ptr(), need
+    torch.cuda.synchronize()
+    rc = S.lib().b200_paged_attention(C.byref(a), None)
+    torch.cuda.synchronize()
+    assert rc == 0, rc
+    return out.double().cpu()
+
+
+def sequences(g, lens, G, M, d, dv, PR):
+    """keys and values per sequence, and pools in shuffled pages whose foreign rows are NaN: reading one would show"""
+    k = [torch.randn(n, G, M, d, generator=g).bfloat16().double() for n in lens]
+    v = [torch.randn(n, G, dv, generator=g).bfloat16().double() for n in lens]
+    need = [(n + PR - 1) // PR for n in lens]
+    order = torch.randperm(sum(need) + 2, generator=g).tolist()
+    table = torch.zeros(len(lens), max(need), dtype=torch.int32)
+    kp = torch.full(((sum(need) + 2) * PR, G, M, d), float("nan"))
+    vp = torch.full(((sum(need) + 2) * PR, G, dv), float("nan"))
+    for b, n in enumerate(lens):
+        for i in range(need[b]):
+            pg, m = order.pop(), min(PR, n - i * PR)
+            table[b, i] = pg
+            kp[pg * PR:pg * PR + m], vp[pg * PR:pg * PR + m] = k[b][i * PR:i * PR + m], v[b][i * PR:i * PR + m]
+    return k, v, kp.bfloat16().cuda(), vp.bfloat16().cuda(), table.cuda()
+
+
+FORMS = {"plain": {}, "capped": dict(cap=3.0, denom=1.0), "biased": dict(sink=1, bias=40), "blocks": dict(chunk=100), "sigmoid": dict(window=70, sigmoid=1)}
+
+
+def options(form, H, d, g):
+    o = dict(FORMS[form], scale=1.3 / math.sqrt(d))
+    if o.get("bias"):
+        o["bias"], o["sink"] = torch.randn(H, o["bias"], generator=g).float().double(), torch.randn(H, generator=g).float().double() * 3
+    if o.get("sigmoid"):
+        o["head_bias"] = torch.randn(H, generator=g).float().double() - 2
+    return o
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("H,G,M,d,dv,PR", [(2, 2, 1, 128, 128, 64), (8, 4, 1, 128, 128, 16), (6, 2, 1, 64, 64, 64), (8, 1, 1, 64, 128, 48), (4, 2, 2, 128, 256, 64)])
+def test_single_tokens_share_their_context_in_a_cluster(S, form, H, G, M, d, dv, PR):
+    """contexts that end at, before and behind a step of 16 keys, a page and a warp's share. The weights keep 24 bits, so the fp32
+    output is as exact as fp32 sums of a thousand products: 2e-5 of the result's norm"""
+    if M > 1 and FORMS[form].get("sigmoid"):
+        pytest.skip("sigmoid weights have one map")
+    g = torch.Generator().manual_seed(H * d + PR)
+    lens = [1, 15, 16, 17, 63, 65, 300, 1100]
+    o = options(form, H, d, g)
+    k, v, kp, vp, table = sequences(g, lens, G, M, d, dv, PR)
+    q = torch.randn(len(lens), H, M, d, generator=g).bfloat16().double()
+    got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, list(range(len(lens))), [n - 1 for n in lens], o, 1)
+    one = run(S, q[6:7].bfloat16().cuda(), kp, vp, table, PR, [6], [lens[6] - 1], o, 1, workspace=False)
+    for b, n in enumerate(lens):
+        want = reference(q[b:b + 1], k[b], v[b], [n - 1], o)[0]
+        assert float((got[b] - want).norm() / want.norm()) < 2e-5, (b, n)
+        if b == 6:
+            assert float((one[0] - want).norm() / want.norm()) < 2e-5
