@@ -1,17 +1,16 @@
 // tcgen05 / TMEM GEMM for fp16 linears with more than B200_GEMV_MAX_TOKENS rows:
 //   prefill QKV / o / gate_up / down / LM-head (launchLinearGemm, src/kernels/linear.cu:39-104 ->
 //   cublasWrapper::Gemm, cublas_utils.cc:32-71, call sites context_attention.cpp:99,166, ffn.cpp:72,88)
-//   and the batched decode step (8 < B <= 256 sequences), where the same kernel runs "swapped".
+//   and the batched decode step (8 < B <= 256 sequences), where the weights are the tiles' rows.
 //
 //   D[128, BN] (fp32, TMEM) += A_tile[128, 64] * B_tile[BN, 64]^T      (both operands K-major fp16)
 //
-//   normal  : A = x [Nt, K] (tokens on the MMA M axis), B = W [N, K]    -> y[tok, n]   tensor-bound
-//   swapped : A = W [N, K] (weight rows on the M axis), B = x [Nt, K]   -> y[tok, n]   HBM-bound:
-//             every weight byte is read once, Nt <= 256 tokens ride along as the MMA N extent;
-//             optional split-K over gridDim-level units so that N = 4096 projections still fill
-//             148 SMs (fp32 partials in a workspace, reduced by a small epilogue kernel).
+//   normal  : A = x [Nt, K] (tokens on the MMA M axis), B = W [N, K]    -> y[tok, n]   tensor-bound (gemm_tcgen05_kernel)
+//   stream  : A = W [N, K] (weight rows on the M axis), B = x [Nt, K]   -> y[tok, n]   HBM-bound (gemm_stream_kernel, below):
+//             every weight byte is read once, Nt <= 256 tokens ride along as the MMA N extent; the K range of a tile is shared by
+//             a cluster, so that narrow projections still fill the GPU.
 //
-// Structure (one persistent CTA per SM, 192 threads):
+// Structure of gemm_tcgen05_kernel (one persistent CTA per SM, 192 threads):
 //   warp 0    TMA producer: cp.async.bulk.tensor.2d (UTMALDG) of 128B-swizzled [rows x 64] boxes
 //             into a STAGES-deep smem ring, completion on mbarriers (expect_tx);
 //   warp 1    allocates TMEM, then one elected lane issues tcgen05.mma.cta_group::1.kind::f16
@@ -19,6 +18,9 @@
 //             of a tile, publishes the accumulator;
 //   warps 2-5 epilogue: tcgen05.ld (LDTM) 32 lanes x 32 columns per instruction, convert, store;
 //             two accumulator stages in TMEM so the epilogue of tile i overlaps the MMAs of i+1.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -27,6 +29,7 @@
 #include "tc_common.cuh"
 
 namespace b200 {
+namespace cg = cooperative_groups;
 
 constexpr int kBM = 128;           // MMA M (rows of A per tile)
 constexpr int kBK = 64;            // K per stage: 64 fp16 = one 128-byte swizzle row
@@ -34,19 +37,20 @@ constexpr int kGemmThreads = 192;  // producer, MMA, 4 epilogue warps
 
 struct GemmParams {
     void* C;            // fp16 [tokens, ldc]
-    float* partial;     // split-K workspace [splits][tokens][ldc] (swapped mode), or nullptr
     const void* bias;   // fp16 [N_out] or nullptr
-    int rows_a;         // valid rows of the A operand (tokens in normal mode, N_out in swapped mode)
+    int rows_a;         // valid rows of the A operand (tokens in normal mode, N_out in stream mode)
     int rows_b;         // valid rows of the B operand
     int K;
     int ldc;            // = N_out
     int tokens;
-    int m_tiles, n_tiles, splits, k_blocks;
+    int m_tiles, n_tiles, k_blocks;
+    int splits;         // stream mode: CTAs (one cluster) that share a tile's K range
     int in_bf16;        // operands are bfloat16 instead of fp16 (same tiles, other instruction descriptor)
     int out_kind;       // element type of C: 0 fp16 (rounding points of the reference sequence), 1 bfloat16, 2 fp32
+    int wide_store;     // stream mode: C is 16-byte aligned
     int glu_act;        // GLU epilogue: 0 silu, 1 gelu in its tanh form, 2 clamped at glu_limit (out_kind 1 / 2 only)
     float glu_limit;
-    int unary;          // plain epilogue: 0 none, 1 the square of relu on every output (after the split-K sum, if any)
+    int unary;          // plain epilogue: 0 none, 1 the square of relu on every output
 };
 __device__ __forceinline__ float gemm_unary(float v, int unary) {
     if (unary == 1) { v = fmaxf(v, 0.f); v *= v; }
@@ -90,7 +94,7 @@ __device__ __forceinline__ void store1(void* C, size_t idx, float f, int kind) {
 // accumulator holds gate in columns [0,128) and up in [128,256) of the same 128 features, and the epilogue
 // writes silu(gate)*up (launchAct, act_kernel.cu:57) straight to out [tokens, inter]: the [tokens, 2*inter]
 // intermediate of ffn.cpp:72-80 is never stored.
-template <int BN, bool SWAP, bool GLU = false>
+template <int BN, bool GLU = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const GemmParams p) {
@@ -128,18 +132,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     pdl_launch_dependents();
     pdl_wait();   // x (and, for PDL chains, the previous kernel's output) must be complete
 
-    const int units = p.m_tiles * p.n_tiles * p.splits;
+    const int units = p.m_tiles * p.n_tiles;
 
     if (warp == 0) {
         // ================= TMA producer =================
         int stage = 0;
         uint32_t phase = 0;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
-            const int mt = u % p.m_tiles, rest = u / p.m_tiles;
-            const int nt = rest % p.n_tiles, sp = rest / p.n_tiles;
-            const int kb0 = (int)((long long)p.k_blocks * sp / p.splits);
-            const int kb1 = (int)((long long)p.k_blocks * (sp + 1) / p.splits);
-            for (int kb = kb0; kb < kb1; ++kb) {
+            const int mt = u % p.m_tiles, nt = u / p.m_tiles;
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
                 mbar_wait(&empty_bar[stage], phase ^ 1);
                 if (lane == 0) {
                     unsigned char* sa = tiles + (size_t)stage * S::kStageBytes;
@@ -165,13 +166,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         int acc = 0;
         uint32_t acc_phase = 0;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
-            const int sp = (u / p.m_tiles) / p.n_tiles;
-            const int kb0 = (int)((long long)p.k_blocks * sp / p.splits);
-            const int kb1 = (int)((long long)p.k_blocks * (sp + 1) / p.splits);
             mbar_wait(&acc_empty[acc], acc_phase ^ 1);   // epilogue has drained this accumulator
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-            for (int kb = kb0; kb < kb1; ++kb) {
+            for (int kb = 0; kb < p.k_blocks; ++kb) {
                 mbar_wait(&full_bar[stage], phase);
                 tc_fence_after();
                 if (lane == 0) {
@@ -181,14 +179,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k)
                         umma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
-                                 (kb > kb0 || k > 0) ? 1u : 0u);
+                                 (kb > 0 || k > 0) ? 1u : 0u);
                     umma_commit(&empty_bar[stage]);                 // smem stage reusable when the MMAs retire
-                    if (kb == kb1 - 1) umma_commit(&acc_full[acc]);  // accumulator complete
+                    if (kb == p.k_blocks - 1) umma_commit(&acc_full[acc]);  // accumulator complete
                 }
                 __syncwarp();
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
-            if (kb1 == kb0 && lane == 0) umma_commit(&acc_full[acc]);  // empty K range (never with K > 0)
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1;
         }
@@ -201,8 +198,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int ok = p.out_kind;
         const __half* bias = reinterpret_cast<const __half*>(p.bias);
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
-            const int mt = u % p.m_tiles, rest = u / p.m_tiles;
-            const int nt = rest % p.n_tiles, sp = rest / p.n_tiles;
+            const int mt = u % p.m_tiles, nt = u / p.m_tiles;
             mbar_wait(&acc_full[acc], acc_phase);
             tc_fence_after();
             const int row = mt * kBM + quarter * 32 + lane;   // row of the A operand / of D
@@ -241,48 +237,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 uint32_t v[32];
                 tmem_ld_32x32(taddr + (uint32_t)c0, v);
                 const int col0 = nt * BN + c0;   // first row of the B operand covered by this chunk
-                if (!SWAP) {
-                    // row = token, col = output feature: 32 consecutive features per thread
-                    if (row < p.tokens && col0 < p.rows_b) {
-                        const size_t dst = (size_t)row * p.ldc + col0;
-                        if (col0 + 32 <= p.rows_b && (p.ldc & 7) == 0) {
+                // row = token, col = output feature: 32 consecutive features per thread
+                if (row < p.tokens && col0 < p.rows_b) {
+                    const size_t dst = (size_t)row * p.ldc + col0;
+                    if (col0 + 32 <= p.rows_b && (p.ldc & 7) == 0) {
 #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                                float f[8];
+                        for (int q = 0; q < 4; ++q) {
+                            float f[8];
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) {
-                                    f[e] = __uint_as_float(v[q * 8 + e]);
-                                    if (bias) f[e] += __half2float(bias[col0 + q * 8 + e]);
-                                    f[e] = gemm_unary(f[e], p.unary);
-                                }
-                                store8(C, dst + q * 8, f, ok);
+                            for (int e = 0; e < 8; ++e) {
+                                f[e] = __uint_as_float(v[q * 8 + e]);
+                                if (bias) f[e] += __half2float(bias[col0 + q * 8 + e]);
+                                f[e] = gemm_unary(f[e], p.unary);
                             }
-                        } else {
-                            // unrolled with a predicate: a run-time index would move v[] to local memory (no L1 behind
-                            // it with the 227 KB carve-out) for EVERY path of the epilogue
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                if (col0 + j >= p.rows_b) continue;
-                                float f = __uint_as_float(v[j]);
-                                if (bias) f += __half2float(bias[col0 + j]);
-                                store1(C, dst + j, gemm_unary(f, p.unary), ok);
-                            }
+                            store8(C, dst + q * 8, f, ok);
                         }
-                    }
-                } else {
-                    // row = output feature, col = token: lanes write consecutive features of one token
-                    if (row < p.rows_a) {
-                        const float bv = (bias && !p.partial) ? __half2float(bias[row]) : 0.f;
+                    } else {
+                        // unrolled with a predicate: a run-time index would move v[] to local memory (no L1 behind
+                        // it with the 227 KB carve-out) for EVERY path of the epilogue
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
-                            const int tok = col0 + j;
-                            if (tok < p.tokens) {
-                                const float f = __uint_as_float(v[j]);
-                                if (p.partial)
-                                    p.partial[((size_t)sp * p.tokens + tok) * p.ldc + row] = f;
-                                else
-                                    store1(C, (size_t)tok * p.ldc + row, gemm_unary(f + bv, p.unary), ok);
-                            }
+                            if (col0 + j >= p.rows_b) continue;
+                            float f = __uint_as_float(v[j]);
+                            if (bias) f += __half2float(bias[col0 + j]);
+                            store1(C, dst + j, gemm_unary(f, p.unary), ok);
                         }
                     }
                 }
@@ -302,36 +280,179 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
-// split-K reduction: y[tok, n] = half(sum_s partial[s, tok, n] + bias[n])
-__global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* __restrict__ partial, const __half* __restrict__ bias, void* __restrict__ y,
-                     int splits, size_t elems, int ldc, int out_kind, int unary) {
-    pdl_wait();
-    const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (i >= elems) return;
-    float4 acc = *reinterpret_cast<const float4*>(partial + i);
-    for (int s = 1; s < splits; ++s) {
-        const float4 t = *reinterpret_cast<const float4*>(partial + (size_t)s * elems + i);
-        acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+// Few token rows: the weights stream through the M axis, 128 rows of W per tile, and a cluster of `splits` CTAs shares a tile's K range.
+// What bounds it is the weights' way from HBM, so what counts is how much of them is in flight and how few things follow: every CTA has
+// up to 100 KB of its share under way before the first product, two CTAs fit an SM, and the partial sums meet in shared memory (rank
+// order) instead of a workspace and a second launch.
+// GLU: a tile is 64 gate rows and the 64 up rows of the same features (W = [2 * rows_a, K], rows_a = features).
+// Measured, 8 rows, 2048 -> 4096, fp32 out: the persistent kernel with partial sums in global memory and a reduction launch 11.2 us, this 8.5 us.
+template <int BN>
+struct StreamSmem {
+    static constexpr int kStageBytes = (kBM + BN) * kBK * 2;
+    static constexpr int kStages = BN <= 32 ? 5 : BN <= 64 ? 4 : BN <= 128 ? 3 : 4;
+    static constexpr int kPerSm = BN <= 128 ? 2 : 1;
+    static constexpr int kTotal = kStages * kStageBytes + (2 * kStages + 1) * 8 + 16 + 1024;
+    static_assert(BN * kBM * 4 <= kStages * kStageBytes, "the partial sums take the place of the stages");
+};
+constexpr int kStreamMaxSplits = 8;
+
+template <int BN, bool GLU>
+__global__ void __launch_bounds__(kGemmThreads, StreamSmem<BN>::kPerSm)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+    using S = StreamSmem<BN>;
+    constexpr int STAGES = S::kStages;
+    constexpr uint32_t A_BYTES = kBM * kBK * 2, B_BYTES = BN * kBK * 2;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * S::kStageBytes);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_full = empty_bar + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* om = reinterpret_cast<float*>(tiles);   // [tokens][128]: this CTA's sums, once the stages have been used
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sp = blockIdx.x % p.splits, mt = blockIdx.x / p.splits;
+    const int kb0 = (int)((long long)p.k_blocks * sp / p.splits), kb1 = (int)((long long)p.k_blocks * (sp + 1) / p.splits);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        *dead = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&map_a);
+        tma_prefetch_desc(&map_b);
     }
-    if (bias) {
-        const int n = (int)(i % (size_t)ldc);
-        acc.x += __half2float(bias[n]); acc.y += __half2float(bias[n + 1]);
-        acc.z += __half2float(bias[n + 2]); acc.w += __half2float(bias[n + 3]);
-    }
+    if (warp == 1) tmem_alloc(tmem_slot, BN);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
     pdl_launch_dependents();
-    acc.x = gemm_unary(acc.x, unary); acc.y = gemm_unary(acc.y, unary);
-    acc.z = gemm_unary(acc.z, unary); acc.w = gemm_unary(acc.w, unary);
-    if (out_kind == 0) {
-        __half2* out = reinterpret_cast<__half2*>(reinterpret_cast<__half*>(y) + i);
-        out[0] = __floats2half2_rn(acc.x, acc.y);
-        out[1] = __floats2half2_rn(acc.z, acc.w);
-    } else if (out_kind == 1) {
-        __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(y) + i);
-        out[0] = __floats2bfloat162_rn(acc.x, acc.y);
-        out[1] = __floats2bfloat162_rn(acc.z, acc.w);
-    } else
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + i) = acc;
+    pdl_wait();
+
+    if (warp == 0) {
+        int stage = 0;
+        uint32_t phase = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            mbar_wait_or_leave(&empty_bar[stage], phase ^ 1, dead);
+            if (lane == 0) {
+                unsigned char* sa = tiles + (size_t)stage * S::kStageBytes;
+                mbar_expect_tx(&full_bar[stage], A_BYTES + B_BYTES);
+                if (GLU) {
+                    tma_load_2d(sa, &map_a, kb * kBK, mt * 64, &full_bar[stage]);
+                    tma_load_2d(sa + A_BYTES / 2, &map_a, kb * kBK, p.rows_a + mt * 64, &full_bar[stage]);
+                } else
+                    tma_load_2d(sa, &map_a, kb * kBK, mt * kBM, &full_bar[stage]);
+                tma_load_2d(sa + A_BYTES, &map_b, kb * kBK, 0, &full_bar[stage]);
+            }
+            __syncwarp();
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc_f16(kBM, BN) | (p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+        int stage = 0;
+        uint32_t phase = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
+            mbar_wait_or_leave(&full_bar[stage], phase, dead);
+            tc_fence_after();
+            if (lane == 0) {
+                const uint32_t sa = smem_u32(tiles + (size_t)stage * S::kStageBytes);
+                const uint64_t da = make_kmajor_sw128_desc(sa), db = make_kmajor_sw128_desc(sa + A_BYTES);
+#pragma unroll
+                for (int k = 0; k < kBK / kUmmaK; ++k)
+                    umma_f16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                umma_commit(&empty_bar[stage]);
+                if (kb == kb1 - 1) umma_commit(acc_full);
+            }
+            __syncwarp();
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+    } else {
+        const int quarter = warp & 3;
+        mbar_wait_or_leave(acc_full, 0, dead);   // every load has landed and every product has read its stage
+        const bool gone = *dead != 0;
+        tc_fence_after();
+        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN && c0 < p.tokens; c0 += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(taddr + (uint32_t)c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (c0 + j < p.tokens) om[(c0 + j) * kBM + quarter * 32 + lane] = gone ? __int_as_float(0x7fffffff) : __uint_as_float(v[j]);
+        }
+        tc_fence_before();
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    if (p.splits > 1) cluster.sync();
+    else __syncthreads();
+    {
+        constexpr int F = GLU ? 64 : kBM;                 // output features of the tile
+        const int total = p.tokens * (F / 4), share = (total + p.splits - 1) / p.splits;
+        const float* part[kStreamMaxSplits];
+#pragma unroll
+        for (int q = 0; q < kStreamMaxSplits; ++q) part[q] = q < p.splits ? cluster.map_shared_rank(om, q) : nullptr;
+        auto sum4 = [&](int at) {
+            float4 t[kStreamMaxSplits], acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < kStreamMaxSplits; ++q)
+                if (q < p.splits) t[q] = *reinterpret_cast<const float4*>(part[q] + at);
+#pragma unroll
+            for (int q = 0; q < kStreamMaxSplits; ++q)
+                if (q < p.splits) {
+                    if (q == 0) acc = t[0];
+                    else { acc.x += t[q].x; acc.y += t[q].y; acc.z += t[q].z; acc.w += t[q].w; }
+                }
+            return acc;
+        };
+        const __half* bias = reinterpret_cast<const __half*>(p.bias);
+        for (int i = sp * share + (int)threadIdx.x; i < min(total, (sp + 1) * share); i += kGemmThreads) {
+            const int tok = i / (F / 4), f0 = i % (F / 4) * 4, n = mt * F + f0;
+            if (n >= p.rows_a) continue;
+            const float4 s4 = sum4(tok * kBM + f0);
+            float f[4] = {s4.x, s4.y, s4.z, s4.w};
+            if (GLU) {
+                const float4 u4 = sum4(tok * kBM + 64 + f0);
+                const float u[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    f[e] = p.glu_act == 2 ? glu_clamp_f(f[e], u[e], p.glu_limit) : (p.glu_act ? gelu_tanh_f(f[e]) : f[e] / (1.f + expf(-f[e]))) * u[e];
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (bias && n + e < p.rows_a) f[e] += __half2float(bias[n + e]);
+                    f[e] = gemm_unary(f[e], p.unary);
+                }
+            }
+            const size_t dst = (size_t)tok * p.ldc + n;
+            if (n + 4 <= p.rows_a && (p.ldc & 3) == 0 && p.wide_store) {
+                if (p.out_kind == 2) *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C) + dst) = make_float4(f[0], f[1], f[2], f[3]);
+                else {
+                    uint2 v;
+                    if (p.out_kind == 0) {
+                        const __half2 a = __floats2half2_rn(f[0], f[1]), b = __floats2half2_rn(f[2], f[3]);
+                        v = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+                    } else {
+                        const __nv_bfloat162 a = __floats2bfloat162_rn(f[0], f[1]), b = __floats2bfloat162_rn(f[2], f[3]);
+                        v = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+                    }
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.C) + dst) = v;
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < p.rows_a) store1(p.C, dst + e, f[e], p.out_kind);
+            }
+        }
+    }
+    if (p.splits > 1) cluster.sync();   // nobody leaves while its sums are read
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, BN);
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -391,9 +512,9 @@ bool make_tma_map_2d(CUtensorMap* out, const void* ptr, long long rows, int K, i
     return true;
 }
 
-template <int BN, bool SWAP, bool GLU = false>
+template <int BN, bool GLU = false>
 static int gemm_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int grid, cudaStream_t s) {
-    auto kern = gemm_tcgen05_kernel<BN, SWAP, GLU>;
+    auto kern = gemm_tcgen05_kernel<BN, GLU>;
     static unsigned long long attr_done = 0;   // per instantiation, one bit per device
     {
         cudaError_t e = ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), GemmSmem<BN>::kTotal, attr_done);
@@ -404,17 +525,49 @@ static int gemm_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
     return (int)e;
 }
 
-// split-K factor for the swapped (weight-streaming) mode: minimise rounds x K-blocks per unit
-static int pick_splits(int m_tiles, int k_blocks, int sms) {
-    int best = 1;
-    long long best_cost = -1;
-    for (int s = 1; s <= 16 && k_blocks / s >= 4; ++s) {
-        const long long rounds = ((long long)m_tiles * s + sms - 1) / sms;
-        const long long per = (k_blocks + s - 1) / s;
-        const long long cost = rounds * (per + 2) + (s > 1 ? s : 0);   // +2: tile prologue/epilogue; +s: partial traffic
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
+template <int BN, bool GLU>
+static int stream_launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, cudaStream_t s) {
+    auto kern = gemm_stream_kernel<BN, GLU>;
+    static unsigned long long attr_done = 0;
+    cudaError_t e = ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), StreamSmem<BN>::kTotal, attr_done);
+    if (e != cudaSuccess) return (int)e;
+    // as many CTAs per tile as one wave takes, each with two K blocks at least
+    p.splits = std::max(1, std::min({kStreamMaxSplits, sm_count() * StreamSmem<BN>::kPerSm / p.m_tiles, p.k_blocks / 2}));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(p.m_tiles * p.splits));
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = StreamSmem<BN>::kTotal;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)p.splits;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (pdl_enabled()) {
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
     }
-    return best;
+    e = cudaLaunchKernelEx(&cfg, kern, ma, mb, p);
+    count_launch();
+    return (int)e;
+}
+
+// M <= 256 token rows (GLU: 128) against W = [N, K] (GLU: [2 N, K], N % 64 == 0)
+static int gemm_stream(const void* x, const void* W, GemmParams p, int M, int N, int K, bool glu, cudaStream_t s) {
+    const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256, F = glu ? 64 : kBM;
+    p.rows_a = N; p.rows_b = M;
+    p.m_tiles = (N + F - 1) / F; p.n_tiles = 1;
+    p.wide_store = (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
+    CUtensorMap ma, mb;
+    if (!make_tma_map_2d(&ma, W, glu ? 2ll * N : N, K, F) || !make_tma_map_2d(&mb, x, M, K, BN)) return B200_EUNSUPPORTED;
+    switch (BN) {
+        case 32: return glu ? stream_launch<32, true>(ma, mb, p, s) : stream_launch<32, false>(ma, mb, p, s);
+        case 64: return glu ? stream_launch<64, true>(ma, mb, p, s) : stream_launch<64, false>(ma, mb, p, s);
+        case 128: return glu ? stream_launch<128, true>(ma, mb, p, s) : stream_launch<128, false>(ma, mb, p, s);
+        default: return stream_launch<256, false>(ma, mb, p, s);
+    }
 }
 
 int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, cudaStream_t s,
@@ -426,6 +579,19 @@ int gemm_min_tokens() {
     static int v = -1;
     if (v < 0) { const char* e = getenv("B200_GEMM_MIN_TOKENS"); v = e ? atoi(e) : 5; if (v < 1) v = 1; }
     return v;
+}
+
+// the number of K shares that the sizes of the split-K workspaces count with
+static int pick_splits(int m_tiles, int k_blocks, int sms) {
+    int best = 1;
+    long long best_cost = -1;
+    for (int s = 1; s <= 16 && k_blocks / s >= 4; ++s) {
+        const long long rounds = ((long long)m_tiles * s + sms - 1) / sms;
+        const long long per = (k_blocks + s - 1) / s;
+        const long long cost = rounds * (per + 2) + (s > 1 ? s : 0);   // +2: tile prologue/epilogue; +s: partial traffic
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
+    }
+    return best;
 }
 
 size_t gemm_tcgen05_workspace_bytes(int M, int N, int K) {
@@ -448,41 +614,14 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     p.k_blocks = (K + kBK - 1) / kBK;
     CUtensorMap ma, mb;
     // 161..256 token rows against a wide weight matrix (>= 60 column tiles of 256: most of the 74 cluster slots busy): one row
-    // tile of the two-CTA kernel beats the swapped kernel's 2 waves of 128 x 256 tiles (measured, us: 22016 x 4096 at 192 /
-    // 256 rows: 60.9 / 61.4 vs 75.8 / 87.6; 12288 x 4096 at 256: 35.5 vs 44.0; narrow outputs stay swapped: 4096 x 11008 at
+    // tile of the two-CTA kernel beats a weight-streaming kernel's 2 waves of 128 x 256 tiles (measured, us: 22016 x 4096 at 192 /
+    // 256 rows: 60.9 / 61.4 vs 75.8 / 87.6; 12288 x 4096 at 256: 35.5 vs 44.0; narrow outputs keep streaming their weights: 4096 x 11008 at
     // 256: 38.4 vs 65.5)
     if (M > 160 && M <= 256 && (N + 255) / 256 >= 60) {
         const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, s);
         if (rc2 != B200_EUNSUPPORTED) return rc2;
     }
-    if (M <= 256) {
-        // swapped: weights stream through the M axis, tokens are the N extent
-        const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-        p.rows_a = N; p.rows_b = M;
-        p.m_tiles = (N + kBM - 1) / kBM; p.n_tiles = 1;
-        p.splits = pick_splits(p.m_tiles, p.k_blocks, sms);
-        if (p.splits > 1) {
-            const size_t need = (size_t)p.splits * M * N * sizeof(float);
-            if (!workspace || workspace_bytes < need || (N & 3)) p.splits = 1;
-            else p.partial = reinterpret_cast<float*>(workspace);
-        }
-        if (!make_tma_map_2d(&ma, W, N, K, kBM) || !make_tma_map_2d(&mb, x, M, K, BN)) return B200_EUNSUPPORTED;
-        const int units = p.m_tiles * p.splits;
-        const int grid = units < sms ? units : sms;
-        int rc;
-        switch (BN) {
-            case 32: rc = gemm_launch<32, true>(ma, mb, p, grid, s); break;
-            case 64: rc = gemm_launch<64, true>(ma, mb, p, grid, s); break;
-            case 128: rc = gemm_launch<128, true>(ma, mb, p, grid, s); break;
-            default: rc = gemm_launch<256, true>(ma, mb, p, grid, s); break;
-        }
-        if (rc != 0 || p.splits == 1) return rc;
-        const size_t elems = (size_t)M * N;
-        cudaError_t e = launch_k(splitk_reduce_kernel, dim3((unsigned)((elems / 4 + 255) / 256)), dim3(256), 0, s, true,
-                                 (const float*)p.partial, (const __half*)bias, y, p.splits, elems, N, 0, 0);
-        count_launch();
-        return (int)e;
-    }
+    if (M <= 256) return gemm_stream(x, W, p, M, N, K, false, s);
     // normal: tokens on the M axis; large shapes go to the two-CTA kernel (gemm2_tcgen05.cu)
     {
         const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, s);
@@ -490,15 +629,15 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     }
     const int BN = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : 32;
     p.rows_a = M; p.rows_b = N;
-    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN; p.splits = 1;
+    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN;
     if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, N, K, BN)) return B200_EUNSUPPORTED;
     const int units = p.m_tiles * p.n_tiles;
     const int grid = units < sms ? units : sms;
     switch (BN) {
-        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
-        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
-        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
-        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
+        case 32: return gemm_launch<32>(ma, mb, p, grid, s);
+        case 64: return gemm_launch<64>(ma, mb, p, grid, s);
+        case 128: return gemm_launch<128>(ma, mb, p, grid, s);
+        default: return gemm_launch<256>(ma, mb, p, grid, s);
     }
 }
 
@@ -506,7 +645,7 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
 // fp32 (out_kind as GemmParams), optionally with the GLU epilogue (glu 1 silu, 2 tanh-gelu: W = [2 N, K], gate rows then up
 // rows, N % 128 == 0; glu 4: the clamped gated unit of common.cuh with its limit) or with the square of relu on every output
 // (glu 3: not a GLU, W = [N, K]).
-// Up to 256 token rows the weights stream through the M axis (swapped, split-K); above, tokens are the M axis.
+// Up to 256 token rows (gated units: 128) the weights stream through the M axis; above, tokens are the M axis.
 int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, int glu, void* workspace,
                     size_t workspace_bytes, cudaStream_t s, float glu_limit) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
@@ -523,50 +662,25 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
     CUtensorMap ma, mb;
     if (glu) {
         if (N < 128 || (N & 127)) return B200_EUNSUPPORTED;
+        if (M <= 128) return gemm_stream(x, W, p, M, N, K, true, s);
         p.rows_a = M; p.rows_b = N;
-        p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = N / 128; p.splits = 1;
+        p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = N / 128;
         if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * N, K, 128)) return B200_EUNSUPPORTED;
         const int units = p.m_tiles * p.n_tiles;
-        return gemm_launch<256, false, true>(ma, mb, p, units < sms ? units : sms, s);
+        return gemm_launch<256, true>(ma, mb, p, units < sms ? units : sms, s);
     }
-    if (M <= 256) {
-        const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-        p.rows_a = N; p.rows_b = M;
-        p.m_tiles = (N + kBM - 1) / kBM; p.n_tiles = 1;
-        p.splits = pick_splits(p.m_tiles, p.k_blocks, sms);
-        if (p.splits > 1) {
-            const size_t need = (size_t)p.splits * M * N * sizeof(float);
-            if (!workspace || workspace_bytes < need || (N & 3)) p.splits = 1;
-            else p.partial = reinterpret_cast<float*>(workspace);
-        }
-        if (!make_tma_map_2d(&ma, W, N, K, kBM) || !make_tma_map_2d(&mb, x, M, K, BN)) return B200_EUNSUPPORTED;
-        const int units = p.m_tiles * p.splits;
-        const int grid = units < sms ? units : sms;
-        int rc;
-        switch (BN) {
-            case 32: rc = gemm_launch<32, true>(ma, mb, p, grid, s); break;
-            case 64: rc = gemm_launch<64, true>(ma, mb, p, grid, s); break;
-            case 128: rc = gemm_launch<128, true>(ma, mb, p, grid, s); break;
-            default: rc = gemm_launch<256, true>(ma, mb, p, grid, s); break;
-        }
-        if (rc != 0 || p.splits == 1) return rc;
-        const size_t elems = (size_t)M * N;
-        cudaError_t e = launch_k(splitk_reduce_kernel, dim3((unsigned)((elems / 4 + 255) / 256)), dim3(256), 0, s, true,
-                                 (const float*)p.partial, (const __half*)nullptr, y, p.splits, elems, N, out_kind, p.unary);
-        count_launch();
-        return (int)e;
-    }
+    if (M <= 256) return gemm_stream(x, W, p, M, N, K, false, s);
     const int BN = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : 32;
     p.rows_a = M; p.rows_b = N;
-    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN; p.splits = 1;
+    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN;
     if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, N, K, BN)) return B200_EUNSUPPORTED;
     const int units = p.m_tiles * p.n_tiles;
     const int grid = units < sms ? units : sms;
     switch (BN) {
-        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
-        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
-        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
-        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
+        case 32: return gemm_launch<32>(ma, mb, p, grid, s);
+        case 64: return gemm_launch<64>(ma, mb, p, grid, s);
+        case 128: return gemm_launch<128>(ma, mb, p, grid, s);
+        default: return gemm_launch<256>(ma, mb, p, grid, s);
     }
 }
 size_t gemm_tcgen05_ex_workspace_bytes(int M, int N, int K) {
@@ -590,11 +704,11 @@ int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int 
     p.C = out; p.bias = nullptr; p.K = K; p.ldc = inter; p.tokens = M;
     p.k_blocks = (K + kBK - 1) / kBK;
     p.rows_a = M; p.rows_b = inter;
-    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = inter / 128; p.splits = 1;
+    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = inter / 128;
     CUtensorMap ma, mb;
     if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * inter, K, 128)) return B200_EUNSUPPORTED;
     const int units = p.m_tiles * p.n_tiles, sms = sm_count();
-    return gemm_launch<256, false, true>(ma, mb, p, units < sms ? units : sms, s);
+    return gemm_launch<256, true>(ma, mb, p, units < sms ? units : sms, s);
 }
 
 // y[M, N] = residual[M, N] + half(x W^T): launchLinearGemm followed by launchAddResidual (ffn.cpp:88 +
