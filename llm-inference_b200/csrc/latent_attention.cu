@@ -19,6 +19,8 @@
 //                              scores and the weighted sum (prompt portions and decoded tokens alike; the default for
 //                              bf16 caches); decode batches split long contexts over several CTAs
 //   latent_attn_combine_kernel merges the shares of a split launch and the sink
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "b200_serve.h"
@@ -27,6 +29,7 @@
 #include "rotary.cuh"
 
 namespace b200 {
+namespace cg = cooperative_groups;
 
 constexpr int kMaxRankPerLane = 20;   // rank <= 640 (a latent of 512 with a rotated part of 64 or 128)
 
@@ -438,6 +441,243 @@ __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* _
     }
 }
 
+// ---- bf16, single tokens (decode batches) ------------------------------------------------------------------------------
+// A cluster of CTAs shares one token's cached rows; a CTA holds up to 16 heads of it, the M rows of one mma tile. What bounds it is
+// the way to the rows (a few MB per launch) and the length of the chain behind them, so the rows are requested before anything else,
+// two half tiles of 32 at once, two CTAs fit an SM, and the shares meet in distributed shared memory (rank order) in the same launch.
+//   scores   warp w: keys [16 (w & 1), +16) x 16 heads over a quarter (w >> 1) of the row; the four partial sums meet in shared memory
+//   softmax  warp w: heads 2w, 2w + 1, a key per lane; the weights leave as bfloat16 (as in the tile kernel)
+//   values   warp w: an eighth of the output columns, the rows read transposed by ldmatrix
+// The sink joins in the merge. Measured, 8 sequences of up to 1024 rows of 576, 16 heads, 512 columns out: the tile kernel with its
+// combine launch 53.3 us, this 20.5 us.
+constexpr int kLdMaxCluster = 16;
+
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+
+template <int NT>   // n8 column tiles of the output per warp: out_cols <= 64 * NT
+__global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __restrict__ qa, float* __restrict__ out, const __nv_bfloat16* __restrict__ pool,
+                                                               const int* __restrict__ pages, int max_pages, int page_rows, const int* __restrict__ slot,
+                                                               const int* __restrict__ pos, const float* __restrict__ sink, float scale, int heads, int rank,
+                                                               int window, int out_cols) {
+    using bf = __nv_bfloat16;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int rpad = (rank + 15) & ~15, RS = rpad + 8, splits = gridDim.x;
+    bf* Ks = reinterpret_cast<bf*>(smraw);                     // [2][32][RS]
+    bf* Qs = Ks + 2 * kHalfKeys * RS;                          // [16][RS]
+    float* Ss = reinterpret_cast<float*>(Qs + 16 * RS);        // [4][16][36]: partial scores [head][key]
+    bf* Ps = reinterpret_cast<bf*>(Ss + 4 * 16 * 36);          // [16][40]
+    float* al_s = reinterpret_cast<float*>(Ps + 16 * 40);      // [16]
+    float* ms = al_s + 16;                                     // [16]
+    float* ls = ms + 16;                                       // [16]
+    float* om = reinterpret_cast<float*>(smraw);               // [16][out_cols]: this CTA's share, once the rows have been used
+    const int t = blockIdx.z, h0 = blockIdx.y * 16, warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane / 4, tig = lane % 4;
+    const int p = pos[t], n = min(16, heads - h0), chunks = rpad / 8;
+    const int* list = pages + (size_t)slot[t] * max_pages;
+    const int lo = window > 0 ? max(0, p - window + 1) : 0, first = lo & ~(kHalfKeys - 1);
+    const int halves = (p - first) / kHalfKeys + 1, per = (halves + splits - 1) / splits;
+    const int b0 = blockIdx.x * per, b1 = min(halves, b0 + per);
+    const bool one_page = page_rows % kHalfKeys == 0;
+    auto load_half = [&](int b) {
+        const int k0 = first + b * kHalfKeys;
+        bf* dst0 = Ks + ((b - b0) & 1) * kHalfKeys * RS;
+        const size_t base = one_page ? (size_t)list[k0 / page_rows] * page_rows + k0 % page_rows : 0;
+        for (int i = threadIdx.x; i < kHalfKeys * chunks; i += 256) {
+            const int kr = i / chunks, ch = i - kr * chunks, j = k0 + kr;
+            const bool ok = j <= p && j >= lo && ch * 8 < rank;
+            const size_t row = !ok ? 0 : one_page ? base + kr : (size_t)list[j / page_rows] * page_rows + j % page_rows;
+            const bf* src = ok ? pool + row * rank + ch * 8 : pool;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(dst0 + kr * RS + ch * 8);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+        }
+    };
+    auto close_group = [&]() {
+        __syncwarp();   // the lanes close their group of copies together
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (b0 < b1) load_half(b0);
+    close_group();
+    if (b0 + 1 < b1) load_half(b0 + 1);
+    close_group();
+    for (int i = threadIdx.x; i < 16 * (rpad / 4); i += 256) {   // rank % 8 == 0: four floats lie inside a head's row or behind it
+        const int r = i / (rpad / 4), c = (i - r * (rpad / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < n && c < rank) v = *reinterpret_cast<const float4*>(qa + ((size_t)t * heads + h0 + r) * rank + c);
+        const __nv_bfloat162 x = __floats2bfloat162_rn(v.x, v.y), y = __floats2bfloat162_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>(Qs + r * RS + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
+    }
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f}, o[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    const int steps = rpad / 16, kq = warp >> 1, ks0 = steps * kq / 4, ks1 = steps * (kq + 1) / 4;
+    const int n8 = out_cols / 8, ntw = ((n8 + kTileWarps - 1) / kTileWarps + 1) & ~1, tile0 = warp * ntw;   // pairs of column tiles
+    for (int b = b0; b < b1; ++b) {
+        const bf* Kb = Ks + ((b - b0) & 1) * kHalfKeys * RS;
+        const int k0 = first + b * kHalfKeys;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();   // half b has landed for everybody (and, the first time, the query rows)
+        {
+            float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            const bf* ka = Kb + ((warp & 1) * 16 + (lane & 15)) * RS + (lane >> 4) * 8;
+            const bf* qb = Qs + ((lane & 7) + (lane >> 4) * 8) * RS + ((lane >> 3) & 1) * 8;
+#pragma unroll 3
+            for (int ks = ks0; ks < ks1; ++ks) {
+                uint32_t a[4], q[4];
+                ldsm_x4(a, ka + ks * 16);
+                ldsm_x4(q, qb + ks * 16);
+                const uint32_t q0[2] = {q[0], q[1]}, q1[2] = {q[2], q[3]};
+                mma_bf16_16816(s[0], a, q0);
+                mma_bf16_16816(s[1], a, q1);
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) Ss[(kq * 16 + x * 8 + tig * 2 + (e & 1)) * 36 + (warp & 1) * 16 + gid + (e >> 1) * 8] = s[x][e];
+        }
+        __syncthreads();
+        const int j = k0 + lane;
+        const bool seen = j <= p && j >= lo;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int r = 2 * warp + x;
+            const float* sr = Ss + r * 36 + lane;
+            const float v = seen ? ((sr[0] + sr[16 * 36]) + (sr[32 * 36] + sr[48 * 36])) * scale : -INFINITY;
+            float mx = v;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+            const float mn = fmaxf(m_run[x], mx);
+            const float pv = seen ? expf(v - mn) : 0.f, al = m_run[x] == mn ? 1.f : expf(m_run[x] - mn);
+            float sum = pv;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+            l_run[x] = l_run[x] * al + sum;
+            m_run[x] = mn;
+            Ps[r * 40 + lane] = __float2bfloat16_rn(pv);
+            if (lane == 0) al_s[r] = al;
+        }
+        __syncthreads();
+        {
+            const float a0 = al_s[gid], a1 = al_s[gid + 8];
+#pragma unroll
+            for (int i = 0; i < NT; ++i) { o[i][0] *= a0; o[i][1] *= a0; o[i][2] *= a1; o[i][3] *= a1; }
+#pragma unroll
+            for (int kk = 0; kk < kHalfKeys; kk += 16) {
+                uint32_t a[4];
+                ldsm_x4(a, Ps + (lane & 15) * 40 + kk + (lane >> 4) * 8);
+#pragma unroll
+                for (int i = 0; i < NT; i += 2) {
+                    if (i < ntw && tile0 + i < n8) {   // n8 is even: a pair of column tiles is inside or outside together
+                        uint32_t v[4];
+                        ldsm_x4_trans(v, Kb + (kk + (lane & 15)) * RS + (tile0 + i + (lane >> 4)) * 8);
+                        const uint32_t v0[2] = {v[0], v[1]}, v1[2] = {v[2], v[3]};
+                        mma_bf16_16816(o[i], a, v0);
+                        mma_bf16_16816(o[i + 1], a, v1);
+                    }
+                }
+            }
+        }
+        __syncthreads();   // nobody reads half b any more
+        if (b + 2 < b1) load_half(b + 2);
+        close_group();
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const int c = (tile0 + i) * 8 + tig * 2;
+        if (i < ntw && c < out_cols) {
+            *reinterpret_cast<float2*>(om + gid * out_cols + c) = make_float2(o[i][0], o[i][1]);
+            *reinterpret_cast<float2*>(om + (gid + 8) * out_cols + c) = make_float2(o[i][2], o[i][3]);
+        }
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) { ms[2 * warp + x] = m_run[x]; ls[2 * warp + x] = l_run[x]; }
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    float* fs = Ss;   // [16 heads][16 shares]: what a share counts with
+    {
+        const int r = threadIdx.x / kLdMaxCluster, q = threadIdx.x % kLdMaxCluster;
+        const bool on = q < splits && r < n;
+        const float sk = sink && r < n ? sink[h0 + r] : -INFINITY;
+        const float mq = on ? cluster.map_shared_rank(ms, q)[r] : -INFINITY, lq = on ? cluster.map_shared_rank(ls, q)[r] : 0.f;
+        float M = fmaxf(sk, mq);
+#pragma unroll
+        for (int d = kLdMaxCluster / 2; d > 0; d >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, d));
+        const float f = mq == -INFINITY ? 0.f : expf(mq - M);
+        float den = lq * f;
+#pragma unroll
+        for (int d = kLdMaxCluster / 2; d > 0; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
+        if (sk != -INFINITY) den += expf(sk - M);
+        fs[threadIdx.x] = f / den;
+    }
+    __syncthreads();
+    const int total = n * (out_cols / 4), share = (total + splits - 1) / splits;
+    for (int i = blockIdx.x * share + threadIdx.x; i < min(total, ((int)blockIdx.x + 1) * share); i += 256) {
+        const int r = i / (out_cols / 4), c = (i - r * (out_cols / 4)) * 4;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int q = 0; q < splits; ++q) {
+            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(om, q) + r * out_cols + c);
+            const float f = fs[r * kLdMaxCluster + q];
+            acc.x = fmaf(v.x, f, acc.x); acc.y = fmaf(v.y, f, acc.y); acc.z = fmaf(v.z, f, acc.z); acc.w = fmaf(v.w, f, acc.w);
+        }
+        *reinterpret_cast<float4*>(out + ((size_t)t * heads + h0 + r) * rank + c) = acc;
+    }
+    cluster.sync();   // nobody leaves while its share is read
+}
+
+template <int NT>
+static int launch_latent_decode(const b200_latent_attention_args& a, int out_cols, int splits, cudaStream_t s) {
+    const int rpad = (a.rank + 15) & ~15, RS = rpad + 8;
+    const size_t smem = (size_t)(2 * kHalfKeys + 16) * RS * 2 + 4 * 16 * 36 * 4 + 16 * 40 * 2 + 3 * 16 * 4;
+    static unsigned long long done = 0, wide = 0;
+    cudaError_t e = ensure_max_dynamic_smem((const void*)latent_decode_kernel<NT>, 114 * 1024, done);
+    if (e == cudaSuccess && splits > 8) {
+        const int dev = current_device();
+        if (!(wide & (1ull << dev))) {
+            e = cudaFuncSetAttribute((const void*)latent_decode_kernel<NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e == cudaSuccess) wide |= 1ull << dev;
+        }
+    }
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)splits, (unsigned)((a.heads + 15) / 16), (unsigned)a.n_tokens);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)splits;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, latent_decode_kernel<NT>, a.qa, a.out, (const __nv_bfloat16*)a.pool, a.pages, a.max_pages, a.page_rows, a.slot, a.pos,
+                           a.sink, a.scale, a.heads, a.rank, a.window, out_cols);
+    if (e != cudaSuccess) return (int)e;
+    count_launch();
+    return (int)cudaGetLastError();
+}
+
+// -1: not built for these sizes
+static int latent_decode(const b200_latent_attention_args& a, int out_cols, int longest_seen, cudaStream_t s) {
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    if ((a.rank & 7) || (out_cols & 15) || a.n_tokens > 65535 || !al16(a.qa) || !al16(a.out) || !al16(a.pool)) return -1;
+    // two CTAs per SM, as long as every CTA keeps a half tile of its own
+    const long long ctas = (long long)a.n_tokens * ((a.heads + 15) / 16);
+    int splits = 1;
+    while (splits < kLdMaxCluster && ctas * splits < 2ll * sm_count() && (longest_seen <= 0 ? splits < 8 : splits * kHalfKeys < longest_seen)) splits *= 2;
+    const int nt = ((out_cols / 8 + kTileWarps - 1) / kTileWarps + 1) & ~1;
+    if (nt <= 2) return launch_latent_decode<2>(a, out_cols, splits, s);
+    if (nt <= 4) return launch_latent_decode<4>(a, out_cols, splits, s);
+    if (nt <= 8) return launch_latent_decode<8>(a, out_cols, splits, s);
+    if (nt <= 10) return launch_latent_decode<10>(a, out_cols, splits, s);
+    return -1;
+}
+
 static bool tile_attention_enabled() {
     static int v = -1;
     if (v < 0) {
@@ -530,6 +770,11 @@ extern "C" int b200_latent_attention_ex(const b200_latent_attention_args* ap, vo
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem = ((size_t)5 * rank + 8) * sizeof(float);
     dim3 grid(n_tokens, heads);
+    // single tokens: a cluster per token whatever the batch (the tile kernel spends half of its 32 rows on nothing there)
+    if (dtype == B200_BF16 && tile_attention_enabled() && longest_entry == 1) {
+        const int rc = latent_decode(*ap, out_cols, longest_context, s);
+        if (rc >= 0) return rc;
+    }
     if (dtype == B200_BF16 && tile_attention_enabled()) {
         // tensor-core form: 32 rows of (token, head) per CTA
         // every entry a single token (a decode batch): one token per CTA, its heads the only rows
