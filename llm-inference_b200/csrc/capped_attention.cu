@@ -378,6 +378,12 @@ extern "C" int b200_paged_attention(const b200_paged_attention_args* p, void* st
     if (smem > 48 * 1024) return B200_EUNSUPPORTED;
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     const char* env = getenv("B200_ATTN_ROWS");   // 1: every batch on the row kernel (debugging aid)
+    int longest_seen = p->chunk > 0 ? std::min(p->longest_context, p->chunk) : p->longest_context;
+    if (p->window > 0) longest_seen = std::min(longest_seen, p->window);
+    if (p->dtype == B200_BF16 && p->longest_entry != 1 && al16(p->q) && al16(p->out) && al16(p->k_pool) && al16(p->v_pool) && !(env && env[0] == '1')) {
+        const int rc = paged_attention_tc(a, p->longest_entry, longest_seen, s);
+        if (rc >= 0) return rc;
+    }
     if (p->dtype == B200_BF16 && p->longest_entry != 1 && (p->sink || p->dist_bias) && !(p->softcap > 0.f) && p->dim % 8 == 0 && p->vdim % 8 == 0 && al16(p->q) && al16(p->out) &&
         al16(p->k_pool) && al16(p->v_pool) && !(env && env[0] == '1')) {
         const int rc = biased_tile(a, s);
@@ -391,12 +397,10 @@ extern "C" int b200_paged_attention(const b200_paged_attention_args* p, void* st
         if (rc == 0) count_launch();
         if (rc >= 0) return rc;
     }
-    int longest_seen = p->chunk > 0 ? std::min(p->longest_context, p->chunk) : p->longest_context;
-    if (p->window > 0) longest_seen = std::min(longest_seen, p->window);
     // bfloat16 single tokens with up to eight query heads per key head: one cluster per (token, key head), whatever the batch (the group
     // kernel below splits contexts only while the rows leave the GPU idle: 32 sequences took 383 us there, 88 us on the clusters)
     if (p->dtype == B200_BF16 && p->longest_entry == 1 && al16(p->q) && al16(p->k_pool) && al16(p->v_pool) && !(env && env[0] == '1')) {
-        const int rc = paged_decode(a, longest_seen, s);
+        const int rc = paged_decode(a, longest_seen, false, s);
         if (rc >= 0) return rc;
     }
     // single tokens whose heads come in groups of 1, 2, 4 or 8 per key head: one pass over K / V serves the whole group

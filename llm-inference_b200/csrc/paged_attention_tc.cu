@@ -1,0 +1,459 @@
+// bfloat16 prompt portions of b200_paged_attention on tcgen05 / TMEM: 128 (token, query head) rows per tile, keys 64 at a time.
+//
+// What bounds it: per 128 x 64 scores of 128-wide heads the tensor pipe needs 640 clocks (the scores are 64 columns wide, so their
+// operands bound them) and the special-function unit 512 for the exponentials; one tile alone is a chain of both, so two CTAs share an
+// SM (96 KB of shared memory and 256 TMEM columns each) and fill each other's gaps.
+//   rows        TQ tokens x the R query heads of one key head (TQ = 128 / R), so a key tile is read once for the whole group and a
+//               causal edge wastes little. A CTA's window of TQ packed rows may hold the end of one sequence and the start of
+//               the next: they are separate tiles, walked by neighbouring CTAs (gridDim.y is doubled when there is more than one entry).
+//               Sequences that bring a single token are left to the cluster kernel of paged_decode.cu.
+//   warp 0      TMA: K and V tiles of 64 rows out of their page (one list lookup per tile), two stages each
+//   warp 1      tcgen05.mma: S_{j+1} = Q K^T is issued before O += P_j V_j, so the tensor pipe works under the softmax
+//   warps 2-5   softmax, a thread per row: scores are read from TMEM once, P_j goes back over its own scores as bfloat16 and is the A operand
+//               of the second product. O stays in TMEM: it is rescaled only when a row's maximum has grown by more than 2^8 since the
+//               last rescaling (weights up to 256, sums in fp32, the final division makes them exact again).
+// Rows of a page beyond the context may hold anything, so the V rows of the last tile are cleared before they are multiplied by zero weights.
+#include <cuda_bf16.h>
+
+#include "b200_serve.h"
+#include "common.cuh"
+#include "launch_count.h"
+#include "paged_attention.cuh"
+#include "tc_common.cuh"
+
+namespace b200 {
+
+enum { kTcPlain = 0, kTcCapped = 1, kTcBiased = 2, kTcSigmoid = 3 };
+constexpr int kTcRows = 128, kTcKeys = 64, kTcThreads = 192;
+constexpr int kTcBox = kTcKeys * 128;         // bytes of 64 rows x 64 columns
+constexpr int kTcBiasPad = 64 + 128 + 64;     // distances in front of and behind a head's table (below)
+constexpr int kTcBiasFloats = 4096;           // at most this many staged bias numbers per CTA
+
+template <int D, int DV>
+struct TcSmem {
+    static constexpr int kQ = kTcRows * D * 2, kK = kTcKeys * D * 2, kV = kTcKeys * DV * 2;
+    static constexpr int kOffK = kQ, kOffV = kOffK + 2 * kK, kOffBar = kOffV + 2 * kV, kOffSlot = kOffBar + 16 * 8;
+    static constexpr int kOffBias = kOffSlot + (kTcRows + 2 + 16) * 4;
+    static constexpr int kTmemCols = 2 * kTcKeys + DV <= 256 ? 256 : 512;
+};
+
+template <int D, int DV, int FORM>
+__global__ void __launch_bounds__(kTcThreads, TcSmem<D, DV>::kTmemCols == 256 ? 2 : 1)
+paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int TQ, int parts, int skip_singles) {
+    using bf = __nv_bfloat16;
+    using L = TcSmem<D, DV>;
+    extern __shared__ __align__(1024) unsigned char tc_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
+    uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 6, *s_full = bars + 8, *p_full = bars + 10, *o_done = bars + 12;
+    int* slots = reinterpret_cast<int*>(smem + L::kOffSlot);        // of the window's rows and one on either side
+    uint32_t* masks = reinterpret_cast<uint32_t*>(slots + kTcRows + 2);   // [0..3] rows that begin a sequence, [4..7] those that begin a tile
+    uint32_t* tmem_slot = masks + 8;
+    volatile int* dead = reinterpret_cast<volatile int*>(masks + 9);
+    float* bias_s = reinterpret_cast<float*>(smem + L::kOffBias);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ku = blockIdx.x, g = ku / a.maps, mp = ku % a.maps, R = a.heads / a.kv_heads, q_units = a.heads * a.maps;
+    // the last rows of a prompt see the most keys: those windows come first
+    const int yy = gridDim.y - 1 - blockIdx.y, part = yy % parts, t0 = yy / parts * TQ, rows = min(TQ, a.n_tokens - t0);
+
+    // ---- the window's tiles
+    if (threadIdx.x < TQ + 2) {
+        const int t = t0 - 1 + (int)threadIdx.x;
+        slots[threadIdx.x] = t >= 0 && t < a.n_tokens ? a.slot[t] : -1;
+    }
+    __syncthreads();
+    if (warp < 4) {
+        const int i = threadIdx.x;   // row of the window; slots[i + 1] is its own
+        const bool in = i < rows, starts = in && (i == 0 || slots[i] != slots[i + 1]);
+        const bool single = in && skip_singles && slots[i] != slots[i + 1] && slots[i + 2] != slots[i + 1];
+        const uint32_t b = __ballot_sync(0xffffffffu, starts), tb = __ballot_sync(0xffffffffu, starts && !single);
+        if (lane == 0) { masks[warp] = b; masks[4 + warp] = tb; }
+    }
+    if (threadIdx.x == 0) *dead = 0;
+    __syncthreads();
+    int n_tiles = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) n_tiles += __popc(masks[4 + i]);
+    if (n_tiles <= part) return;   // nothing here for this CTA (no barrier, no TMEM yet)
+
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1);
+            mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+            mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 4);
+            mbar_init(&o_done[s], 1);
+        }
+        mbar_fence_init();
+        tma_prefetch_desc(&map_k);
+        tma_prefetch_desc(&map_v);
+    }
+    pdl_launch_dependents();   // the kernel for single tokens may move in (it waits for this one before it ends)
+    if (warp == 1) tmem_alloc(tmem_slot, L::kTmemCols);
+    if (FORM == kTcBiased && a.dist_bias) {
+        // per head: entry 64 + distance; distances below 0 (masked keys) and beyond the table repeat its ends, so that no index needs a clamp
+        const int n = a.dist_n + kTcBiasPad;
+        for (int i = threadIdx.x; i < R * n; i += kTcThreads)
+            bias_s[i] = a.dist_bias[(size_t)(g * R + i / n) * a.dist_n + min(max(i % n - 64, 0), a.dist_n - 1)] * 1.4426950408889634f;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot, o_tmem = tmem + 2 * kTcKeys;
+
+    int it0 = 0, ordinal = 0;   // key tiles walked so far (stage and phase of every ring); tiles of the window seen so far
+    for (int first = 0; first < rows;) {
+        // the next tile: rows [first, end) of the window
+        int w = first >> 5;
+        uint32_t left = w < 4 ? masks[4 + w] & (0xffffffffu << (first & 31)) : 0u;
+        while (left == 0u && ++w < 4) left = masks[4 + w];
+        if (left == 0u || w >= 4) break;
+        first = w * 32 + __ffs(left) - 1;
+        int end = rows;
+        {
+            int v = (first + 1) >> 5;
+            uint32_t nx = v < 4 ? masks[v] & (0xffffffffu << ((first + 1) & 31)) : 0u;
+            while (nx == 0u && ++v < 4) nx = masks[v];
+            if (nx != 0u && v < 4) end = min(end, v * 32 + __ffs(nx) - 1);
+        }
+        if (ordinal++ % parts != part) { first = end; continue; }
+        const int tA = t0 + first, count = end - first;
+        const int pA = a.pos[tA], pZ = a.pos[tA + count - 1];
+        const int key0 = pa_first_key(a, pA) & ~(kTcKeys - 1), n_kt = (pZ - key0) / kTcKeys + 1;
+        const int* plist = a.pages + (size_t)slots[first + 1] * a.max_pages;
+
+        // ---- Q rows into the K-major swizzled operand (rows that this tile does not have: zeros)
+        {
+            constexpr int CH = D / 8;
+            for (int i = threadIdx.x; i < kTcRows * CH; i += kTcThreads) {
+                const int r = i / CH, c = i % CH, tl = r / R, h = g * R + r % R;
+                Pack16 v{{0u, 0u, 0u, 0u}};
+                if (tl < count) {
+                    v = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)(tA + tl) * q_units + h * a.maps + mp) * D + c * 8);
+                    if (pa_scale(a, h) < 0.f) {   // the softmax works with |scale|
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v.w[e] ^= 0x80008000u;
+                    }
+                }
+                st16(smem + (c / 8) * (kTcRows * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), v);
+            }
+            fence_proxy_async_smem();
+        }
+        __syncthreads();
+
+        if (warp == 0) {
+            for (int j = 0; j < n_kt; ++j) {
+                const int it = it0 + j, s = it & 1, k0 = key0 + j * kTcKeys;
+                const uint32_t ph = (uint32_t)(it >> 1) & 1u;
+                const int row = plist[k0 / a.page_rows] * a.page_rows + k0 % a.page_rows;
+                mbar_wait_or_leave(&k_empty[s], ph ^ 1u, dead);
+                if (lane == 0) {
+                    mbar_expect_tx(&k_full[s], L::kK);
+#pragma unroll
+                    for (int c = 0; c < D / 64; ++c) tma_load_2d(smem + L::kOffK + s * L::kK + c * kTcBox, &map_k, ku * D + c * 64, row, &k_full[s]);
+                }
+                mbar_wait_or_leave(&v_empty[s], ph ^ 1u, dead);
+                if (lane == 0) {
+                    mbar_expect_tx(&v_full[s], L::kV);
+#pragma unroll
+                    for (int c = 0; c < DV / 64; ++c) tma_load_2d(smem + L::kOffV + s * L::kV + c * kTcBox, &map_v, g * DV + c * 64, row, &v_full[s]);
+                }
+                __syncwarp();
+            }
+        } else if (warp == 1) {
+            constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
+            constexpr uint32_t idesc_s = make_idesc_f16(kTcRows, kTcKeys) | kBf16, idesc_o = make_idesc_f16(kTcRows, DV) | kBf16 | (1u << 16);
+            auto issue_s = [&](int j) {
+                const int it = it0 + j, s = it & 1;
+                mbar_wait_or_leave(&k_full[s], (uint32_t)(it >> 1) & 1u, dead);
+                tc_fence_after();
+                if (lane == 0) {
+                    const uint32_t qa = smem_u32(smem), ka = smem_u32(smem + L::kOffK + s * L::kK);
+#pragma unroll
+                    for (int ks = 0; ks < D / kUmmaK; ++ks)
+                        umma_f16(tmem + (uint32_t)(s * kTcKeys), make_kmajor_sw128_desc(qa + (ks >> 2) * (kTcRows * 128)) + (uint64_t)(2 * (ks & 3)),
+                                 make_kmajor_sw128_desc(ka + (ks >> 2) * kTcBox) + (uint64_t)(2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
+                    umma_commit(&k_empty[s]);
+                    umma_commit(&s_full[s]);
+                }
+                __syncwarp();
+            };
+            issue_s(0);
+            for (int j = 0; j < n_kt; ++j) {
+                // (the score buffer of j + 1 last held P_{j-1}, whose product is ahead of it in the tensor pipe)
+                if (j + 1 < n_kt) issue_s(j + 1);
+                const int it = it0 + j, s = it & 1;
+                const uint32_t ph = (uint32_t)(it >> 1) & 1u;
+                mbar_wait_or_leave(&v_full[s], ph, dead);
+                mbar_wait_or_leave(&p_full[s], ph, dead);
+                tc_fence_after();
+                if (lane == 0) {
+                    const uint32_t va = smem_u32(smem + L::kOffV + s * L::kV);
+#pragma unroll
+                    for (int ks = 0; ks < kTcKeys / kUmmaK; ++ks)
+                        umma_f16_ts(o_tmem, tmem + (uint32_t)(s * kTcKeys + ks * 8), make_mnmajor_sw128_desc(va + ks * 2048u, kTcBox, 1024u), idesc_o,
+                                    j > 0 || ks > 0 ? 1u : 0u);
+                    umma_commit(&v_empty[s]);
+                    umma_commit(&o_done[s]);
+                }
+                __syncwarp();
+            }
+        } else {
+            // ================= softmax: a thread per row =================
+            const int quarter = warp & 3, r = quarter * 32 + lane, tl = r / R, hr = r % R, h = g * R + hr;
+            const uint32_t my = (uint32_t)(quarter * 32) << 16;
+            const bool mine = tl < count;
+            const int p = mine ? a.pos[tA + tl] : -1, f = mine ? pa_first_key(a, p) : 0;
+            const float sc = fabsf(pa_scale(a, h));
+            constexpr float kLog2E = 1.4426950408889634f;
+            // scores leave TMEM as q . k; plain: p = 2^(q . k * sl - m * sl), m the largest q . k; capped, biased: first x = the score times log2 e
+            const float sl = sc * kLog2E;
+            const float over_cap = FORM == kTcCapped ? sc / a.softcap : 0.f, cap2 = a.softcap * kLog2E;
+            const float hb2 = FORM == kTcSigmoid && a.head_bias ? a.head_bias[h] * kLog2E : 0.f;
+            const float* brow = nullptr;
+            float far_bias = 0.f;
+            if (FORM == kTcBiased && a.dist_bias) {
+                brow = bias_s + hr * (a.dist_n + kTcBiasPad) + 64;
+                far_bias = brow[a.dist_n - 1];
+            }
+            float m = -1e30f, l = 0.f;   // m: what the exponents are taken against (the scores of FORM plain unscaled)
+            const float step = FORM == kTcPlain ? sl : 1.f;   // log2 units per unit of m
+            for (int j = 0; j < n_kt; ++j) {
+                const int it = it0 + j, s = it & 1, k0 = key0 + j * kTcKeys;
+                const uint32_t ph = (uint32_t)(it >> 1) & 1u, st = tmem + my + (uint32_t)(s * kTcKeys);
+                mbar_wait_or_leave(&s_full[s], ph, dead);
+                tc_fence_after();
+                if (j == n_kt - 1 && (pZ + 1) % kTcKeys != 0) {
+                    // V rows behind the context: 0 * NaN must stay 0. (After the wait above: these scores follow the product two tiles before in
+                    // the tensor pipe, so the stage has seen its last but one load and its barrier can be waited on by parity.)
+                    mbar_wait_or_leave(&v_full[s], ph, dead);
+                    const int valid = pZ + 1 - k0;
+                    for (int i = threadIdx.x - 64; i < (kTcKeys - valid) * (DV / 8); i += 128) {
+                        const int vr = valid + i / (DV / 8), c = i % (DV / 8);
+                        st_shared_v4(smem_u32(smem + L::kOffV + s * L::kV + (c / 8) * kTcBox) + (uint32_t)(vr * 128 + (c & 7) * 16), 0u, 0u, 0u, 0u);
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                }
+                uint32_t sv[64];
+                tmem_ld_32x32_async(st, sv);
+                tmem_ld_32x32_async(st + 32u, sv + 32);
+                tmem_wait_ld<64>(sv);
+                auto S = [&](int e) { return __uint_as_float(sv[e]); };
+                const bool whole = __all_sync(0xffffffffu, k0 + kTcKeys - 1 <= p && k0 >= f);
+                if (FORM == kTcCapped) {
+                    // cap * tanh(v / cap): the odd series below |x| = 0.25 (exact to fp32 rounding), else (t - 1) / (t + 1), t = e^(2x)
+                    float big = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 64; ++e) {
+                        const float x = S(e) * over_cap;
+                        sv[e] = __float_as_uint(x);
+                        big = fmaxf(big, fabsf(x));
+                    }
+                    if (__all_sync(0xffffffffu, big < 0.25f)) {
+#pragma unroll
+                        for (int e = 0; e < 64; ++e) {
+                            const float x = S(e), x2 = x * x;
+                            sv[e] = __float_as_uint(cap2 * x * fmaf(x2, fmaf(x2, fmaf(x2, -17.f / 315.f, 2.f / 15.f), -1.f / 3.f), 1.f));
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 64; ++e) {
+                            const float t = ex2_approx(fminf(fmaxf(S(e) * (2.f * kLog2E), -43.f), 43.f));
+                            sv[e] = __float_as_uint(cap2 * __fdividef(t - 1.f, t + 1.f));
+                        }
+                    }
+                } else if (FORM == kTcBiased) {
+                    if (brow && !__all_sync(0xffffffffu, p < 0 || p - (k0 + kTcKeys - 1) >= a.dist_n - 1)) {
+                        const int most = a.dist_n - 1 + 64 + 127;
+                        const float* b = brow + max(min(p - k0, most), 0);   // rows without a token: any place of the table
+                        if (__all_sync(0xffffffffu, p - k0 <= most)) {
+#pragma unroll
+                            for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, b[-e]));
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, brow[min(max(p - k0 - e, 0), a.dist_n - 1)]));
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, far_bias));
+                    }
+                }
+                uint32_t pk[32];
+                if (FORM == kTcSigmoid) {   // weights that are not normalised over the keys
+#pragma unroll
+                    for (int e = 0; e < 64; e += 2) {
+                        float w[2];
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const float v = __fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e + x), sl, hb2)));
+                            const int key = k0 + e + x;
+                            w[x] = whole || (key <= p && key >= f) ? v : 0.f;
+                        }
+                        pk[e / 2] = pa_pack(w[0], w[1]);
+                    }
+                } else {
+                    float mx[4] = {-1e30f, -1e30f, -1e30f, -1e30f};
+                    if (whole) {
+#pragma unroll
+                        for (int e = 0; e < 64; ++e) mx[e & 3] = fmaxf(mx[e & 3], S(e));
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 64; ++e) mx[e & 3] = k0 + e <= p && k0 + e >= f ? fmaxf(mx[e & 3], S(e)) : mx[e & 3];
+                    }
+                    const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                    const bool grown = (top - m) * step > 8.f;
+                    if (j > 0 && __any_sync(0xffffffffu, grown)) {
+                        mbar_wait_or_leave(&o_done[s ^ 1], (uint32_t)((it - 1) >> 1) & 1u, dead);
+                        tc_fence_after();
+                        __syncwarp();
+                        const float alpha = grown ? ex2_approx((m - top) * step) : 1.f;
+#pragma unroll 1
+                        for (int c = 0; c < DV; c += 32) {
+                            uint32_t ov[32];
+                            tmem_ld_32x32_async(o_tmem + my + (uint32_t)c, ov);
+                            tmem_wait_ld<32>(ov);
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
+                            tmem_st_32x32(o_tmem + my + (uint32_t)c, ov);
+                        }
+                        l *= alpha;
+                    }
+                    if (grown) m = top;
+                    const float ms = -m * step;
+                    const uint64_t sl2 = pack2f(step, step), nm2 = pack2f(ms, ms);
+                    uint64_t rs2 = 0ull;
+                    if (whole) {
+#pragma unroll
+                        for (int e = 0; e < 64; e += 2) {
+                            float a0, a1;
+                            unpack2(FORM == kTcPlain ? fma2(pack2(sv[e], sv[e + 1]), sl2, nm2) : add2(pack2(sv[e], sv[e + 1]), nm2), a0, a1);
+                            a0 = ex2_approx(a0);
+                            a1 = ex2_approx(a1);
+                            rs2 = add2(rs2, pack2f(a0, a1));
+                            pk[e / 2] = pa_pack(a0, a1);
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 64; e += 2) {
+                            float w[2];
+#pragma unroll
+                            for (int x = 0; x < 2; ++x) {
+                                const float v = ex2_approx(fmaf(S(e + x), step, ms));
+                                w[x] = k0 + e + x <= p && k0 + e + x >= f ? v : 0.f;
+                            }
+                            rs2 = add2(rs2, pack2f(w[0], w[1]));
+                            pk[e / 2] = pa_pack(w[0], w[1]);
+                        }
+                    }
+                    float r0, r1;
+                    unpack2(rs2, r0, r1);
+                    l += r0 + r1;
+                }
+                tmem_st_32x32(st, pk);
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_full[s]);
+            }
+            // ---- division by the weights' sum, in which the sink counts, and the rows' stores
+            // (a wait by parity must be neither two phases behind nor ahead: a barrier per stage, whose last but one product these scores imply)
+            const int last = it0 + n_kt - 1;
+            mbar_wait_or_leave(&o_done[last & 1], (uint32_t)(last >> 1) & 1u, dead);
+            tc_fence_after();
+            __syncwarp();
+            float inv = 1.f;
+            if (FORM != kTcSigmoid) {
+                const float m2 = m * step, w = a.sink ? 1.f : a.denom_bias;
+                const float s2 = a.sink ? a.sink[h] * kLog2E : 0.f;
+                if (w > 0.f) {
+                    const float M = fmaxf(m2, s2), fo = ex2_approx(m2 - M);
+                    inv = fo / (l * fo + w * ex2_approx(s2 - M));
+                } else
+                    inv = 1.f / l;
+            }
+            if (*dead) inv = __int_as_float(0x7fffffff);
+            const size_t dst = ((size_t)(tA + tl) * q_units + h * a.maps + mp) * DV;
+#pragma unroll 1
+            for (int c = 0; c < DV; c += 32) {
+                uint32_t ov[32];
+                tmem_ld_32x32_async(o_tmem + my + (uint32_t)c, ov);
+                tmem_wait_ld<32>(ov);
+                if (mine) {
+                    if (a.out_f32) {
+                        float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + dst + c);
+#pragma unroll
+                        for (int e = 0; e < 32; e += 4)
+                            d[e / 4] = make_float4(__uint_as_float(ov[e]) * inv, __uint_as_float(ov[e + 1]) * inv, __uint_as_float(ov[e + 2]) * inv, __uint_as_float(ov[e + 3]) * inv);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            Pack16 v;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) v.w[e] = pa_pack(__uint_as_float(ov[q * 8 + 2 * e]) * inv, __uint_as_float(ov[q * 8 + 2 * e + 1]) * inv);
+                            st16(reinterpret_cast<bf*>(a.out) + dst + c + q * 8, v);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            tc_fence_before();
+        }
+        it0 += n_kt;
+        first = end;
+        __syncthreads();   // the next tile's Q rows and products come after everybody is done with this one's
+        tc_fence_after();
+    }
+    if (warp == 1) tmem_dealloc(tmem, L::kTmemCols);
+}
+
+template <int D, int DV, int FORM>
+static int launch_tc(const PA& a, int longest_entry, cudaStream_t s) {
+    using L = TcSmem<D, DV>;
+    const int R = a.heads / a.kv_heads, TQ = kTcRows / R;
+    int bias = 0;
+    if (FORM == kTcBiased && a.dist_bias) {
+        if (a.dist_n > kTcBiasFloats) return -1;
+        bias = R * (a.dist_n + kTcBiasPad);
+    }
+    if (bias > kTcBiasFloats) return -1;
+    const int smem = L::kOffBias + bias * 4 + 1024;
+    const bool several = a.n_tokens != longest_entry;   // more than one entry, as far as the host knows
+    const long long windows = (a.n_tokens + TQ - 1) / TQ;
+    if (windows * 2 > 65535) return -1;
+    static unsigned long long done = 0;
+    const cudaError_t e = ensure_max_dynamic_smem((const void*)paged_attn_tc_kernel<D, DV, FORM>, L::kOffBias + kTcBiasFloats * 4 + 1024, done);
+    if (e != cudaSuccess) return (int)e;
+    CUtensorMap mk, mv;
+    // the pool's height is not part of the call: any row that an int can name
+    constexpr long long kAnyRow = (1ll << 31) - 1;
+    if (!make_tma_map_2d(&mk, a.k_pool, kAnyRow, a.kv_heads * a.maps * D, kTcKeys) || !make_tma_map_2d(&mv, a.v_pool, kAnyRow, a.kv_heads * DV, kTcKeys)) return -1;
+    const int parts = several ? 2 : 1;
+    paged_attn_tc_kernel<D, DV, FORM><<<dim3((unsigned)(a.kv_heads * a.maps), (unsigned)(windows * parts)), kTcThreads, smem, s>>>(mk, mv, a, TQ, parts, several ? 1 : 0);
+    return (int)cudaGetLastError();
+}
+
+template <int D, int DV>
+static int launch_tc_for(const PA& a, int longest_entry, cudaStream_t s) {
+    if (a.sigmoid) return launch_tc<D, DV, kTcSigmoid>(a, longest_entry, s);
+    if (a.softcap > 0.f) return launch_tc<D, DV, kTcCapped>(a, longest_entry, s);
+    if (a.dist_bias) return launch_tc<D, DV, kTcBiased>(a, longest_entry, s);
+    return launch_tc<D, DV, kTcPlain>(a, longest_entry, s);
+}
+
+int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStream_t s) {
+    const int R = a.heads / a.kv_heads;
+    // a cap beside a sink or a bias keeps the row kernel, whose weights stay in 32 bits
+    if (R > 8 || a.page_rows % kTcKeys || (a.softcap > 0.f && (a.dist_bias || a.sink)) || a.kv_heads * a.maps > 65535) return -1;
+    int rc = -1;
+    if (a.dim == 128 && a.vdim == 128) rc = launch_tc_for<128, 128>(a, longest_entry, s);
+    else if (a.dim == 64 && a.vdim == 64) rc = launch_tc_for<64, 64>(a, longest_entry, s);
+    else if (a.dim == 128 && a.vdim == 256) rc = launch_tc_for<128, 256>(a, longest_entry, s);
+    if (rc != 0) return rc;
+    count_launch();
+    if (a.n_tokens != longest_entry) return paged_decode(a, longest_seen, true, s);   // the sequences that bring one token
+    return 0;
+}
+
+}  // namespace b200

@@ -35,7 +35,9 @@ __device__ __forceinline__ uint32_t pd_transpose(uint32_t v) {   // 8 x 8 tile o
     return r;
 }
 
-template <int D, int VD>
+// MIXED: a batch that also holds prompt portions, which other kernels take. Cluster z looks after the tokens z, z + gridDim.z, ... and serves
+// those that are their sequence's only token in the batch.
+template <int D, int VD, bool MIXED>
 __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_kernel(const PA a) {
     using bf = __nv_bfloat16;
     constexpr int KC = D / 32;        // 16-byte pieces of a key row per thread
@@ -46,22 +48,13 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
     float* om = pd_sm;                                 // [warps][R][VD], then this CTA's share in the first [R][VD]
     float* ms = om + kPdWarps * R * VD;                // [warps][R], then [R]
     float* ls = ms + kPdWarps * R;
-    const int t = blockIdx.z, ku = blockIdx.y, g = ku / a.maps, mp = ku % a.maps;
+    const int ku = blockIdx.y, g = ku / a.maps, mp = ku % a.maps;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane >> 2, tig = lane & 3;
-    const int p = a.pos[t], k_units = a.kv_heads * a.maps, q_units = a.heads * a.maps;
-    const int* plist = a.pages + (size_t)a.slot[t] * a.max_pages;
+    const int k_units = a.kv_heads * a.maps, q_units = a.heads * a.maps;
     const bf* K = reinterpret_cast<const bf*>(a.k_pool) + (size_t)ku * D + tig * 8;
     const bf* V = reinterpret_cast<const bf*>(a.v_pool) + (size_t)g * VD + gid * (VD / 8);
     const size_t k_row = (size_t)k_units * D, v_row = (size_t)a.kv_heads * VD;
 
-    uint32_t qf[KC][4];               // query head gid (heads beyond the group: zeros)
-#pragma unroll
-    for (int c = 0; c < KC; ++c) {
-        Pack16 v{{0u, 0u, 0u, 0u}};
-        if (gid < R) v = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)t * q_units + (g * R + gid) * a.maps + mp) * D + c * 32 + tig * 8);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) qf[c][e] = v.w[e];
-    }
     // this thread's two heads (columns of S^T and O^T)
     float sc[2], hb[2];
     const float* bias[2];
@@ -72,226 +65,264 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
         hb[x] = (a.sigmoid && a.head_bias) ? a.head_bias[h] : 0.f;
         bias[x] = a.dist_bias ? a.dist_bias + (size_t)h * a.dist_n : nullptr;
     }
-    float m[2], l[2] = {0.f, 0.f}, o[MT][4];
-    m[0] = m[1] = a.sigmoid ? 0.f : -INFINITY;
-#pragma unroll
-    for (int j = 0; j < MT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    for (int base = blockIdx.z; base < a.n_tokens; base += 32 * gridDim.z) {
+        uint32_t todo = 1u;
+        if (MIXED) {
+            const long long c = base + (long long)lane * gridDim.z;
+            const bool in = c < a.n_tokens;
+            const int sl = in ? a.slot[c] : -1;
+            todo = __ballot_sync(0xffffffffu, in && (c == 0 || a.slot[c - 1] != sl) && (c + 1 >= a.n_tokens || a.slot[c + 1] != sl));
+        }
+        for (; todo; todo &= todo - 1) {
+            const int t = MIXED ? base + (__ffs(todo) - 1) * (int)gridDim.z : base;
+            uint32_t qf[KC][4];               // query head gid (heads beyond the group: zeros)
+        #pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                Pack16 v{{0u, 0u, 0u, 0u}};
+                if (gid < R) v = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)t * q_units + (g * R + gid) * a.maps + mp) * D + c * 32 + tig * 8);
+        #pragma unroll
+                for (int e = 0; e < 4; ++e) qf[c][e] = v.w[e];
+            }
+            const int p = a.pos[t];
+            const int* plist = a.pages + (size_t)a.slot[t] * a.max_pages;
+            float m[2], l[2] = {0.f, 0.f}, o[MT][4];
+            m[0] = m[1] = a.sigmoid ? 0.f : -INFINITY;
+        #pragma unroll
+            for (int j = 0; j < MT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
 
-    // this warp's run of 16-key steps; a step lies inside one page (page_rows is a multiple of 16)
-    const int j_lo = pa_first_key(a, p), first = j_lo & ~(kPdStep - 1), steps = (p - first) / kPdStep + 1;
-    const int per = (steps + splits * kPdWarps - 1) / (splits * kPdWarps), w = blockIdx.x * kPdWarps + warp;
-    const int s0 = w * per, s1 = min(steps, s0 + per);
-    int j0 = first + s0 * kPdStep;
-    int page_at = j0 / a.page_rows, off = j0 - page_at * a.page_rows;    // of the step that is fetched next
-    uint4 kf[2][KC], vf[4][VP];
-    int page = s0 < s1 ? plist[page_at] : 0;
-    size_t row_next = 0;
-    auto advance = [&](bool more) {   // the fetched step's first row; then one step on, its page requested ahead
-        row_next = (size_t)page * a.page_rows + off;
-        off += kPdStep;
-        if (off == a.page_rows) { off = 0; ++page_at; if (more) page = plist[page_at]; }
-    };
-    auto load_k = [&]() {
-        const bf* r0 = K + (row_next + gid) * k_row;
-        const bf* r1 = r0 + 8 * k_row;
-#pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            kf[0][c] = *reinterpret_cast<const uint4*>(r0 + c * 32);
-            kf[1][c] = *reinterpret_cast<const uint4*>(r1 + c * 32);
-        }
-    };
-    auto load_v = [&]() {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const bf* r = V + (row_next + 2 * tig + (i & 1) + (i >> 1) * 8) * v_row;
-#pragma unroll
-            for (int x = 0; x < VP; ++x) vf[i][x] = *reinterpret_cast<const uint4*>(r + x * 8);
-        }
-    };
-    if (s0 < s1) {
-        advance(s0 + 1 < s1);
-        load_k();
-        load_v();
-    }
-    for (int s = s0; s < s1; ++s, j0 += kPdStep) {
-        float st[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < KC; ++c) {
-            const uint32_t a0[4] = {kf[0][c].x, kf[1][c].x, kf[0][c].y, kf[1][c].y}, a1[4] = {kf[0][c].z, kf[1][c].z, kf[0][c].w, kf[1][c].w};
-            const uint32_t b0[2] = {qf[c][0], qf[c][1]}, b1[2] = {qf[c][2], qf[c][3]};
-            pa_mma(st, a0, b0);
-            pa_mma(st, a1, b1);
-        }
-        const bool more = s + 1 < s1;
-        if (more) {
-            advance(s + 2 < s1);
-            load_k();
-        }
-        const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p;
-        float pr[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {   // key j0 + gid (+ 8), head 2 tig (+ 1)
-            const int j = j0 + gid + (e >> 1) * 8, x = e & 1;
-            float v = st[e] * sc[x];
-            if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
-            const bool seen = whole || (j >= j_lo && j <= p);
-            if (bias[x] && seen) v += bias[x][min(p - j, a.dist_n - 1)];
-            pr[e] = seen ? v : -INFINITY;
-        }
-        if (a.sigmoid) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : 1.f / (1.f + expf(-(pr[e] + hb[e & 1])));
-        } else {
-            float mx[2] = {fmaxf(pr[0], pr[2]), fmaxf(pr[1], pr[3])}, alpha[2];
-#pragma unroll
+            // this warp's run of 16-key steps; a step lies inside one page (page_rows is a multiple of 16)
+            const int j_lo = pa_first_key(a, p), first = j_lo & ~(kPdStep - 1), steps = (p - first) / kPdStep + 1;
+            const int per = (steps + splits * kPdWarps - 1) / (splits * kPdWarps), w = blockIdx.x * kPdWarps + warp;
+            const int s0 = w * per, s1 = min(steps, s0 + per);
+            int j0 = first + s0 * kPdStep;
+            int page_at = j0 / a.page_rows, off = j0 - page_at * a.page_rows;    // of the step that is fetched next
+            uint4 kf[2][KC], vf[4][VP];
+            int page = s0 < s1 ? plist[page_at] : 0;
+            size_t row_next = 0;
+            auto advance = [&](bool more) {   // the fetched step's first row; then one step on, its page requested ahead
+                row_next = (size_t)page * a.page_rows + off;
+                off += kPdStep;
+                if (off == a.page_rows) { off = 0; ++page_at; if (more) page = plist[page_at]; }
+            };
+            auto load_k = [&]() {
+                const bf* r0 = K + (row_next + gid) * k_row;
+                const bf* r1 = r0 + 8 * k_row;
+        #pragma unroll
+                for (int c = 0; c < KC; ++c) {
+                    kf[0][c] = *reinterpret_cast<const uint4*>(r0 + c * 32);
+                    kf[1][c] = *reinterpret_cast<const uint4*>(r1 + c * 32);
+                }
+            };
+            auto load_v = [&]() {
+        #pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const bf* r = V + (row_next + 2 * tig + (i & 1) + (i >> 1) * 8) * v_row;
+        #pragma unroll
+                    for (int x = 0; x < VP; ++x) vf[i][x] = *reinterpret_cast<const uint4*>(r + x * 8);
+                }
+            };
+            if (s0 < s1) {
+                advance(s0 + 1 < s1);
+                load_k();
+                load_v();
+            }
+            for (int s = s0; s < s1; ++s, j0 += kPdStep) {
+                float st[4] = {0.f, 0.f, 0.f, 0.f};
+        #pragma unroll
+                for (int c = 0; c < KC; ++c) {
+                    const uint32_t a0[4] = {kf[0][c].x, kf[1][c].x, kf[0][c].y, kf[1][c].y}, a1[4] = {kf[0][c].z, kf[1][c].z, kf[0][c].w, kf[1][c].w};
+                    const uint32_t b0[2] = {qf[c][0], qf[c][1]}, b1[2] = {qf[c][2], qf[c][3]};
+                    pa_mma(st, a0, b0);
+                    pa_mma(st, a1, b1);
+                }
+                const bool more = s + 1 < s1;
+                if (more) {
+                    advance(s + 2 < s1);
+                    load_k();
+                }
+                const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p;
+                float pr[4];
+        #pragma unroll
+                for (int e = 0; e < 4; ++e) {   // key j0 + gid (+ 8), head 2 tig (+ 1)
+                    const int j = j0 + gid + (e >> 1) * 8, x = e & 1;
+                    float v = st[e] * sc[x];
+                    if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
+                    const bool seen = whole || (j >= j_lo && j <= p);
+                    if (bias[x] && seen) v += bias[x][min(p - j, a.dist_n - 1)];
+                    pr[e] = seen ? v : -INFINITY;
+                }
+                if (a.sigmoid) {
+        #pragma unroll
+                    for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : 1.f / (1.f + expf(-(pr[e] + hb[e & 1])));
+                } else {
+                    float mx[2] = {fmaxf(pr[0], pr[2]), fmaxf(pr[1], pr[3])}, alpha[2];
+        #pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 4));
+                        mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 8));
+                        mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 16));
+                        const float mn = fmaxf(m[x], mx[x]);
+                        alpha[x] = m[x] == mn ? 1.f : expf(m[x] - mn);   // a step holds a visible key; scores of -inf leave the state alone
+                        m[x] = mn;
+                    }
+        #pragma unroll
+                    for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : expf(pr[e] - m[e & 1]);
+                    l[0] = l[0] * alpha[0] + (pr[0] + pr[2]);
+                    l[1] = l[1] * alpha[1] + (pr[1] + pr[3]);
+                    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+        #pragma unroll
+                        for (int j = 0; j < MT; ++j) { o[j][0] *= alpha[0]; o[j][1] *= alpha[1]; o[j][2] *= alpha[0]; o[j][3] *= alpha[1]; }
+                    }
+                }
+                uint32_t b[3][2];   // hi, mid, lo: p = hi + mid + lo to 24 bits
+        #pragma unroll
+                for (int q = 0; q < 3; ++q)
+        #pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const __nv_bfloat162 h2 = __floats2bfloat162_rn(pr[2 * hf], pr[2 * hf + 1]);
+                        const float2 f = __bfloat1622float2(h2);
+                        pr[2 * hf] -= f.x;
+                        pr[2 * hf + 1] -= f.y;
+                        b[q][hf] = pd_transpose(*reinterpret_cast<const uint32_t*>(&h2));
+                    }
+                if (!whole) {   // rows that are not this token's may hold anything: 0 * NaN must stay 0
+        #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int j = j0 + 2 * tig + (i & 1) + (i >> 1) * 8;
+                        if (j < j_lo || j > p) {
+        #pragma unroll
+                            for (int x = 0; x < VP; ++x) vf[i][x] = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                    }
+                }
+        #pragma unroll
+                for (int j = 0; j < MT; ++j) {
+                    const int x = j / 4, e = j % 4;
+                    auto word = [&](int i) { const uint4& v = vf[i][x]; return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+                    const uint32_t af[4] = {__byte_perm(word(0), word(1), 0x5410), __byte_perm(word(0), word(1), 0x7632),
+                                            __byte_perm(word(2), word(3), 0x5410), __byte_perm(word(2), word(3), 0x7632)};
+                    pa_mma(o[j], af, b[2]);
+                    pa_mma(o[j], af, b[1]);
+                    pa_mma(o[j], af, b[0]);
+                }
+                if (more) load_v();
+            }
+        #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 4));
-                mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 8));
-                mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 16));
-                const float mn = fmaxf(m[x], mx[x]);
-                alpha[x] = m[x] == mn ? 1.f : expf(m[x] - mn);   // a step holds a visible key; scores of -inf leave the state alone
-                m[x] = mn;
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : expf(pr[e] - m[e & 1]);
-            l[0] = l[0] * alpha[0] + (pr[0] + pr[2]);
-            l[1] = l[1] * alpha[1] + (pr[1] + pr[3]);
-            if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-#pragma unroll
-                for (int j = 0; j < MT; ++j) { o[j][0] *= alpha[0]; o[j][1] *= alpha[1]; o[j][2] *= alpha[0]; o[j][3] *= alpha[1]; }
-            }
-        }
-        uint32_t b[3][2];   // hi, mid, lo: p = hi + mid + lo to 24 bits
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-#pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(pr[2 * hf], pr[2 * hf + 1]);
-                const float2 f = __bfloat1622float2(h2);
-                pr[2 * hf] -= f.x;
-                pr[2 * hf + 1] -= f.y;
-                b[q][hf] = pd_transpose(*reinterpret_cast<const uint32_t*>(&h2));
-            }
-        if (!whole) {   // rows that are not this token's may hold anything: 0 * NaN must stay 0
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int j = j0 + 2 * tig + (i & 1) + (i >> 1) * 8;
-                if (j < j_lo || j > p) {
-#pragma unroll
-                    for (int x = 0; x < VP; ++x) vf[i][x] = make_uint4(0u, 0u, 0u, 0u);
+                l[x] += __shfl_xor_sync(0xffffffffu, l[x], 4);
+                l[x] += __shfl_xor_sync(0xffffffffu, l[x], 8);
+                l[x] += __shfl_xor_sync(0xffffffffu, l[x], 16);
+                const int h = 2 * tig + x;
+                if (h < R) {
+                    if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = l[x]; }
+                    float* dst = om + (size_t)(warp * R + h) * VD + gid * (VD / 8);
+        #pragma unroll
+                    for (int j = 0; j < MT; ++j) *reinterpret_cast<float2*>(dst + 2 * j) = make_float2(o[j][x], o[j][2 + x]);
                 }
             }
-        }
-#pragma unroll
-        for (int j = 0; j < MT; ++j) {
-            const int x = j / 4, e = j % 4;
-            auto word = [&](int i) { const uint4& v = vf[i][x]; return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
-            const uint32_t af[4] = {__byte_perm(word(0), word(1), 0x5410), __byte_perm(word(0), word(1), 0x7632),
-                                    __byte_perm(word(2), word(3), 0x5410), __byte_perm(word(2), word(3), 0x7632)};
-            pa_mma(o[j], af, b[2]);
-            pa_mma(o[j], af, b[1]);
-            pa_mma(o[j], af, b[0]);
-        }
-        if (more) load_v();
-    }
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-        l[x] += __shfl_xor_sync(0xffffffffu, l[x], 4);
-        l[x] += __shfl_xor_sync(0xffffffffu, l[x], 8);
-        l[x] += __shfl_xor_sync(0xffffffffu, l[x], 16);
-        const int h = 2 * tig + x;
-        if (h < R) {
-            if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = l[x]; }
-            float* dst = om + (size_t)(warp * R + h) * VD + gid * (VD / 8);
-#pragma unroll
-            for (int j = 0; j < MT; ++j) *reinterpret_cast<float2*>(dst + 2 * j) = make_float2(o[j][x], o[j][2 + x]);
-        }
-    }
-    __syncthreads();
-    // the CTA's share: every output is added by one thread, which alone reads and writes its places
-    for (int i = threadIdx.x; i < R * VD; i += blockDim.x) {
-        const int h = i / VD;
-        float M = ms[h];
-#pragma unroll
-        for (int v = 1; v < kPdWarps; ++v) M = fmaxf(M, ms[v * R + h]);
-        float acc = 0.f;
-#pragma unroll
-        for (int v = 0; v < kPdWarps; ++v) {
-            const float mv = ms[v * R + h];
-            if (mv != -INFINITY) acc += om[(size_t)(v * R + h) * VD + i % VD] * expf(mv - M);
-        }
-        om[i] = acc;
-    }
-    __syncthreads();
-    float cm = 0.f, cl = 0.f;
-    if (threadIdx.x < R) {
-        cm = ms[threadIdx.x];
-        for (int v = 1; v < kPdWarps; ++v) cm = fmaxf(cm, ms[v * R + threadIdx.x]);
-        for (int v = 0; v < kPdWarps; ++v) {
-            const float mv = ms[v * R + threadIdx.x];
-            if (mv != -INFINITY) cl += ls[v * R + threadIdx.x] * expf(mv - cm);
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < R) { ms[threadIdx.x] = cm; ls[threadIdx.x] = cl; }
-    cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();
-    const int total = R * VD, share = (total + splits - 1) / splits;
-    for (int i = blockIdx.x * share + threadIdx.x; i < min(total, ((int)blockIdx.x + 1) * share); i += blockDim.x) {
-        const int h = i / VD, qh = g * R + h;
-        // the sink joins here: a score without key and value
-        float M = a.sigmoid ? 0.f : a.sink ? a.sink[qh] : a.denom_bias > 0.f ? 0.f : -INFINITY;
-        const float sink_at = M, sink_l = a.sigmoid || a.sink ? 1.f : a.denom_bias;
-        float mr[kPdMaxCluster];
-#pragma unroll
-        for (int r = 0; r < kPdMaxCluster; ++r)
-            if (r < splits) { mr[r] = cluster.map_shared_rank(ms, r)[h]; M = fmaxf(M, mr[r]); }
-        float L = sink_at == -INFINITY ? 0.f : sink_l * expf(sink_at - M), acc = 0.f;
-#pragma unroll
-        for (int r = 0; r < kPdMaxCluster; ++r)
-            if (r < splits && mr[r] != -INFINITY) {
-                const float f = expf(mr[r] - M);
-                L += cluster.map_shared_rank(ls, r)[h] * f;
-                acc += cluster.map_shared_rank(om, r)[i] * f;
+            __syncthreads();
+            // the CTA's share: every output is added by one thread, which alone reads and writes its places
+            for (int i = threadIdx.x; i < R * VD; i += blockDim.x) {
+                const int h = i / VD;
+                float M = ms[h];
+        #pragma unroll
+                for (int v = 1; v < kPdWarps; ++v) M = fmaxf(M, ms[v * R + h]);
+                float acc = 0.f;
+        #pragma unroll
+                for (int v = 0; v < kPdWarps; ++v) {
+                    const float mv = ms[v * R + h];
+                    if (mv != -INFINITY) acc += om[(size_t)(v * R + h) * VD + i % VD] * expf(mv - M);
+                }
+                om[i] = acc;
             }
-        pa_store<bf>(a, ((size_t)t * q_units + (size_t)qh * a.maps + mp) * VD + i % VD, acc / L);
+            __syncthreads();
+            float cm = 0.f, cl = 0.f;
+            if (threadIdx.x < R) {
+                cm = ms[threadIdx.x];
+                for (int v = 1; v < kPdWarps; ++v) cm = fmaxf(cm, ms[v * R + threadIdx.x]);
+                for (int v = 0; v < kPdWarps; ++v) {
+                    const float mv = ms[v * R + threadIdx.x];
+                    if (mv != -INFINITY) cl += ls[v * R + threadIdx.x] * expf(mv - cm);
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x < R) { ms[threadIdx.x] = cm; ls[threadIdx.x] = cl; }
+            cg::cluster_group cluster = cg::this_cluster();
+            cluster.sync();
+            const int total = R * VD, share = (total + splits - 1) / splits;
+            for (int i = blockIdx.x * share + threadIdx.x; i < min(total, ((int)blockIdx.x + 1) * share); i += blockDim.x) {
+                const int h = i / VD, qh = g * R + h;
+                // the sink joins here: a score without key and value
+                float M = a.sigmoid ? 0.f : a.sink ? a.sink[qh] : a.denom_bias > 0.f ? 0.f : -INFINITY;
+                const float sink_at = M, sink_l = a.sigmoid || a.sink ? 1.f : a.denom_bias;
+                float mr[kPdMaxCluster];
+        #pragma unroll
+                for (int r = 0; r < kPdMaxCluster; ++r)
+                    if (r < splits) { mr[r] = cluster.map_shared_rank(ms, r)[h]; M = fmaxf(M, mr[r]); }
+                float L = sink_at == -INFINITY ? 0.f : sink_l * expf(sink_at - M), acc = 0.f;
+        #pragma unroll
+                for (int r = 0; r < kPdMaxCluster; ++r)
+                    if (r < splits && mr[r] != -INFINITY) {
+                        const float f = expf(mr[r] - M);
+                        L += cluster.map_shared_rank(ls, r)[h] * f;
+                        acc += cluster.map_shared_rank(om, r)[i] * f;
+                    }
+                pa_store<bf>(a, ((size_t)t * q_units + (size_t)qh * a.maps + mp) * VD + i % VD, acc / L);
+            }
+            cluster.sync();   // nobody leaves (or starts its next token) while its shared memory is read
+        }
+        if (!MIXED) break;
     }
-    cluster.sync();   // nobody leaves while its shared memory is read
+    if (MIXED) pdl_wait();   // the prompt portions' kernel runs beside this one: done only when both are
 }
 
-template <int D, int VD>
-static int launch_paged_decode(const PA& a, int splits, cudaStream_t s) {
+template <int D, int VD, bool MIXED>
+static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s) {
     const int R = a.heads / a.kv_heads;
     const size_t smem = ((size_t)kPdWarps * R * VD + 2 * kPdWarps * R) * sizeof(float);
     static_assert(((size_t)kPdWarps * kPdHeads * VD + 2 * kPdWarps * kPdHeads) * sizeof(float) <= 48 * 1024, "no shared-memory opt-in needed");
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.kv_heads * a.maps), (unsigned)a.n_tokens);
+    cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.kv_heads * a.maps), (unsigned)rows);
     cfg.blockDim = dim3(kPdWarps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)splits;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD>, a);
+    if (MIXED && pdl_enabled()) {
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs = 2;
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, a);
     if (e != cudaSuccess) return (int)e;
     count_launch();
     return (int)cudaGetLastError();
 }
 
-int paged_decode(const PA& a, int longest_seen, cudaStream_t s) {
-    if (a.heads / a.kv_heads > kPdHeads || a.page_rows % kPdStep || a.n_tokens > 65535 || a.kv_heads * a.maps > 65535) return -1;
-    // CTAs for three per SM, as long as every warp of a cluster keeps a step of its own
-    const long long pairs = (long long)a.n_tokens * a.kv_heads * a.maps;
-    int splits = 1;
-    while (splits < kPdMaxCluster && pairs * splits < 3ll * sm_count() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
-    if (a.dim == 128 && a.vdim == 128) return launch_paged_decode<128, 128>(a, splits, s);
-    if (a.dim == 64 && a.vdim == 64) return launch_paged_decode<64, 64>(a, splits, s);
-    if (a.dim == 128 && a.vdim == 256) return launch_paged_decode<128, 256>(a, splits, s);
-    if (a.dim == 64 && a.vdim == 128) return launch_paged_decode<64, 128>(a, splits, s);
+template <bool MIXED>
+static int paged_decode_for(const PA& a, int splits, int rows, cudaStream_t s) {
+    if (a.dim == 128 && a.vdim == 128) return launch_paged_decode<128, 128, MIXED>(a, splits, rows, s);
+    if (a.dim == 64 && a.vdim == 64) return launch_paged_decode<64, 64, MIXED>(a, splits, rows, s);
+    if (a.dim == 128 && a.vdim == 256) return launch_paged_decode<128, 256, MIXED>(a, splits, rows, s);
+    if (a.dim == 64 && a.vdim == 128) return launch_paged_decode<64, 128, MIXED>(a, splits, rows, s);
     return -1;
+}
+
+int paged_decode(const PA& a, int longest_seen, bool mixed, cudaStream_t s) {
+    if (a.heads / a.kv_heads > kPdHeads || a.page_rows % kPdStep || a.kv_heads * a.maps > 65535) return -1;
+    // how many tokens of a mixed batch are single ones is only known on the device: sixteen rows of clusters share them
+    const int rows = mixed ? std::min(a.n_tokens, 16) : a.n_tokens;
+    if (rows > 65535) return -1;
+    // at least four CTAs per SM (three fit at a time), as long as every warp of a cluster keeps a step of its own
+    // (32 sequences of up to 2048 tokens, CTAs per SM aimed at and us: 1: 104, 2 and 3: 89, 4 and 6: 82, 12: 97)
+    const long long pairs = (long long)rows * a.kv_heads * a.maps;
+    int splits = 1;
+    while (splits < kPdMaxCluster && (mixed || pairs * splits < 4ll * sm_count()) && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+    return mixed ? paged_decode_for<true>(a, splits, rows, s) : paged_decode_for<false>(a, splits, rows, s);
 }
 
 }  // namespace b200

@@ -166,6 +166,7 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t* v)
 }
 // mbarrier wait that gives up after ~2 s: it sets *dead (shared memory) and returns, and with *dead set every further wait returns at
 // once, so a broken pipeline runs to its end, frees its TMEM and leaves. The caller then stores NaN instead of results.
+// Called by whole warps; their lanes leave together (warp-wide instructions follow).
 __device__ __forceinline__ void mbar_wait_or_leave(uint64_t* bar, uint32_t parity, volatile int* dead) {
     uint32_t done, spins = 0;
     uint64_t t0 = 0;
@@ -179,15 +180,16 @@ __device__ __forceinline__ void mbar_wait_or_leave(uint64_t* bar, uint32_t parit
             : "=r"(done)
             : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
-        if (done) return;
+        if (done) break;
         if ((++spins & 0xFFu) == 0) {
-            if (*dead) return;
+            if (*dead) break;
             uint64_t now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
             if (t0 == 0) t0 = now;
-            else if (now - t0 > 2000000000ull) { *dead = 1; return; }
+            else if (now - t0 > 2000000000ull) { *dead = 1; break; }
         }
     }
+    __syncwarp();
 }
 
 __device__ __forceinline__ float ex2_approx(float x) {
