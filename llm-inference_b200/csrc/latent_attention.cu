@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* _
 //   softmax  warp w: heads 2w, 2w + 1, a key per lane; the weights leave as bfloat16 (as in the tile kernel)
 //   values   warp w: an eighth of the output columns, the rows read transposed by ldmatrix
 // The sink joins in the merge. Measured, 8 sequences of up to 1024 rows of 576, 16 heads, 512 columns out: the tile kernel with its
-// combine launch 53.3 us, this 20.5 us.
+// combine launch 53.3 us, this 18.4 us (clusters of at most 2 / 4 / 8 CTAs: 51 / 31 / 20.5 us).
 constexpr int kLdMaxCluster = 16;
 
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
@@ -474,23 +474,39 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
     float* ls = ms + 16;                                       // [16]
     float* om = reinterpret_cast<float*>(smraw);               // [16][out_cols]: this CTA's share, once the rows have been used
     const int t = blockIdx.z, h0 = blockIdx.y * 16, warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane / 4, tig = lane % 4;
-    const int p = pos[t], n = min(16, heads - h0), chunks = rpad / 8;
+    const int n = min(16, heads - h0), chunks = rpad / 8;
+    // the query rows are requested first, ahead of the chain position -> page -> rows; a warp brings two heads
+    constexpr int kQv = (32 * kMaxRankPerLane / 4 + 31) / 32;
+    float4 qv[2][kQv];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int i = 0; i < kQv; ++i) {
+            const int r = 2 * warp + x, c = (i * 32 + lane) * 4;   // rank % 8 == 0: four floats lie inside a head's row or behind it
+            qv[x][i] = r < n && c < rank ? *reinterpret_cast<const float4*>(qa + ((size_t)t * heads + h0 + r) * rank + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    const int p = pos[t];
     const int* list = pages + (size_t)slot[t] * max_pages;
     const int lo = window > 0 ? max(0, p - window + 1) : 0, first = lo & ~(kHalfKeys - 1);
     const int halves = (p - first) / kHalfKeys + 1, per = (halves + splits - 1) / splits;
     const int b0 = blockIdx.x * per, b1 = min(halves, b0 + per);
     const bool one_page = page_rows % kHalfKeys == 0;
+    // a warp brings four whole rows, its lanes the 16-byte pieces of a row (one place in the pool per row, no division per piece)
     auto load_half = [&](int b) {
         const int k0 = first + b * kHalfKeys;
-        bf* dst0 = Ks + ((b - b0) & 1) * kHalfKeys * RS;
         const size_t base = one_page ? (size_t)list[k0 / page_rows] * page_rows + k0 % page_rows : 0;
-        for (int i = threadIdx.x; i < kHalfKeys * chunks; i += 256) {
-            const int kr = i / chunks, ch = i - kr * chunks, j = k0 + kr;
-            const bool ok = j <= p && j >= lo && ch * 8 < rank;
-            const size_t row = !ok ? 0 : one_page ? base + kr : (size_t)list[j / page_rows] * page_rows + j % page_rows;
-            const bf* src = ok ? pool + row * rank + ch * 8 : pool;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(dst0 + kr * RS + ch * 8);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+        const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(Ks + ((b - b0) & 1) * kHalfKeys * RS);
+#pragma unroll
+        for (int i = 0; i < kHalfKeys / 8; ++i) {
+            const int kr = i * 8 + warp, j = k0 + kr;
+            const bool in = j <= p && j >= lo;
+            const size_t row = !in ? 0 : one_page ? base + kr : (size_t)list[j / page_rows] * page_rows + j % page_rows;
+            const bf* src = pool + row * rank;
+            const uint32_t dst = dst0 + (uint32_t)(kr * RS) * 2u;
+            for (int ch = lane; ch < chunks; ch += 32) {
+                const bool ok = in && ch * 8 < rank;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)ch * 16u), "l"(ok ? src + ch * 8 : pool), "r"(ok ? 16 : 0) : "memory");
+            }
         }
     };
     auto close_group = [&]() {
@@ -501,13 +517,16 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
     close_group();
     if (b0 + 1 < b1) load_half(b0 + 1);
     close_group();
-    for (int i = threadIdx.x; i < 16 * (rpad / 4); i += 256) {   // rank % 8 == 0: four floats lie inside a head's row or behind it
-        const int r = i / (rpad / 4), c = (i - r * (rpad / 4)) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < n && c < rank) v = *reinterpret_cast<const float4*>(qa + ((size_t)t * heads + h0 + r) * rank + c);
-        const __nv_bfloat162 x = __floats2bfloat162_rn(v.x, v.y), y = __floats2bfloat162_rn(v.z, v.w);
-        *reinterpret_cast<uint2*>(Qs + r * RS + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
-    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int i = 0; i < kQv; ++i) {
+            const int c = (i * 32 + lane) * 4;
+            if (c < rpad) {
+                const __nv_bfloat162 u = __floats2bfloat162_rn(qv[x][i].x, qv[x][i].y), v = __floats2bfloat162_rn(qv[x][i].z, qv[x][i].w);
+                *reinterpret_cast<uint2*>(Qs + (2 * warp + x) * RS + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&u), *reinterpret_cast<const uint32_t*>(&v));
+            }
+        }
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f}, o[NT][4];
 #pragma unroll
     for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;

@@ -6,14 +6,15 @@
 //   S^T = K Q^T   mma.sync m16n8k16, keys on the M axis, the R <= 8 query heads of the key head on the N axis. The order of the
 //                 contraction is free, so a thread's fragment is one 16-byte piece of its key row straight from global memory.
 //   softmax       fp32 in registers, a running (maximum, denominator) per warp; cap, bias, temperature and masks as in the row kernel
-//   O^T = V^T P^T value dimensions on the M axis: a thread loads 32-byte pieces of four value rows and pairs them with PRMT. The
+//   O^T = V^T P^T value dimensions on the M axis: a thread loads 16-byte pieces of four value rows and pairs them with PRMT. The
 //                 weights keep 24 bits: p = hi + mid + lo (three bfloat16, the difference exact at every step), three products
 //                 with fp32 accumulation, so nothing is rounded to 16 bits on the way. movmatrix turns the weights' fragments.
 // The next step's keys are requested before the softmax, the next step's values before the following scores: 8 KB per warp in flight,
 // twelve warps per SM. Warps merge through shared memory, CTAs through distributed shared memory (rank order, so the sum does not
 // depend on timing). The merge adds the sink.
 // Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128:
-// 20.5 -> 8.2 us; 32 sequences of up to 2048 tokens, 16 / 8 heads x 128, bias and sink (190 MB): 383 -> 88 us.
+// 20.5 -> 8.2 us; 32 sequences of up to 2048 tokens, 16 / 8 heads x 128, bias and sink (190 MB): 383 -> 69 us (84 us with one chain of
+// score products, the maximum reduced at every step and three dependent products per output tile: the step's latency was what counted).
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane >> 2, tig = lane & 3;
     const int k_units = a.kv_heads * a.maps, q_units = a.heads * a.maps;
     const bf* K = reinterpret_cast<const bf*>(a.k_pool) + (size_t)ku * D + tig * 8;
-    const bf* V = reinterpret_cast<const bf*>(a.v_pool) + (size_t)g * VD + gid * (VD / 8);
+    const bf* V = reinterpret_cast<const bf*>(a.v_pool) + (size_t)g * VD + gid * 8;
     const size_t k_row = (size_t)k_units * D, v_row = (size_t)a.kv_heads * VD;
 
     // this thread's two heads (columns of S^T and O^T)
@@ -76,18 +77,18 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
         for (; todo; todo &= todo - 1) {
             const int t = MIXED ? base + (__ffs(todo) - 1) * (int)gridDim.z : base;
             uint32_t qf[KC][4];               // query head gid (heads beyond the group: zeros)
-        #pragma unroll
+#pragma unroll
             for (int c = 0; c < KC; ++c) {
                 Pack16 v{{0u, 0u, 0u, 0u}};
                 if (gid < R) v = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)t * q_units + (g * R + gid) * a.maps + mp) * D + c * 32 + tig * 8);
-        #pragma unroll
+#pragma unroll
                 for (int e = 0; e < 4; ++e) qf[c][e] = v.w[e];
             }
             const int p = a.pos[t];
             const int* plist = a.pages + (size_t)a.slot[t] * a.max_pages;
             float m[2], l[2] = {0.f, 0.f}, o[MT][4];
             m[0] = m[1] = a.sigmoid ? 0.f : -INFINITY;
-        #pragma unroll
+#pragma unroll
             for (int j = 0; j < MT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
 
             // this warp's run of 16-key steps; a step lies inside one page (page_rows is a multiple of 16)
@@ -107,18 +108,18 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
             auto load_k = [&]() {
                 const bf* r0 = K + (row_next + gid) * k_row;
                 const bf* r1 = r0 + 8 * k_row;
-        #pragma unroll
+#pragma unroll
                 for (int c = 0; c < KC; ++c) {
                     kf[0][c] = *reinterpret_cast<const uint4*>(r0 + c * 32);
                     kf[1][c] = *reinterpret_cast<const uint4*>(r1 + c * 32);
                 }
             };
             auto load_v = [&]() {
-        #pragma unroll
+#pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const bf* r = V + (row_next + 2 * tig + (i & 1) + (i >> 1) * 8) * v_row;
-        #pragma unroll
-                    for (int x = 0; x < VP; ++x) vf[i][x] = *reinterpret_cast<const uint4*>(r + x * 8);
+#pragma unroll
+                    for (int x = 0; x < VP; ++x) vf[i][x] = *reinterpret_cast<const uint4*>(r + x * 64);
                 }
             };
             if (s0 < s1) {
@@ -127,57 +128,63 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                 load_v();
             }
             for (int s = s0; s < s1; ++s, j0 += kPdStep) {
-                float st[4] = {0.f, 0.f, 0.f, 0.f};
-        #pragma unroll
+                const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p, more = s + 1 < s1;
+                float bv[4] = {0.f, 0.f, 0.f, 0.f};
+                if (a.dist_bias) {   // requested before the scores are formed
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) bv[e] = bias[e & 1][min(max(p - (j0 + gid + (e >> 1) * 8), 0), a.dist_n - 1)];
+                }
+                float st[4] = {0.f, 0.f, 0.f, 0.f}, su[4] = {0.f, 0.f, 0.f, 0.f};   // two chains of products
+#pragma unroll
                 for (int c = 0; c < KC; ++c) {
                     const uint32_t a0[4] = {kf[0][c].x, kf[1][c].x, kf[0][c].y, kf[1][c].y}, a1[4] = {kf[0][c].z, kf[1][c].z, kf[0][c].w, kf[1][c].w};
                     const uint32_t b0[2] = {qf[c][0], qf[c][1]}, b1[2] = {qf[c][2], qf[c][3]};
                     pa_mma(st, a0, b0);
-                    pa_mma(st, a1, b1);
+                    pa_mma(su, a1, b1);
                 }
-                const bool more = s + 1 < s1;
                 if (more) {
                     advance(s + 2 < s1);
                     load_k();
                 }
-                const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p;
                 float pr[4];
-        #pragma unroll
+#pragma unroll
                 for (int e = 0; e < 4; ++e) {   // key j0 + gid (+ 8), head 2 tig (+ 1)
                     const int j = j0 + gid + (e >> 1) * 8, x = e & 1;
-                    float v = st[e] * sc[x];
+                    float v = (st[e] + su[e]) * sc[x];
                     if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
-                    const bool seen = whole || (j >= j_lo && j <= p);
-                    if (bias[x] && seen) v += bias[x][min(p - j, a.dist_n - 1)];
-                    pr[e] = seen ? v : -INFINITY;
+                    pr[e] = whole || (j >= j_lo && j <= p) ? v + bv[e] : -INFINITY;
                 }
                 if (a.sigmoid) {
-        #pragma unroll
+#pragma unroll
                     for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : 1.f / (1.f + expf(-(pr[e] + hb[e & 1])));
                 } else {
-                    float mx[2] = {fmaxf(pr[0], pr[2]), fmaxf(pr[1], pr[3])}, alpha[2];
-        #pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 4));
-                        mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 8));
-                        mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 16));
-                        const float mn = fmaxf(m[x], mx[x]);
-                        alpha[x] = m[x] == mn ? 1.f : expf(m[x] - mn);   // a step holds a visible key; scores of -inf leave the state alone
-                        m[x] = mn;
-                    }
-        #pragma unroll
-                    for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : expf(pr[e] - m[e & 1]);
-                    l[0] = l[0] * alpha[0] + (pr[0] + pr[2]);
-                    l[1] = l[1] * alpha[1] + (pr[1] + pr[3]);
-                    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-        #pragma unroll
+                    // the exponents' reference moves only when a score has passed it by 8 ln 2 (weights up to 256; the division at the end makes
+                    // them exact again): seldom after the first step, and no reduction over the keys until then
+                    const float top[2] = {fmaxf(pr[0], pr[2]), fmaxf(pr[1], pr[3])};
+                    if (__any_sync(0xffffffffu, top[0] > m[0] + 5.545f || top[1] > m[1] + 5.545f)) {
+                        float alpha[2];
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            float mx = fmaxf(top[x], __shfl_xor_sync(0xffffffffu, top[x], 4));
+                            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                            const float mn = fmaxf(m[x], mx);
+                            alpha[x] = m[x] == mn ? 1.f : expf(m[x] - mn);
+                            m[x] = mn;
+                            l[x] *= alpha[x];
+                        }
+#pragma unroll
                         for (int j = 0; j < MT; ++j) { o[j][0] *= alpha[0]; o[j][1] *= alpha[1]; o[j][2] *= alpha[0]; o[j][3] *= alpha[1]; }
                     }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : expf(pr[e] - m[e & 1]);
+                    l[0] += pr[0] + pr[2];
+                    l[1] += pr[1] + pr[3];
                 }
                 uint32_t b[3][2];   // hi, mid, lo: p = hi + mid + lo to 24 bits
-        #pragma unroll
+#pragma unroll
                 for (int q = 0; q < 3; ++q)
-        #pragma unroll
+#pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         const __nv_bfloat162 h2 = __floats2bfloat162_rn(pr[2 * hf], pr[2 * hf + 1]);
                         const float2 f = __bfloat1622float2(h2);
@@ -186,28 +193,34 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                         b[q][hf] = pd_transpose(*reinterpret_cast<const uint32_t*>(&h2));
                     }
                 if (!whole) {   // rows that are not this token's may hold anything: 0 * NaN must stay 0
-        #pragma unroll
+#pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int j = j0 + 2 * tig + (i & 1) + (i >> 1) * 8;
                         if (j < j_lo || j > p) {
-        #pragma unroll
+#pragma unroll
                             for (int x = 0; x < VP; ++x) vf[i][x] = make_uint4(0u, 0u, 0u, 0u);
                         }
                     }
                 }
-        #pragma unroll
-                for (int j = 0; j < MT; ++j) {
-                    const int x = j / 4, e = j % 4;
-                    auto word = [&](int i) { const uint4& v = vf[i][x]; return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
-                    const uint32_t af[4] = {__byte_perm(word(0), word(1), 0x5410), __byte_perm(word(0), word(1), 0x7632),
-                                            __byte_perm(word(2), word(3), 0x5410), __byte_perm(word(2), word(3), 0x7632)};
-                    pa_mma(o[j], af, b[2]);
-                    pa_mma(o[j], af, b[1]);
-                    pa_mma(o[j], af, b[0]);
+#pragma unroll
+                for (int x = 0; x < VP; ++x) {   // four tiles of 16 dimensions at a time: consecutive products feed different sums
+                    uint32_t af[4][4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        auto word = [&](int i) { const uint4& v = vf[i][x]; return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+                        af[e][0] = __byte_perm(word(0), word(1), 0x5410);
+                        af[e][1] = __byte_perm(word(0), word(1), 0x7632);
+                        af[e][2] = __byte_perm(word(2), word(3), 0x5410);
+                        af[e][3] = __byte_perm(word(2), word(3), 0x7632);
+                    }
+#pragma unroll
+                    for (int q = 2; q >= 0; --q)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) pa_mma(o[x * 4 + e], af[e], b[q]);
                 }
                 if (more) load_v();
             }
-        #pragma unroll
+#pragma unroll
             for (int x = 0; x < 2; ++x) {
                 l[x] += __shfl_xor_sync(0xffffffffu, l[x], 4);
                 l[x] += __shfl_xor_sync(0xffffffffu, l[x], 8);
@@ -215,9 +228,9 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                 const int h = 2 * tig + x;
                 if (h < R) {
                     if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = l[x]; }
-                    float* dst = om + (size_t)(warp * R + h) * VD + gid * (VD / 8);
-        #pragma unroll
-                    for (int j = 0; j < MT; ++j) *reinterpret_cast<float2*>(dst + 2 * j) = make_float2(o[j][x], o[j][2 + x]);
+                    float* dst = om + (size_t)(warp * R + h) * VD + gid * 8;
+#pragma unroll
+                    for (int j = 0; j < MT; ++j) *reinterpret_cast<float2*>(dst + j / 4 * 64 + j % 4 * 2) = make_float2(o[j][x], o[j][2 + x]);
                 }
             }
             __syncthreads();
@@ -225,10 +238,10 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
             for (int i = threadIdx.x; i < R * VD; i += blockDim.x) {
                 const int h = i / VD;
                 float M = ms[h];
-        #pragma unroll
+#pragma unroll
                 for (int v = 1; v < kPdWarps; ++v) M = fmaxf(M, ms[v * R + h]);
                 float acc = 0.f;
-        #pragma unroll
+#pragma unroll
                 for (int v = 0; v < kPdWarps; ++v) {
                     const float mv = ms[v * R + h];
                     if (mv != -INFINITY) acc += om[(size_t)(v * R + h) * VD + i % VD] * expf(mv - M);
@@ -256,11 +269,11 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                 float M = a.sigmoid ? 0.f : a.sink ? a.sink[qh] : a.denom_bias > 0.f ? 0.f : -INFINITY;
                 const float sink_at = M, sink_l = a.sigmoid || a.sink ? 1.f : a.denom_bias;
                 float mr[kPdMaxCluster];
-        #pragma unroll
+#pragma unroll
                 for (int r = 0; r < kPdMaxCluster; ++r)
                     if (r < splits) { mr[r] = cluster.map_shared_rank(ms, r)[h]; M = fmaxf(M, mr[r]); }
                 float L = sink_at == -INFINITY ? 0.f : sink_l * expf(sink_at - M), acc = 0.f;
-        #pragma unroll
+#pragma unroll
                 for (int r = 0; r < kPdMaxCluster; ++r)
                     if (r < splits && mr[r] != -INFINITY) {
                         const float f = expf(mr[r] - M);
