@@ -1,8 +1,12 @@
 // bfloat16 prompt portions of b200_paged_attention on tcgen05 / TMEM: 128 (token, query head) rows per tile, keys 64 at a time.
 //
-// What bounds it: per 128 x 64 scores of 128-wide heads the tensor pipe needs 640 clocks (the scores are 64 columns wide, so their
-// operands bound them) and the special-function unit 512 for the exponentials; one tile alone is a chain of both, so two CTAs share an
-// SM (96 KB of shared memory and 256 TMEM columns each) and fill each other's gaps.
+// What bounds it: per 128 x 64 scores of 128-wide heads the tensor pipe needs 512 clocks and more (the scores are 64 columns wide, so their
+// operands count) and the special-function unit 512 for the exponentials; one tile alone is a chain of both, so two CTAs share an
+// SM (96 KB of shared memory and 256 TMEM columns each) and fill each other's gaps. A step of 64 keys takes about 1200 clocks with two
+// CTAs on an SM; the longest row tile of a prompt and what comes before its first and after its last step decide.
+// Measured (before: the mma.sync tiles of paged_attention_tile.cuh), 16 / 8 heads x 128, 2048 tokens: 114 -> 33 us. Tried and taken back: 128 keys
+// per tile with one score buffer (52 us: products and softmax take turns), two threads per row (43 us), the keys of a tile shared by a
+// cluster of two (41 us: the fixed part of a CTA counts more than the chain).
 //   rows        TQ tokens x the R query heads of one key head (TQ = 128 / R), so a key tile is read once for the whole group and a
 //               causal edge wastes little. A CTA's window of TQ packed rows may hold the end of one sequence and the start of
 //               the next: they are separate tiles, walked by neighbouring CTAs (gridDim.y is doubled when there is more than one entry).
@@ -22,12 +26,11 @@
 #include "tc_common.cuh"
 
 namespace b200 {
-
 enum { kTcPlain = 0, kTcCapped = 1, kTcBiased = 2, kTcSigmoid = 3 };
 constexpr int kTcRows = 128, kTcKeys = 64, kTcThreads = 192;
 constexpr int kTcBox = kTcKeys * 128;         // bytes of 64 rows x 64 columns
-constexpr int kTcBiasPad = 64 + 128 + 64;     // distances in front of and behind a head's table (below)
-constexpr int kTcBiasFloats = 4096;           // at most this many staged bias numbers per CTA
+constexpr int kTcBiasFront = kTcKeys, kTcBiasPad = kTcBiasFront + 2 * kTcRows;   // distances in front of, and around, a head's staged table
+constexpr int kTcBiasFloats = 12288;          // at most this many staged bias numbers per CTA (from about 3500 on one CTA per SM)
 
 template <int D, int DV>
 struct TcSmem {
@@ -52,31 +55,13 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     volatile int* dead = reinterpret_cast<volatile int*>(masks + 9);
     float* bias_s = reinterpret_cast<float*>(smem + L::kOffBias);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform as the compiler sees it)
     const int ku = blockIdx.x, g = ku / a.maps, mp = ku % a.maps, R = a.heads / a.kv_heads, q_units = a.heads * a.maps;
     // the last rows of a prompt see the most keys: those windows come first
     const int yy = gridDim.y - 1 - blockIdx.y, part = yy % parts, t0 = yy / parts * TQ, rows = min(TQ, a.n_tokens - t0);
 
-    // ---- the window's tiles
-    if (threadIdx.x < TQ + 2) {
-        const int t = t0 - 1 + (int)threadIdx.x;
-        slots[threadIdx.x] = t >= 0 && t < a.n_tokens ? a.slot[t] : -1;
-    }
-    __syncthreads();
-    if (warp < 4) {
-        const int i = threadIdx.x;   // row of the window; slots[i + 1] is its own
-        const bool in = i < rows, starts = in && (i == 0 || slots[i] != slots[i + 1]);
-        const bool single = in && skip_singles && slots[i] != slots[i + 1] && slots[i + 2] != slots[i + 1];
-        const uint32_t b = __ballot_sync(0xffffffffu, starts), tb = __ballot_sync(0xffffffffu, starts && !single);
-        if (lane == 0) { masks[warp] = b; masks[4 + warp] = tb; }
-    }
-    if (threadIdx.x == 0) *dead = 0;
-    __syncthreads();
-    int n_tiles = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) n_tiles += __popc(masks[4 + i]);
-    if (n_tiles <= part) return;   // nothing here for this CTA (no barrier, no TMEM yet)
-
+    // ---- TMEM, barriers, and the window's tiles
+    if (warp == 1) tmem_alloc(tmem_slot, L::kTmemCols);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
@@ -88,19 +73,36 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         mbar_fence_init();
         tma_prefetch_desc(&map_k);
         tma_prefetch_desc(&map_v);
+        *dead = 0;
+    }
+    for (int i = (int)threadIdx.x - 64; i >= 0 && i < TQ + 2; i += kTcThreads - 64) {
+        const int t = t0 - 1 + i;
+        slots[i] = t >= 0 && t < a.n_tokens ? a.slot[t] : -1;
     }
     pdl_launch_dependents();   // the kernel for single tokens may move in (it waits for this one before it ends)
-    if (warp == 1) tmem_alloc(tmem_slot, L::kTmemCols);
-    if (FORM == kTcBiased && a.dist_bias) {
-        // per head: entry 64 + distance; distances below 0 (masked keys) and beyond the table repeat its ends, so that no index needs a clamp
-        const int n = a.dist_n + kTcBiasPad;
-        for (int i = threadIdx.x; i < R * n; i += kTcThreads)
-            bias_s[i] = a.dist_bias[(size_t)(g * R + i / n) * a.dist_n + min(max(i % n - 64, 0), a.dist_n - 1)] * 1.4426950408889634f;
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot, o_tmem = tmem + 2 * kTcKeys;
+    if (warp < 4) {
+        const int i = threadIdx.x;   // row of the window; slots[i + 1] is its own
+        const bool in = i < rows, starts = in && (i == 0 || slots[i] != slots[i + 1]);
+        const bool single = in && skip_singles && slots[i] != slots[i + 1] && slots[i + 2] != slots[i + 1];
+        const uint32_t b = __ballot_sync(0xffffffffu, starts), tb = __ballot_sync(0xffffffffu, starts && !single);
+        if (lane == 0) { masks[warp] = b; masks[4 + warp] = tb; }
+    }
+    int tn = 0;   // staged distances per head: those that a row of the window can have
+    if (FORM == kTcBiased && a.dist_bias) {
+        // per head: entry kTcBiasFront + distance; distances below 0 (masked keys) and beyond the table repeat its ends, so that no index needs a clamp
+        for (int i = lane; i < rows; i += 32) tn = max(tn, a.pos[t0 + i] + 1);
+        tn = min(__reduce_max_sync(0xffffffffu, tn), a.dist_n);
+        for (int x = 0; x < R; ++x) {
+            const float* src = a.dist_bias + (size_t)(g * R + x) * a.dist_n;
+#pragma unroll 4
+            for (int i = threadIdx.x; i < tn + kTcBiasPad; i += kTcThreads) bias_s[x * (tn + kTcBiasPad) + i] = src[min(max(i - kTcBiasFront, 0), tn - 1)] * 1.4426950408889634f;
+        }
+    }
+    __syncthreads();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0), o_tmem = tmem + 2 * kTcKeys;
 
     int it0 = 0, ordinal = 0;   // key tiles walked so far (stage and phase of every ring); tiles of the window seen so far
     for (int first = 0; first < rows;) {
@@ -119,81 +121,104 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         }
         if (ordinal++ % parts != part) { first = end; continue; }
         const int tA = t0 + first, count = end - first;
-        const int pA = a.pos[tA], pZ = a.pos[tA + count - 1];
-        const int key0 = pa_first_key(a, pA) & ~(kTcKeys - 1), n_kt = (pZ - key0) / kTcKeys + 1;
-        const int* plist = a.pages + (size_t)slots[first + 1] * a.max_pages;
-
-        // ---- Q rows into the K-major swizzled operand (rows that this tile does not have: zeros)
-        {
-            constexpr int CH = D / 8;
-            for (int i = threadIdx.x; i < kTcRows * CH; i += kTcThreads) {
-                const int r = i / CH, c = i % CH, tl = r / R, h = g * R + r % R;
-                Pack16 v{{0u, 0u, 0u, 0u}};
-                if (tl < count) {
-                    v = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)(tA + tl) * q_units + h * a.maps + mp) * D + c * 8);
-                    if (pa_scale(a, h) < 0.f) {   // the softmax works with |scale|
+        // ---- warps 2-5: Q rows into the K-major swizzled operand (rows that this tile does not have: zeros), a thread's loads all in
+        // flight together; K and V are on their way meanwhile
+        if (warp >= 2) {
+            constexpr int CH = D / 8, kPass = 128 / CH, kBatch = kTcRows / kPass;   // 16-byte pieces per row; rows per pass of the 128 threads
+            const int tid = threadIdx.x - 64, c = tid % CH, by_r = (65536 + R - 1) / R;
+            unsigned char* dst = smem + (c / 8) * (kTcRows * 128);
+            const int r0 = tid / CH;
+            {
+                Pack16 v[kBatch];
+                uint32_t flip = 0u;
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) v.w[e] ^= 0x80008000u;
+                for (int i = 0; i < kBatch; ++i) {
+                    const int r = r0 + i * kPass, tl = (r * by_r) >> 16, h = g * R + r - tl * R;   // r / R for r < 128
+                    v[i] = Pack16{{0u, 0u, 0u, 0u}};
+                    if (tl < count) {
+                        v[i] = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)(tA + tl) * q_units + h * a.maps + mp) * D + c * 8);
+                        flip |= pa_scale(a, h) < 0.f ? 1u << i : 0u;   // the softmax works with |scale|
                     }
                 }
-                st16(smem + (c / 8) * (kTcRows * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), v);
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) {
+                    const int r = r0 + i * kPass;
+                    if (flip >> i & 1u) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[i].w[e] ^= 0x80008000u;
+                    }
+                    st16(dst + r * 128 + (((c & 7) ^ (r & 7)) << 4), v[i]);
+                }
             }
             fence_proxy_async_smem();
         }
-        __syncthreads();
+        const int pA = a.pos[tA], pZ = a.pos[tA + count - 1];
+        const int key0 = pa_first_key(a, pA) & ~(kTcKeys - 1), n_kt = (pZ - key0) / kTcKeys + 1;
+        const int* plist = a.pages + (size_t)slots[first + 1] * a.max_pages;
+        if (warp >= 1) asm volatile("bar.sync 1, 160;" ::: "memory");
 
         if (warp == 0) {
-            for (int j = 0; j < n_kt; ++j) {
-                const int it = it0 + j, s = it & 1, k0 = key0 + j * kTcKeys;
-                const uint32_t ph = (uint32_t)(it >> 1) & 1u;
-                const int row = plist[k0 / a.page_rows] * a.page_rows + k0 % a.page_rows;
-                mbar_wait_or_leave(&k_empty[s], ph ^ 1u, dead);
+            // K of tile j + 1 goes ahead of V of tile j (which may have to wait for an older product), and a tile's place is looked up one tile
+            // before it is needed
+            auto row_of = [&](int j) {
+                const int k0 = key0 + min(j, n_kt - 1) * kTcKeys;
+                return plist[k0 / a.page_rows] * a.page_rows + k0 % a.page_rows;
+            };
+            auto load = [&](uint64_t* full, uint64_t* empty, int j, int row, const CUtensorMap* map, int x, unsigned char* base, int bytes, int boxes) {
+                const int it = it0 + j, s = it & 1;
+                mbar_wait_or_leave(&empty[s], ((uint32_t)(it >> 1) & 1u) ^ 1u, dead);
                 if (lane == 0) {
-                    mbar_expect_tx(&k_full[s], L::kK);
-#pragma unroll
-                    for (int c = 0; c < D / 64; ++c) tma_load_2d(smem + L::kOffK + s * L::kK + c * kTcBox, &map_k, ku * D + c * 64, row, &k_full[s]);
-                }
-                mbar_wait_or_leave(&v_empty[s], ph ^ 1u, dead);
-                if (lane == 0) {
-                    mbar_expect_tx(&v_full[s], L::kV);
-#pragma unroll
-                    for (int c = 0; c < DV / 64; ++c) tma_load_2d(smem + L::kOffV + s * L::kV + c * kTcBox, &map_v, g * DV + c * 64, row, &v_full[s]);
+                    mbar_expect_tx(&full[s], bytes);
+                    for (int c = 0; c < boxes; ++c) tma_load_2d(base + s * bytes + c * kTcBox, map, x + c * 64, row, &full[s]);
                 }
                 __syncwarp();
+            };
+            int row = row_of(0), row1 = row_of(1), row2;
+            load(k_full, k_empty, 0, row, &map_k, ku * D, smem + L::kOffK, L::kK, D / 64);
+            for (int j = 0; j < n_kt; ++j, row = row1, row1 = row2) {
+                row2 = row_of(j + 2);
+                if (j + 1 < n_kt) load(k_full, k_empty, j + 1, row1, &map_k, ku * D, smem + L::kOffK, L::kK, D / 64);
+                load(v_full, v_empty, j, row, &map_v, g * DV, smem + L::kOffV, L::kV, DV / 64);
             }
         } else if (warp == 1) {
             constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
             constexpr uint32_t idesc_s = make_idesc_f16(kTcRows, kTcKeys) | kBf16, idesc_o = make_idesc_f16(kTcRows, DV) | kBf16 | (1u << 16);
-            auto issue_s = [&](int j) {
-                const int it = it0 + j, s = it & 1;
-                mbar_wait_or_leave(&k_full[s], (uint32_t)(it >> 1) & 1u, dead);
+            // everything that an instruction takes is uniform over the warp and mostly constant: one lane issues twelve of them per tile, and the
+            // softmax waits for the last
+            const uint64_t q_desc = make_kmajor_sw128_desc(smem_u32(smem)), k_desc = make_kmajor_sw128_desc(smem_u32(smem + L::kOffK));
+            const uint64_t v_desc = make_mnmajor_sw128_desc(smem_u32(smem + L::kOffV), kTcBox, 1024u);
+            const int n = __shfl_sync(0xffffffffu, n_kt, 0);
+            int it = __shfl_sync(0xffffffffu, it0, 0);
+            const bool leader = elect_one();
+            auto issue_s = [&](int i) {   // tile i (counted over all tiles of this CTA)
+                const uint32_t s = (uint32_t)i & 1u;
+                mbar_wait_or_leave(&k_full[s], (uint32_t)(i >> 1) & 1u, dead);
                 tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t qa = smem_u32(smem), ka = smem_u32(smem + L::kOffK + s * L::kK);
+                if (leader) {
+                    const uint64_t kd = k_desc + (uint64_t)(s * (L::kK >> 4));
+                    const uint32_t d = tmem + s * kTcKeys;
 #pragma unroll
                     for (int ks = 0; ks < D / kUmmaK; ++ks)
-                        umma_f16(tmem + (uint32_t)(s * kTcKeys), make_kmajor_sw128_desc(qa + (ks >> 2) * (kTcRows * 128)) + (uint64_t)(2 * (ks & 3)),
-                                 make_kmajor_sw128_desc(ka + (ks >> 2) * kTcBox) + (uint64_t)(2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
-                    umma_commit(&k_empty[s]);
+                        umma_f16(d, q_desc + (uint64_t)((ks >> 2) * (kTcRows * 128 >> 4) + 2 * (ks & 3)), kd + (uint64_t)((ks >> 2) * (kTcBox >> 4) + 2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
                     umma_commit(&s_full[s]);
+                    umma_commit(&k_empty[s]);
                 }
                 __syncwarp();
             };
-            issue_s(0);
-            for (int j = 0; j < n_kt; ++j) {
-                // (the score buffer of j + 1 last held P_{j-1}, whose product is ahead of it in the tensor pipe)
-                if (j + 1 < n_kt) issue_s(j + 1);
-                const int it = it0 + j, s = it & 1;
-                const uint32_t ph = (uint32_t)(it >> 1) & 1u;
+            issue_s(it);
+            for (int j = 0; j < n; ++j, ++it) {
+                // (the score buffer of the next tile last held this one's predecessor's weights, whose product is ahead of it in the tensor pipe)
+                if (j + 1 < n) issue_s(it + 1);
+                const uint32_t s = (uint32_t)it & 1u, ph = (uint32_t)(it >> 1) & 1u;
                 mbar_wait_or_leave(&v_full[s], ph, dead);
                 mbar_wait_or_leave(&p_full[s], ph, dead);
                 tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t va = smem_u32(smem + L::kOffV + s * L::kV);
+                if (leader) {
+                    const uint64_t vd = v_desc + (uint64_t)(s * (L::kV >> 4));
+                    const uint32_t pa = tmem + s * kTcKeys;
 #pragma unroll
                     for (int ks = 0; ks < kTcKeys / kUmmaK; ++ks)
-                        umma_f16_ts(o_tmem, tmem + (uint32_t)(s * kTcKeys + ks * 8), make_mnmajor_sw128_desc(va + ks * 2048u, kTcBox, 1024u), idesc_o,
-                                    j > 0 || ks > 0 ? 1u : 0u);
+                        umma_f16_ts(o_tmem, pa + (uint32_t)(ks * 8), vd + (uint64_t)(ks * (2048 >> 4)), idesc_o, ks > 0 || j > 0 ? 1u : 0u);
                     umma_commit(&v_empty[s]);
                     umma_commit(&o_done[s]);
                 }
@@ -208,14 +233,14 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
             const float sc = fabsf(pa_scale(a, h));
             constexpr float kLog2E = 1.4426950408889634f;
             // scores leave TMEM as q . k; plain: p = 2^(q . k * sl - m * sl), m the largest q . k; capped, biased: first x = the score times log2 e
-            const float sl = sc * kLog2E;
+            const float sl = fmaxf(sc * kLog2E, 1e-30f);   // never 0: a masked score is -inf
             const float over_cap = FORM == kTcCapped ? sc / a.softcap : 0.f, cap2 = a.softcap * kLog2E;
             const float hb2 = FORM == kTcSigmoid && a.head_bias ? a.head_bias[h] * kLog2E : 0.f;
             const float* brow = nullptr;
             float far_bias = 0.f;
             if (FORM == kTcBiased && a.dist_bias) {
-                brow = bias_s + hr * (a.dist_n + kTcBiasPad) + 64;
-                far_bias = brow[a.dist_n - 1];
+                brow = bias_s + hr * (tn + kTcBiasPad) + kTcBiasFront;
+                far_bias = a.dist_bias[(size_t)h * a.dist_n + a.dist_n - 1] * kLog2E;
             }
             float m = -1e30f, l = 0.f;   // m: what the exponents are taken against (the scores of FORM plain unscaled)
             const float step = FORM == kTcPlain ? sl : 1.f;   // log2 units per unit of m
@@ -224,7 +249,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                 const uint32_t ph = (uint32_t)(it >> 1) & 1u, st = tmem + my + (uint32_t)(s * kTcKeys);
                 mbar_wait_or_leave(&s_full[s], ph, dead);
                 tc_fence_after();
-                if (j == n_kt - 1 && (pZ + 1) % kTcKeys != 0) {
+                if (k0 + kTcKeys > pZ + 1) {
                     // V rows behind the context: 0 * NaN must stay 0. (After the wait above: these scores follow the product two tiles before in
                     // the tensor pipe, so the stage has seen its last but one load and its barrier can be waited on by parity.)
                     mbar_wait_or_leave(&v_full[s], ph, dead);
@@ -244,70 +269,66 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                 const bool whole = __all_sync(0xffffffffu, k0 + kTcKeys - 1 <= p && k0 >= f);
                 if (FORM == kTcCapped) {
                     // cap * tanh(v / cap): the odd series below |x| = 0.25 (exact to fp32 rounding), else (t - 1) / (t + 1), t = e^(2x)
-                    float big = 0.f;
+                    float big[2] = {0.f, 0.f};
 #pragma unroll
-                    for (int e = 0; e < 64; ++e) {
-                        const float x = S(e) * over_cap;
-                        sv[e] = __float_as_uint(x);
-                        big = fmaxf(big, fabsf(x));
-                    }
-                    if (__all_sync(0xffffffffu, big < 0.25f)) {
+                    for (int e = 0; e < 64; ++e) big[e & 1] = fmaxf(big[e & 1], fabsf(S(e)));
+                    if (__all_sync(0xffffffffu, fmaxf(big[0], big[1]) * over_cap < 0.25f)) {
+                        const uint64_t oc2 = pack2f(over_cap, over_cap), c2 = pack2f(cap2, cap2), one2 = pack2f(1.f, 1.f);
+                        const uint64_t c7 = pack2f(-17.f / 315.f, -17.f / 315.f), c5 = pack2f(2.f / 15.f, 2.f / 15.f), c3 = pack2f(-1.f / 3.f, -1.f / 3.f);
 #pragma unroll
-                        for (int e = 0; e < 64; ++e) {
-                            const float x = S(e), x2 = x * x;
-                            sv[e] = __float_as_uint(cap2 * x * fmaf(x2, fmaf(x2, fmaf(x2, -17.f / 315.f, 2.f / 15.f), -1.f / 3.f), 1.f));
+                        for (int e = 0; e < 64; e += 2) {
+                            const uint64_t x = mul2(pack2(sv[e], sv[e + 1]), oc2), x2 = mul2(x, x);
+                            float y0, y1;
+                            unpack2(mul2(mul2(c2, x), fma2(x2, fma2(x2, fma2(x2, c7, c5), c3), one2)), y0, y1);
+                            sv[e] = __float_as_uint(y0);
+                            sv[e + 1] = __float_as_uint(y1);
                         }
                     } else {
 #pragma unroll
                         for (int e = 0; e < 64; ++e) {
-                            const float t = ex2_approx(fminf(fmaxf(S(e) * (2.f * kLog2E), -43.f), 43.f));
+                            const float t = ex2_approx(fminf(fmaxf(S(e) * over_cap * (2.f * kLog2E), -43.f), 43.f));
                             sv[e] = __float_as_uint(cap2 * __fdividef(t - 1.f, t + 1.f));
                         }
                     }
                 } else if (FORM == kTcBiased) {
                     if (brow && !__all_sync(0xffffffffu, p < 0 || p - (k0 + kTcKeys - 1) >= a.dist_n - 1)) {
-                        const int most = a.dist_n - 1 + 64 + 127;
+                        const int most = tn - 1 + 2 * kTcRows - kTcKeys;
                         const float* b = brow + max(min(p - k0, most), 0);   // rows without a token: any place of the table
                         if (__all_sync(0xffffffffu, p - k0 <= most)) {
 #pragma unroll
                             for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, b[-e]));
                         } else {
 #pragma unroll
-                            for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, brow[min(max(p - k0 - e, 0), a.dist_n - 1)]));
+                            for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, brow[min(max(p - k0 - e, 0), tn - 1)]));
                         }
                     } else {
 #pragma unroll
                         for (int e = 0; e < 64; ++e) sv[e] = __float_as_uint(fmaf(S(e), sl, far_bias));
                     }
                 }
+                if (!whole) {   // keys that the row does not see: -inf, a weight of 0 whatever comes
+                    const int hi = p - k0, lo = f - k0;
+#pragma unroll
+                    for (int e = 0; e < 64; ++e) sv[e] = e <= hi ? sv[e] : 0xff800000u;
+                    if (__any_sync(0xffffffffu, lo > 0)) {
+#pragma unroll
+                        for (int e = 0; e < 64; ++e) sv[e] = e >= lo ? sv[e] : 0xff800000u;
+                    }
+                }
                 uint32_t pk[32];
                 if (FORM == kTcSigmoid) {   // weights that are not normalised over the keys
 #pragma unroll
-                    for (int e = 0; e < 64; e += 2) {
-                        float w[2];
-#pragma unroll
-                        for (int x = 0; x < 2; ++x) {
-                            const float v = __fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e + x), sl, hb2)));
-                            const int key = k0 + e + x;
-                            w[x] = whole || (key <= p && key >= f) ? v : 0.f;
-                        }
-                        pk[e / 2] = pa_pack(w[0], w[1]);
-                    }
+                    for (int e = 0; e < 64; e += 2)
+                        pk[e / 2] = pa_pack(__fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e), sl, hb2))), __fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e + 1), sl, hb2))));
                 } else {
                     float mx[4] = {-1e30f, -1e30f, -1e30f, -1e30f};
-                    if (whole) {
 #pragma unroll
-                        for (int e = 0; e < 64; ++e) mx[e & 3] = fmaxf(mx[e & 3], S(e));
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 64; ++e) mx[e & 3] = k0 + e <= p && k0 + e >= f ? fmaxf(mx[e & 3], S(e)) : mx[e & 3];
-                    }
+                    for (int e = 0; e < 64; ++e) mx[e & 3] = fmaxf(mx[e & 3], S(e));
                     const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
                     const bool grown = (top - m) * step > 8.f;
                     if (j > 0 && __any_sync(0xffffffffu, grown)) {
                         mbar_wait_or_leave(&o_done[s ^ 1], (uint32_t)((it - 1) >> 1) & 1u, dead);
                         tc_fence_after();
-                        __syncwarp();
                         const float alpha = grown ? ex2_approx((m - top) * step) : 1.f;
 #pragma unroll 1
                         for (int c = 0; c < DV; c += 32) {
@@ -323,32 +344,18 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                     if (grown) m = top;
                     const float ms = -m * step;
                     const uint64_t sl2 = pack2f(step, step), nm2 = pack2f(ms, ms);
-                    uint64_t rs2 = 0ull;
-                    if (whole) {
+                    uint64_t rs2[2] = {0ull, 0ull};
 #pragma unroll
-                        for (int e = 0; e < 64; e += 2) {
-                            float a0, a1;
-                            unpack2(FORM == kTcPlain ? fma2(pack2(sv[e], sv[e + 1]), sl2, nm2) : add2(pack2(sv[e], sv[e + 1]), nm2), a0, a1);
-                            a0 = ex2_approx(a0);
-                            a1 = ex2_approx(a1);
-                            rs2 = add2(rs2, pack2f(a0, a1));
-                            pk[e / 2] = pa_pack(a0, a1);
-                        }
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 64; e += 2) {
-                            float w[2];
-#pragma unroll
-                            for (int x = 0; x < 2; ++x) {
-                                const float v = ex2_approx(fmaf(S(e + x), step, ms));
-                                w[x] = k0 + e + x <= p && k0 + e + x >= f ? v : 0.f;
-                            }
-                            rs2 = add2(rs2, pack2f(w[0], w[1]));
-                            pk[e / 2] = pa_pack(w[0], w[1]);
-                        }
+                    for (int e = 0; e < 64; e += 2) {
+                        float a0, a1;
+                        unpack2(FORM == kTcPlain ? fma2(pack2(sv[e], sv[e + 1]), sl2, nm2) : add2(pack2(sv[e], sv[e + 1]), nm2), a0, a1);
+                        a0 = ex2_approx(a0);
+                        a1 = ex2_approx(a1);
+                        rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2f(a0, a1));
+                        pk[e / 2] = pa_pack(a0, a1);
                     }
                     float r0, r1;
-                    unpack2(rs2, r0, r1);
+                    unpack2(add2(rs2[0], rs2[1]), r0, r1);
                     l += r0 + r1;
                 }
                 tmem_st_32x32(st, pk);
@@ -357,46 +364,40 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_full[s]);
             }
-            // ---- division by the weights' sum, in which the sink counts, and the rows' stores
             // (a wait by parity must be neither two phases behind nor ahead: a barrier per stage, whose last but one product these scores imply)
             const int last = it0 + n_kt - 1;
             mbar_wait_or_leave(&o_done[last & 1], (uint32_t)(last >> 1) & 1u, dead);
             tc_fence_after();
-            __syncwarp();
+            const float m2 = m * step, sink_w = FORM == kTcSigmoid ? 0.f : a.sink ? 1.f : a.denom_bias, s2 = a.sink ? a.sink[h] * kLog2E : 0.f;
+            const size_t dst = ((size_t)(tA + tl) * q_units + h * a.maps + mp) * DV;
+            // division by the weights' sum, in which the sink counts
             float inv = 1.f;
             if (FORM != kTcSigmoid) {
-                const float m2 = m * step, w = a.sink ? 1.f : a.denom_bias;
-                const float s2 = a.sink ? a.sink[h] * kLog2E : 0.f;
-                if (w > 0.f) {
-                    const float M = fmaxf(m2, s2), fo = ex2_approx(m2 - M);
-                    inv = fo / (l * fo + w * ex2_approx(s2 - M));
-                } else
-                    inv = 1.f / l;
+                const float M = sink_w > 0.f ? fmaxf(m2, s2) : m2, fo = ex2_approx(m2 - M);
+                inv = fo / (l * fo + (sink_w > 0.f ? sink_w * ex2_approx(s2 - M) : 0.f));
             }
             if (*dead) inv = __int_as_float(0x7fffffff);
-            const size_t dst = ((size_t)(tA + tl) * q_units + h * a.maps + mp) * DV;
 #pragma unroll 1
             for (int c = 0; c < DV; c += 32) {
                 uint32_t ov[32];
+                __syncwarp();
                 tmem_ld_32x32_async(o_tmem + my + (uint32_t)c, ov);
                 tmem_wait_ld<32>(ov);
-                if (mine) {
-                    if (a.out_f32) {
-                        float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + dst + c);
+                if (!mine) continue;
+                if (a.out_f32) {
+                    float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + dst + c);
 #pragma unroll
-                        for (int e = 0; e < 32; e += 4)
-                            d[e / 4] = make_float4(__uint_as_float(ov[e]) * inv, __uint_as_float(ov[e + 1]) * inv, __uint_as_float(ov[e + 2]) * inv, __uint_as_float(ov[e + 3]) * inv);
-                    } else {
+                    for (int e = 0; e < 32; e += 4)
+                        d[e / 4] = make_float4(__uint_as_float(ov[e]) * inv, __uint_as_float(ov[e + 1]) * inv, __uint_as_float(ov[e + 2]) * inv, __uint_as_float(ov[e + 3]) * inv);
+                } else {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            Pack16 v;
+                    for (int q = 0; q < 4; ++q) {
+                        Pack16 w;
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) v.w[e] = pa_pack(__uint_as_float(ov[q * 8 + 2 * e]) * inv, __uint_as_float(ov[q * 8 + 2 * e + 1]) * inv);
-                            st16(reinterpret_cast<bf*>(a.out) + dst + c + q * 8, v);
-                        }
+                        for (int e = 0; e < 4; ++e) w.w[e] = pa_pack(__uint_as_float(ov[q * 8 + 2 * e]) * inv, __uint_as_float(ov[q * 8 + 2 * e + 1]) * inv);
+                        st16(reinterpret_cast<bf*>(a.out) + dst + c + q * 8, w);
                     }
                 }
-                __syncwarp();
             }
             tc_fence_before();
         }
