@@ -1,20 +1,19 @@
 // Single tokens of b200_paged_attention in bfloat16 (decode batches): every (token, key head) is served by one cluster of CTAs that
 // share the token's context, one launch, no workspace.
 //
-// What bounds it: the keys and values, read once (8 KB per 16 keys of 128 x 128), so the kernel has to keep enough 16-byte loads
-// in flight and spend few instructions per byte. A warp walks its own run of keys, 16 at a time, and never waits for another one:
-//   S^T = K Q^T   mma.sync m16n8k16, keys on the M axis, the R <= 8 query heads of the key head on the N axis. The order of the
-//                 contraction is free, so a thread's fragment is one 16-byte piece of its key row straight from global memory.
+// What bounds it: the keys and values, read once (8 KB per 16 keys of 128 x 128), so the kernel has to keep enough of them on their way
+// and spend few instructions per byte. A warp walks its own run of keys, 16 at a time, out of a ring of its own in shared memory that
+// cp.async fills three steps deep (24 KB per warp, two CTAs of four warps per SM), and never waits for another warp:
+//   S^T = K Q^T   mma.sync m16n8k16, keys on the M axis, the R <= 8 query heads of the key head on the N axis
 //   softmax       fp32 in registers, a running (maximum, denominator) per warp; cap, bias, temperature and masks as in the row kernel
-//   O^T = V^T P^T value dimensions on the M axis: a thread loads 16-byte pieces of four value rows and pairs them with PRMT. The
-//                 weights keep 24 bits: p = hi + mid + lo (three bfloat16, the difference exact at every step), three products
-//                 with fp32 accumulation, so nothing is rounded to 16 bits on the way. movmatrix turns the weights' fragments.
-// The next step's keys are requested before the softmax, the next step's values before the following scores: 8 KB per warp in flight,
-// twelve warps per SM. Warps merge through shared memory, CTAs through distributed shared memory (rank order, so the sum does not
-// depend on timing). The merge adds the sink.
-// Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128:
-// 20.5 -> 8.2 us; 32 sequences of up to 2048 tokens, 16 / 8 heads x 128, bias and sink (190 MB): 383 -> 69 us (84 us with one chain of
-// score products, the maximum reduced at every step and three dependent products per output tile: the step's latency was what counted).
+//   O^T = V^T P^T value dimensions on the M axis (ldmatrix.trans). The weights keep 24 bits: p = hi + mid + lo (three bfloat16, the
+//                 difference exact at every step), three products with fp32 accumulation, so nothing is rounded to 16 bits on the way.
+//                 movmatrix turns the weights' fragments.
+// Warps merge through shared memory, CTAs through distributed shared memory (rank order, so the sum does not depend on timing). The merge
+// adds the sink.
+// Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128: 20.5 -> 8.2 us;
+// 32 sequences of up to 2048 tokens, 16 / 8 heads x 128 (190 MB), bias and sink: 384 -> 61 us (69 us with a step's keys and values in
+// registers, requested one step ahead); 128 such sequences without bias run at 5.0 TB/s.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -30,6 +29,13 @@ namespace cg = cooperative_groups;
 
 constexpr int kPdWarps = 4, kPdStep = 16, kPdHeads = 8, kPdMaxCluster = 8;
 
+template <int D, int VD>
+struct PdRing {   // row strides in elements (16 bytes of padding: conflict-free ldmatrix), a step's keys, then its values
+    static constexpr int kRS = D + 8, kRSV = VD + 8, kStages = VD > 128 ? 2 : 3;
+    static constexpr int kStep = kPdStep * (kRS + kRSV), kWarp = kStages * kStep;   // elements
+    static constexpr int kBytes = kPdWarps * kWarp * 2;
+};
+
 __device__ __forceinline__ uint32_t pd_transpose(uint32_t v) {   // 8 x 8 tile of 16-bit numbers, a pair per thread
     uint32_t r;
     asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
@@ -39,25 +45,26 @@ __device__ __forceinline__ uint32_t pd_transpose(uint32_t v) {   // 8 x 8 tile o
 // MIXED: a batch that also holds prompt portions, which other kernels take. Cluster z looks after the tokens z, z + gridDim.z, ... and serves
 // those that are their sequence's only token in the batch.
 template <int D, int VD, bool MIXED>
-__global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_kernel(const PA a) {
+__global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA a) {
     using bf = __nv_bfloat16;
-    constexpr int KC = D / 32;        // 16-byte pieces of a key row per thread
-    constexpr int VP = VD / 64;       // 16-byte pieces of a value row per thread (VD / 8 dimensions)
+    using L = PdRing<D, VD>;
+    constexpr int KS = D / 16;        // k steps of the scores
     constexpr int MT = VD / 16;       // m tiles of the output
-    extern __shared__ float pd_sm[];
+    extern __shared__ __align__(16) float pd_sm[];
     const int R = a.heads / a.kv_heads, splits = gridDim.x;
-    float* om = pd_sm;                                 // [warps][R][VD], then this CTA's share in the first [R][VD]
-    float* ms = om + kPdWarps * R * VD;                // [warps][R], then [R]
-    float* ls = ms + kPdWarps * R;
+    float* om = pd_sm;                                 // once the rings have been used: [warps][R][VD], then this CTA's share in the first [R][VD]
+    __shared__ float ms[kPdWarps * kPdHeads], ls[kPdWarps * kPdHeads];   // [warps][R], then [R]
     const int ku = blockIdx.y, g = ku / a.maps, mp = ku % a.maps;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane >> 2, tig = lane & 3;
     const int k_units = a.kv_heads * a.maps, q_units = a.heads * a.maps;
-    const bf* K = reinterpret_cast<const bf*>(a.k_pool) + (size_t)ku * D + tig * 8;
-    const bf* V = reinterpret_cast<const bf*>(a.v_pool) + (size_t)g * VD + gid * 8;
+    const bf* K = reinterpret_cast<const bf*>(a.k_pool) + (size_t)ku * D;
+    const bf* V = reinterpret_cast<const bf*>(a.v_pool) + (size_t)g * VD;
+    bf* ring = reinterpret_cast<bf*>(pd_sm) + warp * L::kWarp;
     const size_t k_row = (size_t)k_units * D, v_row = (size_t)a.kv_heads * VD;
 
     // this thread's two heads (columns of S^T and O^T)
     float sc[2], hb[2];
+    const float over_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
     const float* bias[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
@@ -76,13 +83,12 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
         }
         for (; todo; todo &= todo - 1) {
             const int t = MIXED ? base + (__ffs(todo) - 1) * (int)gridDim.z : base;
-            uint32_t qf[KC][4];               // query head gid (heads beyond the group: zeros)
+            uint32_t qf[KS][2];               // query head gid (heads beyond the group: zeros)
 #pragma unroll
-            for (int c = 0; c < KC; ++c) {
-                Pack16 v{{0u, 0u, 0u, 0u}};
-                if (gid < R) v = ld16(reinterpret_cast<const bf*>(a.q) + ((size_t)t * q_units + (g * R + gid) * a.maps + mp) * D + c * 32 + tig * 8);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) qf[c][e] = v.w[e];
+            for (int ks = 0; ks < KS; ++ks) {
+                const bf* q = reinterpret_cast<const bf*>(a.q) + ((size_t)t * q_units + (g * R + min(gid, R - 1)) * a.maps + mp) * D + ks * 16 + tig * 2;
+                qf[ks][0] = gid < R ? *reinterpret_cast<const uint32_t*>(q) : 0u;
+                qf[ks][1] = gid < R ? *reinterpret_cast<const uint32_t*>(q + 8) : 0u;
             }
             const int p = a.pos[t];
             const int* plist = a.pages + (size_t)a.slot[t] * a.max_pages;
@@ -97,38 +103,44 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
             const int s0 = w * per, s1 = min(steps, s0 + per);
             int j0 = first + s0 * kPdStep;
             int page_at = j0 / a.page_rows, off = j0 - page_at * a.page_rows;    // of the step that is fetched next
-            uint4 kf[2][KC], vf[4][VP];
             int page = s0 < s1 ? plist[page_at] : 0;
-            size_t row_next = 0;
-            auto advance = [&](bool more) {   // the fetched step's first row; then one step on, its page requested ahead
-                row_next = (size_t)page * a.page_rows + off;
-                off += kPdStep;
-                if (off == a.page_rows) { off = 0; ++page_at; if (more) page = plist[page_at]; }
-            };
-            auto load_k = [&]() {
-                const bf* r0 = K + (row_next + gid) * k_row;
-                const bf* r1 = r0 + 8 * k_row;
+            auto fetch = [&](int s) {   // step s into its stage; keys that the token does not see arrive as zeros (their rows may hold anything)
+                bf* dst = ring + (s - s0) % L::kStages * L::kStep;
+                const size_t row0 = (size_t)page * a.page_rows + off;
+                const int j = first + s * kPdStep;
 #pragma unroll
-                for (int c = 0; c < KC; ++c) {
-                    kf[0][c] = *reinterpret_cast<const uint4*>(r0 + c * 32);
-                    kf[1][c] = *reinterpret_cast<const uint4*>(r1 + c * 32);
+                for (int i = 0; i < kPdStep * (D / 8) / 32; ++i) {
+                    const int at = i * 32 + lane, r = at / (D / 8), c = at % (D / 8) * 8;
+                    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * L::kRS + c);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(K + (row0 + r) * k_row + c), "r"(j + r >= j_lo && j + r <= p ? 16 : 0) : "memory");
                 }
-            };
-            auto load_v = [&]() {
+                dst += kPdStep * L::kRS;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const bf* r = V + (row_next + 2 * tig + (i & 1) + (i >> 1) * 8) * v_row;
-#pragma unroll
-                    for (int x = 0; x < VP; ++x) vf[i][x] = *reinterpret_cast<const uint4*>(r + x * 64);
+                for (int i = 0; i < kPdStep * (VD / 8) / 32; ++i) {
+                    const int at = i * 32 + lane, r = at / (VD / 8), c = at % (VD / 8) * 8;
+                    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * L::kRSV + c);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(V + (row0 + r) * v_row + c), "r"(j + r >= j_lo && j + r <= p ? 16 : 0) : "memory");
                 }
+                off += kPdStep;   // the page of the step after is looked up now
+                if (off == a.page_rows) { off = 0; ++page_at; if (s + 1 < s1) page = plist[page_at]; }
             };
-            if (s0 < s1) {
-                advance(s0 + 1 < s1);
-                load_k();
-                load_v();
+            auto close_group = [&]() {
+                __syncwarp();   // the lanes close their group of copies together
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            };
+#pragma unroll
+            for (int i = 0; i < L::kStages - 1; ++i) {
+                if (s0 + i < s1) fetch(s0 + i);
+                close_group();
             }
             for (int s = s0; s < s1; ++s, j0 += kPdStep) {
-                const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p, more = s + 1 < s1;
+                const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p;
+                if (s + L::kStages - 1 < s1) fetch(s + L::kStages - 1);
+                close_group();
+                asm volatile("cp.async.wait_group %0;" ::"n"(L::kStages - 1) : "memory");
+                __syncwarp();   // step s has landed for every lane
+                const bf* Ks = ring + (s - s0) % L::kStages * L::kStep;
+                const bf* Vs = Ks + kPdStep * L::kRS;
                 float bv[4] = {0.f, 0.f, 0.f, 0.f};
                 if (a.dist_bias) {   // requested before the scores are formed
 #pragma unroll
@@ -136,23 +148,36 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                 }
                 float st[4] = {0.f, 0.f, 0.f, 0.f}, su[4] = {0.f, 0.f, 0.f, 0.f};   // two chains of products
 #pragma unroll
-                for (int c = 0; c < KC; ++c) {
-                    const uint32_t a0[4] = {kf[0][c].x, kf[1][c].x, kf[0][c].y, kf[1][c].y}, a1[4] = {kf[0][c].z, kf[1][c].z, kf[0][c].w, kf[1][c].w};
-                    const uint32_t b0[2] = {qf[c][0], qf[c][1]}, b1[2] = {qf[c][2], qf[c][3]};
-                    pa_mma(st, a0, b0);
-                    pa_mma(su, a1, b1);
+                for (int ks = 0; ks < KS; ks += 2) {
+                    uint32_t k0[4], k1[4];
+                    pa_ldsm_x4(k0, Ks + (lane & 15) * L::kRS + (lane >> 4) * 8 + ks * 16);
+                    pa_ldsm_x4(k1, Ks + (lane & 15) * L::kRS + (lane >> 4) * 8 + ks * 16 + 16);
+                    pa_mma(st, k0, qf[ks]);
+                    pa_mma(su, k1, qf[ks + 1]);
                 }
-                if (more) {
-                    advance(s + 2 < s1);
-                    load_k();
+#pragma unroll
+                for (int e = 0; e < 4; ++e) st[e] = (st[e] + su[e]) * sc[e & 1];
+                if (a.softcap > 0.f) {
+                    // cap * tanh(v / cap): the odd series up to x^7 while every |x| is below 0.2 (its next term is below 2^-24 of x there)
+                    float x[4], big = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { x[e] = st[e] * over_cap; big = fmaxf(big, fabsf(x[e])); }
+                    if (__all_sync(0xffffffffu, big < 0.2f)) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float x2 = x[e] * x[e];
+                            st[e] = a.softcap * x[e] * fmaf(x2, fmaf(x2, fmaf(x2, -17.f / 315.f, 2.f / 15.f), -1.f / 3.f), 1.f);
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) st[e] = a.softcap * tanhf(x[e]);
+                    }
                 }
                 float pr[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {   // key j0 + gid (+ 8), head 2 tig (+ 1)
-                    const int j = j0 + gid + (e >> 1) * 8, x = e & 1;
-                    float v = (st[e] + su[e]) * sc[x];
-                    if (a.softcap > 0.f) v = a.softcap * tanhf(v / a.softcap);
-                    pr[e] = whole || (j >= j_lo && j <= p) ? v + bv[e] : -INFINITY;
+                    const int j = j0 + gid + (e >> 1) * 8;
+                    pr[e] = whole || (j >= j_lo && j <= p) ? st[e] + bv[e] : -INFINITY;
                 }
                 if (a.sigmoid) {
 #pragma unroll
@@ -192,34 +217,20 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                         pr[2 * hf + 1] -= f.y;
                         b[q][hf] = pd_transpose(*reinterpret_cast<const uint32_t*>(&h2));
                     }
-                if (!whole) {   // rows that are not this token's may hold anything: 0 * NaN must stay 0
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int j = j0 + 2 * tig + (i & 1) + (i >> 1) * 8;
-                        if (j < j_lo || j > p) {
-#pragma unroll
-                            for (int x = 0; x < VP; ++x) vf[i][x] = make_uint4(0u, 0u, 0u, 0u);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int x = 0; x < VP; ++x) {   // four tiles of 16 dimensions at a time: consecutive products feed different sums
+                for (int j = 0; j < MT; j += 4) {   // four tiles of 16 dimensions at a time: consecutive products feed different sums
                     uint32_t af[4][4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        auto word = [&](int i) { const uint4& v = vf[i][x]; return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
-                        af[e][0] = __byte_perm(word(0), word(1), 0x5410);
-                        af[e][1] = __byte_perm(word(0), word(1), 0x7632);
-                        af[e][2] = __byte_perm(word(2), word(3), 0x5410);
-                        af[e][3] = __byte_perm(word(2), word(3), 0x7632);
-                    }
+                    for (int e = 0; e < 4; ++e) pa_ldsm_x4_trans(af[e], Vs + ((lane & 7) + (lane >> 4) * 8) * L::kRSV + (j + e) * 16 + ((lane >> 3) & 1) * 8);
 #pragma unroll
                     for (int q = 2; q >= 0; --q)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) pa_mma(o[x * 4 + e], af[e], b[q]);
+                        for (int e = 0; e < 4; ++e) pa_mma(o[j + e], af[e], b[q]);
                 }
-                if (more) load_v();
+                __syncwarp();   // the stage may be filled again
             }
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();    // the rings' place is taken by the sums
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 l[x] += __shfl_xor_sync(0xffffffffu, l[x], 4);
@@ -228,9 +239,12 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
                 const int h = 2 * tig + x;
                 if (h < R) {
                     if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = l[x]; }
-                    float* dst = om + (size_t)(warp * R + h) * VD + gid * 8;
+                    float* dst = om + (size_t)(warp * R + h) * VD + gid;
 #pragma unroll
-                    for (int j = 0; j < MT; ++j) *reinterpret_cast<float2*>(dst + j / 4 * 64 + j % 4 * 2) = make_float2(o[j][x], o[j][2 + x]);
+                    for (int j = 0; j < MT; ++j) {
+                        dst[j * 16] = o[j][x];
+                        dst[j * 16 + 8] = o[j][2 + x];
+                    }
                 }
             }
             __syncthreads();
@@ -291,9 +305,11 @@ __global__ void __launch_bounds__(kPdWarps * 32, VD > 128 ? 2 : 3) paged_decode_
 
 template <int D, int VD, bool MIXED>
 static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s) {
-    const int R = a.heads / a.kv_heads;
-    const size_t smem = ((size_t)kPdWarps * R * VD + 2 * kPdWarps * R) * sizeof(float);
-    static_assert(((size_t)kPdWarps * kPdHeads * VD + 2 * kPdWarps * kPdHeads) * sizeof(float) <= 48 * 1024, "no shared-memory opt-in needed");
+    constexpr int smem = PdRing<D, VD>::kBytes;
+    static_assert(kPdWarps * kPdHeads * VD * 4 <= smem, "the warps' sums take the rings' place");
+    static unsigned long long done = 0;
+    cudaError_t e = ensure_max_dynamic_smem((const void*)paged_decode_kernel<D, VD, MIXED>, smem, done);
+    if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)splits, (unsigned)(a.kv_heads * a.maps), (unsigned)rows);
     cfg.blockDim = dim3(kPdWarps * 32);
@@ -310,7 +326,7 @@ static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, a);
+    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, a);
     if (e != cudaSuccess) return (int)e;
     count_launch();
     return (int)cudaGetLastError();
@@ -330,11 +346,12 @@ int paged_decode(const PA& a, int longest_seen, bool mixed, cudaStream_t s) {
     // how many tokens of a mixed batch are single ones is only known on the device: sixteen rows of clusters share them
     const int rows = mixed ? std::min(a.n_tokens, 16) : a.n_tokens;
     if (rows > 65535) return -1;
-    // at least four CTAs per SM (three fit at a time), as long as every warp of a cluster keeps a step of its own
-    // (32 sequences of up to 2048 tokens, CTAs per SM aimed at and us: 1: 104, 2 and 3: 89, 4 and 6: 82, 12: 97)
+    // three CTAs for every two SMs, as long as every warp of a cluster keeps a step of its own (32 sequences of up to 2048 tokens, 16 / 8
+    // heads: 256 / 512 / 1024 CTAs 49 / 51 / 63 us; 8 of up to 1024: 256 / 512 CTAs 14.5 / 20.6 us)
     const long long pairs = (long long)rows * a.kv_heads * a.maps;
+    const int most = mixed ? 4 : kPdMaxCluster;
     int splits = 1;
-    while (splits < kPdMaxCluster && (mixed || pairs * splits < 4ll * sm_count()) && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+    while (splits < most && (mixed || 2 * pairs * splits < 3ll * sm_count()) && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
     return mixed ? paged_decode_for<true>(a, splits, rows, s) : paged_decode_for<false>(a, splits, rows, s);
 }
 
