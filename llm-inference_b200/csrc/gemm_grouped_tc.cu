@@ -1,0 +1,212 @@
+// The routed products of b200_gemm_grouped (groups of gathered rows, bfloat16, W [N, K] per group) on tcgen05 / TMEM.
+//
+// What bounds it: the weights, read once (a group owns a few to a few hundred rows), so they lie on the M axis of the products, 128 rows
+// (gated units: 64 gate rows and the 64 up rows of the same features) per CTA, and a group's rows ride along as the N extent, up to 128 of
+// them, in an instruction just wide enough. Weights come by TMA; the rows, which lie anywhere, by cp.async into the same swizzled layout
+// (warps 2-5, 16 bytes at a time, a few stages ahead). Two CTAs share an SM. The sums leave TMEM through shared memory, so that a token's
+// features are stored side by side and the epilogue sees one element like the other kernels of this entry point.
+//   grid: feature tiles x groups x blocks of rows; what lies behind a group's rows leaves at once
+// Measured (before: the mma.sync tiles of gemm_grouped.cu): 400 rows, four of 16 experts each, 2048 -> gated 1024 -> 2048, with routing, dispatch
+// and combine: 246 -> 109 us.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "b200_serve.h"
+#include "common.cuh"
+#include "gemm_grouped.cuh"
+#include "launch_count.h"
+#include "tc_common.cuh"
+
+namespace b200 {
+
+constexpr int kGtM = 128, kGtK = 64, kGtThreads = 192;
+
+template <int BN>
+struct GtSmem {
+    static constexpr int kStageBytes = (kGtM + BN) * kGtK * 2;
+    static constexpr int kStages = BN <= 32 ? 5 : 3, kLag = kStages - 1;   // kLag: stages of rows under way before the first is announced
+    static constexpr int kTotal = kStages * kStageBytes + (2 * kStages + 1) * 8 + 16 + 1024;
+    static_assert(BN * kGtM * 4 <= kStages * kStageBytes, "the sums take the place of the stages");
+};
+
+template <int BN, typename TC, bool GLU>
+__global__ void __launch_bounds__(kGtThreads, 2) gemm_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const GG g) {
+    using S = GtSmem<BN>;
+    using bf = __nv_bfloat16;
+    constexpr int STAGES = S::kStages, LAG = S::kLag;
+    constexpr uint32_t A_BYTES = kGtM * kGtK * 2;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * S::kStageBytes);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_full = empty_bar + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float* om = reinterpret_cast<float*>(tiles);   // [rows][128]: the sums, once the stages have been used
+
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    pdl_wait();
+    const int z = blockIdx.y, row0 = g.group_off[z] + (int)blockIdx.z * BN, rows = min(BN, g.group_off[z + 1] - row0);
+    if (rows <= 0) return;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], 1 + 4);   // the weights, and the four warps that bring the rows
+            mbar_init(&empty_bar[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        *dead = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&map_w);
+    }
+    if (warp == 1) tmem_alloc(tmem_slot, BN);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    pdl_launch_dependents();
+    const int k_blocks = (g.K + kGtK - 1) / kGtK;
+
+    if (warp == 0) {
+        const int wrow = z * (GLU ? 2 * g.N : g.N) + (int)blockIdx.x * (GLU ? 64 : kGtM);
+        for (int kb = 0; kb < k_blocks; ++kb) {
+            const int s = kb % STAGES;
+            mbar_wait_or_leave(&empty_bar[s], ((uint32_t)(kb / STAGES) & 1u) ^ 1u, dead);
+            if (lane == 0) {
+                unsigned char* sa = tiles + (size_t)s * S::kStageBytes;
+                mbar_expect_tx(&full_bar[s], A_BYTES);
+                tma_load_2d(sa, &map_w, kb * kGtK, wrow, &full_bar[s]);
+                tma_load_2d(sa + A_BYTES / 2, &map_w, kb * kGtK, GLU ? wrow + g.N : wrow + 64, &full_bar[s]);
+            }
+            __syncwarp();
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc_f16(kGtM, 16) + ((uint32_t)((rows + 15) / 16 - 1) << 18) + ((1u << 7) | (1u << 10));   // N: rows rounded up to 16
+        const bool leader = elect_one();
+        const uint64_t a0 = make_kmajor_sw128_desc(smem_u32(tiles)), b0 = make_kmajor_sw128_desc(smem_u32(tiles + A_BYTES));
+        for (int kb = 0; kb < k_blocks; ++kb) {
+            const int s = kb % STAGES;
+            mbar_wait_or_leave(&full_bar[s], (uint32_t)(kb / STAGES) & 1u, dead);
+            tc_fence_after();
+            if (leader) {
+                const uint64_t off = (uint64_t)(s * (S::kStageBytes >> 4));
+#pragma unroll
+                for (int k = 0; k < kGtK / kUmmaK; ++k) umma_f16(tmem, a0 + off + (uint64_t)(2 * k), b0 + off + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                umma_commit(&empty_bar[s]);
+                if (kb == k_blocks - 1) umma_commit(acc_full);
+            }
+            __syncwarp();
+        }
+    } else {
+        // ---- rows: a thread brings 16-byte piece c of rows r, r + 16, ...
+        constexpr int NR = BN / 16;
+        const int tid = threadIdx.x - 64, c = tid % 8, r0 = tid / 8;
+        const bf* src[NR];
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            const int r = r0 + i * 16;
+            src[i] = nullptr;
+            if (r < rows) src[i] = reinterpret_cast<const bf*>(g.A) + (size_t)(g.a_rows ? g.a_rows[row0 + r] : row0 + r) * g.lda + c * 8;
+        }
+        const uint32_t dst0 = smem_u32(tiles + A_BYTES) + (uint32_t)(r0 * 128 + ((c ^ (r0 & 7)) << 4));   // (rows 16 apart share r & 7)
+        auto announce = [&](int kb) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_bar[kb % STAGES]);
+        };
+        for (int kb = 0; kb < k_blocks; ++kb) {
+            const int s = kb % STAGES;
+            mbar_wait_or_leave(&empty_bar[s], ((uint32_t)(kb / STAGES) & 1u) ^ 1u, dead);
+            const bool in = kb * kGtK + c * 8 < g.K;
+#pragma unroll
+            for (int i = 0; i < NR; ++i) {
+                const bool ok = in && src[i] != nullptr;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst0 + (uint32_t)(s * S::kStageBytes + i * 16 * 128)),
+                             "l"(ok ? src[i] + kb * kGtK : reinterpret_cast<const bf*>(g.A)), "r"(ok ? 16 : 0) : "memory");
+            }
+            __syncwarp();   // the lanes close their group of copies together
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (kb >= LAG) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
+                announce(kb - LAG);
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        for (int kb = max(0, k_blocks - LAG); kb < k_blocks; ++kb) announce(kb);
+        // ---- sums to shared memory
+        const int quarter = warp & 3;
+        mbar_wait_or_leave(acc_full, 0, dead);
+        const bool gone = *dead != 0;
+        tc_fence_after();
+        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+        for (int c0 = 0; c0 < rows; c0 += 32) {
+            uint32_t v[32];
+            tmem_ld_32x32(taddr + (uint32_t)c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (c0 + j < rows) om[(c0 + j) * kGtM + quarter * 32 + lane] = gone ? __int_as_float(0x7fffffff) : __uint_as_float(v[j]);
+        }
+        tc_fence_before();
+    }
+    __syncthreads();
+    constexpr int F = GLU ? 64 : kGtM;
+    const int n0 = blockIdx.x * F;
+    TC* C = reinterpret_cast<TC*>(g.C);
+    const bool wide = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15u) == 0;
+    for (int i = threadIdx.x; i < rows * (F / 4); i += kGtThreads) {
+        const int r = i / (F / 4), f0 = i % (F / 4) * 4, n = n0 + f0;
+        const long long row = row0 + r;
+        const float4 a = *reinterpret_cast<const float4*>(om + r * kGtM + f0);
+        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (GLU) u = *reinterpret_cast<const float4*>(om + r * kGtM + 64 + f0);
+        float v[4] = {a.x, a.y, a.z, a.w};
+        const float v2[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (n + e < g.N) v[e] = gg_value(g, row, n + e, v[e], v2[e], 0);
+        if (wide && n + 4 <= g.N) {
+            if constexpr (sizeof(TC) == 4) *reinterpret_cast<float4*>(C + row * g.ldc + n) = make_float4(v[0], v[1], v[2], v[3]);
+            else {
+                const __nv_bfloat162 x = __floats2bfloat162_rn(v[0], v[1]), y = __floats2bfloat162_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(C + row * g.ldc + n) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (n + e < g.N) C[row * g.ldc + n + e] = DT<TC>::from_f(v[e]);
+        }
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, BN);
+    }
+}
+
+template <int BN, typename TC, bool GLU>
+static int launch_gt(const GG& g, int groups, cudaStream_t s) {
+    CUtensorMap map;
+    if (!make_tma_map_2d(&map, g.W, (long long)groups * (GLU ? 2 * g.N : g.N), g.K, 64)) return -1;
+    auto kern = gemm_grouped_tc_kernel<BN, TC, GLU>;
+    static unsigned long long done = 0;
+    const cudaError_t e = ensure_max_dynamic_smem((const void*)kern, GtSmem<BN>::kTotal, done);
+    if (e != cudaSuccess) return (int)e;
+    const int F = GLU ? 64 : kGtM;
+    const dim3 grid((g.N + F - 1) / F, groups, (g.M + BN - 1) / BN);
+    if (grid.z > 65535) return -1;
+    return (int)launch_k(kern, grid, dim3(kGtThreads), (size_t)GtSmem<BN>::kTotal, s, true, map, g);
+}
+
+template <typename TC>
+int gg_launch_tc(const GG& g, int groups, cudaStream_t s) {
+    const bool glu = gg_is_glu(g.epi);
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    // weights of all groups as one matrix without gaps, rows that 16-byte pieces can fetch
+    if (!g.group_off || (g.K & 7) || (g.lda & 7) || g.ldw != g.K || g.sW != (long long)(glu ? 2 : 1) * g.N * g.K || !al16(g.A) || !al16(g.W) || (glu && g.N % 64) || groups > 65535) return -1;
+    if (g.M <= 32) return glu ? launch_gt<32, TC, true>(g, groups, s) : launch_gt<32, TC, false>(g, groups, s);
+    return glu ? launch_gt<128, TC, true>(g, groups, s) : launch_gt<128, TC, false>(g, groups, s);
+}
+template int gg_launch_tc<float>(const GG&, int, cudaStream_t);
+template int gg_launch_tc<__nv_bfloat16>(const GG&, int, cudaStream_t);
+
+}  // namespace b200
