@@ -25,6 +25,7 @@
 
 #include "b200_serve.h"
 #include "common.cuh"
+#include "latent_attention.cuh"
 #include "launch_count.h"
 #include "rotary.cuh"
 
@@ -792,6 +793,12 @@ extern "C" int b200_latent_attention_ex(const b200_latent_attention_args* ap, vo
     // single tokens: a cluster per token whatever the batch (the tile kernel spends half of its 32 rows on nothing there)
     if (dtype == B200_BF16 && tile_attention_enabled() && longest_entry == 1) {
         const int rc = latent_decode(*ap, out_cols, longest_context, s);
+        if (rc >= 0) return rc;
+    }
+    // prompt portions over rows of whole 64-dimension chunks with 256 or 512 columns of output (2048 tokens, 16 heads, rows of 576: 160 us there, 856 us
+    // on the tiles below)
+    if (dtype == B200_BF16 && tile_attention_enabled() && longest_entry != 1) {
+        const int rc = latent_attention_tc(*ap, out_cols, s);
         if (rc >= 0) return rc;
     }
     if (dtype == B200_BF16 && tile_attention_enabled()) {
