@@ -79,10 +79,12 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         const int t = t0 - 1 + i;
         slots[i] = t >= 0 && t < a.n_tokens ? a.slot[t] : -1;
     }
-    pdl_launch_dependents();   // the kernel for single tokens may move in (it waits for this one before it ends)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // the kernel for single tokens may move in (it waits for this one before it ends); TMEM has been allocated: a product kernel that moved in ahead of
+    // that would wait for this one while holding it
+    pdl_launch_dependents();
     if (warp < 4) {
         const int i = threadIdx.x;   // row of the window; slots[i + 1] is its own
         const bool in = i < rows, starts = in && (i == 0 || slots[i] != slots[i + 1]);
@@ -351,8 +353,8 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                         unpack2(FORM == kTcPlain ? fma2(pack2(sv[e], sv[e + 1]), sl2, nm2) : add2(pack2(sv[e], sv[e + 1]), nm2), a0, a1);
                         a0 = ex2_approx(a0);
                         a1 = ex2_approx(a1);
-                        rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2f(a0, a1));
                         pk[e / 2] = pa_pack(a0, a1);
+                        rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2(pk[e / 2] << 16, pk[e / 2] & 0xffff0000u));   // the weights as they are used: they add up to 1
                     }
                     float r0, r1;
                     unpack2(add2(rs2[0], rs2[1]), r0, r1);
