@@ -12,6 +12,8 @@ namespace b200 {
 template <typename T>
 __global__ void diff_combine_kernel(const float* __restrict__ a, float lambda, float eps, float out_scale, T* __restrict__ out,
                                     int units, int vdim) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int u = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (u >= units) return;
     const float* a1 = a + (size_t)u * 2 * vdim;
@@ -30,6 +32,8 @@ __global__ void diff_combine_kernel(const float* __restrict__ a, float lambda, f
 template <typename T>
 __global__ void sigmoid_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long ld_gate, T* __restrict__ out,
                                     int n, size_t total) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / n, c = i % n;
@@ -43,6 +47,8 @@ template <typename T>
 __global__ void unrotate_gate_kernel(const float* __restrict__ o, const float* __restrict__ cs, const float* __restrict__ sn, int layout,
                                      const float* __restrict__ gate, long long ld_gate, T* __restrict__ out, int heads, int vdim,
                                      size_t total) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int half = vdim / 2, per = half + (vdim & 1);
@@ -71,8 +77,8 @@ extern "C" int b200_unrotate_gate(const float* o, const float* cos, const float*
     const size_t total = (size_t)n_tokens * heads * (vdim / 2 + (vdim & 1));
     const unsigned grid = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == B200_BF16) unrotate_gate_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(o, cos, sin, rot_layout, gate, ld_gate, (__nv_bfloat16*)out, heads, vdim, total);
-    else if (out_dtype == B200_F32) unrotate_gate_kernel<float><<<grid, 256, 0, s>>>(o, cos, sin, rot_layout, gate, ld_gate, (float*)out, heads, vdim, total);
+    if (out_dtype == B200_BF16) launch_chained(unrotate_gate_kernel<__nv_bfloat16>, grid, 256, 0, s, o, cos, sin, rot_layout, gate, ld_gate, (__nv_bfloat16*)out, heads, vdim, total);
+    else if (out_dtype == B200_F32) launch_chained(unrotate_gate_kernel<float>, grid, 256, 0, s, o, cos, sin, rot_layout, gate, ld_gate, (float*)out, heads, vdim, total);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();
@@ -85,8 +91,8 @@ extern "C" int b200_diff_combine(const float* a, float lambda, float eps, float 
     const int units = n_tokens * heads;
     const dim3 grid((units + 3) / 4);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == B200_BF16) diff_combine_kernel<__nv_bfloat16><<<grid, 128, 0, s>>>(a, lambda, eps, out_scale, (__nv_bfloat16*)out, units, vdim);
-    else if (out_dtype == B200_F32) diff_combine_kernel<float><<<grid, 128, 0, s>>>(a, lambda, eps, out_scale, (float*)out, units, vdim);
+    if (out_dtype == B200_BF16) launch_chained(diff_combine_kernel<__nv_bfloat16>, grid, 128, 0, s, a, lambda, eps, out_scale, (__nv_bfloat16*)out, units, vdim);
+    else if (out_dtype == B200_F32) launch_chained(diff_combine_kernel<float>, grid, 128, 0, s, a, lambda, eps, out_scale, (float*)out, units, vdim);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();
@@ -99,8 +105,8 @@ extern "C" int b200_sigmoid_gate(const float* o, const float* gate, long long ld
     const size_t total = (size_t)n_tokens * n;
     const unsigned grid = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == B200_BF16) sigmoid_gate_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(o, gate, ld_gate, (__nv_bfloat16*)out, n, total);
-    else if (out_dtype == B200_F32) sigmoid_gate_kernel<float><<<grid, 256, 0, s>>>(o, gate, ld_gate, (float*)out, n, total);
+    if (out_dtype == B200_BF16) launch_chained(sigmoid_gate_kernel<__nv_bfloat16>, grid, 256, 0, s, o, gate, ld_gate, (__nv_bfloat16*)out, n, total);
+    else if (out_dtype == B200_F32) launch_chained(sigmoid_gate_kernel<float>, grid, 256, 0, s, o, gate, ld_gate, (float*)out, n, total);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();

@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* _
 //   softmax  warp w: heads 2w, 2w + 1, a key per lane; the weights leave as bfloat16 (as in the tile kernel)
 //   values   warp w: an eighth of the output columns, the rows read transposed by ldmatrix
 // The sink joins in the merge. Measured, 8 sequences of up to 1024 rows of 576, 16 heads, 512 columns out: the tile kernel with its
-// combine launch 53.3 us, this 18.4 us (clusters of at most 2 / 4 / 8 CTAs: 51 / 31 / 20.5 us).
+// combine launch 53.3 us, this 16.2 us (clusters of at most 2 / 4 / 8 CTAs: 51 / 31 / 20.5 us).
 constexpr int kLdMaxCluster = 16;
 
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
@@ -465,6 +465,8 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
                                                                int window, int out_cols) {
     using bf = __nv_bfloat16;
     extern __shared__ __align__(16) unsigned char smraw[];
+    pdl_wait();
+    pdl_launch_dependents();
     const int rpad = (rank + 15) & ~15, RS = rpad + 8, splits = gridDim.x;
     bf* Ks = reinterpret_cast<bf*>(smraw);                     // [2][32][RS]
     bf* Qs = Ks + 2 * kHalfKeys * RS;                          // [16][RS]
@@ -669,12 +671,14 @@ static int launch_latent_decode(const b200_latent_attention_args& a, int out_col
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)splits;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
     e = cudaLaunchKernelEx(&cfg, latent_decode_kernel<NT>, a.qa, a.out, (const __nv_bfloat16*)a.pool, a.pages, a.max_pages, a.page_rows, a.slot, a.pos,
                            a.sink, a.scale, a.heads, a.rank, a.window, out_cols);
     if (e != cudaSuccess) return (int)e;

@@ -10,6 +10,8 @@ namespace b200 {
 template <typename T>
 __global__ void embed_positions_kernel(const int* __restrict__ ids, const int* __restrict__ pos, const T* __restrict__ table,
                                        const T* __restrict__ pos_table, float* __restrict__ out, int width) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x;
     const T* e = table + (size_t)ids[t] * width;
     if (!pos_table) {
@@ -39,6 +41,8 @@ __global__ void __launch_bounds__(256) layernorm_pair_kernel(const float* __rest
                                                              const float* __restrict__ b1, T* __restrict__ out1,
                                                              const float* __restrict__ w2, const float* __restrict__ b2,
                                                              T* __restrict__ out2) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ float row[];
     __shared__ float red[8];
     const int i = blockIdx.x;
@@ -69,6 +73,8 @@ __global__ void __launch_bounds__(256) layernorm_residual_kernel(float* __restri
                                                                  float eps, float mult, const float* __restrict__ w,
                                                                  const float* __restrict__ b, const float* __restrict__ w2,
                                                                  const float* __restrict__ b2, T* __restrict__ out2) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ float row[];
     __shared__ float red[8];
     const size_t base = (size_t)blockIdx.x * width;
@@ -111,6 +117,8 @@ __global__ void __launch_bounds__(256) layernorm_residual_reg_kernel(float* __re
                                                                      float eps, float mult, const float* __restrict__ w,
                                                                      const float* __restrict__ b, const float* __restrict__ w2,
                                                                      const float* __restrict__ b2, T* __restrict__ out2) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float red[8];
     const size_t base = (size_t)blockIdx.x * width;
     float xv[kLnPerThread], yv[kLnPerThread], wv[kLnPerThread], bv[kLnPerThread], w2v[kLnPerThread], b2v[kLnPerThread];
@@ -164,6 +172,8 @@ __global__ void __launch_bounds__(256) layernorm_residual_reg_kernel(float* __re
 
 template <typename T>
 __global__ void concat_cast_kernel(const float* __restrict__ a, const float* __restrict__ b, T* __restrict__ out, int width) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t t = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         out[t * 2 * width + c] = DT<T>::from_f(a[t * width + c]);
@@ -175,6 +185,8 @@ __global__ void concat_cast_kernel(const float* __restrict__ a, const float* __r
 // computed without the fused epilogue (small batches stream the stacked weight once through the split-K GEMM)
 template <typename T>
 __global__ void glu_act_kernel(const float* __restrict__ gu, T* __restrict__ out, int n, size_t total, int gelu) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / n, j = i - t * n;
@@ -184,6 +196,8 @@ __global__ void glu_act_kernel(const float* __restrict__ gu, T* __restrict__ out
 
 template <typename T>
 __global__ void glu_act_clamped_kernel(const float* __restrict__ gu, T* __restrict__ out, int n, size_t total, float limit) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const size_t t = i / n, j = i - t * n;
@@ -191,6 +205,8 @@ __global__ void glu_act_clamped_kernel(const float* __restrict__ gu, T* __restri
 }
 
 __global__ void scale_kernel(float* __restrict__ v, size_t n, float f) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] *= f;
 }
@@ -200,6 +216,8 @@ template <typename T>
 __global__ void embed_pair_hash_kernel(const int* __restrict__ ids, const int* __restrict__ prev, const T* __restrict__ table, float scale,
                                        const T* __restrict__ pair_table, int buckets, int mul_prev, int mul_cur, float* __restrict__ out,
                                        T* __restrict__ out_cast, int width) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x;
     const T* e = table + (size_t)ids[t] * width;
     if (!pair_table) {
@@ -224,6 +242,8 @@ __global__ void embed_pair_hash_kernel(const int* __restrict__ ids, const int* _
 }
 
 __global__ void softcap_kernel(float* __restrict__ v, size_t n, float cap) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) v[i] = cap * tanhf(v[i] / cap);
 }
@@ -242,20 +262,20 @@ extern "C" int b200_layernorm_residual(float* x, const float* y, int n_rows, int
     cudaStream_t s = (cudaStream_t)stream;
     if (width <= 256 * kLnPerThread && (out_dtype == B200_BF16 || out_dtype == B200_F32)) {
         if (out_dtype == B200_BF16)
-            layernorm_residual_reg_kernel<__nv_bfloat16><<<n_rows, 256, 0, s>>>(x, y, width, eps, mult, w, b, w2, b2, (__nv_bfloat16*)out2);
+            launch_chained(layernorm_residual_reg_kernel<__nv_bfloat16>, n_rows, 256, 0, s, x, y, width, eps, mult, w, b, w2, b2, (__nv_bfloat16*)out2);
         else
-            layernorm_residual_reg_kernel<float><<<n_rows, 256, 0, s>>>(x, y, width, eps, mult, w, b, w2, b2, (float*)out2);
+            launch_chained(layernorm_residual_reg_kernel<float>, n_rows, 256, 0, s, x, y, width, eps, mult, w, b, w2, b2, (float*)out2);
         count_launch();
         return (int)cudaGetLastError();
     }
     if (out_dtype == B200_BF16) {
         static unsigned long long done = 0;
         if (smem > 48 * 1024) ensure_max_dynamic_smem((const void*)layernorm_residual_kernel<__nv_bfloat16>, 200 * 1024, done);
-        layernorm_residual_kernel<__nv_bfloat16><<<n_rows, 256, smem, s>>>(x, y, width, eps, mult, w, b, w2, b2, (__nv_bfloat16*)out2);
+        launch_chained(layernorm_residual_kernel<__nv_bfloat16>, n_rows, 256, smem, s, x, y, width, eps, mult, w, b, w2, b2, (__nv_bfloat16*)out2);
     } else if (out_dtype == B200_F32) {
         static unsigned long long done = 0;
         if (smem > 48 * 1024) ensure_max_dynamic_smem((const void*)layernorm_residual_kernel<float>, 200 * 1024, done);
-        layernorm_residual_kernel<float><<<n_rows, 256, smem, s>>>(x, y, width, eps, mult, w, b, w2, b2, (float*)out2);
+        launch_chained(layernorm_residual_kernel<float>, n_rows, 256, smem, s, x, y, width, eps, mult, w, b, w2, b2, (float*)out2);
     } else
         return B200_EINVAL;
     count_launch();
@@ -266,8 +286,8 @@ extern "C" int b200_concat_cast(const float* a, const float* b, void* out, int n
     if (!a || !b || !out || n_rows < 0 || width < 1) return B200_EINVAL;
     if (n_rows == 0) return B200_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == B200_BF16) concat_cast_kernel<__nv_bfloat16><<<n_rows, 256, 0, s>>>(a, b, (__nv_bfloat16*)out, width);
-    else if (out_dtype == B200_F32) concat_cast_kernel<float><<<n_rows, 256, 0, s>>>(a, b, (float*)out, width);
+    if (out_dtype == B200_BF16) launch_chained(concat_cast_kernel<__nv_bfloat16>, n_rows, 256, 0, s, a, b, (__nv_bfloat16*)out, width);
+    else if (out_dtype == B200_F32) launch_chained(concat_cast_kernel<float>, n_rows, 256, 0, s, a, b, (float*)out, width);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();
@@ -279,8 +299,8 @@ extern "C" int b200_glu_act(const float* gu, void* out, int n_rows, int n, int e
     const size_t total = (size_t)n_rows * n;
     const unsigned grid = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == B200_BF16) glu_act_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(gu, (__nv_bfloat16*)out, n, total, epi == B200_GG_GLU_GELU);
-    else if (out_dtype == B200_F32) glu_act_kernel<float><<<grid, 256, 0, s>>>(gu, (float*)out, n, total, epi == B200_GG_GLU_GELU);
+    if (out_dtype == B200_BF16) launch_chained(glu_act_kernel<__nv_bfloat16>, grid, 256, 0, s, gu, (__nv_bfloat16*)out, n, total, epi == B200_GG_GLU_GELU);
+    else if (out_dtype == B200_F32) launch_chained(glu_act_kernel<float>, grid, 256, 0, s, gu, (float*)out, n, total, epi == B200_GG_GLU_GELU);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();
@@ -292,8 +312,8 @@ extern "C" int b200_glu_act_clamped(const float* gu, void* out, int n_rows, int 
     const size_t total = (size_t)n_rows * n;
     const unsigned grid = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dtype == B200_BF16) glu_act_clamped_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(gu, (__nv_bfloat16*)out, n, total, limit);
-    else if (out_dtype == B200_F32) glu_act_clamped_kernel<float><<<grid, 256, 0, s>>>(gu, (float*)out, n, total, limit);
+    if (out_dtype == B200_BF16) launch_chained(glu_act_clamped_kernel<__nv_bfloat16>, grid, 256, 0, s, gu, (__nv_bfloat16*)out, n, total, limit);
+    else if (out_dtype == B200_F32) launch_chained(glu_act_clamped_kernel<float>, grid, 256, 0, s, gu, (float*)out, n, total, limit);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();
@@ -302,7 +322,7 @@ extern "C" int b200_glu_act_clamped(const float* gu, void* out, int n_rows, int 
 extern "C" int b200_scale(float* v, size_t n, float f, void* stream) {
     if (!v) return B200_EINVAL;
     if (n == 0) return B200_OK;
-    scale_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(v, n, f);
+    launch_chained(scale_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, v, n, f);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -313,10 +333,10 @@ extern "C" int b200_embed_pair_hash(const int* ids, const int* prev, const void*
     if (n_tokens == 0) return B200_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == B200_BF16)
-        embed_pair_hash_kernel<__nv_bfloat16><<<n_tokens, 128, 0, s>>>(ids, prev, (const __nv_bfloat16*)table, scale, (const __nv_bfloat16*)pair_table,
+        launch_chained(embed_pair_hash_kernel<__nv_bfloat16>, n_tokens, 128, 0, s, ids, prev, (const __nv_bfloat16*)table, scale, (const __nv_bfloat16*)pair_table,
                                                                       buckets, mul_prev, mul_cur, out, (__nv_bfloat16*)out_cast, width);
     else if (dtype == B200_F32)
-        embed_pair_hash_kernel<float><<<n_tokens, 128, 0, s>>>(ids, prev, (const float*)table, scale, (const float*)pair_table, buckets, mul_prev,
+        launch_chained(embed_pair_hash_kernel<float>, n_tokens, 128, 0, s, ids, prev, (const float*)table, scale, (const float*)pair_table, buckets, mul_prev,
                                                               mul_cur, out, (float*)out_cast, width);
     else
         return B200_EINVAL;
@@ -327,7 +347,7 @@ extern "C" int b200_embed_pair_hash(const int* ids, const int* prev, const void*
 extern "C" int b200_softcap(float* v, size_t n, float cap, void* stream) {
     if (!v || !(cap > 0.f)) return B200_EINVAL;
     if (n == 0) return B200_OK;
-    softcap_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(v, n, cap);
+    launch_chained(softcap_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, v, n, cap);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -338,10 +358,10 @@ extern "C" int b200_embed_positions(const int* ids, const int* pos, const void* 
     if (n_tokens == 0) return B200_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == B200_BF16)
-        embed_positions_kernel<__nv_bfloat16><<<n_tokens, 128, 0, s>>>(ids, pos, (const __nv_bfloat16*)table,
+        launch_chained(embed_positions_kernel<__nv_bfloat16>, n_tokens, 128, 0, s, ids, pos, (const __nv_bfloat16*)table,
                                                                       (const __nv_bfloat16*)pos_table, out, width);
     else if (dtype == B200_F32)
-        embed_positions_kernel<float><<<n_tokens, 128, 0, s>>>(ids, pos, (const float*)table, (const float*)pos_table, out, width);
+        launch_chained(embed_positions_kernel<float>, n_tokens, 128, 0, s, ids, pos, (const float*)table, (const float*)pos_table, out, width);
     else
         return B200_EINVAL;
     count_launch();
@@ -360,12 +380,12 @@ extern "C" int b200_layernorm_pair(const float* x, const int* rows, int n_rows, 
     if (out_dtype == B200_BF16) {
         static unsigned long long done = 0;
         if (smem > 48 * 1024) ensure_max_dynamic_smem((const void*)layernorm_pair_kernel<__nv_bfloat16>, 200 * 1024, done);
-        layernorm_pair_kernel<__nv_bfloat16><<<n_rows, 256, smem, s>>>(x, rows, width, eps, w1, b1, (__nv_bfloat16*)out1, w2, b2,
+        launch_chained(layernorm_pair_kernel<__nv_bfloat16>, n_rows, 256, smem, s, x, rows, width, eps, w1, b1, (__nv_bfloat16*)out1, w2, b2,
                                                                       (__nv_bfloat16*)out2);
     } else if (out_dtype == B200_F32) {
         static unsigned long long done = 0;
         if (smem > 48 * 1024) ensure_max_dynamic_smem((const void*)layernorm_pair_kernel<float>, 200 * 1024, done);
-        layernorm_pair_kernel<float><<<n_rows, 256, smem, s>>>(x, rows, width, eps, w1, b1, (float*)out1, w2, b2, (float*)out2);
+        launch_chained(layernorm_pair_kernel<float>, n_rows, 256, smem, s, x, rows, width, eps, w1, b1, (float*)out1, w2, b2, (float*)out2);
     } else
         return B200_EINVAL;
     count_launch();

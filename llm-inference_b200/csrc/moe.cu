@@ -84,6 +84,8 @@ __global__ void __launch_bounds__(MAX_THREADS) moe_route_kernel(const T* __restr
                                                         int on_logits, int width, int n_out, int top,
                                                         float scale, int groups, int keep, int* __restrict__ chosen,
                                                         float* __restrict__ weight, int sigmoids = 0, int n_gates = 0, float* __restrict__ gates = nullptr) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ float z[];   // z[n_out] | pick[n_out] | x[width]
     const int n_all = n_out + n_gates;   // the rows of w_router behind the experts' are gates of their own
     float* pick = z + n_all;
@@ -176,6 +178,8 @@ __global__ void __launch_bounds__(1024) moe_dispatch_kernel(const int* __restric
                                                             int top, int* __restrict__ group_off, int* __restrict__ src_row,
                                                             int* __restrict__ dest, const float* __restrict__ weight,
                                                             float* __restrict__ row_weight) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ int cnt[];   // count[n_experts] | cursor[n_experts]
     int* cursor = cnt + n_experts;
     for (int e = threadIdx.x; e < n_experts; e += blockDim.x) cnt[e] = 0;
@@ -212,6 +216,8 @@ __global__ void __launch_bounds__(256) residual_combine_kernel(float* __restrict
                                                                const float* __restrict__ shared, const float* __restrict__ eo,
                                                                const int* __restrict__ dest, const float* __restrict__ weight,
                                                                const T* __restrict__ h, int width, int top) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         const size_t i = (size_t)t * width + c;
@@ -234,6 +240,8 @@ __global__ void __launch_bounds__(256) residual_combine_kernel(float* __restrict
 template <typename T>
 __global__ void __launch_bounds__(256) gather_rows_scaled_kernel(const T* __restrict__ src, const int* __restrict__ rows, const float* __restrict__ scale,
                                                                 T* __restrict__ dst, int width, int vec) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int P = DT<T>::kPer16B;
     const T* s = src + (size_t)rows[blockIdx.x] * width;
     T* d = dst + (size_t)blockIdx.x * width;
@@ -254,6 +262,8 @@ __global__ void __launch_bounds__(256) gather_rows_scaled_kernel(const T* __rest
 // dst[i, :] = src[rows[i], :]: the rows of every expert's group side by side, so that a dense GEMM can read a group
 __global__ void __launch_bounds__(256) gather_rows_kernel(const unsigned char* __restrict__ src, const int* __restrict__ rows,
                                                          unsigned char* __restrict__ dst, size_t row_bytes, int vec) {
+    pdl_wait();
+    pdl_launch_dependents();
     const unsigned char* s = src + (size_t)rows[blockIdx.x] * row_bytes;
     unsigned char* d = dst + (size_t)blockIdx.x * row_bytes;
     if (vec) {
@@ -272,7 +282,7 @@ extern "C" int b200_gather_rows(const void* src, const int* rows, void* dst, int
     if (n_rows == 0) return B200_OK;
     const size_t row_bytes = (size_t)width * (dtype == B200_BF16 ? 2 : 4);
     const int vec = row_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
-    gather_rows_kernel<<<n_rows, 256, 0, (cudaStream_t)stream>>>((const unsigned char*)src, rows, (unsigned char*)dst, row_bytes, vec);
+    launch_chained(gather_rows_kernel, n_rows, 256, 0, (cudaStream_t)stream, (const unsigned char*)src, rows, (unsigned char*)dst, row_bytes, vec);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -282,8 +292,8 @@ extern "C" int b200_gather_rows_scaled(const void* src, const int* rows, const f
     if (n_rows == 0) return B200_OK;
     const int vec = ((size_t)width * (dtype == B200_BF16 ? 2 : 4)) % 16 == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dtype == B200_BF16) gather_rows_scaled_kernel<__nv_bfloat16><<<n_rows, 256, 0, s>>>((const __nv_bfloat16*)src, rows, scale, (__nv_bfloat16*)dst, width, vec);
-    else gather_rows_scaled_kernel<float><<<n_rows, 256, 0, s>>>((const float*)src, rows, scale, (float*)dst, width, vec);
+    if (dtype == B200_BF16) launch_chained(gather_rows_scaled_kernel<__nv_bfloat16>, n_rows, 256, 0, s, (const __nv_bfloat16*)src, rows, scale, (__nv_bfloat16*)dst, width, vec);
+    else launch_chained(gather_rows_scaled_kernel<float>, n_rows, 256, 0, s, (const float*)src, rows, scale, (float*)dst, width, vec);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -300,10 +310,10 @@ extern "C" int b200_moe_route_sigmoid(const void* h, int h_dtype, const float* w
     // a warp per output where 32 warps suffice; else rounds of equal length
     const int n_all = n_out + n_gates, rounds = (n_all + 31) / 32, threads = 32 * std::max(4, (n_all + rounds - 1) / rounds);
     if (h_dtype == B200_BF16)
-        moe_route_kernel<__nv_bfloat16, 1024><<<n_tokens, threads, smem, s>>>((const __nv_bfloat16*)h, w_router, nullptr, nullptr, 0, width, n_out, top,
+        launch_chained(moe_route_kernel<__nv_bfloat16, 1024>, n_tokens, threads, smem, s, (const __nv_bfloat16*)h, w_router, nullptr, nullptr, 0, width, n_out, top,
                                                                              1.f, 0, 0, chosen, weight, 1, n_gates, gates);
     else if (h_dtype == B200_F32)
-        moe_route_kernel<float, 1024><<<n_tokens, threads, smem, s>>>((const float*)h, w_router, nullptr, nullptr, 0, width, n_out, top, 1.f, 0, 0,
+        launch_chained(moe_route_kernel<float, 1024>, n_tokens, threads, smem, s, (const float*)h, w_router, nullptr, nullptr, 0, width, n_out, top, 1.f, 0, 0,
                                                                      chosen, weight, 1, n_gates, gates);
     else
         return B200_EINVAL;
@@ -321,11 +331,11 @@ extern "C" int b200_moe_route(const void* h, int h_dtype, const float* w_router,
     const size_t smem = ((size_t)2 * n_out + width) * sizeof(float);
     if (smem > 48 * 1024) return B200_EUNSUPPORTED;
     if (h_dtype == B200_BF16)
-        moe_route_kernel<__nv_bfloat16><<<n_tokens, 512, smem, s>>>((const __nv_bfloat16*)h, w_router, correction, nullptr, 0, width, n_out, top,
-                                                                   scale, 0, 0, chosen, weight);
+        launch_chained(moe_route_kernel<__nv_bfloat16>, n_tokens, 512, smem, s, (const __nv_bfloat16*)h, w_router, correction, nullptr, 0, width, n_out, top,
+                                                                   scale, 0, 0, chosen, weight, 0, 0, nullptr);
     else if (h_dtype == B200_F32)
-        moe_route_kernel<float><<<n_tokens, 512, smem, s>>>((const float*)h, w_router, correction, nullptr, 0, width, n_out, top, scale, 0, 0, chosen,
-                                                           weight);
+        launch_chained(moe_route_kernel<float>, n_tokens, 512, smem, s, (const float*)h, w_router, correction, nullptr, 0, width, n_out, top, scale, 0, 0, chosen,
+                                                           weight, 0, 0, nullptr);
     else
         return B200_EINVAL;
     count_launch();
@@ -341,10 +351,10 @@ extern "C" int b200_moe_route_logits(const void* h, int h_dtype, const float* w_
     const size_t smem = ((size_t)2 * n_out + width) * sizeof(float);
     if (smem > 48 * 1024) return B200_EUNSUPPORTED;
     if (h_dtype == B200_BF16)
-        moe_route_kernel<__nv_bfloat16><<<n_tokens, 512, smem, s>>>((const __nv_bfloat16*)h, w_router, nullptr, bias, 1, width, n_out, top, 1.f,
-                                                                   0, 0, chosen, weight);
+        launch_chained(moe_route_kernel<__nv_bfloat16>, n_tokens, 512, smem, s, (const __nv_bfloat16*)h, w_router, nullptr, bias, 1, width, n_out, top, 1.f,
+                                                                   0, 0, chosen, weight, 0, 0, nullptr);
     else if (h_dtype == B200_F32)
-        moe_route_kernel<float><<<n_tokens, 512, smem, s>>>((const float*)h, w_router, nullptr, bias, 1, width, n_out, top, 1.f, 0, 0, chosen, weight);
+        launch_chained(moe_route_kernel<float>, n_tokens, 512, smem, s, (const float*)h, w_router, nullptr, bias, 1, width, n_out, top, 1.f, 0, 0, chosen, weight, 0, 0, nullptr);
     else
         return B200_EINVAL;
     count_launch();
@@ -362,11 +372,11 @@ extern "C" int b200_moe_route_groups(const void* h, int h_dtype, const float* w_
     const size_t smem = ((size_t)2 * n_out + width) * sizeof(float);
     if (smem > 48 * 1024) return B200_EUNSUPPORTED;
     if (h_dtype == B200_BF16)
-        moe_route_kernel<__nv_bfloat16><<<n_tokens, 512, smem, s>>>((const __nv_bfloat16*)h, w_router, nullptr, nullptr, 0, width, n_out, top, 1.f,
-                                                                   groups, keep, chosen, weight);
+        launch_chained(moe_route_kernel<__nv_bfloat16>, n_tokens, 512, smem, s, (const __nv_bfloat16*)h, w_router, nullptr, nullptr, 0, width, n_out, top, 1.f,
+                                                                   groups, keep, chosen, weight, 0, 0, nullptr);
     else if (h_dtype == B200_F32)
-        moe_route_kernel<float><<<n_tokens, 512, smem, s>>>((const float*)h, w_router, nullptr, nullptr, 0, width, n_out, top, 1.f, groups, keep,
-                                                           chosen, weight);
+        launch_chained(moe_route_kernel<float>, n_tokens, 512, smem, s, (const float*)h, w_router, nullptr, nullptr, 0, width, n_out, top, 1.f, groups, keep,
+                                                           chosen, weight, 0, 0, nullptr);
     else
         return B200_EINVAL;
     count_launch();
@@ -383,8 +393,7 @@ extern "C" int b200_moe_dispatch_weighted(const int* chosen, const float* weight
     if (row_weight && !weight) return B200_EINVAL;
     if (!chosen || !group_off || !src_row || !dest || n_tokens < 0 || top < 1 || n_experts < 0) return B200_EINVAL;
     if (n_experts > 4096) return B200_EUNSUPPORTED;
-    moe_dispatch_kernel<<<1, 1024, (size_t)2 * (n_experts + 1) * sizeof(int), (cudaStream_t)stream>>>(
-        chosen, n_tokens * top, n_experts, top, group_off, src_row, dest, weight, row_weight);
+    launch_chained(moe_dispatch_kernel, 1, 1024, (size_t)2 * (n_experts + 1) * sizeof(int), (cudaStream_t)stream, chosen, n_tokens * top, n_experts, top, group_off, src_row, dest, weight, row_weight);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -397,10 +406,10 @@ extern "C" int b200_residual_combine(float* x, const float* mix, const float* sh
     if (n_tokens == 0) return B200_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (h_dtype == B200_BF16)
-        residual_combine_kernel<__nv_bfloat16><<<n_tokens, 256, 0, s>>>(x, mix, shared, expert_out, dest, weight,
+        launch_chained(residual_combine_kernel<__nv_bfloat16>, n_tokens, 256, 0, s, x, mix, shared, expert_out, dest, weight,
                                                                        (const __nv_bfloat16*)h, width, top);
     else if (h_dtype == B200_F32)
-        residual_combine_kernel<float><<<n_tokens, 256, 0, s>>>(x, mix, shared, expert_out, dest, weight, (const float*)h, width, top);
+        launch_chained(residual_combine_kernel<float>, n_tokens, 256, 0, s, x, mix, shared, expert_out, dest, weight, (const float*)h, width, top);
     else
         return B200_EINVAL;
     count_launch();

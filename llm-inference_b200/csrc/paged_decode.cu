@@ -11,8 +11,8 @@
 //                 movmatrix turns the weights' fragments.
 // Warps merge through shared memory, CTAs through distributed shared memory (rank order, so the sum does not depend on timing). The merge
 // adds the sink.
-// Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128: 20.5 -> 8.2 us;
-// 32 sequences of up to 2048 tokens, 16 / 8 heads x 128 (190 MB), bias and sink: 384 -> 61 us (69 us with a step's keys and values in
+// Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128: 20.5 -> 7.1 us;
+// 32 sequences of up to 2048 tokens, 16 / 8 heads x 128 (190 MB), bias and sink: 384 -> 59 us (69 us with a step's keys and values in
 // registers, requested one step ahead); 128 such sequences without bias run at 5.0 TB/s.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -51,6 +51,10 @@ __global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA
     constexpr int KS = D / 16;        // k steps of the scores
     constexpr int MT = VD / 16;       // m tiles of the output
     extern __shared__ __align__(16) float pd_sm[];
+    if (!MIXED) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     const int R = a.heads / a.kv_heads, splits = gridDim.x;
     float* om = pd_sm;                                 // once the rings have been used: [warps][R][VD], then this CTA's share in the first [R][VD]
     __shared__ float ms[kPdWarps * kPdHeads], ls[kPdWarps * kPdHeads];   // [warps][R], then [R]
@@ -321,7 +325,7 @@ static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (MIXED && pdl_enabled()) {
+    if (pdl_enabled()) {
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;

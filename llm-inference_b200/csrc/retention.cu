@@ -36,6 +36,8 @@ constexpr int kWalkTokens = 8;   // tokens whose q / k are staged per synchronis
 
 template <int DIM>
 __global__ void __launch_bounds__(128) retention_walk_kernel(const RT a) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ float sm[];
     const int dim = a.dim;
     float* raw = sm;                              // [2][dim] un-rotated q, k of the token being staged
@@ -119,6 +121,8 @@ __device__ __forceinline__ void stage_rotated(const RT& a, float* dst, int col_o
 
 template <int NACC>   // accumulators per thread (a multiple of 4): dim <= 4 * NACC
 __global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) float sm[];
     const RT& a = rc.a;
     const int e = blockIdx.x / rc.col_blocks, cb = blockIdx.x % rc.col_blocks;
@@ -172,6 +176,8 @@ __global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc)
 
 // element-wise over (dim, vdim): walks the entry's chunks, leaves S at each chunk's start in place of its U
 __global__ void __launch_bounds__(256) retention_chunk_scan_kernel(const RC rc) {
+    pdl_wait();
+    pdl_launch_dependents();
     const RT& a = rc.a;
     const int e = blockIdx.x, h = blockIdx.y, i = blockIdx.z * blockDim.x + threadIdx.x;
     const int per = a.dim * a.vdim;
@@ -200,6 +206,8 @@ __global__ void __launch_bounds__(256) retention_chunk_scan_kernel(const RC rc) 
 }
 
 __global__ void __launch_bounds__(256) retention_chunk_out_kernel(const RC rc) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) float sm[];
     const RT& a = rc.a;
     const int e = blockIdx.x / rc.col_blocks, cb = blockIdx.x % rc.col_blocks;
@@ -289,6 +297,8 @@ __global__ void __launch_bounds__(256) retention_chunk_out_kernel(const RC rc) {
 template <typename T, bool SIG>
 __global__ void unit_rms_gate_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long ld_gate, const float* __restrict__ w,
                                      T* __restrict__ out, int units, int heads, int vdim, float eps) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int u = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (u >= units) return;
     const int t = u / heads, h = u % heads;
@@ -311,6 +321,8 @@ template <typename T, bool SIG, int PER>
 __global__ void __launch_bounds__(128) unit_rms_gate_reg_kernel(const float* __restrict__ o, const float* __restrict__ gate, long long ld_gate,
                                                                 const float* __restrict__ w, T* __restrict__ out, int units, int heads, int vdim,
                                                                 float eps) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int u = blockIdx.x * 4 + threadIdx.x / 32, lane = threadIdx.x % 32, quads = vdim / 4;
     if (u >= units) return;
     const int t = u / heads, h = u % heads;
@@ -355,11 +367,11 @@ static void launch_unit_rms(const float* o, const float* gate, long long ld_gate
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     const unsigned grid = (unsigned)((units + 3) / 4);
     if (vdim % 4 == 0 && vdim <= 512 && ld_gate % 4 == 0 && al16(o) && al16(gate) && al16(w) && al16(out)) {
-        if (vdim <= 128) unit_rms_gate_reg_kernel<T, SIG, 1><<<grid, 128, 0, s>>>(o, gate, ld_gate, w, out, units, heads, vdim, eps);
-        else if (vdim <= 256) unit_rms_gate_reg_kernel<T, SIG, 2><<<grid, 128, 0, s>>>(o, gate, ld_gate, w, out, units, heads, vdim, eps);
-        else unit_rms_gate_reg_kernel<T, SIG, 4><<<grid, 128, 0, s>>>(o, gate, ld_gate, w, out, units, heads, vdim, eps);
+        if (vdim <= 128) launch_chained(unit_rms_gate_reg_kernel<T, SIG, 1>, grid, 128, 0, s, o, gate, ld_gate, w, out, units, heads, vdim, eps);
+        else if (vdim <= 256) launch_chained(unit_rms_gate_reg_kernel<T, SIG, 2>, grid, 128, 0, s, o, gate, ld_gate, w, out, units, heads, vdim, eps);
+        else launch_chained(unit_rms_gate_reg_kernel<T, SIG, 4>, grid, 128, 0, s, o, gate, ld_gate, w, out, units, heads, vdim, eps);
     } else
-        unit_rms_gate_kernel<T, SIG><<<grid, 128, 0, s>>>(o, gate, ld_gate, w, out, units, heads, vdim, eps);
+        launch_chained(unit_rms_gate_kernel<T, SIG>, grid, 128, 0, s, o, gate, ld_gate, w, out, units, heads, vdim, eps);
 }
 
 }  // namespace b200
@@ -398,13 +410,13 @@ extern "C" int b200_retention(const b200_retention_args* p, void* stream) {
         cudaError_t e = ensure_max_dynamic_smem((const void*)retention_chunk_out_kernel, kMax3, done3);
         if (e != cudaSuccess) return (int)e;
         rc.col_blocks = col_blocks;
-        if (p->dim <= 32) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<8>, kMax1, done1[0]); retention_chunk_state_kernel<8><<<grid, 256, smem1, s>>>(rc); }
-        else if (p->dim <= 64) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<16>, kMax1, done1[1]); retention_chunk_state_kernel<16><<<grid, 256, smem1, s>>>(rc); }
-        else if (p->dim <= 128) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<32>, kMax1, done1[2]); retention_chunk_state_kernel<32><<<grid, 256, smem1, s>>>(rc); }
-        else { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<64>, kMax1, done1[3]); retention_chunk_state_kernel<64><<<grid, 256, smem1, s>>>(rc); }
+        if (p->dim <= 32) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<8>, kMax1, done1[0]); launch_chained(retention_chunk_state_kernel<8>, grid, 256, smem1, s, rc); }
+        else if (p->dim <= 64) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<16>, kMax1, done1[1]); launch_chained(retention_chunk_state_kernel<16>, grid, 256, smem1, s, rc); }
+        else if (p->dim <= 128) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<32>, kMax1, done1[2]); launch_chained(retention_chunk_state_kernel<32>, grid, 256, smem1, s, rc); }
+        else { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<64>, kMax1, done1[3]); launch_chained(retention_chunk_state_kernel<64>, grid, 256, smem1, s, rc); }
         const int per = p->dim * p->vdim;
-        retention_chunk_scan_kernel<<<dim3(p->n_entries, p->heads, (per + 255) / 256), 256, 0, s>>>(rc);
-        retention_chunk_out_kernel<<<grid, 256, smem3, s>>>(rc);
+        launch_chained(retention_chunk_scan_kernel, dim3(p->n_entries, p->heads, (per + 255) / 256), 256, 0, s, rc);
+        launch_chained(retention_chunk_out_kernel, grid, 256, smem3, s, rc);
         count_launch(3);
         return (int)cudaGetLastError();
     }
@@ -412,10 +424,10 @@ extern "C" int b200_retention(const b200_retention_args* p, void* stream) {
     const dim3 grid(p->n_entries, p->heads, (p->vdim + threads - 1) / threads);
     if (grid.y > 65535 || grid.z > 65535) return B200_EUNSUPPORTED;
     const size_t smem = (size_t)(2 + 2 * kWalkTokens) * p->dim * sizeof(float);
-    if (p->dim <= 32) retention_walk_kernel<32><<<grid, threads, smem, s>>>(a);
-    else if (p->dim <= 64) retention_walk_kernel<64><<<grid, threads, smem, s>>>(a);
-    else if (p->dim <= 128) retention_walk_kernel<128><<<grid, threads, smem, s>>>(a);
-    else retention_walk_kernel<256><<<grid, threads, smem, s>>>(a);
+    if (p->dim <= 32) launch_chained(retention_walk_kernel<32>, grid, threads, smem, s, a);
+    else if (p->dim <= 64) launch_chained(retention_walk_kernel<64>, grid, threads, smem, s, a);
+    else if (p->dim <= 128) launch_chained(retention_walk_kernel<128>, grid, threads, smem, s, a);
+    else launch_chained(retention_walk_kernel<256>, grid, threads, smem, s, a);
     count_launch();
     return (int)cudaGetLastError();
 }

@@ -13,6 +13,8 @@ namespace b200 {
 
 __global__ void rope_angles_kernel(const int* __restrict__ pos, const double* __restrict__ freq, int n_freq, int total,
                                    double amplitude, float* __restrict__ cos_out, float* __restrict__ sin_out) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const double a = (double)pos[i / n_freq] * freq[i % n_freq];
@@ -49,6 +51,8 @@ __device__ __forceinline__ float query_temp(const QkPrep& a, int p) {
 constexpr int kPrepWarps = 4, kMaxTapsUnrolled = 4;   // longer filters take the plain loop
 template <typename T>
 __global__ void __launch_bounds__(kPrepWarps * 32) qk_prepare_kernel(const QkPrep a, int n_units) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ float prep_sm[];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, dim = a.dim;
     const int unit = blockIdx.x * kPrepWarps + warp, per_token = a.heads + a.kv_heads;
@@ -186,6 +190,8 @@ __device__ __forceinline__ void prep_load(float (&v)[VEC], const float* src) {
 }
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kRowPrepThreads) qk_row_prepare_kernel(const QkPrep a) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ __align__(16) float prep_sm[];   // rotated designs: the normed q and k of the token
     __shared__ float red[2][kRowPrepThreads / 32];
     const int t = blockIdx.x, dim = a.dim, nq = a.heads * dim, nk = a.kv_heads * dim, nv = a.v_heads * a.vdim, p = a.pos[t];
@@ -255,6 +261,8 @@ __global__ void __launch_bounds__(kRowPrepThreads) qk_row_prepare_kernel(const Q
 // values and the weights are loaded up front and live in registers (one round trip to memory instead of two passes).
 template <typename T, int THREADS, int PER>
 __global__ void __launch_bounds__(THREADS) qk_row_prepare_reg_kernel(const QkPrep a) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float red[2][THREADS / 32];
     const int t = blockIdx.x, nq = a.heads * a.dim, nk = a.kv_heads * a.dim, nv = a.v_heads * a.vdim, p = a.pos[t];
     const float* row = a.proj + (size_t)t * a.ld_proj;
@@ -313,9 +321,9 @@ __global__ void __launch_bounds__(THREADS) qk_row_prepare_reg_kernel(const QkPre
 template <typename T>
 static bool launch_row_prepare_reg(const QkPrep& a, int n_tokens, cudaStream_t s) {
     const int quads = (a.heads + a.kv_heads) * a.dim / 4;
-    if (quads <= 256) qk_row_prepare_reg_kernel<T, 256, 1><<<n_tokens, 256, 0, s>>>(a);
-    else if (quads <= 1024) qk_row_prepare_reg_kernel<T, 512, 2><<<n_tokens, 512, 0, s>>>(a);
-    else if (quads <= 2048) qk_row_prepare_reg_kernel<T, 512, 4><<<n_tokens, 512, 0, s>>>(a);
+    if (quads <= 256) launch_chained(qk_row_prepare_reg_kernel<T, 256, 1>, n_tokens, 256, 0, s, a);
+    else if (quads <= 1024) launch_chained(qk_row_prepare_reg_kernel<T, 512, 2>, n_tokens, 512, 0, s, a);
+    else if (quads <= 2048) launch_chained(qk_row_prepare_reg_kernel<T, 512, 4>, n_tokens, 512, 0, s, a);
     else return false;
     return true;
 }
@@ -325,6 +333,8 @@ static bool launch_row_prepare_reg(const QkPrep& a, int n_tokens, cudaStream_t s
 // four of its rotate-half partner with 16-byte loads, and stores four values of the serving dtype at once.
 template <typename T>
 __global__ void __launch_bounds__(256) qk_rotate_store_kernel(const QkPrep a, long long total, int quads_per_token) {
+    pdl_wait();
+    pdl_launch_dependents();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int t = (int)(idx / quads_per_token), qd = (int)(idx % quads_per_token);
@@ -367,6 +377,8 @@ __global__ void __launch_bounds__(256) qk_rotate_store_kernel(const QkPrep a, lo
 __global__ void rotate_part_kernel(const float* __restrict__ src, long long ld_src, long long src_off, long long src_stride,
                                    float* __restrict__ dst, long long ld_dst, long long dst_off, long long dst_stride,
                                    const float* __restrict__ cs, const float* __restrict__ sn, int layout, int heads, int dims, size_t total) {
+    pdl_wait();
+    pdl_launch_dependents();
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= total) return;
     const int i = (int)(idx % dims), h = (int)((idx / dims) % heads);
@@ -379,6 +391,8 @@ __global__ void rotate_part_kernel(const float* __restrict__ src, long long ld_s
 __global__ void conv_state_update_kernel(const float* __restrict__ proj, long long ld_proj, float* __restrict__ state,
                                          const int* __restrict__ slot, const int* __restrict__ pos, const int* __restrict__ end,
                                          int channels, int taps) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int t = blockIdx.x, p = pos[t];
     if (p < end[t] - (taps - 1)) return;   // only the last taps-1 inputs of a sequence are carried
     float* dst = state + ((size_t)slot[t] * (taps - 1) + p % (taps - 1)) * channels;
@@ -394,7 +408,7 @@ extern "C" int b200_rope_angles_amp(const int* pos, int n_tokens, const double* 
     if (!pos || !freq || !cos_out || !sin_out || n_tokens < 0 || n_freq < 0) return B200_EINVAL;
     const int total = n_tokens * n_freq;
     if (total == 0) return B200_OK;
-    rope_angles_kernel<<<(total + 255) / 256, 256, 0, (cudaStream_t)stream>>>(pos, freq, n_freq, total, amplitude, cos_out, sin_out);
+    launch_chained(rope_angles_kernel, (total + 255) / 256, 256, 0, (cudaStream_t)stream, pos, freq, n_freq, total, amplitude, cos_out, sin_out);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -435,11 +449,11 @@ extern "C" int b200_qk_prepare(const b200_qk_prepare_args* p, void* stream) {
         const bool reg = vec && !p->rot_dims && !p->bias && (!p->q_norm || al16(p->q_norm)) && (!p->k_norm || al16(p->k_norm));
         if (reg && (p->dtype == B200_BF16 ? launch_row_prepare_reg<__nv_bfloat16>(a, p->n_tokens, s) : p->dtype == B200_F32 && launch_row_prepare_reg<float>(a, p->n_tokens, s))) {
         } else if (p->dtype == B200_BF16) {
-            if (vec) qk_row_prepare_kernel<__nv_bfloat16, 4><<<p->n_tokens, kRowPrepThreads, smem, s>>>(a);
-            else qk_row_prepare_kernel<__nv_bfloat16, 1><<<p->n_tokens, kRowPrepThreads, smem, s>>>(a);
+            if (vec) launch_chained(qk_row_prepare_kernel<__nv_bfloat16, 4>, p->n_tokens, kRowPrepThreads, smem, s, a);
+            else launch_chained(qk_row_prepare_kernel<__nv_bfloat16, 1>, p->n_tokens, kRowPrepThreads, smem, s, a);
         } else if (p->dtype == B200_F32) {
-            if (vec) qk_row_prepare_kernel<float, 4><<<p->n_tokens, kRowPrepThreads, smem, s>>>(a);
-            else qk_row_prepare_kernel<float, 1><<<p->n_tokens, kRowPrepThreads, smem, s>>>(a);
+            if (vec) launch_chained(qk_row_prepare_kernel<float, 4>, p->n_tokens, kRowPrepThreads, smem, s, a);
+            else launch_chained(qk_row_prepare_kernel<float, 1>, p->n_tokens, kRowPrepThreads, smem, s, a);
         } else
             return B200_EINVAL;
         count_launch();
@@ -454,8 +468,8 @@ extern "C" int b200_qk_prepare(const b200_qk_prepare_args* p, void* stream) {
             const int quads = (p->heads + p->kv_heads) * (p->dim / 4) + p->v_heads * (p->vdim / 4);
             const long long total = (long long)p->n_tokens * quads;
             const unsigned grid = (unsigned)((total + 255) / 256);
-            if (p->dtype == B200_BF16) qk_rotate_store_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(a, total, quads);
-            else qk_rotate_store_kernel<float><<<grid, 256, 0, s>>>(a, total, quads);
+            if (p->dtype == B200_BF16) launch_chained(qk_rotate_store_kernel<__nv_bfloat16>, grid, 256, 0, s, a, total, quads);
+            else launch_chained(qk_rotate_store_kernel<float>, grid, 256, 0, s, a, total, quads);
             count_launch();
             return (int)cudaGetLastError();
         }
@@ -465,8 +479,8 @@ extern "C" int b200_qk_prepare(const b200_qk_prepare_args* p, void* stream) {
     const unsigned grid = (unsigned)((units + kPrepWarps - 1) / kPrepWarps);
     const size_t smem = (size_t)kPrepWarps * a.vals_per_warp * sizeof(float);
     if (smem > 48 * 1024) return B200_EUNSUPPORTED;
-    if (p->dtype == B200_BF16) qk_prepare_kernel<__nv_bfloat16><<<grid, kPrepWarps * 32, smem, s>>>(a, (int)units);
-    else if (p->dtype == B200_F32) qk_prepare_kernel<float><<<grid, kPrepWarps * 32, smem, s>>>(a, (int)units);
+    if (p->dtype == B200_BF16) launch_chained(qk_prepare_kernel<__nv_bfloat16>, grid, kPrepWarps * 32, smem, s, a, (int)units);
+    else if (p->dtype == B200_F32) launch_chained(qk_prepare_kernel<float>, grid, kPrepWarps * 32, smem, s, a, (int)units);
     else return B200_EINVAL;
     count_launch();
     return (int)cudaGetLastError();
@@ -479,7 +493,7 @@ extern "C" int b200_rotate_part(const float* src, long long ld_src, long long sr
     if (rot_layout != B200_ROPE_HALF && rot_layout != B200_ROPE_INTERLEAVED) return B200_EINVAL;
     if (n_tokens == 0) return B200_OK;
     const size_t total = (size_t)n_tokens * heads * dims;
-    rotate_part_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(src, ld_src, src_off, src_stride, dst, ld_dst, dst_off,
+    launch_chained(rotate_part_kernel, (unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream, src, ld_src, src_off, src_stride, dst, ld_dst, dst_off,
                                                                                          dst_stride, cos, sin, rot_layout, heads, dims, total);
     count_launch();
     return (int)cudaGetLastError();
@@ -490,7 +504,7 @@ extern "C" int b200_conv_state_update(const float* proj, long long ld_proj, floa
     if (!proj || !slot || !pos || !end || n_tokens < 0 || channels < 1 || taps < 1) return B200_EINVAL;
     if (n_tokens == 0 || taps == 1) return B200_OK;
     if (!conv_state) return B200_EINVAL;
-    conv_state_update_kernel<<<n_tokens, 128, 0, (cudaStream_t)stream>>>(proj, ld_proj, conv_state, slot, pos, end, channels, taps);
+    launch_chained(conv_state_update_kernel, n_tokens, 128, 0, (cudaStream_t)stream, proj, ld_proj, conv_state, slot, pos, end, channels, taps);
     count_launch();
     return (int)cudaGetLastError();
 }
