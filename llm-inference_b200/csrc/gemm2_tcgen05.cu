@@ -11,7 +11,6 @@
 //   warps 2-5 epilogue (both CTAs): own 128 rows from own TMEM, then a remote arrive on the leader's
 //             accumulator-empty barrier
 // GLU: as in gemm_tcgen05.cu — the leader's B half is 128 gate rows, the peer's the matching 128 up rows.
-#include <cstdio>
 #include "common.cuh"
 #include "launch_count.h"
 #include "tc_common.cuh"
@@ -222,13 +221,7 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
     }
 }
 
-// QUAD: a cluster of FOUR CTAs = two MMA pairs on the same 256 rows of A and two neighbouring column tiles. Every CTA
-// loads a 64-row box of A and multicasts it to its counterpart in the other pair, so a cluster reads A from L2 once
-// instead of twice: 48 KB instead of 64 KB per pair and K step (the cuBLAS kernel of this shape, nvjet ..._2x2_2cta, moves
-// the same 4.83 GB against the pair kernel's 6.44 GB at 8192 x 12288 x 4096). On a power-capped B200 the bytes moved set
-// the clock. A stage is free when BOTH pairs' MMAs have read it (empty barriers count two commits); each pair
-// keeps its own full barriers, accumulators and epilogue.
-template <bool GLU, bool QUAD>
+template <bool GLU>
 __global__ void __launch_bounds__(k2Threads, 1)
 gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Gemm2Params p) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -238,16 +231,12 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     uint64_t* acc_empty = acc_full + 2;          // [2], used in the leader only
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + k2OffSlot);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t crank = cluster_ctarank();
-    const uint32_t rank = crank & 1u;            // position in the MMA pair, 0 = pair leader
-    const uint32_t pair = QUAD ? crank >> 1 : 0u;
-    const uint32_t leader = crank & ~1u;         // cluster rank of this pair's leader
-    constexpr int CS = QUAD ? 4 : 2;
+    const uint32_t rank = cluster_ctarank();     // 0 = leader
     if (threadIdx.x == 0) {
         if (smem_u32(smem) & 1023u) __trap();
         for (int s = 0; s < k2Stages; ++s) {
             mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], QUAD ? 2 : 1);   // one commit per pair that reads the stage
+            mbar_init(&empty_bar[s], 1);
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&acc_full[a], 1);
@@ -266,9 +255,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     pdl_launch_dependents();
     pdl_wait();
 
-    const int n_tiles = QUAD ? p.n_tiles >> 1 : p.n_tiles;   // QUAD: a unit is two neighbouring column tiles
-    const int units = p.m_tiles * n_tiles;
-    const int cluster_id = blockIdx.x / CS, n_clusters = gridDim.x / CS;
+    const int units = p.m_tiles * p.n_tiles;
+    const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
 
     if (warp == 0) {
         // ================= TMA producer (both CTAs) =================
@@ -276,21 +264,16 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         uint32_t phase = 0;
         for (int u = cluster_id; u < units; u += n_clusters) {
             int mt, nt;
-            tile_of_unit(p, n_tiles, u, mt, nt);
-            if (QUAD) nt = 2 * nt + (int)pair;
-            const int a_row = mt * 256 + (int)rank * 128 + (QUAD ? (int)pair * 64 : 0);
+            tile_of_unit(p, p.n_tiles, u, mt, nt);
+            const int a_row = mt * 256 + (int)rank * 128;
             const int b_row = GLU ? (rank == 0 ? nt * 128 : p.n_out + nt * 128) : nt * 256 + (int)rank * 128;
             for (int kb = 0; kb < p.k_blocks; ++kb) {
                 mbar_wait_bounded(&empty_bar[stage], phase ^ 1);
                 if (lane == 0) {
                     unsigned char* sa = smem + (size_t)stage * k2StageBytes;
-                    const uint32_t leader_full = mapa_shared(smem_u32(&full_bar[stage]), leader);
+                    const uint32_t leader_full = mapa_shared(smem_u32(&full_bar[stage]), 0);
                     if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * k2StageBytes);   // both CTAs' boxes
-                    if (QUAD)   // my 64 rows of this position's A half, to me and to my counterpart in the other pair
-                        tma_load_2d_pair_multicast(sa + pair * (k2ABytes / 2), &map_a, kb * k2BK, a_row, leader_full,
-                                                   (uint16_t)((1u << rank) | (1u << (rank + 2))));
-                    else
-                        tma_load_2d_pair(sa, &map_a, kb * k2BK, a_row, leader_full);
+                    tma_load_2d_pair(sa, &map_a, kb * k2BK, a_row, leader_full);
                     tma_load_2d_pair(sa + k2ABytes, &map_b, kb * k2BK, b_row, leader_full);
                 }
                 __syncwarp();
@@ -317,8 +300,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 #pragma unroll
                         for (int k = 0; k < k2BK / kUmmaK; ++k)
                             umma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        umma_commit_pair(&empty_bar[stage], QUAD ? 0xF : 3);         // the producers may refill
-                        if (kb == p.k_blocks - 1) umma_commit_pair(&acc_full[acc], (uint16_t)(3u << (2 * pair)));   // both epilogues of the pair may read
+                        umma_commit_pair(&empty_bar[stage], 3);         // the producers may refill
+                        if (kb == p.k_blocks - 1) umma_commit_pair(&acc_full[acc], 3);   // both epilogues may read
                     }
                     __syncwarp();
                     if (++stage == k2Stages) { stage = 0; phase ^= 1; }
@@ -334,8 +317,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         uint32_t acc_phase = 0;
         for (int u = cluster_id; u < units; u += n_clusters) {
             int mt, nt;
-            tile_of_unit(p, n_tiles, u, mt, nt);
-            if (QUAD) nt = 2 * nt + (int)pair;
+            tile_of_unit(p, p.n_tiles, u, mt, nt);
             mbar_wait_bounded(&acc_full[acc], acc_phase);
             tc_fence_after();
             const int row = mt * 256 + (int)rank * 128 + quarter * 32 + lane;
@@ -345,7 +327,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                                  smem_u32(smem + k2OffStg + (uint32_t)(warp - 2) * kStgBytes), lane);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[acc]), leader));
+            if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[acc]), 0));
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1;
         }
@@ -547,43 +529,6 @@ static void fill_cluster_cfg(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr,
     cfg.numAttrs = na;
 }
 
-// clusters of four CTAs that can be resident at once (a cluster lives inside one GPC: fewer than sm_count / 4 where a GPC's
-// SM count is not a multiple of 4), asked from the runtime once per device and instantiation; 0 = not launchable
-template <bool GLU>
-static int quad_clusters() {
-    static int cached[64];
-    static bool have[64];
-    const int dev = current_device();
-    if (dev < 0 || dev >= 64) return 0;
-    if (!have[dev]) {
-        auto kern = gemm2_tcgen05_kernel<GLU, true>;
-        static unsigned long long attr_done = 0;
-        int n = 0;
-        if (ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), (int)k2Smem, attr_done) == cudaSuccess) {
-            prefer_max_smem_carveout(reinterpret_cast<const void*>(kern));
-            cudaLaunchConfig_t cfg;
-            cudaLaunchAttribute attr[2];
-            fill_cluster_cfg(cfg, attr, 4 * (sm_count() / 4), 4, nullptr, false);
-            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { n = 0; cudaGetLastError(); }
-        }
-        if (getenv("B200_GEMM2_VERBOSE")) fprintf(stderr, "[b200] gemm2 quad: %d clusters of 4 CTAs resident (of %d SMs)\n", n, sm_count());
-        cached[dev] = n;
-        have[dev] = true;
-    }
-    return cached[dev];
-}
-
-template <bool GLU>
-static int gemm2_launch_quad(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params& p, int clusters, cudaStream_t s) {
-    auto kern = gemm2_tcgen05_kernel<GLU, true>;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[2];
-    fill_cluster_cfg(cfg, attr, 4 * clusters, 4, s, pdl_enabled());
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ma, mb, p);
-    count_launch();
-    return (int)e;
-}
-
 template <bool GLU>
 static int gemm2_launch_wide(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params& p, int clusters, cudaStream_t s) {
     auto kern = gemm2w_tcgen05_kernel<GLU>;
@@ -603,7 +548,7 @@ static int gemm2_launch_wide(const CUtensorMap& ma, const CUtensorMap& mb, const
 
 template <bool GLU>
 static int gemm2_launch(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params& p, int grid, cudaStream_t s) {
-    auto kern = gemm2_tcgen05_kernel<GLU, false>;
+    auto kern = gemm2_tcgen05_kernel<GLU>;
     static unsigned long long attr_done = 0;   // per instantiation, one bit per device
     {
         cudaError_t e = ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), (int)k2Smem, attr_done);
@@ -660,14 +605,6 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
         p.group_m = group_env >= 0 ? group_env : 16;
     }
     CUtensorMap ma, mb;
-    // Opt-in (B200_GEMM2_QUAD=1, read per call so that tests can switch it): four-CTA clusters with the A tile multicast
-    // between two MMA pairs. Needs an even number of column tiles and >= 2 units per cluster. Measured on the B200 at
-    // 8192 x 12288 x 4096 (tools/gemm_power.py, 3 s back to back, board at its 1 kW cap): L2 -> SM bytes 6.44 -> 4.83 GB and
-    // the SM clock rises 1335 -> 1455 MHz (cuBLAS' clock), but only 33 clusters of 4 are resident (132 of 148 SMs: a cluster
-    // lives inside one GPC) and the throughput per clock drops 891 -> 782 TFLOP/s/GHz: 1137 vs 1190 TFLOP/s sustained, 1262
-    // vs 1305 burst. The pair kernel stays the default.
-    const char* quad_s = getenv("B200_GEMM2_QUAD");
-    const int quad_env = (quad_s && quad_s[0] == '1') ? 1 : 0;
     // Opt-in (B200_GEMM2_WIDE=1, read per call so that tests can compare): 256 x 512 pair tiles (gemm2w_tcgen05_kernel); needs
     // an even number of column tiles and at least one unit per cluster. Measured at 8192 x 12288 x 4096 (tools/gemm_power.py,
     // three interleaved 2 s rounds per variant, board at its 1 kW cap): 1194 TFLOP/s at 1417 MHz against the 256 x 256
@@ -676,7 +613,7 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
     // kernels (more L2 traffic = more energy) and was removed again.
     const char* wide_s = getenv("B200_GEMM2_WIDE");
     const int wide_env = (wide_s && wide_s[0] == '1') ? 1 : 0;
-    if (wide_env && !quad_env && M >= 512 && (p.n_tiles & 1) == 0) {
+    if (wide_env && M >= 512 && (p.n_tiles & 1) == 0) {
         int clusters = sm_count() / 2;
         const int units_w = p.m_tiles * (p.n_tiles / 2);
         if (units_w >= clusters) {
@@ -685,15 +622,6 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
             p.wide_full = (rem > 0 && 2 * rem <= clusters) ? units_w - rem : units_w;
             if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, 128)) return B200_EUNSUPPORTED;
             return glu ? gemm2_launch_wide<true>(ma, mb, p, clusters, s) : gemm2_launch_wide<false>(ma, mb, p, clusters, s);
-        }
-    }
-    if (quad_env && M >= 512 && (p.n_tiles & 1) == 0) {
-        int clusters = glu ? quad_clusters<true>() : quad_clusters<false>();
-        const int units4 = p.m_tiles * (p.n_tiles / 2);
-        if (clusters > units4) clusters = units4;
-        if (clusters >= 8 && units4 >= 2 * clusters) {
-            if (!make_tma_map_2d(&ma, x, M, K, 64) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, 128)) return B200_EUNSUPPORTED;
-            return glu ? gemm2_launch_quad<true>(ma, mb, p, clusters, s) : gemm2_launch_quad<false>(ma, mb, p, clusters, s);
         }
     }
     if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, 128)) return B200_EUNSUPPORTED;

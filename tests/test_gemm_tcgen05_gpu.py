@@ -60,17 +60,6 @@ def test_one_row_tile_of_the_pair_kernel(ops, m, n, k):
     assert rel_err(got, want) < 4e-3
 
 
-@pytest.mark.parametrize("m,n,k", [(2048, 12288, 4096), (4000, 2504, 328), (4100, 2500, 72), (8192, 1024, 512)])
-def test_quad_cluster_multicast_variant(ops, m, n, k, monkeypatch):
-    """B200_GEMM2_QUAD=1: clusters of four CTAs, the A tile multicast between the two MMA pairs (opt-in, gemm2_tcgen05.cu);
-    must give the pair kernel's result bit for bit (same MMAs in the same order) and match the oracle"""
-    got0, want = case(ops, m, n, k, m + n * 3)
-    monkeypatch.setenv("B200_GEMM2_QUAD", "1")
-    got1, _ = case(ops, m, n, k, m + n * 3)
-    assert_close(got1, want, "fp16", f"tcgen05 quad {m}x{n}x{k}")
-    assert np.array_equal(got0, got1)
-
-
 @pytest.mark.parametrize("m,n,k", [(8192, 12288, 512), (5000, 5120, 328), (19000, 1024, 72), (2048, 12288, 4096)])
 def test_wide_pair_tile_equals_the_256x256_tile(ops, m, n, k, monkeypatch):
     """B200_GEMM2_WIDE=1: the 256 x 512 pair tile (gemm2w_tcgen05_kernel, opt-in), incl. shapes whose last wave is split
@@ -155,13 +144,13 @@ def test_linear_with_residual_epilogue(ops, m, n, k):
     assert_close(out.float().cpu().numpy(), want, "fp16", f"linear + residual {m}x{n}x{k}")
 
 
-@pytest.mark.parametrize("knob", ["B200_GEMM2_WIDE", "B200_GEMM2_QUAD"])
+@pytest.mark.parametrize("knob", ["B200_GEMM2_WIDE"])
 def test_opt_in_tile_shapes_with_swiglu_and_residual_epilogues(ops, knob, monkeypatch):
-    """the opt-in 256 x 512 pair tile / four-CTA multicast cluster also carry the SwiGLU and the residual epilogue: their
+    """the opt-in 256 x 512 pair tile also carries the SwiGLU and the residual epilogue: its
     outputs must equal the default 256 x 256 tile's bit for bit (same MMAs, same K order, same rounding points); the default
     is pinned to the oracle by the tests above"""
     g = torch.Generator(device="cpu").manual_seed(3)
-    m, inter, k = 2048, 11008, 1024      # 86 GLU column tiles: 344 wide units / quad units
+    m, inter, k = 2048, 11008, 1024      # 86 GLU column tiles: 344 wide units
     x = (torch.rand(m, k, generator=g) * 2 - 1).half().cuda()
     w = (torch.randn(2 * inter, k, generator=g) * 0.05).half().cuda()
     m2, n2, k2 = 4096, 4096, 520          # 16 x 8 units, ragged K

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""usage: gemm_power.py [N] [VARIANT ...], VARIANT = comma-separated B200_GEMM2_* knobs without the prefix, e.g. WIDE=1 or QUAD=1,GROUP_M=8
+"""usage: gemm_power.py [N] [VARIANT ...], VARIANT = comma-separated B200_GEMM2_* knobs without the prefix, e.g. WIDE=1,GROUP_M=8
 SM clock and board power while one GEMM runs back to back for a few seconds: gemm2_tcgen05_kernel vs the cuBLAS kernel
 on the same 7B prefill shape (both are power-capped on a B200: the clock they settle at is part of the comparison)."""
 import os
@@ -57,7 +57,7 @@ def run(name, fn, secs=4.0):
           f"  -> {2 * m * n * k / ms / 1e9 / med(0) * 1000:7.1f} TFLOP/s per GHz", flush=True)
 
 
-variants = [dict(kv.split("=") for kv in a.split(",") if kv) for a in sys.argv[2:]] or [{}, {"WIDE": "1"}, {"QUAD": "1"}]
+variants = [dict(kv.split("=") for kv in a.split(",") if kv) for a in sys.argv[2:]] or [{}, {"WIDE": "1"}]
 variants = [{("B200_GEMM2_" + k_): v for k_, v in d.items()} for d in variants]
 # the board drifts (temperature, power-cap controller): every variant is timed in ROUNDS interleaved rounds, means are printed last
 ROUNDS, SECS = 3, 2.0
@@ -80,7 +80,7 @@ def run(name, fn, secs=3.0):   # noqa: F811 - keeps the one-line report, collect
 for r in range(ROUNDS):
     acc["cuBLAS"].append(run("cuBLAS (torch linear)", lambda i: torch.nn.functional.linear(x, ws[i % 4]), SECS))
     for env, nm in zip(variants, names[1:]):
-        for k_ in ("B200_GEMM2_WIDE", "B200_GEMM2_QUAD", "B200_GEMM2_GROUP_M"):
+        for k_ in ("B200_GEMM2_WIDE", "B200_GEMM2_GROUP_M"):
             os.environ.pop(k_, None)
         os.environ.update(env)
         acc[nm].append(run("gemm2 " + nm, lambda i: ops.launchLinearGemm(x, ws[i % 4], y, trans_b=True), SECS))
