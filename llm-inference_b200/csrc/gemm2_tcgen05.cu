@@ -51,80 +51,13 @@ __device__ __forceinline__ void tile_of_unit(const Gemm2Params& p, int n_tiles, 
     mt = band * p.group_m + (r - nt * rows);
 }
 
-// One thread's row of one accumulator tile: TMEM (taddr: this warp's lane quarter, the tile's first column) -> fp16 -> C.
-// nt: column tile (256 features, GLU: 128 features with gate in columns [0,128) and up in [128,256) of the accumulator).
-template <bool GLU>
-__device__ __forceinline__ void store_tile_row(const Gemm2Params& p, uint32_t taddr, int row, int nt) {
-    if (GLU) {
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 32) {
-            uint32_t g[32], uu[32];
-            tmem_ld_32x32(taddr + (uint32_t)c0, g);
-            tmem_ld_32x32(taddr + (uint32_t)(128 + c0), uu);
-            const int col0 = nt * 128 + c0;
-            if (row < p.tokens && col0 < p.n_out) {
-                __half* dst = p.C + (size_t)row * p.ldc + col0;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    float f[8];
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float gv = __half2float(__float2half_rn(__uint_as_float(g[q * 8 + e])));
-                        const float uv = __half2float(__float2half_rn(__uint_as_float(uu[q * 8 + e])));
-                        const float sv = __half2float(__float2half_rn(gv / (1.f + expf(-gv))));
-                        f[e] = sv * uv;
-                    }
-                    if (col0 + q * 8 + 8 <= p.n_out) st16(dst + q * 8, Unpack<__half>::put(f));
-                }
-            }
-        }
-    } else {
-#pragma unroll 1
-        for (int c0 = 0; c0 < 256; c0 += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(taddr + (uint32_t)c0, v);
-            const int col0 = nt * 256 + c0;
-            if (row < p.tokens && col0 < p.n_out) {
-                __half* dst = p.C + (size_t)row * p.ldc + col0;
-                if (col0 + 32 <= p.n_out && (p.ldc & 7) == 0) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        float f[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            f[e] = __uint_as_float(v[q * 8 + e]);
-                            if (p.bias) f[e] += __half2float(p.bias[col0 + q * 8 + e]);
-                        }
-                        if (p.residual) {   // the linear's output is rounded to fp16 first, as the unfused pair does
-                            float r[8];
-                            Unpack<__half>::get(ld16(p.residual + (size_t)row * p.ldc + col0 + q * 8), r);
-#pragma unroll
-                            for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e])) + r[e];
-                        }
-                        st16(dst + q * 8, Unpack<__half>::put(f));
-                    }
-                } else {
-                    // (fully unrolled with a predicate: a run-time index would put v[] into local memory - with the
-                    // 227 KB carve-out there is no L1 behind it, and the whole epilogue crawled at L2 latency: STACK 128 -> 0)
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (col0 + j >= p.n_out) continue;
-                        float f = __uint_as_float(v[j]);
-                        if (p.bias) f += __half2float(p.bias[col0 + j]);
-                        if (p.residual) f = __half2float(__float2half_rn(f)) + __half2float(p.residual[(size_t)row * p.ldc + col0 + j]);
-                        dst[j] = __float2half_rn(f);
-                    }
-                }
-            }
-        }
-    }
-}
-
-// The same tile part for a whole WARP (32 rows x the tile's columns), with the stores coalesced: every thread owns an
+// One warp's part of an accumulator tile (32 rows x the tile's columns): TMEM (taddr: this warp's lane quarter, the tile's first column) -> fp16 -> C.
+// nt: column tile (256 features, GLU: 128 features with gate in columns [0,128) and up in [128,256) of the accumulator). Every thread owns an
 // accumulator ROW in TMEM, so storing straight from registers makes each store instruction touch 32 rows x 16 bytes - 8192
 // sixteen-byte transactions per 128 x 512 CTA tile, ~20 k clocks that the 256 x 512 kernel cannot hide. Here 64 output
 // columns of the warp's 32 rows are rounded to fp16, staged in 4 KB of shared memory (16-byte chunks XOR-swizzled by row:
-// conflict-free both ways), then written as 4 rows x 128 contiguous bytes per instruction. Rounding points as above.
+// conflict-free both ways), then written as 4 rows x 128 contiguous bytes per instruction. Rounding points of the unfused sequence: the linear's
+// output, silu of the gate and the product of gate and up are each rounded to fp16.
 __device__ __forceinline__ void stg_st_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
@@ -149,6 +82,7 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
         for (int sub = 0; sub < 2; ++sub) {
             const int cc = c0 + sub * 32;
             uint32_t h[16];
+            __syncwarp();   // the loads of tensor memory are warp-wide: lanes that took different ways through the divisions meet first
             if (GLU) {
                 uint32_t g[32], uu[32];
                 tmem_ld_32x32(taddr + (uint32_t)cc, g);

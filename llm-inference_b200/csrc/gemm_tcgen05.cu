@@ -101,12 +101,14 @@ template <int KIND>
 __device__ __forceinline__ void store_glu_row(const GemmParams& p, uint32_t taddr, int row, int nt) {
     if (row - (int)(threadIdx.x & 31) >= p.tokens) return;   // (rows behind the tokens are zeros, which take the long way through the division: not here, and not below)
     uint32_t g[16], u[16];
+    __syncwarp();   // (the loads and waits of tensor memory are warp-wide: lanes that left a branch or a wait one by one meet first, here and below)
     tmem_ld_32x16_async(taddr, g);
     tmem_ld_32x16_async(taddr + 128u, u);
 #pragma unroll 1
     for (int c0 = 0; c0 < 128; c0 += 16) {
         float f[16];
         uint32_t gc[16], uc[16];
+        __syncwarp();
         tmem_wait_ld<16>(g);
         tmem_wait_ld<16>(u);
 #pragma unroll
@@ -254,6 +256,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 uint32_t v[32];
+                __syncwarp();   // as in store_glu_row
                 tmem_ld_32x32(taddr + (uint32_t)c0, v);
                 const int col0 = nt * BN + c0;   // first row of the B operand covered by this chunk
                 // row = token, col = output feature: 32 consecutive features per thread

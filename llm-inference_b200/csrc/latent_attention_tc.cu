@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
                 for (int i = 0; i < 8; ++i) pack8(x[i], y[i], v[i]);
                 if (o + 1 < NCH) load(o + 1);
                 const uint32_t base = smem_u32(smem + (o < QT ? o : o - QT) * kLtQChunk);
+                __syncwarp();   // lanes without a row skipped its loads; the barriers and tensor memory stores are warp-wide
                 if (QT > 0 && o == QT) asm volatile("bar.sync 2, 128;" ::: "memory");   // those chunks have gone to TMEM
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {

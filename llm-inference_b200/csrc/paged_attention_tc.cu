@@ -157,6 +157,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         const int pA = a.pos[tA], pZ = a.pos[tA + count - 1];
         const int key0 = pa_first_key(a, pA) & ~(kTcKeys - 1), n_kt = (pZ - key0) / kTcKeys + 1;
         const int* plist = a.pages + (size_t)slots[first + 1] * a.max_pages;
+        __syncwarp();   // lanes without a row skipped its loads; the barrier is warp-wide
         if (warp >= 1) asm volatile("bar.sync 1, 160;" ::: "memory");
 
         if (warp == 0) {
