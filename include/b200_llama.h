@@ -154,7 +154,7 @@ int b200_scale_mask_softmax(const void* qk, const void* mask, void* score, int b
  *   trans_b = 0: W is [K, N] row-major (tests/unittests/test_linear.cu)
  * Dispatch: n_tokens <= B200_GEMV_MAX_TOKENS and trans_b -> weight-streaming GEMV (bulk-async
  * smem ring); fp16 with large n_tokens -> tcgen05/TMEM GEMM; everything else -> SIMT tiled GEMM.
- * workspace may be NULL when b200_linear_workspace_bytes() returns 0.
+ * b200_linear_workspace_bytes() is 0 for every call: the workspace is not read and may be NULL.
  * ------------------------------------------------------------------------------------ */
 #define B200_GEMV_MAX_TOKENS 8
 size_t b200_linear_workspace_bytes(int n_tokens, int N, int K, int trans_b, int dtype);

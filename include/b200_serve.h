@@ -78,7 +78,7 @@ int b200_gemm_grouped(const b200_gemm_grouped_args* args, void* stream);
  * output), or the GLU form with W [2N, K] (B200_GG_GLU, B200_GG_GLU_GELU). bfloat16 operands run on the tcgen05 / TMEM GEMM of the LLaMA path (weights streamed once through the
  * M axis up to 256 token rows, tokens on the M axis above; fp32 accumulation; out_dtype B200_BF16 or B200_F32) when the
  * shape allows (K % 8 == 0, 16-byte aligned pointers, GLU: N % 128 == 0); everything else, and B200_F32 operands, goes
- * to b200_gemm_grouped. workspace: split-K partials of the weight-streaming mode (may be NULL: single split). */
+ * to b200_gemm_grouped. No workspace is needed: the size is 0 and the two arguments are not read. */
 size_t b200_linear_ex_workspace_bytes(int n_tokens, int N, int K);
 int b200_linear_ex(const void* x, const void* W, void* y, int n_tokens, int N, int K, int in_dtype, int out_dtype, int epi,
                    void* workspace, size_t workspace_bytes, void* stream);
@@ -194,8 +194,8 @@ int b200_layernorm_residual(float* x, const float* y, int n_rows, int width, flo
 /* out[t, 0:width] = a[t,:], out[t, width:2 width] = b[t,:], as out_dtype (the operand of a projection of two streams) */
 int b200_concat_cast(const float* a, const float* b, void* out, int n_rows, int width, int out_dtype, void* stream);
 /* out[t, j] = act(gu[t, j]) * gu[t, n + j], act by epi (B200_GG_GLU: silu, B200_GG_GLU_GELU: tanh-gelu); gu fp32 [n_rows, 2 n]:
- * the GLU of a [gate | up] product computed without the fused epilogue (small batches, where the stacked weight streams
- * once through the split-K GEMM) */
+ * the GLU of a [gate | up] product computed without the fused epilogue (small batches, whose stacked weight
+ * is one plain product) */
 int b200_glu_act(const float* gu, void* out, int n_rows, int n, int epi, int out_dtype, void* stream);
 /* v[i] <- cap * tanh(v[i] / cap) */
 int b200_softcap(float* v, size_t n, float cap, void* stream);

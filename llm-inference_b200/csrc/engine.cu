@@ -83,8 +83,6 @@ struct b200_engine {
     float* rope_den;
     void* attn_ws;
     size_t attn_ws_bytes;
-    void* lin_ws;          // split-K partials of the tcgen05 weight-streaming linears (batch > 8)
-    size_t lin_ws_bytes;
     int* pinned_ids = nullptr;
     // prefill scratch (grown on demand by b200_engine_prefill)
     char* pf_arena = nullptr;
@@ -583,15 +581,6 @@ extern "C" b200_engine* b200_engine_create_paged(const b200_model_config* c, int
     const size_t o_fin = off; off += align256(B);
     const size_t o_den = off; off += align256((size_t)c->rotary_dim / 2 * sizeof(float) + 64);
     const size_t o_ws = off; off += align256(e->attn_ws_bytes);
-    e->lin_ws_bytes = 0;
-    {
-        const int shapes[5][2] = {{e->qkv_n, e->H}, {e->H, e->h * e->d}, {2 * e->I, e->H}, {e->H, e->I}, {e->V, e->H}};
-        for (auto& sh : shapes) {
-            const size_t w = b200_linear_workspace_bytes(batch, sh[0], sh[1], 1, c->dtype);
-            if (w > e->lin_ws_bytes) e->lin_ws_bytes = w;
-        }
-    }
-    const size_t o_lws = off; off += align256(e->lin_ws_bytes + 256);
     if ((err = cudaMalloc(&e->act_arena, off)) != cudaSuccess) return fail_free("cudaMalloc(act)", err);
     cudaMemset(e->act_arena, 0, off);
     char* a = e->act_arena;
@@ -602,7 +591,6 @@ extern "C" b200_engine* b200_engine_create_paged(const b200_model_config* c, int
     e->finished = (unsigned char*)(a + o_fin);
     e->seq_cached.assign(B, 0);
     e->attn_ws = a + o_ws;
-    e->lin_ws = a + o_lws;
     e->rope_den = (float*)(a + o_den);
     b200_rope_table(e->rope_den, c->rotary_dim, c->rotary_base, nullptr);
     if ((err = cudaMallocHost(&e->pinned_ids, 2 * B * sizeof(int))) != cudaSuccess) return fail_free("cudaMallocHost", err);
@@ -1040,7 +1028,7 @@ static int enqueue_step_body(b200_engine* e) {
     const bool fused = (e->mode & B200_ENGINE_FUSED) && B <= (dt == B200_F16 && !tp ? 4 : B200_GEMV_MAX_TOKENS) && !e->kv_fp8 &&
                        !e->kv_paged;
     auto linear = [&](const void* x, const void* W, void* y, int N, int K) {
-        return b200_linear(x, W, nullptr, y, B, N, K, 1, dt, e->lin_ws, e->lin_ws_bytes, s);
+        return b200_linear(x, W, nullptr, y, B, N, K, 1, dt, nullptr, 0, s);
     };
     RC(b200_embedding(e->ids_cur, e->embed, e->hidden, B, H, e->V, dt, s));
     for (int l = 0; l < e->cfg.num_layers; ++l) {
@@ -1297,12 +1285,6 @@ static int prefill_impl(b200_engine* e, const int* ids_host, const int* lens_hos
     const size_t o_gu = take((size_t)Nt * 2 * e->I * es), o_act = take((size_t)Nt * e->I * es);
     const size_t o_ids = take((size_t)Nt * 4), o_pad = take((size_t)Nt * 4), o_cum = take((size_t)(B + 1) * 4),
                  o_len = take((size_t)B * 4), o_hist = take((size_t)B * 4), o_ctx = take((size_t)B * 4);
-    size_t lin_ws = 0;
-    {
-        const int shapes[4][2] = {{e->qkv_n, H}, {H, e->h * e->d}, {2 * e->I, H}, {H, e->I}};
-        for (auto& sh : shapes) lin_ws = std::max(lin_ws, b200_linear_workspace_bytes(Nt, sh[0], sh[1], 1, dt));
-    }
-    const size_t o_lws = take(lin_ws + 256);
     const bool flash = dt == B200_F16 && e->d == 128 && !(getenv("B200_NO_TCGEN05") && getenv("B200_NO_TCGEN05")[0] == '1');
     if (any_zero && !flash)
         return fail("prefill: sequences that sit a pass out need the flash context attention (fp16, head size 128)", B200_EUNSUPPORTED);
@@ -1357,7 +1339,7 @@ static int prefill_impl(b200_engine* e, const int* ids_host, const int* lens_hos
     }
     char* a = e->pf_arena;
     void *x = a + o_x, *res = a + o_res, *qkv = a + o_qkv, *q = a + o_q, *k = a + o_k, *v = a + o_v, *att = a + o_att,
-         *gu = a + o_gu, *act = a + o_act, *lws = a + o_lws;
+         *gu = a + o_gu, *act = a + o_act;
     int *ids = (int*)(a + o_ids), *pad = (int*)(a + o_pad), *cum = (int*)(a + o_cum), *lens = (int*)(a + o_len),
         *hists = (int*)(a + o_hist), *ctxs = (int*)(a + o_ctx);
     // ---- host -> device: token ids and the three length vectors (contiguous in the arena)
@@ -1381,7 +1363,7 @@ static int prefill_impl(b200_engine* e, const int* ids_host, const int* lens_hos
             if (len_b[b] > 0) CU(cudaMemsetAsync(e->finished + b, 0, 1, s));   // ... every sequence that takes part in it
     }
     auto linear = [&](const void* in, const void* W, void* out, int N, int K) {
-        return b200_linear(in, W, nullptr, out, Nt, N, K, 1, dt, lws, lin_ws + 256, s);
+        return b200_linear(in, W, nullptr, out, Nt, N, K, 1, dt, nullptr, 0, s);
     };
     const bool tp = e->cfg.tp_size > 1 && (e->allreduce || e->p2p);
     RC(b200_cal_padding_offset(pad, cum, lens, B, len, s));
@@ -1471,7 +1453,7 @@ static int prefill_impl(b200_engine* e, const int* ids_host, const int* lens_hos
     }
     CU(cudaMemcpyAsync(e->partial, e->hidden, (size_t)B * H * es, cudaMemcpyDeviceToDevice, s));
     RC(b200_rmsnorm(e->partial, nullptr, e->final_norm, B, H, e->cfg.rms_eps, dt, s));
-    RC(b200_linear(e->partial, e->lm_head, nullptr, e->logits, B, e->V, H, 1, dt, e->lin_ws, e->lin_ws_bytes, s));
+    RC(b200_linear(e->partial, e->lm_head, nullptr, e->logits, B, e->V, H, 1, dt, nullptr, 0, s));
     RC(b200_argmax(e->logits, e->ids_next, B, e->V, dt, s));
     CU(launch_k(set_ids_step_kernel, dim3(1), dim3(1024), 0, s, false, e->ids_cur, e->ids_next, e->step_dev, B, ctx + 1,
                 any_zero ? (const int*)lens : (const int*)nullptr));

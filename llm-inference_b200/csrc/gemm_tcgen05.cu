@@ -603,28 +603,8 @@ int gemm_min_tokens() {
     return v;
 }
 
-// the number of K shares that the sizes of the split-K workspaces count with
-static int pick_splits(int m_tiles, int k_blocks, int sms) {
-    int best = 1;
-    long long best_cost = -1;
-    for (int s = 1; s <= 16 && k_blocks / s >= 4; ++s) {
-        const long long rounds = ((long long)m_tiles * s + sms - 1) / sms;
-        const long long per = (k_blocks + s - 1) / s;
-        const long long cost = rounds * (per + 2) + (s > 1 ? s : 0);   // +2: tile prologue/epilogue; +s: partial traffic
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
-    }
-    return best;
-}
-
-size_t gemm_tcgen05_workspace_bytes(int M, int N, int K) {
-    if (M < gemm_min_tokens() || M > 256) return 0;
-    const int splits = pick_splits((N + kBM - 1) / kBM, (K + kBK - 1) / kBK, sm_count());
-    return splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
-}
-
 // y[M, N] = x[M, K] * W[N, K]^T (+ bias), fp16 in / fp32 accumulate / fp16 out
-int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, void* workspace,
-                     size_t workspace_bytes, cudaStream_t s) {
+int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, cudaStream_t s) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     if (M < 1 || N < 8 || K < 8 || (K & 7) || !al(x) || !al(W)) return B200_EUNSUPPORTED;
     static int disabled = -1;
@@ -668,8 +648,8 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
 // rows, N % 128 == 0; glu 4: the clamped gated unit of common.cuh with its limit) or with the square of relu on every output
 // (glu 3: not a GLU, W = [N, K]).
 // Up to 256 token rows (gated units: 128) the weights stream through the M axis; above, tokens are the M axis.
-int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, int glu, void* workspace,
-                    size_t workspace_bytes, cudaStream_t s, float glu_limit) {
+int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, int glu, cudaStream_t s,
+                    float glu_limit) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     if (M < 1 || N < 8 || K < 8 || (K & 7) || !al(x) || !al(W) || !al(y)) return B200_EUNSUPPORTED;
     const char* env = getenv("B200_NO_TCGEN05");
@@ -705,12 +685,6 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
         default: return gemm_launch<256>(ma, mb, p, grid, s);
     }
 }
-size_t gemm_tcgen05_ex_workspace_bytes(int M, int N, int K) {
-    if (M > 256) return 0;
-    const int splits = pick_splits((N + kBM - 1) / kBM, (K + kBK - 1) / kBK, sm_count());
-    return splits > 1 ? (size_t)splits * M * N * sizeof(float) : 0;
-}
-
 // out[M, inter] = silu(x W_gate^T) * (x W_up^T), W = [2*inter, K] (gate rows, then up rows): the gate_up GEMM of
 // ffn.cpp:72 with launchAct (ffn.cpp:80) as its epilogue. Prefill shapes only (M > 256, inter % 128 == 0).
 int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int inter, int K, cudaStream_t s) {

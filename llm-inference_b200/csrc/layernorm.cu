@@ -182,7 +182,7 @@ __global__ void concat_cast_kernel(const float* __restrict__ a, const float* __r
 }
 
 // out[t, j] = act(gu[t, j]) * gu[t, n + j] (act: silu or gelu in its tanh form): the GLU of a [gate | up] product that was
-// computed without the fused epilogue (small batches stream the stacked weight once through the split-K GEMM)
+// computed without the fused epilogue (small batches, whose stacked weight is one plain product)
 template <typename T>
 __global__ void glu_act_kernel(const float* __restrict__ gu, T* __restrict__ out, int n, size_t total, int gelu) {
     pdl_wait();

@@ -14,9 +14,7 @@ namespace b200 {
 int gemv_plain(const void* x, const void* W, const void* bias, void* y, int n_tokens, int N, int K,
                int dtype, cudaStream_t s);
 // tcgen05 path (gemm_tcgen05.cu); returns B200_EUNSUPPORTED when the shape does not fit
-int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K,
-                     void* workspace, size_t workspace_bytes, cudaStream_t s);
-size_t gemm_tcgen05_workspace_bytes(int M, int N, int K);
+int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, cudaStream_t s);
 int gemm_min_tokens();
 int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int inter, int K, cudaStream_t s);
 int gemm_tcgen05_f16_residual(const void* x, const void* W, const void* residual, void* y, int M, int N, int K, cudaStream_t s);
@@ -115,16 +113,12 @@ static int gemm_simt(const void* A, const void* B, const void* bias, void* C, in
 
 using namespace b200;
 
-// split-K partials of the tcgen05 weight-streaming mode (fp16, 8 < n_tokens <= 256); 0 otherwise.
-// Without a workspace the call still succeeds (single-split schedule, less SM coverage).
-extern "C" size_t b200_linear_workspace_bytes(int n_tokens, int N, int K, int trans_b, int dtype) {
-    if (!trans_b || dtype != B200_F16) return 0;
-    return gemm_tcgen05_workspace_bytes(n_tokens, N, K);
-}
+// no kernel behind b200_linear needs scratch: partial sums of a shared K range meet in shared memory (gemm_stream_kernel)
+extern "C" size_t b200_linear_workspace_bytes(int, int, int, int, int) { return 0; }
 
 extern "C" int b200_linear(const void* x, const void* W, const void* bias, void* y, int n_tokens,
-                           int N, int K, int trans_b, int dtype, void* workspace,
-                           size_t workspace_bytes, void* stream) {
+                           int N, int K, int trans_b, int dtype, void* /*workspace*/,
+                           size_t /*workspace_bytes*/, void* stream) {
     B200_RETURN_IF(!x || !W || !y || n_tokens < 0 || N <= 0 || K <= 0, B200_EINVAL);
     B200_RETURN_IF(dtype != B200_F32 && dtype != B200_F16, B200_EINVAL);
     if (n_tokens == 0) return B200_OK;
@@ -135,7 +129,7 @@ extern "C" int b200_linear(const void* x, const void* W, const void* bias, void*
     // halves = weights streamed twice); the tcgen05 weight-streaming GEMM reads every weight byte once, so it takes
     // these shapes. Up to 4 rows the GEMV (tensor-core consumer from 2 rows on) is as fast or faster (route_sweep.sh).
     if (trans_b && dtype == B200_F16 && n_tokens >= b200::gemm_min_tokens() && n_tokens <= B200_GEMV_MAX_TOKENS) {
-        int rc = gemm_tcgen05_f16(x, W, bias, y, n_tokens, N, K, workspace, workspace_bytes, s);
+        int rc = gemm_tcgen05_f16(x, W, bias, y, n_tokens, N, K, s);
         if (rc != B200_EUNSUPPORTED) return rc;
     }
     if (trans_b && n_tokens <= B200_GEMV_MAX_TOKENS && K % E == 0 && al(x) && al(W)) {
@@ -143,7 +137,7 @@ extern "C" int b200_linear(const void* x, const void* W, const void* bias, void*
         if (rc != B200_EUNSUPPORTED) return rc;
     }
     if (trans_b && dtype == B200_F16) {
-        int rc = gemm_tcgen05_f16(x, W, bias, y, n_tokens, N, K, workspace, workspace_bytes, s);
+        int rc = gemm_tcgen05_f16(x, W, bias, y, n_tokens, N, K, s);
         if (rc != B200_EUNSUPPORTED) return rc;
     }
     if (dtype == B200_F16)

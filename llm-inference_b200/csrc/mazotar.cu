@@ -43,7 +43,7 @@ namespace b200 {
 namespace {
 
 constexpr int kPageRows = 64;
-constexpr int kStreamRows = 256;   // up to here a stacked [gate; up] streams once through the split-K GEMM
+constexpr int kStreamRows = 256;   // up to here a stacked [gate; up] is one plain product whose weights stream through the M axis
 constexpr double kPi = 3.14159265358979323846;
 
 struct MzConnect {   // one sublayer's connections to the streams
@@ -504,7 +504,7 @@ int Mazotar::memory_mixer(MzLayer& L, int T, int longest_entry, std::string& err
 
 // out = W_down (silu(W_gate h) * (W_up h)) on lane k
 int Mazotar::gated_unit(const void* w_gu, const void* w_down, int ff, int T, float* gu, void* act, float* out, int k, std::string& err) {
-    if (dtype_ == B200_BF16 && T <= kStreamRows) {   // few rows: the stacked [gate; up] streams once through the split-K GEMM
+    if (dtype_ == B200_BF16 && T <= kStreamRows) {   // few rows: the stacked [gate; up] is one plain product whose weights stream through the M axis
         MZ_OP(gemm(h_, w_gu, gu, B200_F32, T, 2 * ff, D_, B200_GG_NONE, 0.f, k));
         MZ_OP(b200_glu_act(gu, act, T, ff, B200_GG_GLU, dtype_, lane(k)));
     } else

@@ -153,7 +153,6 @@ StepRunner::~StepRunner() {
         if (l.stream) { cudaStreamSynchronize(l.stream); cudaStreamDestroy(l.stream); }
         if (l.forked) cudaEventDestroy(l.forked);
         if (l.joined) cudaEventDestroy(l.joined);
-        cudaFree(l.ws);
     }
     for (void* p : owned_) cudaFree(p);
     cudaFree(attn_ws_);
@@ -221,17 +220,7 @@ int StepRunner::ensure_logits_host(int W) {
 }
 
 int StepRunner::gemm(const void* A, const void* W, void* C, int c_dt, int M, int N, int K, int epi, float epi_param, int k) {
-    const size_t need = b200_linear_ex_workspace_bytes(M, N, K);
-    Lane& l = lanes_[k];
-    if (need > l.ws_bytes && !capturing_) {
-        cudaStreamSynchronize(lane(k));
-        ++buffers_epoch_;
-        cudaFree(l.ws);
-        l.ws = nullptr;
-        l.ws_bytes = 0;
-        if (cudaMalloc(&l.ws, need) == cudaSuccess) l.ws_bytes = need;   // without it the call runs with a single split
-    }
-    return b200_linear_ex2(A, W, C, M, N, K, dtype_, c_dt, epi, epi_param, l.ws, l.ws_bytes, lane(k));
+    return b200_linear_ex2(A, W, C, M, N, K, dtype_, c_dt, epi, epi_param, nullptr, 0, lane(k));
 }
 
 int StepRunner::fork(int k, std::string& err) {
@@ -283,7 +272,6 @@ int StepRunner::expert_products(const ExpertGroups& g, int k, std::string& err) 
         const int off = group_off_host_[e], n = group_off_host_[e + 1] - off;
         if (n <= 0) continue;
         cudaStream_t s = side_[used++ % kExpertStreams];
-        // no split-K workspace: the products of different streams run at the same time and must not share one
         rc = b200_linear_ex((const char*)g.gathered + (size_t)off * D_ * ez, (const char*)g.w_up + (size_t)e * up_rows * D_ * ez,
                             (char*)g.act + (size_t)off * g.ff * ez, n, g.ff, D_, dtype_, dtype_, g.epi, nullptr, 0, s);
         if (rc == B200_OK)

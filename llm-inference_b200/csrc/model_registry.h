@@ -157,8 +157,7 @@ protected:
     int gemm(const void* A, const void* W, void* C, int c_dt, int M, int N, int K, int epi = B200_GG_NONE, float epi_param = 0.f,
              int lane = 0);
     // Lanes: lane 0 is stream_; sublayers that read the same input can run on lanes 1 .. kLanes - 1 beside it (captured into the
-    // step's graph as parallel branches). fork(lane) orders the lane behind everything on stream_, join(lane) the reverse. Every
-    // lane has its own split-K workspace.
+    // step's graph as parallel branches). fork(lane) orders the lane behind everything on stream_, join(lane) the reverse.
     static constexpr int kLanes = 3;
     cudaStream_t lane(int k) const { return k == 0 ? stream_ : lanes_[k].stream; }
     int fork(int k, std::string& err);
@@ -201,8 +200,6 @@ private:
     struct Lane {
         cudaStream_t stream = nullptr;              // lane 0 runs on stream_
         cudaEvent_t forked = nullptr, joined = nullptr;
-        void* ws = nullptr;                         // split-K partials of the weight-streaming GEMM
-        size_t ws_bytes = 0;
     };
     Lane lanes_[kLanes];
     // side streams of expert_products

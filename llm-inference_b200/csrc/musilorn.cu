@@ -40,7 +40,7 @@ namespace b200 {
 namespace {
 
 constexpr int kPageRows = 64;
-constexpr int kStreamRows = 256;   // up to here b200_linear_ex streams weights through its M axis (split-K)
+constexpr int kStreamRows = 256;   // up to here b200_linear_ex streams weights through its M axis
 constexpr double kPi = 3.14159265358979323846;
 
 struct MuRot {
@@ -446,7 +446,7 @@ int Musilorn::enqueue(int T, int W, int longest_entry, int longest_context, bool
         const MuLayer* next = (r + 1 < runs_.size() && !runs_[r + 1].pass_start) ? &layers_[runs_[r + 1].layer] : nullptr;
         if (L.has_mlp) {
             MU_OP(b200_layernorm_residual(x_, y_, T, D, eps_, mult_, L.n1bw, L.n1bb, L.n2w, L.n2b, h2_, dt, stream_));
-            if (dt == B200_BF16 && T <= kStreamRows) {   // few rows: the stacked [gate; up] streams once through the split-K GEMM
+            if (dt == B200_BF16 && T <= kStreamRows) {   // few rows: the stacked [gate; up] is one plain product whose weights stream through the M axis
                 MU_OP(gemm(h2_, L.w_gu, gu_, B200_F32, T, 2 * L.ff, D));
                 MU_OP(b200_glu_act(gu_, act_, T, L.ff, B200_GG_GLU_GELU, dt, stream_));
             } else

@@ -32,7 +32,7 @@
 //              out) -> turn back + head gates -> W_o (its bias joins in the norm kernel)
 //   latent:  [q | latent | key part] = h W^T -> normed latent + rotated key part to the pages; per head q W_uk beside the
 //            rotated query part -> windowed attention over the rows -> per head W_uv -> W_o
-//   x += N1(y) with h = x out of the same kernel -> [gate ; up] GEMM with the clamped unit (fused epilogue, or split-K GEMM +
+//   x += N1(y) with h = x out of the same kernel -> [gate ; up] GEMM with the clamped unit (fused epilogue, or a plain GEMM +
 //   activation kernel for few rows) -> W_down -> x += N2(y), h = x.
 #include <cuda_bf16.h>
 
@@ -52,7 +52,7 @@ namespace b200 {
 namespace {
 
 constexpr int kPageRows = 64;
-constexpr int kStreamRows = 256;   // up to here b200_linear_ex2 streams weights through its M axis (split-K)
+constexpr int kStreamRows = 256;   // up to here b200_linear_ex2 streams weights through its M axis
 constexpr double kPi = 3.14159265358979323846;
 
 struct SkFreq {
@@ -538,7 +538,7 @@ int Sakevik::enqueue(int T, int W, int longest_entry, int longest_context, bool 
         SK_OP(gemm(mid_, L.w_o, y_, B200_F32, T, D, L.n_mid));
         SK_OP(add_normed(L.n1, L.o_bias));
         if (L.ff > 0) {
-            if (dt == B200_BF16 && T <= kStreamRows) {   // few rows: the stacked [gate; up] streams once through the split-K GEMM
+            if (dt == B200_BF16 && T <= kStreamRows) {   // few rows: the stacked [gate; up] is one plain product whose weights stream through the M axis
                 SK_OP(gemm(h_, L.w_gu, gu_, B200_F32, T, 2 * L.ff, D));
                 SK_OP(b200_glu_act_clamped(gu_, act_, T, L.ff, L.limit, dt, stream_));
             } else
