@@ -1,17 +1,17 @@
 #!/usr/bin/env python
-"""bench.py — LLaMA-2-7B fp16 decode tok/s on B200 (BASELINE.json metric), one JSON line.
+"""bench.py — LLaMA-2-7B fp16 decode tok/s on B200, one JSON line.
 
     python bench.py --gpus N --steps K --warmup W [--workload cfg2|cfg3|cfg4] [--impl reference]
 
 A "step" is one decode step of the whole model for the whole batch (one new token per sequence).
-Workloads (BASELINE.json configs):
+Workloads:
   cfg2 (default): LLaMA-2-7B fp16 random-init full model, batch 1 greedy decode at a 512-token
         context. N GPUs = N independent requests (weights replicated, no communication): weak.
   cfg4: batch 32 x KV length 4096, 32/N sequences per GPU (strong), no communication.
   cfg5: LLaMA-2-70B-shaped GQA (64 q / 8 kv heads, 80 layers) fp16 decode, tensor parallel over the N GPUs
         (strong scaling: heads / FFN columns split, allreduce after o_proj and down_proj only);
         --comm p2p = the fused one-shot NVLink allreduce + residual kernel, --comm nccl = the NCCL baseline.
-  nekodra, musilorn: not BASELINE.json configs: prefill and decode tokens/s of the Nekodra / Musilorn family
+  nekodra, musilorn: prefill and decode tokens/s of the Nekodra / Musilorn family
         (include/b200_serve.h, random weights, --size s|m) beside the LLaMA engine at equal size; a line of its own shape.
   tomalix: the same for the Tomalix family, beside the Musilorn family at equal size.
   sakevik, filipel, mazotar: the same for the Sakevik / Filipel / Mazotar family, beside the Tomalix family at equal size
@@ -72,15 +72,15 @@ def parse():
 
 def workload(args):
     if args.workload == "cfg3":
-        return dict(name="LLaMA-2-7B fp16 prefill: context attention + tcgen05 GEMMs, batch 4 x seq 2048 (configs[2])",
+        return dict(name="LLaMA-2-7B fp16 prefill: context attention + tcgen05 GEMMs, batch 4 x seq 2048",
                     batch=4, context=args.context or 2048, scaling="weak")
     if args.workload == "cfg5":
-        return dict(name="LLaMA-2-70B-shaped GQA (64 q / 8 kv heads) fp16 decode, tensor-parallel (configs[4])",
+        return dict(name="LLaMA-2-70B-shaped GQA (64 q / 8 kv heads) fp16 decode, tensor-parallel",
                     batch=args.batch or 1, context=args.context or 512, scaling="strong")
     if args.workload == "cfg4":
-        return dict(name="LLaMA-2-7B fp16 decode, batch 32 x KV 4096 (configs[3])", batch=args.batch or 32,
+        return dict(name="LLaMA-2-7B fp16 decode, batch 32 x KV 4096", batch=args.batch or 32,
                     context=args.context or 4096, scaling="strong")
-    return dict(name="LLaMA-2-7B fp16 random-init full model, batch 1 greedy decode, 512-token context (configs[1])",
+    return dict(name="LLaMA-2-7B fp16 random-init full model, batch 1 greedy decode, 512-token context",
                 batch=1, context=args.context or 512, scaling="weak")
 
 
@@ -195,9 +195,9 @@ def cpu_baseline_port(wl, budget_s=10.0):
 
 
 def cpu_baseline_hf(wl, n_layers=8, n_decode=12):
-    """The torch-CPU `LlamaForCausalLM` leg north_star names (reference: modeling_llama.py + test_llama_run.py:1-29;
+    """The torch-CPU `LlamaForCausalLM` leg (reference: modeling_llama.py + test_llama_run.py:1-29;
     the vendored modeling_llama.py is not importable on its own - relative imports into the transformers package -
-    so the container's transformers LlamaForCausalLM stands in, BASELINE.md section 4.2). fp32, use_cache=True, LLaMA-2-7B
+    so the container's transformers LlamaForCausalLM stands in). fp32, use_cache=True, LLaMA-2-7B
     geometry with `n_layers` of the 32 layers (host memory / time bound), batch 1: prefill of the workload's
     context, then greedy decode steps; the per-token time is scaled to 32 layers (the LM head is timed inside the
     steps and not scaled)."""
@@ -256,7 +256,7 @@ class RefCpu:
     oracle/_ref/libref.so) composed into a decode-layer sample. CPUlinear is a single-threaded
     triple loop over W[K,N]; the output columns are sliced over all host cores (one slice per
     thread, ctypes releases the GIL). Attention / RoPE use the oracle port: the reference's
-    CPUMaskedAttn / CPUfunc are unsound outside their toy shapes (SURVEY §4)."""
+    CPUMaskedAttn / CPUfunc are unsound outside their toy shapes."""
 
     def __init__(self):
         self.lib = C.CDLL(os.path.join(ROOT, "oracle", "_ref", "libref.so"))
@@ -278,7 +278,7 @@ def reference_arm(args, wl):
     they lie) composed into WHOLE decode steps of the 7B-shaped model on the host cores and timed as they run:
     per layer its CPU RMSNorm, CPUlinear for qkv / o / gate_up / down (output columns sliced over all cores, one
     slice per thread), its CPU SwiGLU, and decode attention + RoPE through the oracle port (the reference's
-    CPUMaskedAttn / CPUfunc are unsound outside their toy shapes, SURVEY section 4); then the LM head through CPUlinear.
+    CPUMaskedAttn / CPUfunc are unsound outside their toy shapes); then the LM head through CPUlinear.
     The 32 layers share ONE 0.8 GB set of fp32 layer weights (far larger than the host caches, so every layer still
     streams them from DRAM). A step is a whole token when the run fits the wall-clock budget; otherwise a step is
     the first `sample_layers` layers and the line says so (`extrapolated`, `scale`): `ms_per_step` is always the
@@ -724,7 +724,7 @@ def bench_tp(args, wl, rank, world, local_rank):
 
 
 # --------------------------------------------------------------------------------------------
-# proof that the timed launch order did the work ("make the timed region prove it")
+# proof that the timed launch order did the work
 # --------------------------------------------------------------------------------------------
 def verify_decode(pkg, eng, model_shape, weight_seed, ctx, kv_seed, ids0, n_steps=6):
     """After the timed region: rewind the timed engine to the cache state it was timed from and let it decode
@@ -784,7 +784,7 @@ def verify_decode(pkg, eng, model_shape, weight_seed, ctx, kv_seed, ids0, n_step
 
 
 # --------------------------------------------------------------------------------------------
-# N > 1 only: the partitioned workloads of north_star in the SAME process group and JSON line
+# N > 1 only: the partitioned workloads in the SAME process group and JSON line
 # --------------------------------------------------------------------------------------------
 def tp_step_bytes(eng, B, ctx_mid, world, n_layers):
     kv = B * n_layers * 2 * max(1, 8 // world) * 128 * 2 * ctx_mid
@@ -858,7 +858,7 @@ def extras_multi_gpu(pkg, args, rank, world, local_rank, peak):
             logits[kind] = eng.logits().float().clone()
             bytes_ = tp_step_bytes(eng, B, ctx + W + K // 2, world, cfg["num_layers"])
             ach = bytes_ / (ms * 1e-3) / 1e9
-            out["tp_" + kind] = {"workload": f"LLaMA-2-70B-shaped GQA fp16 decode, tp{world}, batch 1, context 512 (configs[4])",
+            out["tp_" + kind] = {"workload": f"LLaMA-2-70B-shaped GQA fp16 decode, tp{world}, batch 1, context 512",
                                  "comm": {"p2p": "GEMV epilogue pushes partial rows to the peers + one-shot NVLink reduce+residual kernel",
                                           "p2p_persistent": "persistent step kernel: K-split accumulators exchanged as low-latency "
                                                             "lines over NVLink inside the kernel (kOpExchange), 1 launch per token",
@@ -891,7 +891,7 @@ def extras_multi_gpu(pkg, args, rank, world, local_rank, peak):
         bytes_ = eng.weight_bytes - 2 * 32000 * 4096 + Bl * 2 * 32 * 4096 * 2 * (ctx + W + K // 2)
         ach = bytes_ / (ms * 1e-3) / 1e9
         out["cfg4_shard"] = {"workload": f"LLaMA-2-7B fp16 decode, 32 sequences x KV 4096 split {Bl} per GPU over {world} GPUs, "
-                                         "no collective (configs[3])",
+                                         "no collective",
                              "value": round(Bt / (ms * 1e-3), 1), "unit": "tok/s", "ms_per_step": round(ms, 4), "steps": K,
                              "warmup": W, "launches_per_step": eng.launches_per_step,
                              "roofline": {"bound": "hbm", "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
@@ -1101,8 +1101,8 @@ def main():
         roof = {"bound": "hbm", "kernel": "gemv_stream_kernel", "achieved": round(achieved, 1), "peak": peak,
                 "unit": "GB/s", "frac": round(achieved / peak, 4),
                 # dram__bytes_read+write per launch, mean of the four GEMVs of a layer, from the committed
-                # `ncu --set full` capture (profiles/r01_gemv_full.md): 101.2 MB read + 2.6 MB written
-                "traffic": 103.8e6, "traffic_unit": "bytes/launch (ncu, profiles/r01_gemv_full.md)",
+                # `ncu --set full` capture (profiles/gemv_full.md): 101.2 MB read + 2.6 MB written
+                "traffic": 103.8e6, "traffic_unit": "bytes/launch (ncu, profiles/gemv_full.md)",
                 "per_launch_us": round(g_ms * 1e3 / n_launch, 2), "per_launch_MB": round(tot_bytes / n_launch / 1e6, 2),
                 "peak_source": peak_src,
                 "algorithmic_bytes_per_launch": round(tot_bytes / n_launch),
@@ -1128,12 +1128,12 @@ def main():
         achieved = step_bytes / (per_launch_ms * 1e-3) / 1e9
         traffic = None
         try:   # dram__bytes_read.sum + dram__bytes_write.sum of one launch, from the committed ncu capture
-            traffic = float(json.load(open(os.path.join(ROOT, "profiles", "r02_decode_step_traffic.json")))["dram_bytes_per_launch"])
+            traffic = float(json.load(open(os.path.join(ROOT, "profiles", "decode_step_traffic.json")))["dram_bytes_per_launch"])
         except Exception:
             pass
         roof = {"bound": "hbm", "kernel": "decode_step_kernel", "achieved": round(achieved, 1), "peak": peak,
                 "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
-                "traffic_unit": "bytes/launch (ncu --set full, profiles/r02_decode_step_full.md)" if traffic else None,
+                "traffic_unit": "bytes/launch (ncu --set full, profiles/decode_step_full.md)" if traffic else None,
                 "per_launch_us": round(per_launch_ms * 1e3, 1), "algorithmic_bytes_per_launch": int(step_bytes),
                 "peak_source": peak_src,
                 "note": "persistent whole-step kernel: one cooperative launch per token; per-launch time = the "

@@ -68,7 +68,7 @@ enum {
 };
 
 /* creation flags for b200_engine_create_ex */
-#define B200_ENGINE_KV_FP8 1u  /* KV cache in fp8 e4m3 with one fp32 scale per cached row (SURVEY 8 f4; replaces the T-typed
+#define B200_ENGINE_KV_FP8 1u  /* KV cache in fp8 e4m3 with one fp32 scale per cached row (replaces the T-typed
                                 * [layers,B,hk,max_seq,d] caches of llama.cpp:77-78). fp16 models, head size 128,
                                 * head_num / kv_head_num in {1,2,4}. A row is rounded once, when it enters the cache; decode
                                 * runs the reference launch order (RoPE -> b200_kv_append_fp8 -> b200_decode_attention_fp8);
@@ -76,7 +76,7 @@ enum {
                                 * cache: tests/test_kv_fp8_gpu.py pins it to the oracle run on the same rounded rows. */
 
 #define B200_ENGINE_KV_PAGED 2u /* KV cache as page pools [layers][n_pages, hk, 128 rows, d] + one page list per sequence
-                                * (SURVEY 8 f4 "paged blocks"; b200_llama.h, csrc/kv_paged.cu) instead of max_seq rows
+                                * (b200_llama.h, csrc/kv_paged.cu) instead of max_seq rows
                                 * reserved per sequence slot. fp16 models, head size 128, head_num / kv_head_num in
                                 * {1,2,4,8}. Bit-identical results to the dense cache on the same launch order
                                 * (tests/test_kv_paged_gpu.py). With KV_FP8 as well: fp8 pages + scale pools
@@ -91,8 +91,8 @@ enum {
 #define B200_ENGINE_GRAPH 2u   /* CUDA-graph replay of the whole step (default)               */
 #define B200_ENGINE_PERSISTENT 4u /* with FUSED: ONE persistent cooperative kernel per step     */
 /* Default: all three for fp16 batches 1-2 (and fp32 / tensor-parallel engines, where PERSISTENT only applies once a
- * b200_p2p communicator is attached and the mode asks for it); FUSED | GRAPH for fp16 batches >= 3 (the measured best,
- * DESIGN 4c): fused tensor-core GEMVs up to 4 token rows; above, the reference launch order on the tcgen05
+ * b200_p2p communicator is attached and the mode asks for it); FUSED | GRAPH for fp16 batches >= 3 (the measured
+ * best): fused tensor-core GEMVs up to 4 token rows; above, the reference launch order on the tcgen05
  * weight-streaming GEMM. */
                                   /* (fp16, batch <= 4, tp_size 1; default where it applies)   */
 /* without FUSED the engine issues the reference's kernel sequence one launch* at a time
@@ -198,7 +198,7 @@ int b200_engine_decode_step_host(b200_engine* e, const int* ids_in_host, int* id
  * then no host sync) receives them. */
 int b200_engine_prefill(b200_engine* e, const int* ids_host, int len, int* ids_out_host);
 
-/* Ragged batch (per-sequence lengths: the `step` per request SURVEY 8f-2 asks for instead of the
+/* Ragged batch (per-sequence lengths: a `step` per request instead of the
  * reference's single host scalar, llama.h): sequence b gets lens_host[b] >= 1 prompt tokens,
  * ids_host holds them packed back to back (sum(lens) ids, the padding-free layout the context
  * decoder works on, llama.cpp:158-185), each appended after what THAT sequence has cached. When

@@ -267,7 +267,7 @@ int b200_decode_attention_static(const void* qkv, void* k_cache_layer, void* v_c
                                  int max_seq_len, int step, int append_kv, int dtype, void* stream);
 
 /* ------------------------------------------------------------------------------------
- * fp8 (e4m3) KV cache, SURVEY 8 f4 - the evolution of the reference's T-typed cache
+ * fp8 (e4m3) KV cache - the evolution of the reference's T-typed cache
  * [layers,B,hk,max_seq,d] (src/models/llama/llama.cpp:77-78,102-103): one byte per element + one fp32 scale
  * per cached row ([B, hk, max_seq] per layer), value = scale * e4m3, scale = amax(row) / 448 fixed at append.
  * fp16 models, head size 128, head_num / kv_head_num in {1,2,4}.
@@ -291,7 +291,7 @@ int b200_kv_quantize_fp8(const void* src, void* dst8, float* scale, const int* n
 int b200_kv_dequant_fp8(const void* src8, const float* scale, void* dst, size_t rows, int head_size, void* stream);
 
 /* ------------------------------------------------------------------------------------
- * Paged KV cache, SURVEY 8 f4 - the other evolution of [layers,B,hk,max_seq,d] (src/models/llama/llama.cpp:77-78):
+ * Paged KV cache - the other evolution of [layers,B,hk,max_seq,d] (src/models/llama/llama.cpp:77-78):
  * a layer's K (V) is a pool of pages [n_pages, hk, B200_KV_PAGE_ROWS, d]; sequence b owns the pages listed in
  * page_table[b * max_pages + i] (DEVICE int, one list for all layers), cache row r of the sequence = row r % 128 of
  * page r / 128. No reference counterpart: the reference reserves max_seq rows per sequence slot.
@@ -358,7 +358,7 @@ int b200_context_attention(const void* q, const void* k_cache_layer, const void*
 void b200_context_attention_set_trace(void* dev_buf);
 
 /* ------------------------------------------------------------------------------------
- * next-tier ops bracketing a decode step (SURVEY §8f rank 1)
+ * next-tier ops bracketing a decode step
  * launchInputEmbedding   src/kernels/input_embedding.cu:30   out[t,:] = table[ids[t],:]
  * greedy pick            src/kernels/topK.cu:147 (K=1 case): lowest index wins ties
  * ------------------------------------------------------------------------------------ */

@@ -2,7 +2,7 @@
 // Replaces launchDecoderMaskedMHA (src/kernels/fused_decoder_self_attention.cu:80-291, 317-365):
 //   append k,v of the new token at row step-1; s_j = (q . K_j) * rsqrt(d), j < step;
 //   p = exp(s - max s) / (sum + 1e-6) (:203-221); out = sum_j p_j V_j (:272-287).
-// SURVEY defects D1-D6 resolved: kv head = q head / (h/hk), element-correct addressing, layer
+// Where the reference kernel is wrong, this one is not: kv head = q head / (h/hk), element-correct addressing, layer
 // slice includes kv_head_num, softmax over the full length, token-major qkv, fp16 implemented.
 //
 // HBM-bound: algorithmic bytes = 2*B*hk*step*d*sizeof(T). Layout of the work:
@@ -682,7 +682,7 @@ extern "C" int b200_decode_attention(const void* qkv, void* k_cache_layer, void*
 }
 
 // ------------------------------------------------------------------------------------------
-// Paged cache (SURVEY 8 f4 "paged blocks"): the reference's dense [layers, B, hk, max_seq, d] (llama.cpp:77-78) reserves
+// Paged cache: the reference's dense [layers, B, hk, max_seq, d] (llama.cpp:77-78) reserves
 // max_seq rows for every sequence slot; here a layer's K (V) is a pool of pages [n_pages, hk, 128 rows, d] and a
 // sequence owns the pages its page list names ([batch, max_pages] int, shared by all layers). Same kernel, same
 // split / combine, same semantics as b200_decode_attention_ragged; the only difference is the row address. fp16,

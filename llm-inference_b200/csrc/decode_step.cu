@@ -27,11 +27,11 @@ namespace b200 {
 constexpr int kStepWarps = 8;                         // consumer warps
 constexpr int kStepThreads = (kStepWarps + 1) * 32;   // + producer warp
 constexpr int kStepConsumers = kStepWarps * 32;
-// K-segment bytes per row per stage = the size of one bulk copy. 4 KB (round 2; was 2 KB): a stage is 64 KB, the ring
+// K-segment bytes per row per stage = the size of one bulk copy. 4 KB (2 KB before): a stage is 64 KB, the ring
 // 3 stages. The SM's copy engine costs ~27 ns + bytes / 124 GB/s per copy, so 2 KB copies cap an SM at 47.8 GB/s - just
 // under its fair share of HBM - and 4 KB copies at 68 GB/s; the consumers pay their ~200-cycle hand-over once per 64 KB
-// instead of once per 32 KB. Round 1 measured 4 KB copies SLOWER (HBM saturated -> uneven service -> every one of the 5
-// grid barriers per layer waits for the slowest CTA); with 2 barriers per layer the balance flips: 2.70 -> 2.53 ms.
+// instead of once per 32 KB. With five grid barriers per layer 4 KB copies were SLOWER (HBM saturated -> uneven service -> every one of the
+// barriers waits for the slowest CTA); with 2 barriers per layer the balance flips: 2.70 -> 2.53 ms.
 #ifndef B200_STEP_SEG_KB
 #define B200_STEP_SEG_KB 4
 #endif
@@ -289,7 +289,7 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 // Producer warp: issues bulk copies global -> ring stage as the consumers free slots, in program order and
 // without ever stopping at an op boundary. (An L2-prefetch cursor running ahead of the ring while the consumers
 // sit at a barrier was measured not to help - 2.88 -> 3.3 ms always on, no gain when stalled only: an SM ingests
-// 2 KB bulk copies at 47.8 GB/s from L2 exactly as from HBM, DESIGN section 4 - and is gone from the code.)
+// 2 KB bulk copies at 47.8 GB/s from L2 exactly as from HBM - and is gone from the code.)
 __device__ __noinline__ void step_producer(const StepParams& p, Ring rg, int lane) {
     unsigned char* const r_base = rg.base;
     uint64_t* const r_full = rg.full;

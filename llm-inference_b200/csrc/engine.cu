@@ -258,7 +258,7 @@ static void build_program(b200_engine* e) {
     if (c.dtype != B200_F16 || e->batch > 4) return;
     std::vector<StepOp> ops;
     const int H = e->H, L = c.num_layers;
-    // Fused FFN (gate_up + SwiGLU + K-split down in one op, DESIGN section 4): needs whole W2 rows per ring stage
+    // Fused FFN (gate_up + SwiGLU + K-split down in one op): needs whole W2 rows per ring stage
     // (H a power of two <= 16384) and the per-thread accumulators in registers (batch tile x packets per thread <= 8)
     const int nb_t = e->batch <= 1 ? 1 : e->batch <= 2 ? 2 : 4;
     const int ppt = (H / 8 + 255) / 256;
@@ -599,7 +599,7 @@ extern "C" b200_engine* b200_engine_create_paged(const b200_model_config* c, int
     cudaMemcpy(e->step_dev, &ref_step0, sizeof(int), cudaMemcpyHostToDevice);
     cudaDeviceSynchronize();
     if (!e->kv_fp8 && !e->kv_paged) build_program(e);   // the persistent step kernel reads and appends a dense fp16 cache
-    // default launch order by batch (measured, tools/order_sweep.sh + route_sweep.sh, 7B fp16, ms per step at
+    // default launch order by batch (measured, 7B fp16, ms per step at
     // context 512 / 4096; GEMV = the tensor-core consumer, gemv.cu):
     //   batch 2: persistent 3.53 / 4.72, fused GEMV graph 3.30 / 4.24, reference launch order graph 3.49 / 4.42
     //   batch 3: persistent 4.58 / 6.91, fused GEMV graph 3.69 / 4.91, reference launch order graph 3.82 / 5.03
@@ -607,7 +607,7 @@ extern "C" b200_engine* b200_engine_create_paged(const b200_model_config* c, int
     // (the persistent kernel still runs the scalar FHFMA loop, issue-bound from 2 token rows on). So batch 1 keeps the
     // persistent kernel, fp16 batches 2-4 default to the graphed fused-GEMV order; batches >= 5 run the reference
     // launch order on the tcgen05 weight-streaming GEMM whatever the FUSED flag says (enqueue_step).
-    // Round 2 (2 grid barriers per layer, K-split o / down, 4 KB copies): batch 2 persistent 3.13 / 4.37 ms vs fused GEMV
+    // With 2 grid barriers per layer, K-split o / down and 4 KB copies: batch 2 persistent 3.13 / 4.37 ms vs fused GEMV
     // graph 3.31 / 4.38; batch 3 persistent 4.01 / 6.51 vs 3.71 / 5.08 -> the persistent kernel is the default up to batch 2.
     if (c->dtype == B200_F16 && c->tp_size == 1 && batch >= 3) e->mode = B200_ENGINE_FUSED | B200_ENGINE_GRAPH;
     return e;
@@ -1023,7 +1023,7 @@ static int enqueue_step_body(b200_engine* e) {
     // sequence with the linears on the tcgen05 weight-streaming GEMM (weights are read once per
     // step instead of once per 8-token tile).
     // fp16 batches of 5..8 also take the tensor-core path: eight x-rows of K = 11008 crowd the GEMV's weight ring out
-    // of shared memory (measured at batch 8 x KV 4096: 12.0 ms per step fused vs the figure in DESIGN §4c)
+    // of shared memory (measured at batch 8 x KV 4096: 12.0 ms per step fused)
     // (the fused qkv GEMV appends fp16 rows in its epilogue: an fp8 cache takes the reference launch order)
     const bool fused = (e->mode & B200_ENGINE_FUSED) && B <= (dt == B200_F16 && !tp ? 4 : B200_GEMV_MAX_TOKENS) && !e->kv_fp8 &&
                        !e->kv_paged;
@@ -1496,7 +1496,7 @@ extern "C" int b200_engine_get_seq_steps(const b200_engine* e, int* steps_out_ho
 //   <dir>/model.layers.<l>.{input_layernorm,post_attention_layernorm}.weight.bin
 //   <dir>/model.layers.<l>.self_attn.{qkv,o_proj}.weight.bin   <dir>/model.layers.<l>.mlp.{gate_up_proj,down_proj}.weight.bin
 // qkv rows are q heads, k heads, v heads; gate_up rows gate then up (act_kernel.cu:28-29). With
-// tp_size > 1 each rank keeps its head / FFN-column shard (Megatron split, SURVEY §8e): rows of qkv and
+// tp_size > 1 each rank keeps its head / FFN-column shard (Megatron split): rows of qkv and
 // gate_up, columns of o_proj and down_proj.
 // ------------------------------------------------------------------------------------------
 namespace b200 {

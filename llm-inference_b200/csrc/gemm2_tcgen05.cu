@@ -281,7 +281,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // of both accumulators from the same A descriptors. Against the 256 x 256 tile: 24 instead of 32 KB loaded per 128 x 256 x
 // 64 MAC block (L2 -> SM and TMA smem writes -25 %), shared-memory traffic (TMA writes + MMA operand reads) 112 KB per
 // 1024 tensor clocks instead of 128 KB - the 256 x 256 kernel asks for exactly the 128 B/clk an SM's shared memory
-// delivers, which is where its 83 % tensor-pipe ceiling comes from (ncu: profiles/r02_gemm_vs_cublas_full.md; cuBLAS'
+// delivers, which is where its 83 % tensor-pipe ceiling comes from (ncu: profiles/gemm_vs_cublas_full.md; cuBLAS'
 // kernel for this shape has the same 48 KB stages x 4). Price: both accumulators fill all 512 TMEM columns, so the
 // epilogue of a tile is not hidden behind the next tile's MMAs any more; eight epilogue warps (four per accumulator)
 // keep it short, and the first K steps of the next tile's accumulator 0 are issued as soon as ITS half is drained.

@@ -1,4 +1,4 @@
-// fp8 (e4m3) KV cache for the batched long-context decode ("KV-cache layout evolution ... fp8 KV").
+// fp8 (e4m3) KV cache for the batched long-context decode.
 // The reference keeps K and V in T, [layers, B, hk, max_seq, d] (src/models/llama/llama.cpp:77-78); at cfg4
 // (32 sequences x 4096 keys) those rows are 84 % of a decode step's bytes and the split-KV attention already streams
 // them at 0.93 of the measured HBM peak - bytes are the only lever left there.

@@ -1,4 +1,4 @@
-// Paged KV cache ("KV-cache layout evolution ... paged blocks").
+// Paged KV cache: blocks of rows instead of a row per possible position.
 // The reference allocates K and V as [layers, B, hk, max_seq, d] (src/models/llama/llama.cpp:77-78): every sequence
 // slot owns max_seq rows whether it uses them or not. Here a layer's K (V) is a POOL of pages
 //     pool [n_pages, hk, B200_KV_PAGE_ROWS = 128 rows, d]

@@ -1,6 +1,6 @@
 // KV-cache data movement: ConcatKVCache, RepeatKVCache, TransposeOutRemovePadding.
 // Pure copies -> bit-exact. One thread moves one 16-byte packet; K and V are handled by the
-// same launch (blockIdx.y selects which). 64-bit indexing throughout (SURVEY D21).
+// same launch (blockIdx.y selects which). 64-bit indexing throughout.
 // Reference: src/kernels/concat_past_kv.cu:17-56,103-144; repeat_kv.cu:27-70,76-120;
 // fused_transpose_and_remv_pad.cu:18-47.
 #include "common.cuh"

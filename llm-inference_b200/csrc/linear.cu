@@ -127,7 +127,7 @@ extern "C" int b200_linear(const void* x, const void* W, const void* bias, void*
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     // fp16 with 5..8 token rows: at K = 11008 the GEMV's x-rows leave no room for its weight ring (tokens walked in two
     // halves = weights streamed twice); the tcgen05 weight-streaming GEMM reads every weight byte once, so it takes
-    // these shapes. Up to 4 rows the GEMV (tensor-core consumer from 2 rows on) is as fast or faster (route_sweep.sh).
+    // these shapes. Up to 4 rows the GEMV (tensor-core consumer from 2 rows on) is as fast or faster.
     if (trans_b && dtype == B200_F16 && n_tokens >= b200::gemm_min_tokens() && n_tokens <= B200_GEMV_MAX_TOKENS) {
         int rc = gemm_tcgen05_f16(x, W, bias, y, n_tokens, N, K, s);
         if (rc != B200_EUNSUPPORTED) return rc;

@@ -1,6 +1,6 @@
 // RMSNorm family: b200_rmsnorm, b200_fused_add_bias_residual_rmsnorm, b200_add_residual.
 // Reference math: src/kernels/rmsnorm_kernel.cu:63-115, fused_addresidual_norm.cu:62-128,
-// add_residual.cu:9-31 (with SURVEY defects D7-D10 resolved: residual is really saved, the
+// add_residual.cu:9-31 (where those are wrong, this is not: residual is really saved, the
 // block reduce is a correct two-stage reduce, <=1024 threads, half adds out += residual).
 //
 // Layout: one CTA per token row; each thread keeps up to kCache 16-byte packets of the row in

@@ -1,4 +1,4 @@
-// One-shot NVLink allreduce fused with the residual add, for tensor-parallel decode (SURVEY §8e):
+// One-shot NVLink allreduce fused with the residual add, for tensor-parallel decode:
 // after the row-parallel o_proj / down_proj every rank holds a partial [B, H]; the reference has no
 // multi-GPU path, the baseline is ncclAllReduce + launchAddResidual (add_residual.cu:58). Messages
 // are 16 KB (B=1, 70B) .. 512 KB (B=32): latency-bound. Every rank PUSHES its partial straight into a
@@ -11,7 +11,7 @@
 // current call, so there is no separate flag, no system-scope fence and no barrier on the critical
 // path: a line is valid as soon as it is visible. (First version, measured on 2 x B200: payload
 // stores + __threadfence_system + release flag + acquire spin = 11.3 us per 16 KB call, no better
-// than NCCL's 11.8 us; profiles/r01_allreduce_bench_n2.json.)
+// than NCCL's 11.8 us.)
 //
 // Layout of a rank's IPC allocation: [header: call counter, ticket][receive buffer 0: world slots]
 // [receive buffer 1: world slots]; a slot holds 2 x max_message_bytes of lines. The two receive

@@ -1,7 +1,7 @@
 // Rotate-half RoPE: decode (in place on the newest token) and prefill
 // (bias + RoPE + un-pad/transposition into q/k/v buffers).
 // Reference math: src/kernels/qkv_bias_and_RoPE.cu:29-46 (freq + rotation), :323-380 (decode),
-// :50-145 (prefill; SURVEY defects D5, D6, D12 resolved: token-major qkv with stride
+// :50-145 (prefill; where the reference is wrong, this is not: token-major qkv with stride
 // (h+2hk)*d, v is copied, timestep = history_len[b] + local token id).
 //   theta_i = pos / base^(2i/rot_dim), i < rot_dim/2; pair (i, i + head_size/2)
 //   (x_i, x_j) <- (x_i cos - x_j sin, x_j cos + x_i sin)

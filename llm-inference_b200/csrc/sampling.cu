@@ -1,6 +1,6 @@
-// Ops bracketing a decode step (SURVEY §8f rank 1): embedding gather, greedy argmax, top-K.
+// Ops bracketing a decode step: embedding gather, greedy argmax, top-K.
 // Reference: src/kernels/input_embedding.cu:5-44; src/kernels/topK.cu:25-190 + topK.h:7-47
-// (two-pass cub::BlockReduce top-K with K=5; greedy = final_topk_id[b,0], SURVEY D22).
+// (two-pass cub::BlockReduce top-K with K=5; greedy = final_topk_id[b,0]).
 // Index outputs are exact: larger value wins, equal values -> lower index wins.
 #include "common.cuh"
 #include "launch_count.h"

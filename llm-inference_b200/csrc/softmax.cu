@@ -1,7 +1,7 @@
 // Prefill scale-mask-softmax over the last axis:
 //   s = scale*qk + (1-mask)*(-10000);  p = exp(s - max(s)) / (sum + 1e-6)
 // Reference: src/kernels/attn_softmax_kernel.cu:80-173 (fp32), :179-290 (half), :337-372.
-// Deviations (SURVEY D8, D16): correct two-stage block reduce, running max starts at -inf, no
+// Deviations: correct two-stage block reduce, running max starts at -inf, no
 // K < 4096 limit. The additive -10000 mask and the +1e-6 denominator are kept.
 // One CTA per (b, head, q) row; the row lives in registers between the three passes, so qk and
 // mask are read once and the score written once. May run in place (qk == score).

@@ -13,8 +13,8 @@
 
 namespace b200shim {
 
-// The reference launches everything on the legacy default stream (no <<<.., stream>>> anywhere,
-// SURVEY §0); that stays the default. A host application that owns a stream sets it once.
+// The reference launches everything on the legacy default stream (no <<<.., stream>>> anywhere);
+// that stays the default. A host application that owns a stream sets it once.
 inline cudaStream_t& current_stream() {
     static thread_local cudaStream_t s = nullptr;
     return s;

@@ -5,7 +5,7 @@
 #include "src/weights/llama/norm_weights.h"
 
 // decoder_out [num_tokens, hidden] normalised in place; decoder_residual receives the pre-norm
-// input (the intent of the reference header; D7 in SURVEY §2.3). is_last is accepted and unused,
+// input (the intent of the reference header). is_last is accepted and unused,
 // as in the reference.
 template <typename T>
 void launchRMSNorm(TensorWrapper<T>* decoder_out, TensorWrapper<T>* decoder_residual,

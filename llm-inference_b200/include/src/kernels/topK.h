@@ -4,7 +4,7 @@
 #include "src/kernels/b200_shim.h"
 
 // probs [bs*beam, vocab]; final_topk_ids / final_topk_values [bs*beam, K] with K = last dim
-// (<= 8). topk_ids / topK_values (the reference's round-1 scratch) are accepted and unused.
+// (<= 8). topk_ids / topK_values (the scratch of the reference's first pass) are accepted and unused.
 template <typename T>
 void launchTopKforBeamSearch(TensorWrapper<T>* probs, TensorWrapper<int>* topk_ids, TensorWrapper<T>* topK_values,
                              TensorWrapper<int>* final_topk_ids, TensorWrapper<T>* final_topk_values) {

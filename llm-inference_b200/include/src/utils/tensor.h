@@ -1,7 +1,7 @@
 // Tensor carriers at the kernel boundary: Device / DataType enums, Tensor, TensorWrapper<T>,
 // TensorMap. Source-compatible with the reference's src/utils/tensor.h:13-304 (same names, same
 // member layout, same checks), re-written; size64() is added because Tensor::size() is int
-// (the batch-32 x 4096 KV cache has 1.7e10 elements, SURVEY §8 a15).
+// (the batch-32 x 4096 KV cache has 1.7e10 elements).
 #pragma once
 #include <cuda_fp16.h>
 #include <cstdint>

@@ -1,6 +1,6 @@
 // LlamaLayerWeight<T>: one decoder layer's weights (reference src/weights/llama/layer_weights.h:9-43,
-// layer_weights.cc:18-177). Differences, all listed in SURVEY §2.3: down is allocated H*I elements
-// (D19), sizes are exact (D20); everything lives in ONE 256-byte-aligned device arena per layer
+// layer_weights.cc:18-177). Differences: down is allocated H*I elements,
+// sizes are exact; everything lives in ONE 256-byte-aligned device arena per layer
 // so the GEMV's bulk copies and the GEMM's TMA maps see naturally aligned row-major [N,K] tiles.
 // The on-disk format is the reference's: raw little-endian fp32 .bin per tensor named
 // model.layers.<i>.{input_layernorm,post_attention_layernorm}.weight.bin,

@@ -1,4 +1,4 @@
-"""Host-side sharding rules of the decode path across GPUs (SURVEY §8e; the reference itself is
+"""Host-side sharding rules of the decode path across GPUs (the reference itself is
 single-GPU, src/models/llama/llama.cpp has no communicator).
 
 Two ways, one process per GPU in both:

@@ -5,7 +5,7 @@
  * only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs do.
  *
  * Each function follows the reference CUDA kernel (file:line cited, paths relative to the
- * reference repo root) with the SURVEY.md §2.3 defects D1-D22 resolved as listed there.
+ * reference repo root), except where that kernel is wrong (the comment at the function says how).
  * Data are fp32 arrays (fp16 inputs are widened exactly by the caller); sums are accumulated
  * in double so the oracle is at least as accurate as either implementation it arbitrates.
  * Pinned against the reference's own unit-test CPU functions and golden vectors by

@@ -18,7 +18,7 @@ class OracleModel:
     def __init__(self, weights, cfg, batch, max_seq_len, kind, allreduce=None):
         """weights: dict with 'layers' (list of dicts attn_norm,qkv,o,ffn_norm,gate_up,down),
         'embed','final_norm','lm_head' — float32 arrays holding the (already rounded) values.
-        Tensor parallel (SURVEY 8e): cfg holds this rank's head counts / FFN columns plus
+        Tensor parallel: cfg holds this rank's head counts / FFN columns plus
         'hidden_size' (the unsplit H), weights are this rank's shard, and `allreduce(a)` sums a
         [n,H] partial result in place over the ranks after o_proj and after down_proj."""
         self.w, self.cfg, self.B, self.kind = weights, cfg, batch, kind

@@ -8,7 +8,7 @@
 //   ref_cpu_*  the CPU reference functions that live inside tests/unittests/*.cu, reached by
 //              including each test file inside its own namespace with `main` renamed;
 //   ref_gpu_*  the reference's CUDA launchers (src/kernels/*.cu), a live GPU oracle for the
-//              kernels that are not defective at the tested shape (SURVEY.md §8c).
+//              kernels that are not defective at the tested shape.
 // System / reference headers are included first, outside any namespace, so the includes inside
 // the test files are no-ops by the time they are seen in a namespace.
 #include <algorithm>

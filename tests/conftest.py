@@ -35,7 +35,7 @@ def pkg():
     return load_package()
 
 
-# Tolerances stated by BASELINE.json north_star: rel err <= 1e-5 (fp32), <= 2e-2 (fp16), where
+# Tolerances: rel err <= 1e-5 (fp32), <= 2e-2 (fp16), where
 # rel err = max|got - want| / max(|want|)  (normalised max-error; element-wise relative error is
 # meaningless next to zero crossings). Bit-exact ops use np.array_equal instead.
 RTOL = {"fp32": 1e-5, "fp16": 2e-2}

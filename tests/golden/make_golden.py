@@ -4,7 +4,7 @@ run on the reference tests' own input data. Run in the build container only:
 
     python tests/golden/make_golden.py
 
-The fixture pins the oracle (tests/test_oracle_golden.py) wherever /root/reference is absent.
+The fixture pins the oracle (tests/test_oracle_golden.py) wherever the reference is absent.
 """
 import ctypes as C
 import os

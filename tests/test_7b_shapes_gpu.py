@@ -1,4 +1,4 @@
-"""Parity at the BENCHMARKED shapes (VERDICT r1 item 1): the kernels that produce the bench lines —
+"""Parity at the BENCHMARKED shapes: the kernels that produce the bench lines —
 `decode_step_kernel<1,1>` (cfg2), the fused-GEMV graph order and the reference launch order; the
 batched tcgen05 decode path (cfg4) and the prompt pass (cfg3) — on LLaMA-2-7B geometry
 (H 4096, 32/32 heads, d 128, I 11008, V 32000), teacher-forced against the CPU oracle
@@ -86,7 +86,7 @@ def slice_weights(pkg):
 
 @pytest.mark.parametrize("mode", ["persistent", "fused_graph", "unfused"])
 def test_cfg2_7b_slice_batch1_ctx512(pkg, slice_weights, mode):
-    """configs[1] geometry, 4 of the 32 layers: batch 1 from a 512-token cache (4 split-KV chunks per
+    """cfg2 geometry, 4 of the 32 layers: batch 1 from a 512-token cache (4 split-KV chunks per
     head in the persistent kernel), 4 steps, every decode mode."""
     E = pkg.engine
     cfg = dict(num_layers=4, **L7B)
@@ -105,7 +105,7 @@ def test_cfg2_7b_slice_batch1_ctx512(pkg, slice_weights, mode):
 
 @pytest.mark.slow
 def test_cfg2_7b_full_32_layers_persistent(pkg):
-    """configs[1] itself: all 32 layers, batch 1, 512-token cache, the default engine mode (the
+    """cfg2 itself: all 32 layers, batch 1, 512-token cache, the default engine mode (the
     persistent whole-step kernel, 162 ops, ONE launch per token) - 8 teacher-forced steps."""
     if _host_gb() < 48:
         pytest.skip(f"the oracle's fp32 copy of the 7B weights needs ~30 GB of host memory ({_host_gb():.0f} GB free)")
@@ -124,7 +124,7 @@ def test_cfg2_7b_full_32_layers_persistent(pkg):
 
 
 def test_cfg4_7b_batch32_ctx4096(pkg):
-    """configs[3] geometry on 2 layers: 32 sequences x 4096 cached keys, the default batched path
+    """cfg4 geometry on 2 layers: 32 sequences x 4096 cached keys, the default batched path
     (tcgen05 weight-streaming linears + split-KV attention under one CUDA graph), 2 steps."""
     if _host_gb() < 24:
         pytest.skip("needs ~16 GB of host memory for the oracle's fp32 caches")
@@ -141,7 +141,7 @@ def test_cfg4_7b_batch32_ctx4096(pkg):
 
 
 def test_cfg3_7b_prefill_4x2048(pkg, monkeypatch):
-    """configs[2] geometry on 2 layers: 4 x 2048 prompt tokens through b200_engine_prefill (two-CTA
+    """cfg3 geometry on 2 layers: 4 x 2048 prompt tokens through b200_engine_prefill (two-CTA
     tcgen05 GEMMs, SwiGLU / residual epilogues, flash context attention) against the ORACLE prefill
     loop - not against this repo's own unfused GPU sequence."""
     if _host_gb() < 24:

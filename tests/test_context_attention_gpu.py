@@ -1,7 +1,7 @@
 """b200_context_attention (csrc/context_attention.cu: tcgen05 S = QK^T into TMEM, fp32 online softmax,
 P V with V as an MN-major operand) against the CPU oracle's reference-order sequence
 (context_attention.cpp:136-161: RepeatKV -> QK^T -> scale+mask+softmax -> PV -> transpose / remove
-padding) on the same seeded inputs, fp16, rel err <= 2e-2 (north_star); at the cfg3 size
+padding) on the same seeded inputs, fp16, rel err <= 2e-2; at the cfg3 size
 (4 x 2048 tokens, 32 heads) against the unfused GPU sequence of the same library, which the oracle
 pins at small sizes (test_parity_gpu.py)."""
 import numpy as np
@@ -97,7 +97,7 @@ def test_context_attention_rejects_unsupported(ops):
 
 
 def test_context_attention_cfg3_vs_unfused_gpu_sequence(ops):
-    """BASELINE cfg3 geometry for one layer (B 4 x S 2048, 32 heads): the flash kernel against the
+    """cfg3 geometry for one layer (B 4 x S 2048, 32 heads): the flash kernel against the
     library's own reference-order sequence (materialised scores), and the all-ones-V property:
     softmax rows sum to l / (l + 1e-6), so with V = 1 every output element is 1 within fp16 rounding."""
     B, h, hk, S, d = 4, 32, 32, 2048, 128

@@ -24,7 +24,7 @@ def capi(pkg):
 
 def test_decode_attention_reference_test_data(ops):
     """tests/unittests/test_fused_decoder_attention.cu:269-349: B=1, h=hk=2, d=4, max_seq=4, step=4,
-    ramp data (v taken from its declared slot in qkv, SURVEY §4 note on the test's h_v offset)."""
+    ramp data (v taken from its declared slot in qkv: the reference test's own h_v offset is not it)."""
     B, h, hk, d, max_seq, step = 1, 2, 2, 4, 4, 4
     n = B * (h + 2 * hk) * d
     qkv = np.zeros(n, np.float32)

@@ -1,7 +1,7 @@
 """GPU parity of the decode-step driver (include/b200_engine.h) against the CPU oracle of the
 whole decoder stack (oracle/model.py), in all three execution modes: fused + CUDA graph (the
 product path), fused without graph, and the unfused reference launch sequence.
-Covers BASELINE.json configs[0] (one LLaMA-2-7B-shaped fp32 layer, batch 1, 64-token cache) and a
+Covers one layer (LLaMA-2-7B-shaped fp32 layer, batch 1, 64-token cache) and a
 teacher-forced greedy token-ID check on a small LLaMA-shaped model."""
 import numpy as np
 import pytest
@@ -104,7 +104,7 @@ def test_modes_agree_and_graph_replays(pkg):
 
 
 def test_config0_single_7b_layer_fp32(pkg):
-    """BASELINE.json configs[0]: one LLaMA-2-7B-shaped decoder layer (hidden 4096, 32 heads,
+    """one LLaMA-2-7B-shaped decoder layer (hidden 4096, 32 heads,
     head_dim 128), fp32 random weights, batch 1, one decode step on a 64-token KV cache, checked
     against the CPU oracle at rel err <= 1e-5."""
     E = pkg.engine
@@ -243,7 +243,7 @@ def test_persistent_step_kernel_exchange_form_single_rank(pkg, B, ctx):
 
 def test_persistent_step_kernel_70b_geometry(pkg):
     """hidden 8192 (four 16-byte packets per thread in the K-split consumer), 64 q / 8 kv heads (groups of 8): the
-    geometry of BASELINE configs[4], two layers with a narrow FFN, plain and exchange form, vs the oracle."""
+    LLaMA-2-70B geometry, two layers with a narrow FFN, plain and exchange form, vs the oracle."""
     import ctypes as C
     E = pkg.engine
     lib = E._lib()

@@ -1,4 +1,4 @@
-"""fp8 (e4m3) KV cache (SURVEY section 8 f4; csrc/kv_fp8.cu, b200_decode_attention_fp8, B200_ENGINE_KV_FP8).
+"""fp8 (e4m3) KV cache (csrc/kv_fp8.cu, b200_decode_attention_fp8, B200_ENGINE_KV_FP8).
 
 The fp8 cache is an engine option, not bit-compatible with the reference's T-typed cache (llama.cpp:77-78), so its
 contract is stated here: a K / V row is rounded ONCE, when it enters the cache (scale = amax(row) / 448, e4m3 round to
@@ -166,7 +166,7 @@ def test_engine_fp8_prefill_then_decode_vs_oracle(pkg, B, n):
 
 
 def test_cfg4_shape_fp8_cache(pkg):
-    """configs[3] geometry (7B heads, 32 sequences x 4096 cached keys, 2 layers) with the fp8 cache: two teacher-forced
+    """cfg4 geometry (7B heads, 32 sequences x 4096 cached keys, 2 layers) with the fp8 cache: two teacher-forced
     steps against the oracle on the dequantised rows; the cache is half the bytes (+ 4 B per row of scales)."""
     E = pkg.engine
     L7B = dict(head_num=32, kv_head_num=32, head_size=128, inter_size=11008, vocab_size=32000)

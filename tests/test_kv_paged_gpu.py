@@ -1,4 +1,4 @@
-"""Paged KV cache (SURVEY section 8 f4 "paged blocks"; csrc/kv_paged.cu, b200_decode_attention_paged,
+"""Paged KV cache (csrc/kv_paged.cu, b200_decode_attention_paged,
 B200_ENGINE_KV_PAGED).
 
 The reference's cache is dense, [layers, B, hk, max_seq, d] (llama.cpp:77-78): max_seq rows reserved per sequence slot.
@@ -221,7 +221,7 @@ def test_retired_sequences_return_their_pages(pkg):
 
 
 def test_cfg4_shape_paged_equals_dense(pkg):
-    """configs[3] geometry (7B heads, 32 sequences x 4096 cached keys, 2 layers): the same synthetic rows in both caches,
+    """cfg4 geometry (7B heads, 32 sequences x 4096 cached keys, 2 layers): the same synthetic rows in both caches,
     three decode steps (the second one opens page 33 of every sequence), logits bit-identical; the dense engine at this
     shape is pinned to the oracle by tests/test_7b_shapes_gpu.py"""
     E = pkg.engine

@@ -2,7 +2,7 @@
  * against tests/golden/ref_cpu_golden.npz — outputs of the reference's own unit-test CPU
    functions on the reference tests' own data (generated by tests/golden/make_golden.py), and the
    golden vector written in tests/unittests/test_cal_paddingoffset.cu:54-56;
- * against closed forms the reference tests imply (SURVEY.md §8c).
+ * against closed forms the reference tests imply.
 Runs on CPU (no `gpu` marker)."""
 import os
 
@@ -107,7 +107,7 @@ def test_causal_mask_reference_vectors():
     cpu.build_causal_mask(mask, np.array([5], np.int32), np.array([5], np.int32), True)
     assert np.array_equal(mask, G["mask_5x5"])
     assert np.array_equal(mask[0], np.tril(np.ones((5, 5), np.float32)))
-    # the GPU kernel's extra clause agrees when klen == qlen (SURVEY D17)
+    # the GPU kernel's extra clause agrees when klen == qlen
     m2 = np.zeros((1, 5, 5), np.float32)
     cpu.build_causal_mask(m2, np.array([5], np.int32), np.array([5], np.int32), False)
     assert np.array_equal(m2, mask)

@@ -1,7 +1,7 @@
 """GPU parity: every C-ABI op (through ctypes -> libb200llama.so) against the CPU oracle on the
 same seeded inputs. Shapes: the reference unit tests' own (tests/unittests/*.cu) plus
 LLaMA-2-7B / 70B shaped cases and ragged / empty edge cases.
-Tolerance (north_star): normalised max error <= 1e-5 fp32, <= 2e-2 fp16; copies, masks, padding
+Tolerance: normalised max error <= 1e-5 fp32, <= 2e-2 fp16; copies, masks, padding
 offsets and top-K indices are bit-exact."""
 import numpy as np
 import pytest
@@ -131,7 +131,7 @@ def test_rope_decode(ops, kind, b, h, hk, d, step, rot):
     cpu.rope_decode(want, h, hk, step, rot, 10000.0)
     dq = dev(qkv, kind)
     ops.launchRoPE(dq, step, rot, 10000.0, kv_head_num=hk)
-    # cos/sin of large angles differ by a few ulp between libm and CUDA: tolerance per north_star
+    # cos/sin of large angles differ by a few ulp between libm and CUDA: the same tolerance
     assert_close(host(dq), want, "fp16" if kind == "fp16" else "fp32", "rope decode")
     assert np.array_equal(host(dq)[:, h + hk:], qkv[:, h + hk:]), "v heads untouched"
 

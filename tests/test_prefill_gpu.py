@@ -3,7 +3,7 @@ LlamaContextDecoder layers -> final norm -> LM head on the last token -> top-1) 
 oracle's prefill loop (oracle/model.py prefill_layers = context_decoder.cpp:48-140), then decode
 steps continuing from the prefilled cache against the oracle's decode loop. fp16 runs the tcgen05
 GEMMs + the flash context attention; fp32 the reference-order GPU sequence. Tolerances: rel 1e-5
-fp32 / 2e-2 fp16 (north_star); cache rows beyond the prompt stay bit-exact (untouched)."""
+fp32 / 2e-2 fp16; cache rows beyond the prompt stay bit-exact (untouched)."""
 import numpy as np
 import pytest
 

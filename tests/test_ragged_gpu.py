@@ -1,10 +1,10 @@
-"""Ragged batches: one `step` per sequence instead of the reference's single host scalar (llama.h; SURVEY 8f-2).
+"""Ragged batches: one `step` per sequence instead of the reference's single host scalar (llama.h).
 The oracle has no ragged decode of its own, and needs none: sequences of a batch share nothing but the weights, so
 the expected result of sequence b in a ragged batch is the oracle's result for that sequence run ALONE (batch 1).
   * b200_rope_decode_ragged / b200_decode_attention_ragged against oracle rope_decode / decode_attention per sequence;
   * b200_engine_prefill_ragged (+ a second ragged round on top of ragged histories) and the decode steps that follow
     against per-sequence OracleModels: logits, the written cache rows, untouched rows bit-exact zero.
-Tolerances: rel 1e-5 fp32 / 2e-2 fp16 (north_star)."""
+Tolerances: rel 1e-5 fp32 / 2e-2 fp16."""
 import numpy as np
 import pytest
 import torch

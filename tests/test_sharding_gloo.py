@@ -1,4 +1,4 @@
-"""N>1 host logic on CPU, two `gloo` ranks (SURVEY §8e):
+"""N>1 host logic on CPU, two `gloo` ranks:
   * request sharding (independent sequences, no collective) and the max-over-ranks step time the
     bench reports;
   * tensor parallel: every rank runs the CPU oracle on ITS shard of the weights

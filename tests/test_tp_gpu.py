@@ -1,5 +1,5 @@
 """Tensor-parallel decode through the engine's allreduce hook (include/b200_engine.h:
-b200_engine_set_allreduce), two ranks, against the UNSHARDED CPU oracle (SURVEY §8e).
+b200_engine_set_allreduce), two ranks, against the UNSHARDED CPU oracle.
 Each rank owns head_num/2 query heads, kv_head_num/2 kv heads and inter_size/2 FFN columns
 (sharding.tp_shard_layer); the hook sums the partial [B,H] after o_proj and after down_proj.
 With >= 2 GPUs the ranks sit on different devices and the sum is an NCCL allreduce enqueued on the
@@ -154,7 +154,7 @@ def _p2p_unit_worker(rank, world, port, out_dir):
 
 def test_p2p_oneshot_allreduce_two_gpus(tmp_path):
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs two GPUs with peer access (verified with gpurun --gpus 2, profiles/r01_tp2_*.json)")
+        pytest.skip("needs two GPUs with peer access")
     import torch.multiprocessing as mp
     world = 2
     mp.spawn(_p2p_unit_worker, args=(world, free_port(), str(tmp_path)), nprocs=world, join=True)

@@ -1,9 +1,9 @@
 """GPU parity against the REFERENCE'S OWN CUDA kernels (oracle/_ref/libref.so = src/kernels/*.cu
-compiled for sm_100a from where they lie under /root/reference, `make -C oracle ref`), on the
-kernels that are sound at the tested shape (SURVEY §8c): RMSNorm output, SwiGLU fp32, AddResidual
-fp32, fused add+norm with one warp per row (D8), ConcatKV, RepeatKV, transpose-remove-pad,
-padding offset, causal mask at klen==qlen (D17), cuBLAS fp32 linear, decode RoPE fp32 at B=1 (D5),
-scale-mask-softmax with S_k <= 32 (D8). Copies / masks / offsets bit-exact, floats rel <= 1e-5."""
+compiled for sm_100a from where they lie, `make -C oracle ref`), on the
+kernels that are sound at the tested shape: RMSNorm output, SwiGLU fp32, AddResidual
+fp32, fused add+norm with one warp per row, ConcatKV, RepeatKV, transpose-remove-pad,
+padding offset, causal mask at klen==qlen, cuBLAS fp32 linear, decode RoPE fp32 at B=1,
+scale-mask-softmax with S_k <= 32. Copies / masks / offsets bit-exact, floats rel <= 1e-5."""
 import ctypes as C
 import os
 

@@ -1,4 +1,4 @@
-"""Per-shape timing of the weight-streaming GEMV (development aid; run under gpurun).
+"""Per-shape timing of the weight-streaming GEMV (development aid).
 Cycles through enough distinct weight buffers that nothing is served from L2."""
 import json
 import os

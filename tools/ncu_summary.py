@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""Summarise ncu outputs brought back in gpurun_out/ into small tracked files under profiles/.
+"""Summarise ncu outputs into small tracked files under profiles/.
 
-  python tools/ncu_summary.py launches gpurun_out/launches.csv profiles/r01_launches.md
-  python tools/ncu_summary.py full gpurun_out/prof_gemv.ncu-rep profiles/r01_gemv_full.md
+  python tools/ncu_summary.py launches launches.csv profiles/launches.md
+  python tools/ncu_summary.py full prof_gemv.ncu-rep profiles/gemv_full.md
 """
 import collections
 import csv
