@@ -10,10 +10,10 @@
 //   warp 0      TMA: chunks of 64 rows x 64 dimensions out of their page
 //   warp 1      tcgen05.mma, scores of tile j + 1 ahead of the weighted sum of tile j
 //   warps 2-5   the query rows (rounded to bfloat16, as in the mma.sync kernel), then the softmax, a thread per row, as in paged_attention_tc.cu
-// The weights go back over their scores as bfloat16; the sums are rescaled only when a row's maximum has grown by more than 2^8. A window of
+// The weights go back over their scores as the sum of two bfloat16; the sums are rescaled only when a row's maximum has grown by more than 2^8. A window of
 // packed tokens that holds several sequences is walked tile by tile (two CTAs share it when there is more than one entry).
-// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, this 160 us (183 with
-// the query rows loaded a chunk at a time and the results stored from registers). A tile per CTA takes half of that: what is left is mostly the query's way in.
+// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, this 179 us (160 with
+// weights rounded to bfloat16 alone, and 183 then with the query rows loaded a chunk at a time and the results stored from registers). A tile per CTA takes half of that: what is left is mostly the query's way in.
 #include <cuda_bf16.h>
 
 #include "b200_serve.h"
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
                 if (leader) {
                     const uint64_t vd = vm_desc + (uint64_t)(s * (kLtV * kLtChunk >> 4));
 #pragma unroll
-                    for (int ks = 0; ks < kLtKeys / kUmmaK; ++ks)
-                        umma_f16_ts(o_tmem, s_tmem + s * kLtKeys + (uint32_t)(ks * 8), vd + (uint64_t)(ks * (2048 >> 4)), idesc_o, j > 0 || ks > 0 ? 1u : 0u);
+                    for (int ks = 0; ks < 2 * kLtKeys / kUmmaK; ++ks)   // hi, then lo
+                        umma_f16_ts(o_tmem, s_tmem + s * kLtKeys + (uint32_t)(ks * 8), vd + (uint64_t)((ks & 3) * (2048 >> 4)), idesc_o, j > 0 || ks > 0 ? 1u : 0u);
                     umma_commit(&v_empty[s]);
                     umma_commit(&o_done[s]);
                 }
@@ -302,21 +302,21 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
                 const float ms = -m * sl;
                 const uint64_t sl2 = pack2f(sl, sl), nm2 = pack2f(ms, ms);
                 uint64_t rs2[2] = {0ull, 0ull};
-                uint32_t pk[32];
+                uint32_t pk[32], pl[32];
 #pragma unroll
                 for (int e = 0; e < 64; e += 2) {
                     float a0, a1;
                     unpack2(fma2(pack2(sv[e], sv[e + 1]), sl2, nm2), a0, a1);
                     a0 = ex2_approx(a0);
                     a1 = ex2_approx(a1);
-                    const __nv_bfloat162 b = __floats2bfloat162_rn(a0, a1);
-                    pk[e / 2] = *reinterpret_cast<const uint32_t*>(&b);
-                    rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2(pk[e / 2] << 16, pk[e / 2] & 0xffff0000u));   // the weights as they are used
+                    split_bf16x2(a0, a1, pk[e / 2], pl[e / 2]);
+                    rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2f(a0, a1));
                 }
                 float r0, r1;
                 unpack2(add2(rs2[0], rs2[1]), r0, r1);
                 l += r0 + r1;
                 tmem_st_32x32(st, pk);
+                tmem_st_32x32(st + 32u, pl);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();

@@ -4,7 +4,8 @@
 // operands count) and the special-function unit 512 for the exponentials; one tile alone is a chain of both, so two CTAs share an
 // SM (96 KB of shared memory and 256 TMEM columns each) and fill each other's gaps. A step of 64 keys takes about 1200 clocks with two
 // CTAs on an SM; the longest row tile of a prompt and what comes before its first and after its last step decide.
-// Measured (before: the mma.sync tiles of paged_attention_tile.cuh), 16 / 8 heads x 128, 2048 tokens: 114 -> 33 us. Tried and taken back: 128 keys
+// Measured (before: the mma.sync tiles of paged_attention_tile.cuh), 16 / 8 heads x 128, 2048 tokens: 114 -> 36 us (32 with
+// weights rounded to bfloat16 alone). Tried and taken back: 128 keys
 // per tile with one score buffer (52 us: products and softmax take turns), two threads per row (43 us), the keys of a tile shared by a
 // cluster of two (41 us: the fixed part of a CTA counts more than the chain).
 //   rows        TQ tokens x the R query heads of one key head (TQ = 128 / R), so a key tile is read once for the whole group and a
@@ -13,9 +14,12 @@
 //               Sequences that bring a single token are left to the cluster kernel of paged_decode.cu.
 //   warp 0      TMA: K and V tiles of 64 rows out of their page (one list lookup per tile), two stages each
 //   warp 1      tcgen05.mma: S_{j+1} = Q K^T is issued before O += P_j V_j, so the tensor pipe works under the softmax
-//   warps 2-5   softmax, a thread per row: scores are read from TMEM once, P_j goes back over its own scores as bfloat16 and is the A operand
-//               of the second product. O stays in TMEM: it is rescaled only when a row's maximum has grown by more than 2^8 since the
-//               last rescaling (weights up to 256, sums in fp32, the final division makes them exact again).
+//   warps 2-5   softmax, a thread per row: scores are read from TMEM once, P_j goes back over its own scores and is the A operand of the second
+//               product. O stays in TMEM: it is rescaled only when a row's maximum has grown by more than 2^8 since the last rescaling
+//               (weights up to 256, sums in fp32). A row's largest weight is then any number instead of 1, so a weight rounded to
+//               bfloat16 alone would cost more precision than against the running maximum (2.07e-3 of the result's norm, 2.03e-3
+//               there): P_j is the sum of two bfloat16, hi + lo, in the 64 columns of its scores, and both are multiplied (1.61e-3, the
+//               rounding of the outputs).
 // Rows of a page beyond the context may hold anything, so the V rows of the last tile are cleared before they are multiplied by zero weights.
 #include <cuda_bf16.h>
 
@@ -220,8 +224,8 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                     const uint64_t vd = v_desc + (uint64_t)(s * (L::kV >> 4));
                     const uint32_t pa = tmem + s * kTcKeys;
 #pragma unroll
-                    for (int ks = 0; ks < kTcKeys / kUmmaK; ++ks)
-                        umma_f16_ts(o_tmem, pa + (uint32_t)(ks * 8), vd + (uint64_t)(ks * (2048 >> 4)), idesc_o, ks > 0 || j > 0 ? 1u : 0u);
+                    for (int ks = 0; ks < 2 * kTcKeys / kUmmaK; ++ks)   // hi, then lo
+                        umma_f16_ts(o_tmem, pa + (uint32_t)(ks * 8), vd + (uint64_t)((ks & 3) * (2048 >> 4)), idesc_o, ks > 0 || j > 0 ? 1u : 0u);
                     umma_commit(&v_empty[s]);
                     umma_commit(&o_done[s]);
                 }
@@ -318,11 +322,11 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                         for (int e = 0; e < 64; ++e) sv[e] = e >= lo ? sv[e] : 0xff800000u;
                     }
                 }
-                uint32_t pk[32];
+                uint32_t pk[32], pl[32];
                 if (FORM == kTcSigmoid) {   // weights that are not normalised over the keys
 #pragma unroll
                     for (int e = 0; e < 64; e += 2)
-                        pk[e / 2] = pa_pack(__fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e), sl, hb2))), __fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e + 1), sl, hb2))));
+                        split_bf16x2(__fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e), sl, hb2))), __fdividef(1.f, 1.f + ex2_approx(-fmaf(S(e + 1), sl, hb2))), pk[e / 2], pl[e / 2]);
                 } else {
                     float mx[4] = {-1e30f, -1e30f, -1e30f, -1e30f};
 #pragma unroll
@@ -354,14 +358,15 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                         unpack2(FORM == kTcPlain ? fma2(pack2(sv[e], sv[e + 1]), sl2, nm2) : add2(pack2(sv[e], sv[e + 1]), nm2), a0, a1);
                         a0 = ex2_approx(a0);
                         a1 = ex2_approx(a1);
-                        pk[e / 2] = pa_pack(a0, a1);
-                        rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2(pk[e / 2] << 16, pk[e / 2] & 0xffff0000u));   // the weights as they are used: they add up to 1
+                        split_bf16x2(a0, a1, pk[e / 2], pl[e / 2]);
+                        rs2[(e / 2) & 1] = add2(rs2[(e / 2) & 1], pack2f(a0, a1));
                     }
                     float r0, r1;
                     unpack2(add2(rs2[0], rs2[1]), r0, r1);
                     l += r0 + r1;
                 }
                 tmem_st_32x32(st, pk);
+                tmem_st_32x32(st + 32u, pl);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();

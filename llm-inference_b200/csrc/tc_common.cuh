@@ -1,6 +1,8 @@
 // tcgen05 / TMEM / TMA PTX wrappers and descriptor builders shared by the tensor-core kernels
 // (gemm_tcgen05.cu, context_attention.cu). sm_100a only.
 #pragma once
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -242,6 +244,15 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
+}
+// two fp32 numbers as the sums of two bfloat16, hi + lo: hi is cut off (which takes no conversion), the difference is exact, lo is rounded, so each
+// sum is off by at most 2^-16 of its number, 2^-18 on average
+__device__ __forceinline__ void split_bf16x2(float a0, float a1, uint32_t& hi, uint32_t& lo) {
+    hi = __byte_perm(__float_as_uint(a0), __float_as_uint(a1), 0x7632);
+    float r0, r1;
+    unpack2(fma2(pack2(__float_as_uint(a0) & 0xffff0000u, __float_as_uint(a1) & 0xffff0000u), pack2f(-1.f, -1.f), pack2f(a0, a1)), r0, r1);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(r0, r1);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
