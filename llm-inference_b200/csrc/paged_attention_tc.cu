@@ -20,7 +20,8 @@
 //               bfloat16 alone would cost more precision than against the running maximum (2.07e-3 of the result's norm, 2.03e-3
 //               there): P_j is the sum of two bfloat16, hi + lo, in the 64 columns of its scores, and both are multiplied (1.61e-3, the
 //               rounding of the outputs).
-// Rows of a page beyond the context may hold anything, so the V rows of the last tile are cleared before they are multiplied by zero weights.
+// Rows of a page beyond the context, or ahead of what a window or a block mask leaves, may hold anything, so those V rows are cleared in the
+// last and the first tile before they are multiplied by zero weights.
 #include <cuda_bf16.h>
 
 #include "b200_serve.h"
@@ -159,7 +160,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
             fence_proxy_async_smem();
         }
         const int pA = a.pos[tA], pZ = a.pos[tA + count - 1];
-        const int key0 = pa_first_key(a, pA) & ~(kTcKeys - 1), n_kt = (pZ - key0) / kTcKeys + 1;
+        const int fA = pa_first_key(a, pA), key0 = fA & ~(kTcKeys - 1), n_kt = (pZ - key0) / kTcKeys + 1;
         const int* plist = a.pages + (size_t)slots[first + 1] * a.max_pages;
         __syncwarp();   // lanes without a row skipped its loads; the barrier is warp-wide
         if (warp >= 1) asm volatile("bar.sync 1, 160;" ::: "memory");
@@ -256,13 +257,13 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                 const uint32_t ph = (uint32_t)(it >> 1) & 1u, st = tmem + my + (uint32_t)(s * kTcKeys);
                 mbar_wait_or_leave(&s_full[s], ph, dead);
                 tc_fence_after();
-                if (k0 + kTcKeys > pZ + 1) {
-                    // V rows behind the context: 0 * NaN must stay 0. (After the wait above: these scores follow the product two tiles before in
+                if (k0 + kTcKeys > pZ + 1 || k0 < fA) {
+                    // V rows behind the context, and those ahead of the first key that any row sees: 0 * NaN must stay 0. (After the wait above: these scores follow the product two tiles before in
                     // the tensor pipe, so the stage has seen its last but one load and its barrier can be waited on by parity.)
                     mbar_wait_or_leave(&v_full[s], ph, dead);
-                    const int valid = pZ + 1 - k0;
-                    for (int i = threadIdx.x - 64; i < (kTcKeys - valid) * (DV / 8); i += 128) {
-                        const int vr = valid + i / (DV / 8), c = i % (DV / 8);
+                    for (int i = threadIdx.x - 64; i < kTcKeys * (DV / 8); i += 128) {
+                        const int vr = i / (DV / 8), c = i % (DV / 8);
+                        if (k0 + vr >= fA && k0 + vr <= pZ) continue;
                         st_shared_v4(smem_u32(smem + L::kOffV + s * L::kV + (c / 8) * kTcBox) + (uint32_t)(vr * 128 + (c & 7) * 16), 0u, 0u, 0u, 0u);
                     }
                     fence_proxy_async_smem();

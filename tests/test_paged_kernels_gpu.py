@@ -60,7 +60,7 @@ def run(S, q, keys, values, table, PR, slot, pos, o, longest, f32=True, workspac
     a.slot, a.pos, a.n_tokens, a.heads, a.kv_heads, a.dim, a.vdim = keep[0].data_ptr(), keep[1].data_ptr(), T, H, G, d, dv
     a.scale, a.softcap, a.denom_bias, a.dtype, a.longest_entry, a.longest_context = o["scale"], o.get("cap", 0.0), o.get("denom", 0.0), S.BF16, longest, max(pos) + 1
     a.chunk, a.maps, a.out_f32, a.window, a.sigmoid_weights = o.get("chunk", 0), M, int(f32), o.get("window", 0), int(bool(o.get("sigmoid")))
-    for name, key in (("sink", "sink"), ("dist_bias", "bias"), ("head_bias", "head_bias")):
+    for name, key in (("sink", "sink"), ("dist_bias", "bias"), ("head_bias", "head_bias"), ("head_temp", "temp")):
         if o.get(key) is not None:
             keep.append(o[key].float().cuda().contiguous())
             setattr(a, name, keep[-1].data_ptr())
@@ -187,3 +187,42 @@ def test_prompt_weights_are_the_sum_of_two_bfloat16(S, form, H, G, M, d, dv):
     got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * n, list(range(before, before + n)), o, n)
     want = reference(q, k[0], v[0], list(range(before, before + n)), o)
     assert float((got - want).norm() / want.norm()) < 3e-5
+
+
+@pytest.mark.parametrize("form,before", [("blocks", 230), ("blocks", 305), ("sigmoid", 171)])
+@pytest.mark.parametrize("d,dv", [(128, 128), (64, 64), (128, 256)])
+def test_rows_ahead_of_the_first_visible_key_may_hold_anything(S, form, before, d, dv):
+    """a portion whose window or block begins inside a page: what is cached ahead of it is NaN, as it is where only the visible part of a
+    sequence was brought into the cache"""
+    g = torch.Generator().manual_seed(before + dv)
+    o = options(form, 4, d, g)
+    n, PR = 70, 64
+    k, v, kp, vp, table = sequences(g, [before + n], 2, 1, d, dv, PR)
+    first = seen(o, before)
+    for j in range(first):
+        row = int(table[0, j // PR]) * PR + j % PR
+        kp[row], vp[row] = float("nan"), float("nan")
+    q = torch.randn(n, 4, 1, d, generator=g).bfloat16().double()
+    got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * n, list(range(before, before + n)), o, n)
+    want = reference(q, k[0], v[0], list(range(before, before + n)), o)
+    assert float((got - want).norm() / want.norm()) < 3e-5
+
+
+@pytest.mark.parametrize("G", [4, 2, 1])
+@pytest.mark.parametrize("longest", [0, 1, 90])
+def test_head_temperatures_and_an_unknown_longest_entry(S, G, longest):
+    """a factor per head on the scores, negative ones among them; 0: the caller does not know how many tokens an entry brings"""
+    g = torch.Generator().manual_seed(G + longest)
+    H, d, PR = 4, 128, 64
+    before, new = ([250, 63, 10], [1, 1, 1]) if longest == 1 else ([250, 63, 10, 0], [1, 65, 1, 90])
+    o = dict(scale=1.3 / math.sqrt(d), temp=torch.tensor([0.5, -1.0, 1.7, 0.0], dtype=torch.float64))
+    k, v, kp, vp, table = sequences(g, [a + b for a, b in zip(before, new)], G, 1, d, d, PR)
+    q = [torch.randn(n, H, 1, d, generator=g).bfloat16().double() for n in new]
+    slot = [b for b in range(len(new)) for _ in range(new[b])]
+    pos = [before[b] + i for b in range(len(new)) for i in range(new[b])]
+    got = run(S, torch.cat(q).bfloat16().cuda(), kp, vp, table, PR, slot, pos, o, longest)
+    at = 0
+    for b in range(len(new)):
+        want = reference(q[b] * o["temp"][None, :, None, None], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
+        assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 3e-5, b
+        at += new[b]
