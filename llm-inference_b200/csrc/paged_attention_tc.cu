@@ -276,11 +276,12 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                 auto S = [&](int e) { return __uint_as_float(sv[e]); };
                 const bool whole = __all_sync(0xffffffffu, k0 + kTcKeys - 1 <= p && k0 >= f);
                 if (FORM == kTcCapped) {
-                    // cap * tanh(v / cap): the odd series below |x| = 0.25 (exact to fp32 rounding), else (t - 1) / (t + 1), t = e^(2x)
+                    // cap * tanh(v / cap): the odd series up to x^7 while every |x| is below 0.2 (its next term is below 2^-24 of x there), else
+                    // (t - 1) / (t + 1), t = e^(2x)
                     float big[2] = {0.f, 0.f};
 #pragma unroll
                     for (int e = 0; e < 64; ++e) big[e & 1] = fmaxf(big[e & 1], fabsf(S(e)));
-                    if (__all_sync(0xffffffffu, fmaxf(big[0], big[1]) * over_cap < 0.25f)) {
+                    if (__all_sync(0xffffffffu, fmaxf(big[0], big[1]) * over_cap < 0.2f)) {
                         const uint64_t oc2 = pack2f(over_cap, over_cap), c2 = pack2f(cap2, cap2), one2 = pack2f(1.f, 1.f);
                         const uint64_t c7 = pack2f(-17.f / 315.f, -17.f / 315.f), c5 = pack2f(2.f / 15.f, 2.f / 15.f), c3 = pack2f(-1.f / 3.f, -1.f / 3.f);
 #pragma unroll

@@ -180,15 +180,15 @@ __global__ void __launch_bounds__(128, DV <= 128 ? 3 : 2) paged_attn_tile_kernel
                 }
             }
             // cap * tanh(v / cap): when every score of this thread's tile is small against the cap (the usual case) the odd
-            // series x - x^3/3 + 2x^5/15 - 17x^7/315 is exact to fp32 rounding below |x| = 0.25 and costs no special-function
-            // unit; otherwise (t - 1) / (t + 1) with t = e^(2x) (absolute error ~1e-7 * cap)
+            // series x - x^3/3 + 2x^5/15 - 17x^7/315 is exact to fp32 rounding below |x| = 0.2 (the next term is below 2^-24 of x)
+            // and costs no special-function unit; otherwise (t - 1) / (t + 1) with t = e^(2x) (absolute error ~1e-7 * cap)
             if (!BIAS && a.softcap > 0.f) {
                 float big = 0.f;
 #pragma unroll
                 for (int nt = 0; nt < kTileN / 8; ++nt)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) { s[nt][e] *= scale_over_cap; big = fmaxf(big, fabsf(s[nt][e])); }
-                if (__all_sync(0xffffffffu, big < 0.25f)) {
+                if (__all_sync(0xffffffffu, big < 0.2f)) {
 #pragma unroll
                     for (int nt = 0; nt < kTileN / 8; ++nt)
 #pragma unroll
