@@ -189,9 +189,9 @@ __device__ __forceinline__ SsdChunk ssd_chunk_of(const SS& a, int e, int c) {
 // and each is a chain of loads and products. A whole chunk per CTA took 9 us, this three; 2048 tokens, 8 heads x 64 in all 44.9 -> 39.0 us.
 __global__ void __launch_bounds__(128) ssd_cb_kernel(const SS a) {
     extern __shared__ __align__(16) float sm[];
-    const SsdChunk ck = ssd_chunk_of(a, blockIdx.x, blockIdx.y);
+    const SsdChunk ck = ssd_chunk_of(a, blockIdx.x >> 2, blockIdx.y);
     if (!ck.on) return;
-    const int g = blockIdx.z >> 2, m0 = (blockIdx.z & 3) * 16, N = a.n_state, npad = (N + 7) & ~7, st = ssd_stride4(npad);
+    const int g = blockIdx.z, m0 = (blockIdx.x & 3) * 16, N = a.n_state, npad = (N + 7) & ~7, st = ssd_stride4(npad);
     if (m0 >= ck.len) return;
     float* Cs = sm;               // [16][st]
     float* Bs = sm + 16 * st;     // [m0 + 16][st]
@@ -502,7 +502,7 @@ extern "C" int b200_ssd_scan(const b200_ssd_scan_args* p, void* stream) {
         if (e == cudaSuccess) e = ensure_max_dynamic_smem((const void*)ssd_state_kernel, kSsdChunk * (kSsdXs + 264) * 4, d1);
         if (e == cudaSuccess) e = ensure_max_dynamic_smem((const void*)ssd_out_kernel, (kSsdChunk * (kSsdXs + kSsdMs + 260) + 256 * kSsdXs) * 4, d2);
         if (e != cudaSuccess) return (int)e;
-        ssd_cb_kernel<<<dim3(p->n_entries, chunks, 4 * p->groups), 128, sm_cb, s>>>(a);
+        ssd_cb_kernel<<<dim3(4 * p->n_entries, chunks, p->groups), 128, sm_cb, s>>>(a);
         const dim3 grid(p->n_entries * a.col_blocks, chunks, p->heads);
         ssd_state_kernel<<<grid, 128, sm_st, s>>>(a);
         const int per = p->n_state * p->vdim;   // a head's state starts on a multiple of `per` floats
