@@ -98,9 +98,10 @@ int b200_latent_store(const float* raw, long long ld_raw, const float* w, float 
  * (sum_j exp(s_j - m) + exp(sink[h] - m)); out[t,h,:] = sum_j p_j c_j. qa, out fp32 [n_tokens, heads, rank] (qa is the
  * query already multiplied by the key up-projection; the caller applies the value up-projection to out). The sink
  * has no row and no value. Rows come from the page pool as in b200_latent_store.
- * Hints (0 / NULL = unknown): longest_entry = most consecutive tokens of one sequence in the batch (1: a decode batch,
- * one token per CTA); longest_context = most rows any token sees; with a workspace the bfloat16 kernel then splits long
- * contexts of small batches over several CTAs and merges the shares (and the sink) in a second launch. */
+ * Hints (0 / NULL = unknown): longest_entry = most consecutive tokens of one sequence in the batch (1: a decode batch: in
+ * bfloat16 a cluster of CTAs shares each token's rows, in one launch and without the workspace); longest_context = most rows any
+ * token sees; with a workspace a few bfloat16 rows behind long contexts are split over several CTAs, and a second launch merges the
+ * shares (and the sink). */
 size_t b200_latent_attention_workspace_bytes(int n_tokens, int heads, int rank);
 int b200_latent_attention(const float* qa, float* out, const void* pool, const int* pages, int max_pages, int page_rows,
                           const int* slot, const int* pos, const float* sink, float scale, int n_tokens, int heads,
@@ -327,9 +328,10 @@ int b200_conv_state_update(const float* proj, long long ld_proj, float* conv_sta
  * sequence's rows j <= pos[t]; p_j = exp(s_j) / (denom_bias + sum_j exp(s_j)) (denom_bias 1: a sink of score 0 without
  * a value; 0: plain softmax); out[t, h, :] = sum_j p_j v_j. q [n_tokens, heads*dim], out [n_tokens, heads*vdim], pools
  * [n_pages*page_rows, kv_heads, dim | vdim], all of `dtype`; scores, softmax and sums in fp32.
- * longest_entry (0 = unknown): most tokens one sequence brings in this batch; bfloat16 batches with prompt portions run
- * on tensor-core tiles, single tokens and fp32 on the row kernel; with a workspace and longest_context given, a batch of few
- * rows with long contexts (decoding) splits every context over up to 16 CTAs and merges the shares in a second launch. */
+ * longest_entry (0 = unknown): most tokens one sequence brings in this batch. In bfloat16 prompt portions run on tensor-core tiles
+ * and single tokens on clusters of CTAs that share a context (head sizes 64 / 64, 64 / 128, 128 / 128 and 128 / 256, up to eight query heads
+ * per key head; neither needs the workspace). fp32, other head sizes and unaligned operands run on the row kernel; with a workspace and
+ * longest_context given, it splits the contexts of few rows over up to 16 CTAs and merges the shares in a second launch. */
 typedef struct b200_paged_attention_args {
     const void* q; void* out; const void* k_pool; const void* v_pool;
     const int* pages; int max_pages, page_rows;

@@ -711,6 +711,21 @@ static bool tile_attention_enabled() {
     return v == 1;
 }
 
+// Batches with prompt portions: rows of whole 64-dimension chunks with 256 or 512 columns of output go to the tcgen05 tiles (2048 tokens, 16 heads, rows
+// of 576: 180 us there, 856 us on the mma.sync tiles), unless a few rows sit behind long contexts, which only the mma.sync tiles share out. A tcgen05
+// CTA takes about 1.8 us per 64 cached rows of a sequence and walks those of its window that fall to it; an mma.sync CTA, two to an SM, takes 7 times
+// as long at 512 columns and 5 times at 256, over its share and once per sequence of its rows. Measured, rows of 576, 16 heads, tcgen05 / shared out:
+// 2 or 16 tokens behind 8000 rows 255 / 122 us, 64 tokens 254 / 212, 200 tokens behind 4000 147 / 407, 64 behind 1000 51 / 77; 12 single tokens and a
+// portion of 16 over 4000 137 / 144, 64 and 256 over 1000 119 / 338; rows of 320 (256 columns), 16 behind a window of 1024 49 / 42, 200 48 / 58.
+static bool shares_are_shorter(const b200_latent_attention_args& a, int out_cols, int tokens_per_tile, int splits, int longest_context) {
+    if (a.heads > 64) return false;   // not built for the tcgen05 tiles
+    const int tiles = (longest_context + kTileKeys - 1) / kTileKeys, share = (tiles + splits - 1) / splits, halves = out_cols > 256 ? 2 : 1;
+    const int others = std::max(0, a.n_tokens - a.longest_entry);   // tokens of the other entries
+    const int parts = latent_tc_parts(a.n_tokens, a.longest_entry, a.heads, halves), held = std::min(128 / a.heads, others + 1);
+    const int walked = others == 0 ? 1 : (held + parts - 1) / parts, walked_here = std::min(tokens_per_tile, others + 1);
+    return (halves == 2 ? 7 : 5) * share * walked_here < tiles * walked;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -799,12 +814,6 @@ extern "C" int b200_latent_attention_ex(const b200_latent_attention_args* ap, vo
         const int rc = latent_decode(*ap, out_cols, longest_context, s);
         if (rc >= 0) return rc;
     }
-    // prompt portions over rows of whole 64-dimension chunks with 256 or 512 columns of output (2048 tokens, 16 heads, rows of 576: 160 us there, 856 us
-    // on the tiles below)
-    if (dtype == B200_BF16 && tile_attention_enabled() && longest_entry != 1) {
-        const int rc = latent_attention_tc(*ap, out_cols, s);
-        if (rc >= 0) return rc;
-    }
     if (dtype == B200_BF16 && tile_attention_enabled()) {
         // tensor-core form: 32 rows of (token, head) per CTA
         // every entry a single token (a decode batch): one token per CTA, its heads the only rows
@@ -821,6 +830,10 @@ extern "C" int b200_latent_attention_ex(const b200_latent_attention_args* ap, vo
             const int want = (2 * sm_count()) / (int)(tg.x * tg.y);
             splits = std::max(1, std::min({want, tiles / 2, kMaxSplits}));
             if (workspace_bytes < (size_t)n_tokens * heads * splits * (rank + 2) * sizeof(float)) splits = 1;
+        }
+        if (longest_entry != 1 && !(splits > 1 && shares_are_shorter(*ap, out_cols, TQ, splits, longest_context))) {
+            const int rc = latent_attention_tc(*ap, out_cols, s);
+            if (rc >= 0) return rc;
         }
         tg.z = splits;
         float* part = reinterpret_cast<float*>(workspace);

@@ -11,7 +11,7 @@
 //   warp 1      tcgen05.mma, scores of tile j + 1 ahead of the weighted sum of tile j
 //   warps 2-5   the query rows (rounded to bfloat16, as in the mma.sync kernel), then the softmax, a thread per row, as in paged_attention_tc.cu
 // The weights go back over their scores as the sum of two bfloat16; the sums are rescaled only when a row's maximum has grown by more than 2^8. A window of
-// packed tokens that holds several sequences is walked tile by tile (two CTAs share it when there is more than one entry).
+// packed tokens that holds several sequences is walked tile by tile (latent_tc_parts CTAs share it).
 // Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, this 179 us (160 with
 // weights rounded to bfloat16 alone, and 183 then with the query rows loaded a chunk at a time and the results stored from registers). A tile per CTA takes half of that: what is left is mostly the query's way in.
 #include <cuda_bf16.h>
@@ -369,7 +369,7 @@ static int launch_lt(const b200_latent_attention_args& a, int halves, cudaStream
     static unsigned long long done = 0;
     const cudaError_t e = ensure_max_dynamic_smem((const void*)latent_attn_tc_kernel<NCH>, LtSmem<NCH>::kTotal, done);
     if (e != cudaSuccess) return (int)e;
-    const int TQ = kLtRows / a.heads, parts = a.n_tokens == a.longest_entry ? 1 : 2;
+    const int TQ = kLtRows / a.heads, parts = latent_tc_parts(a.n_tokens, a.longest_entry, a.heads, halves);
     const long long windows = (a.n_tokens + TQ - 1) / TQ;
     if (windows * parts > 65535) return -1;
     const LtArgs la{a.qa, a.out, a.pages, a.slot, a.pos, a.sink, a.max_pages, a.page_rows, a.n_tokens, a.heads, a.rank, a.window, TQ, parts, a.scale};
