@@ -457,6 +457,10 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     const int R = a.heads / a.kv_heads;
     // a cap beside a sink or a bias keeps the row kernel, whose weights stay in 32 bits
     if (R > 8 || a.page_rows % kTcKeys || (a.softcap > 0.f && (a.dist_bias || a.sink)) || a.kv_heads * a.maps > 65535) return -1;
+    // a short portion of one sequence, 64-wide heads, a distance bias: the fixed part of a CTA and a bias per score outweigh products half as long, and the
+    // mma.sync tiles are faster (16 / 8 heads, us there / here: 40 tokens 11.2 / 13.3, 400 tokens 17.4 / 20.5, 100 behind 1000 31.7 / 35.8; but 700 tokens
+    // 28.7 / 27.8, 2048 tokens 73 / 48). Where other sequences are beside it their single tokens decide
+    if (a.dist_bias && a.dim == 64 && a.vdim == 64 && a.chunk == 0 && a.window == 0 && a.n_tokens == longest_entry && a.n_tokens <= 512 && longest_seen > 0 && longest_seen <= 1200) return -1;
     int rc = -1;
     if (a.dim == 128 && a.vdim == 128) rc = launch_tc_for<128, 128>(a, longest_entry, s);
     else if (a.dim == 64 && a.vdim == 64) rc = launch_tc_for<64, 64>(a, longest_entry, s);
