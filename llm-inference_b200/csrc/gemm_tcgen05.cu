@@ -9,6 +9,7 @@
 //   stream  : A = W [N, K] (weight rows on the M axis), B = x [Nt, K]   -> y[tok, n]   HBM-bound (gemm_stream_kernel, below):
 //             every weight byte is read once, Nt <= 256 tokens ride along as the MMA N extent; the K range of a tile is shared by
 //             a cluster, so that narrow projections still fill the GPU.
+//   swapped : the same operands on the persistent gemm_tcgen05_kernel, for outputs so wide that every CTA has tiles of its own.
 //
 // Structure of gemm_tcgen05_kernel (one persistent CTA per SM, 192 threads):
 //   warp 0    TMA producer: cp.async.bulk.tensor.2d (UTMALDG) of 128B-swizzled [rows x 64] boxes
@@ -21,6 +22,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 
@@ -45,6 +47,7 @@ struct GemmParams {
     int tokens;
     int m_tiles, n_tiles, k_blocks;
     int splits;         // stream mode: CTAs (one cluster) that share a tile's K range
+    int accs;           // stream mode: chains that a CTA's share of K is formed in, one after another
     int in_bf16;        // operands are bfloat16 instead of fp16 (same tiles, other instruction descriptor)
     int out_kind;       // element type of C: 0 fp16 (rounding points of the reference sequence), 1 bfloat16, 2 fp32
     int wide_store;     // stream mode: C is 16-byte aligned
@@ -137,7 +140,7 @@ __device__ __forceinline__ void store_glu_row(const GemmParams& p, uint32_t tadd
     }
 }
 
-template <int BN, bool GLU = false>
+template <int BN, bool SWAP, bool GLU = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const GemmParams p) {
@@ -259,6 +262,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 __syncwarp();   // as in store_glu_row
                 tmem_ld_32x32(taddr + (uint32_t)c0, v);
                 const int col0 = nt * BN + c0;   // first row of the B operand covered by this chunk
+                if (SWAP) {
+                    // row = output feature, col = token: lanes write consecutive features of one token
+                    if (row < p.rows_a) {
+                        const float bv = bias ? __half2float(bias[row]) : 0.f;
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            if (col0 + j < p.tokens) store1(C, (size_t)(col0 + j) * p.ldc + row, gemm_unary(__uint_as_float(v[j]) + bv, p.unary), ok);
+                    }
+                    continue;
+                }
                 // row = token, col = output feature: 32 consecutive features per thread
                 if (row < p.tokens && col0 < p.rows_b) {
                     const size_t dst = (size_t)row * p.ldc + col0;
@@ -307,29 +320,35 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // up to 100 KB of its share under way before the first product, two CTAs fit an SM, and the partial sums meet in shared memory (rank
 // order) instead of a workspace and a second launch.
 // GLU: a tile is 64 gate rows and the 64 up rows of the same features (W = [2 * rows_a, K], rows_a = features).
+// The tensor core cuts off when it adds to an accumulator, so a sum's error grows with the length of its chain (1.05e-9 of the result's norm per element
+// of K: 2.1e-6 at 2048, 4.7e-7 at 512): for fp32 outputs a long share of K is formed in several chains, which are added in fp32.
 // Measured, 8 rows, 2048 -> 4096, fp32 out: the persistent kernel with partial sums in global memory and a reduction launch 11.2 us, this 8.5 us.
 template <int BN>
 struct StreamSmem {
     static constexpr int kStageBytes = (kBM + BN) * kBK * 2;
     static constexpr int kStages = BN <= 32 ? 5 : BN <= 64 ? 4 : BN <= 128 ? 3 : 4;
-    static constexpr int kPerSm = BN <= 128 ? 2 : 1;
-    static constexpr int kTotal = kStages * kStageBytes + (2 * kStages + 1) * 8 + 16 + 1024;
+    static constexpr int kPerSm = BN <= 128 ? 2 : 1, kAccs = 512 / kPerSm / BN;   // accumulators that fit a CTA's tensor memory
+    // up to 64 rows a CTA's chains have an accumulator each; above, two take turns and eight warps add them up in registers, half a row each
+    static constexpr bool kFold = kAccs == 2;
+    static constexpr int kThreads = kFold ? 320 : 192;
+    static constexpr int kTotal = kStages * kStageBytes + (2 * kStages + 4) * 8 + 16 + 1024;
     static_assert(BN * kBM * 4 <= kStages * kStageBytes, "the partial sums take the place of the stages");
 };
 constexpr int kStreamMaxSplits = 8;
 
 template <int BN, bool GLU>
-__global__ void __launch_bounds__(kGemmThreads, StreamSmem<BN>::kPerSm)
+__global__ void __launch_bounds__(StreamSmem<BN>::kThreads, StreamSmem<BN>::kPerSm)
 gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
     using S = StreamSmem<BN>;
     constexpr int STAGES = S::kStages;
+    constexpr bool FOLD = S::kFold;
     constexpr uint32_t A_BYTES = kBM * kBK * 2, B_BYTES = BN * kBK * 2;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(tiles + (size_t)STAGES * S::kStageBytes);
     uint64_t* empty_bar = full_bar + STAGES;
-    uint64_t* acc_full = empty_bar + STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+    uint64_t *acc_full = empty_bar + STAGES, *acc_empty = acc_full + 2;   // [2] each; without FOLD only the first of acc_full
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* om = reinterpret_cast<float*>(tiles);   // [tokens][128]: this CTA's sums, once the stages have been used
 
@@ -341,13 +360,14 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
-        mbar_init(acc_full, 1);
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
         *dead = 0;
         mbar_fence_init();
         tma_prefetch_desc(&map_a);
         tma_prefetch_desc(&map_b);
     }
-    if (warp == 1) tmem_alloc(tmem_slot, BN);
+    const uint32_t tmem_cols = (uint32_t)(FOLD ? min(p.accs, 2) : p.accs) * BN;
+    if (warp == 1) tmem_alloc(tmem_slot, tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -375,9 +395,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
     } else if (warp == 1) {
         const uint32_t idesc = make_idesc_f16(kBM, BN) | (p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
-        int stage = 0;
+        auto chain_end = [&](int i) { return p.accs == 1 ? kb1 : kb0 + (kb1 - kb0) * (i + 1) / p.accs; };
+        int stage = 0, at = 0, end = chain_end(0);
+        bool fresh = true;   // the first products of a chain
         uint32_t phase = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
+            const int slot = FOLD ? at & 1 : at;
+            if (FOLD && fresh && at >= 2) mbar_wait_or_leave(&acc_empty[slot], (uint32_t)((at >> 1) - 1) & 1u, dead);
             mbar_wait_or_leave(&full_bar[stage], phase, dead);
             tc_fence_after();
             if (lane == 0) {
@@ -385,13 +409,42 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 const uint64_t da = make_kmajor_sw128_desc(sa), db = make_kmajor_sw128_desc(sa + A_BYTES);
 #pragma unroll
                 for (int k = 0; k < kBK / kUmmaK; ++k)
-                    umma_f16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                    umma_f16(tmem + (uint32_t)(slot * BN), da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (!fresh || k > 0) ? 1u : 0u);
                 umma_commit(&empty_bar[stage]);
-                if (kb == kb1 - 1) umma_commit(acc_full);
+                if (FOLD ? kb + 1 == end : kb + 1 == kb1) umma_commit(&acc_full[FOLD ? slot : 0]);
             }
             __syncwarp();
+            fresh = kb + 1 == end;
+            if (fresh && kb + 1 < kb1) end = chain_end(++at);
             if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+    } else if constexpr (FOLD) {
+        constexpr int COLS = BN / 2;
+        const int quarter = warp & 3, first = (warp - 2) / 4 * COLS;
+        const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)first;
+        float sum[COLS];
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+        for (int i = 0; i < p.accs; ++i) {
+            mbar_wait_or_leave(&acc_full[i & 1], (uint32_t)(i >> 1) & 1u, dead);   // (the last: every load has landed and every product has read its stage)
+            tc_fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < COLS; c0 += 16)
+                if (first + c0 < p.tokens) {
+                    uint32_t v[16];
+                    tmem_ld_32x16_async(taddr + (uint32_t)((i & 1) * BN + c0), v);
+                    tmem_wait_ld<16>(v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(v[j]);
+                }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[i & 1]);
+        }
+        const bool gone = *dead != 0;
+#pragma unroll
+        for (int j = 0; j < COLS; ++j)
+            if (first + j < p.tokens) om[(first + j) * kBM + quarter * 32 + lane] = gone ? __int_as_float(0x7fffffff) : sum[j];
     } else {
         const int quarter = warp & 3;
         mbar_wait_or_leave(acc_full, 0, dead);   // every load has landed and every product has read its stage
@@ -402,6 +455,13 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         for (int c0 = 0; c0 < BN && c0 < p.tokens; c0 += 32) {
             uint32_t v[32];
             tmem_ld_32x32(taddr + (uint32_t)c0, v);
+#pragma unroll 1
+            for (int i = 1; i < p.accs; ++i) {
+                uint32_t w[32];
+                tmem_ld_32x32(taddr + (uint32_t)(i * BN + c0), w);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j)
                 if (c0 + j < p.tokens) om[(c0 + j) * kBM + quarter * 32 + lane] = gone ? __int_as_float(0x7fffffff) : __uint_as_float(v[j]);
@@ -431,7 +491,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             return acc;
         };
         const __half* bias = reinterpret_cast<const __half*>(p.bias);
-        for (int i = sp * share + (int)threadIdx.x; i < min(total, (sp + 1) * share); i += kGemmThreads) {
+        for (int i = sp * share + (int)threadIdx.x; i < min(total, (sp + 1) * share); i += S::kThreads) {
             const int tok = i / (F / 4), f0 = i % (F / 4) * 4, n = mt * F + f0;
             if (n >= p.rows_a) continue;
             const float4 s4 = sum4(tok * kBM + f0);
@@ -473,7 +533,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (p.splits > 1) cluster.sync();   // nobody leaves while its sums are read
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, BN);
+        tmem_dealloc(tmem, tmem_cols);
     }
 }
 
@@ -534,9 +594,9 @@ bool make_tma_map_2d(CUtensorMap* out, const void* ptr, long long rows, int K, i
     return true;
 }
 
-template <int BN, bool GLU = false>
+template <int BN, bool SWAP, bool GLU = false>
 static int gemm_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int grid, cudaStream_t s) {
-    auto kern = gemm_tcgen05_kernel<BN, GLU>;
+    auto kern = gemm_tcgen05_kernel<BN, SWAP, GLU>;
     static unsigned long long attr_done = 0;   // per instantiation, one bit per device
     {
         cudaError_t e = ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), GemmSmem<BN>::kTotal, attr_done);
@@ -548,47 +608,139 @@ static int gemm_launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmP
 }
 
 template <int BN, bool GLU>
-static int stream_launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, cudaStream_t s) {
-    auto kern = gemm_stream_kernel<BN, GLU>;
-    static unsigned long long attr_done = 0;
-    cudaError_t e = ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), StreamSmem<BN>::kTotal, attr_done);
-    if (e != cudaSuccess) return (int)e;
-    // as many CTAs per tile as one wave takes, each with two K blocks at least
-    p.splits = std::max(1, std::min({kStreamMaxSplits, sm_count() * StreamSmem<BN>::kPerSm / p.m_tiles, p.k_blocks / 2}));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(p.m_tiles * p.splits));
-    cfg.blockDim = dim3(kGemmThreads);
+static void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int m_tiles, int splits, cudaStream_t s) {
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3((unsigned)(m_tiles * splits));
+    cfg.blockDim = dim3(StreamSmem<BN>::kThreads);
     cfg.dynamicSmemBytes = StreamSmem<BN>::kTotal;
     cfg.stream = s;
-    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)p.splits;
+    at[0].val.clusterDim.x = (unsigned)splits;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+}
+
+// [n]: clusters of n CTAs that run at once, asked for once per device and kernel; nullptr: e says why. A cluster lives inside one GPC, so they are fewer than the
+// SMs alone would hold. (The runtime counts one CTA per SM here, 148 74 45 33 26 22 15 15 clusters of 1 to 8, while kPerSm of them run: its answer is scaled.)
+template <int BN, bool GLU>
+static const int* stream_capacity(int dev, int sms, cudaError_t& e) {
+    static std::atomic<const int*> known[kMaxDevices];
+    const int* c = known[dev].load(std::memory_order_acquire);
+    if (c) return c;
+    auto kern = gemm_stream_kernel<BN, GLU>;
+    prefer_max_smem_carveout(reinterpret_cast<const void*>(kern));
+    e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeMaxDynamicSharedMemorySize, StreamSmem<BN>::kTotal);
+    if (e != cudaSuccess) return nullptr;
+    int* t = new int[kStreamMaxSplits + 1]{};
+    for (int n = 1; n <= kStreamMaxSplits; ++n) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[1];
+        stream_config<BN, GLU>(cfg, at, sms, n, nullptr);
+        if (cudaOccupancyMaxActiveClusters(&t[n], kern, &cfg) != cudaSuccess) { cudaGetLastError(); t[n] = 0; }
+    }
+    for (int n = kStreamMaxSplits; n > 0; --n) t[n] = t[1] > 0 ? t[n] * sms * StreamSmem<BN>::kPerSm / t[1] : 0;
+    if (known[dev].compare_exchange_strong(c, t, std::memory_order_acq_rel)) return t;
+    delete[] t;   // another thread was first
+    return c;
+}
+
+// CTAs per tile: as many as run at once, each with two K blocks at least; more where their chains would be fewer than `shares`
+template <int BN>
+static int stream_splits(const int* capacity, int sms, int m_tiles, int k_blocks, int shares) {
+    const int slots = sms * StreamSmem<BN>::kPerSm;
+    int n = std::max(1, std::min({kStreamMaxSplits, slots / m_tiles, k_blocks / 2})), fit = n;
+    // a second wave costs a whole pass (us, 2048 x 2048 at 256 rows in clusters of 8 / 6: 26.6 / 17.3, 6184 x 2048 at 32 rows of 6 / 5: 20.4 / 16.4), but leaving
+    // more than a quarter of the places empty costs more (11008 x 4096 at 32 rows in clusters of 3 / 2: 28.7 / 36.1)
+    while (fit > 1 && capacity[fit] < m_tiles) --fit;
+    if (4 * fit * m_tiles >= 3 * slots || StreamSmem<BN>::kPerSm == 1) n = fit;
+    return StreamSmem<BN>::kFold ? n : std::max(n, std::min(kStreamMaxSplits, (shares + StreamSmem<BN>::kAccs - 1) / StreamSmem<BN>::kAccs));
+}
+
+template <int BN, bool GLU>
+static int stream_launch(const void* x, const void* W, GemmParams p, int M, int N, int K, int shares, int dev, int sms, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    const int* capacity = stream_capacity<BN, GLU>(dev, sms, e);
+    if (!capacity) return (int)e;
+    CUtensorMap ma, mb;
+    if (!make_tma_map_2d(&ma, W, GLU ? 2ll * N : N, K, GLU ? 64 : kBM) || !make_tma_map_2d(&mb, x, M, K, BN)) return B200_EUNSUPPORTED;
+    p.splits = stream_splits<BN>(capacity, sms, p.m_tiles, p.k_blocks, shares);
+    const int share = p.k_blocks / p.splits;
+    p.accs = 1;
+    if (p.out_kind == 2) {
+        if (StreamSmem<BN>::kFold) p.accs = std::max({1, share / 8, std::min(share, (shares + p.splits - 1) / p.splits)});
+        else while (p.accs < StreamSmem<BN>::kAccs && p.accs * 4 < share) p.accs *= 2;
+    }
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[2];
+    stream_config<BN, GLU>(cfg, at, p.m_tiles, p.splits, s);
     if (pdl_enabled()) {
         at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    e = cudaLaunchKernelEx(&cfg, kern, ma, mb, p);
+    e = cudaLaunchKernelEx(&cfg, gemm_stream_kernel<BN, GLU>, ma, mb, p);
     count_launch();
     return (int)e;
 }
 
-// M <= 256 token rows (GLU: 128) against W = [N, K] (GLU: [2 N, K], N % 64 == 0)
-static int gemm_stream(const void* x, const void* W, GemmParams p, int M, int N, int K, bool glu, cudaStream_t s) {
-    const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256, F = glu ? 64 : kBM;
+template <int BN>
+static int swapped_launch(const void* x, const void* W, const GemmParams& p, int M, int N, int K, cudaStream_t s) {
+    CUtensorMap ma, mb;
+    if (!make_tma_map_2d(&ma, W, N, K, kBM) || !make_tma_map_2d(&mb, x, M, K, BN)) return B200_EUNSUPPORTED;
+    return gemm_launch<BN, true>(ma, mb, p, std::min(p.m_tiles, sm_count()), s);
+}
+
+// the shares of K that fp32 outputs are formed in at least: what fills `sms` CTAs best when every share is a tile of its own (and what the kernel with partial
+// sums in global memory formed them in: no sum is less exact than it was there)
+static int least_shares(int m_tiles, int k_blocks, int sms) {
+    int best = 1;
+    long long best_cost = -1;
+    for (int s = 1; s <= 16 && k_blocks / s >= 4; ++s) {
+        const long long rounds = ((long long)m_tiles * s + sms - 1) / sms;
+        const long long per = (k_blocks + s - 1) / s;
+        const long long cost = rounds * (per + 2) + (s > 1 ? s : 0);
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = s; }
+    }
+    return best;
+}
+
+// M <= 256 token rows against W = [N, K] (GLU: M <= 128, W = [2 N, K], N % 64 == 0)
+static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int N, int K, bool glu, cudaStream_t s) {
+    const int F = glu ? 64 : kBM, sms = sm_count();
+    const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     p.rows_a = N; p.rows_b = M;
     p.m_tiles = (N + F - 1) / F; p.n_tiles = 1;
     p.wide_store = (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
-    CUtensorMap ma, mb;
-    if (!make_tma_map_2d(&ma, W, glu ? 2ll * N : N, K, F) || !make_tma_map_2d(&mb, x, M, K, BN)) return B200_EUNSUPPORTED;
+    // Wide outputs: with a tile or more per CTA there is no K range to share, and the persistent kernel hides a tile's epilogue and set-up under the next
+    // one's products. The lines lie where its time passes the stream kernel's (us, stream / persistent). More than 128 rows, where a CTA fills an SM, from
+    // one CTA per tile on: 11008 x 4096 at 256 rows 57 / 53, 32000 x 1024 55 / 39, 128256 x 2048 222 / 137. 33 to 128 rows from 1.6 tiles per SM on
+    // (25600 x 4096 at 64 rows 55 / 60, 32000 x 4096 67 / 62, 128256 x 2048 118 / 105) and where about one each is left (16384 x 1024 19 / 17). Fewer
+    // only beyond the two tiles per SM that run at once and for short sums: 50304 x 1024 at 32 rows 36 / 32, 128256 x 2048 106 / 109.
+    const bool wide = M > 128 ? 2 * p.m_tiles > sms : M > 32 ? 5 * p.m_tiles > 8 * sms || (5 * p.m_tiles > 4 * sms && p.m_tiles <= sms) : p.m_tiles > 2 * sms && p.k_blocks <= 16;
+    // fp32 outputs are formed in least_shares shares of K at least (the persistent kernel knows one)
+    const int shares = !glu && p.out_kind == 2 ? least_shares(p.m_tiles, p.k_blocks, sms) : 1;
+    // three CTAs per tile whose clusters do not all run at once: 12288 x 4096 fp16 at 32 rows 38.9 us, 31.8 on the persistent kernel
+    const int dev = current_device();
+    bool late = false;
+    if (!glu && shares == 1 && M <= 128 && 2 * sms / p.m_tiles == 3) {
+        cudaError_t e = cudaSuccess;
+        const int* c = BN == 32 ? stream_capacity<32, false>(dev, sms, e) : BN == 64 ? stream_capacity<64, false>(dev, sms, e) : stream_capacity<128, false>(dev, sms, e);
+        late = c && c[3] < p.m_tiles;
+    }
+    if (!glu && (wide || late) && shares == 1) {
+        switch (BN) {
+            case 32: return swapped_launch<32>(x, W, p, M, N, K, s);
+            case 64: return swapped_launch<64>(x, W, p, M, N, K, s);
+            case 128: return swapped_launch<128>(x, W, p, M, N, K, s);
+            default: return swapped_launch<256>(x, W, p, M, N, K, s);
+        }
+    }
     switch (BN) {
-        case 32: return glu ? stream_launch<32, true>(ma, mb, p, s) : stream_launch<32, false>(ma, mb, p, s);
-        case 64: return glu ? stream_launch<64, true>(ma, mb, p, s) : stream_launch<64, false>(ma, mb, p, s);
-        case 128: return glu ? stream_launch<128, true>(ma, mb, p, s) : stream_launch<128, false>(ma, mb, p, s);
-        default: return stream_launch<256, false>(ma, mb, p, s);
+        case 32: return glu ? stream_launch<32, true>(x, W, p, M, N, K, shares, dev, sms, s) : stream_launch<32, false>(x, W, p, M, N, K, shares, dev, sms, s);
+        case 64: return glu ? stream_launch<64, true>(x, W, p, M, N, K, shares, dev, sms, s) : stream_launch<64, false>(x, W, p, M, N, K, shares, dev, sms, s);
+        case 128: return glu ? stream_launch<128, true>(x, W, p, M, N, K, shares, dev, sms, s) : stream_launch<128, false>(x, W, p, M, N, K, shares, dev, sms, s);
+        default: return stream_launch<256, false>(x, W, p, M, N, K, shares, dev, sms, s);
     }
 }
 
@@ -623,7 +775,7 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
         const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, s);
         if (rc2 != B200_EUNSUPPORTED) return rc2;
     }
-    if (M <= 256) return gemm_stream(x, W, p, M, N, K, false, s);
+    if (M <= 256) return gemm_few_rows(x, W, p, M, N, K, false, s);
     // normal: tokens on the M axis; large shapes go to the two-CTA kernel (gemm2_tcgen05.cu)
     {
         const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, s);
@@ -636,10 +788,10 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     const int units = p.m_tiles * p.n_tiles;
     const int grid = units < sms ? units : sms;
     switch (BN) {
-        case 32: return gemm_launch<32>(ma, mb, p, grid, s);
-        case 64: return gemm_launch<64>(ma, mb, p, grid, s);
-        case 128: return gemm_launch<128>(ma, mb, p, grid, s);
-        default: return gemm_launch<256>(ma, mb, p, grid, s);
+        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
+        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
+        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
+        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
     }
 }
 
@@ -664,14 +816,15 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
     CUtensorMap ma, mb;
     if (glu) {
         if (N < 128 || (N & 127)) return B200_EUNSUPPORTED;
-        if (M <= 128) return gemm_stream(x, W, p, M, N, K, true, s);
+        // (96 rows of 28672 gated features: 110 us with the weights streaming in 1.5 waves, 107 with the tokens on the M axis; 72 rows 107 / 108)
+        if (M <= 64 || (M <= 128 && N <= 128 * sms)) return gemm_few_rows(x, W, p, M, N, K, true, s);
         p.rows_a = M; p.rows_b = N;
         p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = N / 128;
         if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * N, K, 128)) return B200_EUNSUPPORTED;
         const int units = p.m_tiles * p.n_tiles;
-        return gemm_launch<256, true>(ma, mb, p, units < sms ? units : sms, s);
+        return gemm_launch<256, false, true>(ma, mb, p, units < sms ? units : sms, s);
     }
-    if (M <= 256) return gemm_stream(x, W, p, M, N, K, false, s);
+    if (M <= 256) return gemm_few_rows(x, W, p, M, N, K, false, s);
     const int BN = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : 32;
     p.rows_a = M; p.rows_b = N;
     p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN;
@@ -679,10 +832,10 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
     const int units = p.m_tiles * p.n_tiles;
     const int grid = units < sms ? units : sms;
     switch (BN) {
-        case 32: return gemm_launch<32>(ma, mb, p, grid, s);
-        case 64: return gemm_launch<64>(ma, mb, p, grid, s);
-        case 128: return gemm_launch<128>(ma, mb, p, grid, s);
-        default: return gemm_launch<256>(ma, mb, p, grid, s);
+        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
+        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
+        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
+        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
     }
 }
 // out[M, inter] = silu(x W_gate^T) * (x W_up^T), W = [2*inter, K] (gate rows, then up rows): the gate_up GEMM of
@@ -704,7 +857,7 @@ int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int 
     CUtensorMap ma, mb;
     if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * inter, K, 128)) return B200_EUNSUPPORTED;
     const int units = p.m_tiles * p.n_tiles, sms = sm_count();
-    return gemm_launch<256, true>(ma, mb, p, units < sms ? units : sms, s);
+    return gemm_launch<256, false, true>(ma, mb, p, units < sms ? units : sms, s);
 }
 
 // y[M, N] = residual[M, N] + half(x W^T): launchLinearGemm followed by launchAddResidual (ffn.cpp:88 +
