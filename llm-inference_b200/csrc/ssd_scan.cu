@@ -13,6 +13,7 @@
 //     ssd_state_kernel     U = sum_j exp(cum_end - cum_j) dt_j B_j x_j^T of every chunk and head, chunks in parallel;
 //     ssd_carry_kernel     S at the start of every chunk, S' = exp(cum_end) S + U, and the state the entry leaves behind;
 //     ssd_out_kernel       y_i = exp(cum_i) S^T C_i + sum_(j<=i) (C_i . B_j) exp(cum_i - cum_j) dt_j x_j + D x_i.
+//   (n_state of 33 to 128 and rows of whole 16-byte pieces take the chunks of 128 tokens in ssd_tc.cu instead, on tcgen05)
 //   cum is the running sum of A dt inside the chunk, kept in double: the differences of two large sums are exact enough to
 //   be exponentiated whatever the step sizes are.
 #include <cuda_bf16.h>
@@ -24,24 +25,9 @@
 #include "b200_serve.h"
 #include "common.cuh"
 #include "launch_count.h"
+#include "ssd_scan.cuh"
 
 namespace b200 {
-
-struct SS {
-    const float* u; long long ld_u; int x_off, b_off, c_off;
-    const float* dt_raw; long long ld_dt; const float* dt_bias;
-    const float* A; const float* D;
-    float* state; float* out;
-    const int* ent_row; const int* ent_len; const int* slot; const int* pos;
-    int heads, groups, vdim, n_state;
-    // chunk form: chunk c of entry e sits at place ent_row[e] / kSsdChunk + e + c
-    float* chunk_state;   // [place, head, n_state, vdim]
-    float* chunk_decay;   // [place, head]
-    float* chunk_cb;      // [place, group, kSsdChunk, kSsdChunk]
-    int col_blocks;
-};
-
-__device__ __forceinline__ float ssd_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 constexpr int kSsdRowGroups = 4, kSsdTokens = 8;
 
@@ -109,23 +95,6 @@ __global__ void __launch_bounds__(kSsdRowGroups * PB) ssd_walk_kernel(const SS a
 // chunk form
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kSsdChunk = 64, kSsdCols = 64, kSsdXs = kSsdCols + 8, kSsdMs = kSsdChunk + 4;
-// row strides in floats: stride % 32 == 4 for operands whose rows run along the fragment's 8-wide index, 8 for those whose
-// rows run along its 4-wide index (every fragment load then touches 32 different banks)
-__host__ __device__ __forceinline__ int ssd_stride4(int n) { return ((n + 31) & ~31) + 4; }
-__host__ __device__ __forceinline__ int ssd_stride8(int n) { return ((n + 31) & ~31) + 8; }
-
-__device__ __forceinline__ float ssd_tf32(float v) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-    return __uint_as_float(r);
-}
-__device__ __forceinline__ void ssd_mma(float (&d)[4], const float (&a)[4], float b0, float b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
-          "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
-}
-
 // the chunk's step sizes and running sums of A dt (double) by warp 0: two tokens per lane; places beyond the chunk hold
 // dt = 0 and the last sum
 __device__ __forceinline__ void ssd_chunk_sums(const SS& a, int h, int row0, int len, float* dts, double* cum) {
@@ -149,31 +118,6 @@ __device__ __forceinline__ void ssd_chunk_sums(const SS& a, int h, int row0, int
         cum[2 * l] = run - v1 + v0;
         cum[2 * l + 1] = run;
     }
-}
-
-// `rows` rows of `cols` columns from global (leading dimension ld) into shared memory, rows beyond `live` and columns beyond
-// cols (up to cpad) zero. Rows that allow it travel by cp.async (nothing waits for a load here: ssd_landed() before the first
-// read); the values are rounded to tf32 when a fragment picks them up.
-__device__ __forceinline__ void ssd_stage(float* dst, int stride, const float* src, long long ld, int rows, int live, int cols, int cpad) {
-    if ((cols & 3) == 0 && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0 && cpad == cols) {
-        const int q = cols / 4;
-        for (int i = threadIdx.x; i < rows * q; i += blockDim.x) {
-            const int r = i / q, c = (i - r * q) * 4;
-            const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + r * stride + c);
-            const float* g = src + (r < live ? (size_t)r * ld + c : 0);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(g), "r"(r < live ? 16 : 0) : "memory");
-        }
-        return;
-    }
-    for (int i = threadIdx.x; i < rows * cpad; i += blockDim.x) {
-        const int r = i / cpad, c = i - r * cpad;
-        dst[r * stride + c] = (r < live && c < cols) ? src[(size_t)r * ld + c] : 0.f;
-    }
-}
-__device__ __forceinline__ void ssd_landed() {
-    __syncwarp();   // the lanes close their group of copies together
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
 }
 
 struct SsdChunk {
@@ -469,10 +413,15 @@ static int launch_walk(const SS& a, int n_entries, cudaStream_t s) {
 
 using namespace b200;
 
-extern "C" size_t b200_ssd_scan_workspace_bytes(int n_tokens, int n_entries, int heads, int groups, int vdim, int n_state) {
+static size_t ssd_parallel_bytes(int n_tokens, int n_entries, int heads, int groups, int vdim, int n_state) {
     if (n_tokens < 2 * kSsdChunk || n_entries < 1 || heads < 1 || groups < 1 || vdim < 1 || n_state < 1) return 0;
     const size_t places = ssd_places(n_tokens, n_entries);
     return places * ((size_t)heads * n_state * vdim + ((heads + 3) & ~3) + (size_t)groups * kSsdChunk * kSsdChunk) * sizeof(float) + 256;
+}
+
+extern "C" size_t b200_ssd_scan_workspace_bytes(int n_tokens, int n_entries, int heads, int groups, int vdim, int n_state) {
+    const size_t need = ssd_parallel_bytes(n_tokens, n_entries, heads, groups, vdim, n_state);
+    return need > 0 ? std::max(need, ssd_scan_tc_bytes(n_tokens, n_entries, heads, groups, vdim, n_state)) : 0;
 }
 
 extern "C" int b200_ssd_scan(const b200_ssd_scan_args* p, void* stream) {
@@ -485,7 +434,11 @@ extern "C" int b200_ssd_scan(const b200_ssd_scan_args* p, void* stream) {
     SS a{p->u, p->ld_u, p->x_off, p->b_off, p->c_off, p->dt_raw, p->ld_dt, p->dt_bias, p->A, p->D, p->state, p->out,
          p->ent_row, p->ent_len, p->slot, p->pos, p->heads, p->groups, p->vdim, p->n_state, nullptr, nullptr, nullptr, 1};
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t need = b200_ssd_scan_workspace_bytes(p->n_tokens, p->n_entries, p->heads, p->groups, p->vdim, p->n_state);
+    if (p->chunked && p->longest_entry >= 2 * kSsdChunk) {
+        const int rc = ssd_scan_tc(a, *p, s);
+        if (rc >= 0) return rc;
+    }
+    const size_t need = ssd_parallel_bytes(p->n_tokens, p->n_entries, p->heads, p->groups, p->vdim, p->n_state);
     const int chunks = (p->longest_entry + kSsdChunk - 1) / kSsdChunk;
     if (p->chunked && p->longest_entry >= 2 * kSsdChunk && need > 0 && p->workspace && p->workspace_bytes >= need && chunks <= 65535) {
         const size_t places = ssd_places(p->n_tokens, p->n_entries);
