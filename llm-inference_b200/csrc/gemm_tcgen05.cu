@@ -705,9 +705,20 @@ static int least_shares(int m_tiles, int k_blocks, int sms) {
     return best;
 }
 
+int gemm_rows(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool bf16, int out_kind, bool glu, int act, int unary, float limit, cudaStream_t s);
+
 // M <= 256 token rows against W = [N, K] (GLU: M <= 128, W = [2 N, K], N % 64 == 0)
 static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int N, int K, bool glu, cudaStream_t s) {
     const int F = glu ? 64 : kBM, sms = sm_count();
+    // Up to 16 rows against few weights, where set-up and latency count: no tensor maps, barriers or tensor memory (gemm_rows.cu). The lines lie where the time of
+    // gemm_stream_kernel is reached (us in a graph, weights from HBM, stream / rows). K <= 2048, plain, up to 8 rows: 4096 x 1024 at 8 rows 5.7 / 3.6, 4096 x 2048
+    // 6.9 / 5.5, 6184 x 2048 8.6 / 8.1, 11008 x 2048 11.3 / 11.9; 9 to 16 rows: 8192 x 1024 7.2 / 6.8, 6184 x 2048 8.8 / 9.5; gated: 2 x 4096 x 2048 9.8 / 7.9,
+    // 2 x 8192 x 2048 15.0 / 15.7. Longer K, as long as every CTA has an SM: 2048 x 5504 8.7 / 6.7, 2048 x 8192 10.7 / 8.6, gated 2 x 2048 x 5504 11.7 / 10.0,
+    // 2 x 2048 x 8192 15.0 / 15.1, 4096 x 11008 18.4 / 23.0.
+    if (M <= 16) {
+        const long long weights = (long long)N * K * (glu ? 2 : 1), most = K > 2048 ? (N <= 16 * sms ? 24000000 : 0) : glu ? 17000000 : M <= 8 ? 13000000 : 8500000;
+        if (weights <= most) return gemm_rows(x, W, p.bias, p.C, M, N, K, p.in_bf16 != 0, p.out_kind, glu, p.glu_act, p.unary, p.glu_limit, s);
+    }
     const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     p.rows_a = N; p.rows_b = M;
     p.m_tiles = (N + F - 1) / F; p.n_tiles = 1;
