@@ -20,6 +20,7 @@
 #include "common.cuh"
 #include "launch_count.h"
 #include "rotary.cuh"
+#include "tc_common.cuh"
 
 namespace b200 {
 
@@ -105,21 +106,63 @@ struct RC {
 
 __host__ __device__ __forceinline__ int chunk_row_stride(int dim) { return ((dim + 3) & ~3) + 4; }   // floats; rows stay 16-byte aligned
 
-// rotated q (or k * k_scale * weight[j]) of a chunk into shared memory; the padding columns are zero
+// rotated q (or k * k_scale * weight[j]) of a chunk into shared memory: TRANS false: [token][rs], the padding columns zero; true: [component][kChunkT].
+// A warp takes two tokens at a time and four components per lane of each, all their loads at once (and none behind a condition: such a load waits for the one
+// before it, which is what a chunk's 64 tokens spent most of their time on).
+constexpr int kChunkT = kChunk + 4;
+template <bool TRANS>
 __device__ __forceinline__ void stage_rotated(const RT& a, float* dst, int col_off, int h, int row0, int len, float mul, const float* rowmul) {
-    const int dim = a.dim, nf = a.rot_dims / 2, rs = chunk_row_stride(dim);
-    for (int i = threadIdx.x; i < len * rs; i += blockDim.x) {
-        const int j = i / rs, d = i - j * rs;
-        const size_t r = (size_t)(row0 + j);
-        float v = 0.f;
-        if (d < dim)
-            v = rotary_component(a.proj + r * a.ld_proj + col_off + h * dim, d, a.rot_dims, a.rot_layout, a.cos + r * nf, a.sin + r * nf) * mul *
-                (rowmul ? rowmul[j] : 1.f);
-        dst[i] = v;
+    const int dim = a.dim, nf = a.rot_dims / 2, rs = chunk_row_stride(dim), lane = threadIdx.x & 31, warps = blockDim.x / 32;
+    const bool halves = a.rot_layout == B200_ROPE_HALF;
+    const float *cosines = nf > 0 ? a.cos : a.decay, *sines = nf > 0 ? a.sin : a.decay;   // (without rotation something that can be read)
+    for (int d0 = lane; d0 < dim; d0 += 128) {
+        int lo[4], hi[4], f[4];
+        bool rot[4], first[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {   // the pair of component d and its place in it
+            const int d = min(d0 + 32 * k, dim - 1);
+            rot[k] = d < a.rot_dims;
+            first[k] = halves ? d < nf : (d & 1) == 0;
+            f[k] = !rot[k] ? 0 : halves ? (d < nf ? d : d - nf) : d / 2;
+            lo[k] = !rot[k] ? d : halves ? f[k] : 2 * f[k];
+            hi[k] = !rot[k] ? d : halves ? f[k] + nf : 2 * f[k] + 1;
+        }
+#pragma unroll 1
+        for (int j0 = threadIdx.x / 32; j0 < len; j0 += 2 * warps) {
+            float u[2][4], v[2][4], cs[2][4], sn[2][4];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const size_t r = (size_t)(row0 + min(j0 + t * warps, len - 1));
+                const float *vals = a.proj + r * a.ld_proj + col_off + h * dim, *c = cosines + r * nf, *s = sines + r * nf;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    u[t][k] = vals[lo[k]];
+                    v[t][k] = vals[hi[k]];
+                    cs[t][k] = __ldg(c + f[k]);
+                    sn[t][k] = __ldg(s + f[k]);
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int j = j0 + t * warps;
+                const float w = rowmul ? rowmul[min(j, len - 1)] : 1.f;
+                float* to = dst + (TRANS ? d0 * kChunkT + j : j * rs + d0);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float x = first[k] ? u[t][k] * cs[t][k] - v[t][k] * sn[t][k] : v[t][k] * cs[t][k] + u[t][k] * sn[t][k];
+                    if (!rot[k]) x = u[t][k];
+                    if (j < len && d0 + 32 * k < dim) to[TRANS ? 32 * k * kChunkT : 32 * k] = x * mul * w;
+                }
+            }
+        }
     }
+    if (!TRANS)
+        for (int i = threadIdx.x; i < len * (rs - dim); i += blockDim.x) dst[i / (rs - dim) * rs + dim + i % (rs - dim)] = 0.f;
 }
 
-template <int NACC>   // accumulators per thread (a multiple of 4): dim <= 4 * NACC
+// What bounds these kernels is fp32 arithmetic (two columns and NACC rows of the state per thread: NACC packed products of two per 16-byte read of Kw), once the
+// loads come in groups. 4 entries of 312 to 512 tokens, 4 heads of 128 x 256: 78 us with a load per token and column, one behind the other, now see below.
+template <int NACC, bool FULL>   // accumulators per thread (a multiple of 4): dim <= 4 * NACC, FULL: equal
 __global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc) {
     pdl_wait();
     pdl_launch_dependents();
@@ -135,77 +178,108 @@ __global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc)
     const float decay = a.decay[h];
     for (int j = threadIdx.x; j < len; j += blockDim.x) pw[j] = powf(decay, (float)(len - 1 - j));
     __syncthreads();
-    stage_rotated(a, Kw, a.k_off, h, row0, len, a.k_scale, pw);
+    stage_rotated<false>(a, Kw, a.k_off, h, row0, len, a.k_scale, pw);
     __syncthreads();
     // thread: kColsPerThread value columns, NACC consecutive rows of the state (read from shared memory four at a time)
     const int c = cb * kChunkCols + (threadIdx.x & 63), d0 = (threadIdx.x >> 6) * NACC, dpad = (dim + 3) & ~3;
-    float acc[kColsPerThread][NACC];
+    uint64_t acc[kColsPerThread][NACC / 2];
 #pragma unroll
     for (int q = 0; q < kColsPerThread; ++q)
 #pragma unroll
-        for (int k = 0; k < NACC; ++k) acc[q][k] = 0.f;
+        for (int k = 0; k < NACC / 2; ++k) acc[q][k] = 0ull;
     if (c < a.vdim && d0 < dim) {
         const float* vcol = a.proj + (size_t)row0 * a.ld_proj + a.v_off + h * a.vdim + c;
-        for (int j = 0; j < len; ++j) {
-            float v[kColsPerThread];
+        constexpr int J = 8;
+        int off[kColsPerThread];
 #pragma unroll
-            for (int q = 0; q < kColsPerThread; ++q) v[q] = c + 64 * q < a.vdim ? vcol[(size_t)j * a.ld_proj + 64 * q] : 0.f;
+        for (int q = 0; q < kColsPerThread; ++q) off[q] = c + 64 * q < a.vdim ? 64 * q : 0;
+        auto load = [&](int j0, float (&v)[J][kColsPerThread]) {
+#pragma unroll
+            for (int x = 0; x < J; ++x)
+#pragma unroll
+                for (int q = 0; q < kColsPerThread; ++q) v[x][q] = vcol[(size_t)min(j0 + x, len - 1) * a.ld_proj + off[q]];
+        };
+        auto product = [&](int j, const float (&v)[kColsPerThread]) {
+            uint64_t v2[kColsPerThread];
+#pragma unroll
+            for (int q = 0; q < kColsPerThread; ++q) v2[q] = pack2f(v[q], v[q]);
             const float* kr = Kw + j * rs + d0;
 #pragma unroll
             for (int k = 0; k < NACC; k += 4)
-                if (d0 + k < dpad) {
-                    const float4 k4 = *reinterpret_cast<const float4*>(kr + k);
+                if (FULL || d0 + k < dpad) {
+                    const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kr + k);
 #pragma unroll
                     for (int q = 0; q < kColsPerThread; ++q) {
-                        acc[q][k] = fmaf(k4.x, v[q], acc[q][k]);
-                        acc[q][k + 1] = fmaf(k4.y, v[q], acc[q][k + 1]);
-                        acc[q][k + 2] = fmaf(k4.z, v[q], acc[q][k + 2]);
-                        acc[q][k + 3] = fmaf(k4.w, v[q], acc[q][k + 3]);
+                        acc[q][k / 2] = fma2(k4.x, v2[q], acc[q][k / 2]);
+                        acc[q][k / 2 + 1] = fma2(k4.y, v2[q], acc[q][k / 2 + 1]);
                     }
                 }
+        };
+        float v[J][kColsPerThread], next[J][kColsPerThread];
+        load(0, next);
+        int j0 = 0;
+        for (; j0 + J <= len; j0 += J) {
+#pragma unroll
+            for (int x = 0; x < J; ++x)
+#pragma unroll
+                for (int q = 0; q < kColsPerThread; ++q) v[x][q] = next[x][q];
+            load(j0 + J, next);
+#pragma unroll
+            for (int x = 0; x < J; ++x) product(j0 + x, v[x]);
         }
+#pragma unroll
+        for (int x = 0; x < J; ++x)
+            if (j0 + x < len) product(j0 + x, next[x]);
         float* U = rc.chunk_state + (((size_t)(row_e / kChunk + e + c_in) * a.heads + h) * dim) * a.vdim + c;
 #pragma unroll
         for (int q = 0; q < kColsPerThread; ++q)
             if (c + 64 * q < a.vdim)
 #pragma unroll
-                for (int k = 0; k < NACC; ++k)
-                    if (d0 + k < dim) U[(size_t)(d0 + k) * a.vdim + 64 * q] = acc[q][k];
+                for (int k = 0; k < NACC; k += 2) {
+                    float lo, hi;
+                    unpack2(acc[q][k / 2], lo, hi);
+                    if (d0 + k < dim) U[(size_t)(d0 + k) * a.vdim + 64 * q] = lo;
+                    if (d0 + k + 1 < dim) U[(size_t)(d0 + k + 1) * a.vdim + 64 * q] = hi;
+                }
     }
 }
 
-// element-wise over (dim, vdim): walks the entry's chunks, leaves S at each chunk's start in place of its U
+// element-wise over (dim, vdim), VEC consecutive elements per thread: walks the entry's chunks, leaves S at each chunk's start in place of its U
+__device__ __forceinline__ float retention_next(float S, float d, float u) { return fmaf(d, S, u); }
+__device__ __forceinline__ float4 retention_next(float4 S, float d, float4 u) { return make_float4(fmaf(d, S.x, u.x), fmaf(d, S.y, u.y), fmaf(d, S.z, u.z), fmaf(d, S.w, u.w)); }
+template <typename V>
 __global__ void __launch_bounds__(256) retention_chunk_scan_kernel(const RC rc) {
     pdl_wait();
     pdl_launch_dependents();
     const RT& a = rc.a;
     const int e = blockIdx.x, h = blockIdx.y, i = blockIdx.z * blockDim.x + threadIdx.x;
-    const int per = a.dim * a.vdim;
+    const int per = a.dim * a.vdim / (int)(sizeof(V) / 4);
     if (i >= per) return;
     const int row_e = a.ent_row[e], n = a.ent_len[e], b = a.slot[row_e], p0 = a.pos[row_e];
     const float decay = a.decay[h];
-    float* sp = a.state + ((size_t)b * a.heads + h) * per + i;
-    float S = p0 > 0 ? *sp : 0.f;
-    const float full = powf(decay, (float)kChunk);
+    V* sp = reinterpret_cast<V*>(a.state) + ((size_t)b * a.heads + h) * per + i;
+    V S{};
+    if (p0 > 0) S = *sp;
     const int chunks = (n + kChunk - 1) / kChunk;
-    float* U = rc.chunk_state + ((size_t)(row_e / kChunk + e) * a.heads + h) * per + i;
+    const float full = powf(decay, (float)kChunk), tail = powf(decay, (float)(n - (chunks - 1) * kChunk));
+    V* U = reinterpret_cast<V*>(rc.chunk_state) + ((size_t)(row_e / kChunk + e) * a.heads + h) * per + i;
     const size_t step = (size_t)a.heads * per;
     for (int c0 = 0; c0 < chunks; c0 += 8) {   // eight loads in flight, then the dependent chain
-        float u[8];
+        V u[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) u[k] = c0 + k < chunks ? U[(size_t)(c0 + k) * step] : 0.f;
+        for (int k = 0; k < 8; ++k) u[k] = __ldcg(U + (size_t)min(c0 + k, chunks - 1) * step);   // (behind a condition each would wait for the one before)
 #pragma unroll
         for (int k = 0; k < 8; ++k)
             if (c0 + k < chunks) {
-                const int len = min(kChunk, n - (c0 + k) * kChunk);
                 U[(size_t)(c0 + k) * step] = S;
-                S = fmaf(len == kChunk ? full : powf(decay, (float)len), S, u[k]);
+                S = retention_next(S, c0 + k + 1 < chunks ? full : tail, u[k]);
             }
     }
     *sp = S;
 }
 
-__global__ void __launch_bounds__(256) retention_chunk_out_kernel(const RC rc) {
+// Thread: columns c, c + 64; sixteen consecutive rows, two per packed product (q and A lie transposed: a 16-byte read is four rows of one j or component).
+__global__ void __launch_bounds__(256, 2) retention_chunk_out_kernel(const RC rc) {
     pdl_wait();
     pdl_launch_dependents();
     extern __shared__ __align__(16) float sm[];
@@ -214,82 +288,114 @@ __global__ void __launch_bounds__(256) retention_chunk_out_kernel(const RC rc) {
     const int c_in = blockIdx.y, h = blockIdx.z;
     const int row_e = a.ent_row[e], n = a.ent_len[e];
     if (c_in * kChunk >= n) return;
-    const int row0 = row_e + c_in * kChunk, len = min(kChunk, n - c_in * kChunk), dim = a.dim, rs = chunk_row_stride(dim);
-    constexpr int AS = kChunk + 4;                // row stride of A in floats
-    float* Qc = sm;                               // [kChunk][rs]
-    float* Kc = Qc + kChunk * rs;                 // [kChunk][rs]
-    float* A = Kc + kChunk * rs;                  // [kChunk][AS]
-    float* pw = A + kChunk * AS;                  // [kChunk + 1]: decay^k
+    const int row0 = row_e + c_in * kChunk, len = min(kChunk, n - c_in * kChunk), dim = a.dim;
+    float* Qt = sm;                               // [dim][kChunkT]
+    float* Kt = Qt + dim * kChunkT;               // [dim][kChunkT]
+    float* At = Kt + dim * kChunkT;               // [j][kChunkT]: row i of A at At[j][i]
+    float* pw = At + kChunk * kChunkT;            // [kChunk + 1]: decay^k
     const float decay = a.decay[h];
     for (int k = threadIdx.x; k <= kChunk; k += blockDim.x) pw[k] = powf(decay, (float)k);
-    stage_rotated(a, Qc, a.q_off, h, row0, len, 1.f, nullptr);
-    stage_rotated(a, Kc, a.k_off, h, row0, len, a.k_scale, nullptr);
+    if (len < kChunk)   // rows and columns behind the entry: the tiles below read them
+        for (int i = threadIdx.x; i < 2 * dim * (kChunk - len); i += blockDim.x) Qt[i / (kChunk - len) * kChunkT + len + i % (kChunk - len)] = 0.f;
+    stage_rotated<true>(a, Qt, a.q_off, h, row0, len, 1.f, nullptr);
+    stage_rotated<true>(a, Kt, a.k_off, h, row0, len, a.k_scale, nullptr);
     __syncthreads();
-    const int dpad = (dim + 3) & ~3;
-    for (int idx = threadIdx.x; idx < kChunk * kChunk; idx += blockDim.x) {
-        const int i = idx / kChunk, j = idx % kChunk;
-        float v = 0.f;
-        if (j <= i && i < len) {
-            const float* q = Qc + i * rs;
-            const float* k = Kc + j * rs;
-            for (int d = 0; d < dpad; d += 4) {
-                const float4 q4 = *reinterpret_cast<const float4*>(q + d), k4 = *reinterpret_cast<const float4*>(k + d);
-                v = fmaf(q4.x, k4.x, v); v = fmaf(q4.y, k4.y, v); v = fmaf(q4.z, k4.z, v); v = fmaf(q4.w, k4.w, v);
+    {   // q . k in tiles of four rows and four columns
+        const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+        uint64_t t[4][2];   // [column][row pair]
+#pragma unroll
+        for (int y = 0; y < 4; ++y) t[y][0] = t[y][1] = 0ull;
+        if (tj <= ti)
+#pragma unroll 4
+            for (int d = 0; d < dim; ++d) {
+                const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(Qt + d * kChunkT + ti * 4);
+                const float4 k4 = *reinterpret_cast<const float4*>(Kt + d * kChunkT + tj * 4);
+                const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const uint64_t k2 = pack2f(kk[y], kk[y]);
+                    t[y][0] = fma2(q4.x, k2, t[y][0]);
+                    t[y][1] = fma2(q4.y, k2, t[y][1]);
+                }
             }
-            v *= pw[i - j];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            float f[4];
+            unpack2(t[y][0], f[0], f[1]);
+            unpack2(t[y][1], f[2], f[3]);
+            const int jj = tj * 4 + y;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int i = ti * 4 + x;
+                f[x] = jj <= i && i < len ? f[x] * pw[i - jj] : 0.f;
+            }
+            *reinterpret_cast<float4*>(At + jj * kChunkT + ti * 4) = make_float4(f[0], f[1], f[2], f[3]);
         }
-        A[i * AS + j] = v;
     }
     __syncthreads();
-    const int c = cb * kChunkCols + (threadIdx.x & 63), rg = threadIdx.x >> 6;   // thread: columns c, c + 64; rows rg, rg + 4, ...
-    if (c >= a.vdim) return;
-    constexpr int NR = kChunk / 4, CP = kColsPerThread;
-    float acc[CP][NR], cross[CP][NR];
+    const int c = cb * kChunkCols + (threadIdx.x & 63), r0 = (threadIdx.x >> 6) * 16;
+    if (c >= a.vdim || r0 >= len) return;
+    constexpr int CP = kColsPerThread, J = 8;
+    uint64_t acc[CP][8], cross[CP][8];
 #pragma unroll
     for (int q = 0; q < CP; ++q)
 #pragma unroll
-        for (int k = 0; k < NR; ++k) acc[q][k] = cross[q][k] = 0.f;
-    const float* vcol = a.proj + (size_t)row0 * a.ld_proj + a.v_off + h * a.vdim + c;
-    for (int j = 0; j < len; j += 4) {
-        float v[CP][4];
+        for (int k = 0; k < 8; ++k) acc[q][k] = cross[q][k] = 0ull;
+    int off[CP];
 #pragma unroll
-        for (int q = 0; q < CP; ++q)
+    for (int q = 0; q < CP; ++q) off[q] = c + 64 * q < a.vdim ? 64 * q : 0;
+    // `rows` rows of `src` (leading dimension ld), eight at a time ahead of the eight in use, times the sixteen of m
+    auto products = [&](const float* src, long long ld, int rows, const float* m, uint64_t (&to)[CP][8]) {
+        float v[J][CP], next[J][CP];
+        auto load = [&](int at, float (&x)[J][CP]) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) v[q][x] = (j + x < len && c + 64 * q < a.vdim) ? vcol[(size_t)(j + x) * a.ld_proj + 64 * q] : 0.f;
+            for (int y = 0; y < J; ++y)
 #pragma unroll
-        for (int k = 0; k < NR; ++k) {
-            const float4 a4 = *reinterpret_cast<const float4*>(A + (rg + 4 * k) * AS + j);
+                for (int q = 0; q < CP; ++q) x[y][q] = src[(size_t)min(at + y, rows - 1) * ld + off[q]];
+        };
+        auto product = [&](int at, const float (&x)[CP]) {
+            uint64_t v2[CP];
 #pragma unroll
-            for (int q = 0; q < CP; ++q) {
-                acc[q][k] = fmaf(a4.x, v[q][0], acc[q][k]); acc[q][k] = fmaf(a4.y, v[q][1], acc[q][k]);
-                acc[q][k] = fmaf(a4.z, v[q][2], acc[q][k]); acc[q][k] = fmaf(a4.w, v[q][3], acc[q][k]);
+            for (int q = 0; q < CP; ++q) v2[q] = pack2f(x[q], x[q]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const ulonglong2 m4 = *reinterpret_cast<const ulonglong2*>(m + at * kChunkT + r0 + 4 * k);
+#pragma unroll
+                for (int q = 0; q < CP; ++q) {
+                    to[q][2 * k] = fma2(m4.x, v2[q], to[q][2 * k]);
+                    to[q][2 * k + 1] = fma2(m4.y, v2[q], to[q][2 * k + 1]);
+                }
             }
+        };
+        load(0, next);
+        int at = 0;
+        for (; at + J <= rows; at += J) {
+#pragma unroll
+            for (int y = 0; y < J; ++y)
+#pragma unroll
+                for (int q = 0; q < CP; ++q) v[y][q] = next[y][q];
+            load(at + J, next);
+#pragma unroll
+            for (int y = 0; y < J; ++y) product(at + y, v[y]);
         }
-    }
-    const float* S = rc.chunk_state + (((size_t)(row_e / kChunk + e + c_in) * a.heads + h) * dim) * a.vdim + c;
-    for (int d = 0; d < dpad; d += 4) {
-        float sv[CP][4];
 #pragma unroll
-        for (int q = 0; q < CP; ++q)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) sv[q][x] = (d + x < dim && c + 64 * q < a.vdim) ? S[(size_t)(d + x) * a.vdim + 64 * q] : 0.f;
-#pragma unroll
-        for (int k = 0; k < NR; ++k) {
-            const float4 q4 = *reinterpret_cast<const float4*>(Qc + (rg + 4 * k) * rs + d);
-#pragma unroll
-            for (int q = 0; q < CP; ++q) {
-                cross[q][k] = fmaf(q4.x, sv[q][0], cross[q][k]); cross[q][k] = fmaf(q4.y, sv[q][1], cross[q][k]);
-                cross[q][k] = fmaf(q4.z, sv[q][2], cross[q][k]); cross[q][k] = fmaf(q4.w, sv[q][3], cross[q][k]);
-            }
-        }
-    }
+        for (int y = 0; y < J; ++y)
+            if (at + y < rows) product(at + y, next[y]);
+    };
+    products(a.proj + (size_t)row0 * a.ld_proj + a.v_off + h * a.vdim + c, a.ld_proj, min(len, r0 + 16), At, acc);
+    products(rc.chunk_state + (((size_t)(row_e / kChunk + e + c_in) * a.heads + h) * dim) * a.vdim + c, a.vdim, dim, Qt, cross);
 #pragma unroll
     for (int q = 0; q < CP; ++q)
 #pragma unroll
-        for (int k = 0; k < NR; ++k) {
-            const int i = rg + 4 * k;
-            if (i < len && c + 64 * q < a.vdim)
-                a.out[(size_t)(row0 + i) * ((size_t)a.heads * a.vdim) + h * a.vdim + c + 64 * q] = fmaf(pw[i + 1], cross[q][k], acc[q][k]);
+        for (int k = 0; k < 8; ++k) {
+            float x[2], y[2];
+            unpack2(cross[q][k], x[0], x[1]);
+            unpack2(acc[q][k], y[0], y[1]);
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+                const int i = r0 + 2 * k + z;
+                if (i < len && c + 64 * q < a.vdim) a.out[(size_t)(row0 + i) * ((size_t)a.heads * a.vdim) + h * a.vdim + c + 64 * q] = fmaf(pw[i + 1], x[z], y[z]);
+            }
         }
 }
 
@@ -403,19 +509,30 @@ extern "C" int b200_retention(const b200_retention_args* p, void* stream) {
         const dim3 grid(p->n_entries * col_blocks, chunks, p->heads);
         const int rs = chunk_row_stride(p->dim);
         const size_t smem1 = ((size_t)kChunk * rs + kChunk) * sizeof(float);
-        const size_t smem3 = ((size_t)2 * kChunk * rs + kChunk * (kChunk + 4) + kChunk + 4) * sizeof(float);
-        static unsigned long long done1[4] = {0, 0, 0, 0}, done3 = 0;
+        const size_t smem3 = ((size_t)2 * p->dim * kChunkT + kChunk * kChunkT + kChunk + 4) * sizeof(float);
+        static unsigned long long done1[8] = {}, done3 = 0;
         // the attribute is set once per kernel: to the most any supported dim (256) needs
-        constexpr int kMax1 = (kChunk * 260 + kChunk) * 4, kMax3 = (2 * kChunk * 260 + kChunk * (kChunk + 4) + kChunk + 4) * 4;
+        constexpr int kMax1 = (kChunk * 260 + kChunk) * 4, kMax3 = (2 * 256 * kChunkT + kChunk * kChunkT + kChunk + 4) * 4;
         cudaError_t e = ensure_max_dynamic_smem((const void*)retention_chunk_out_kernel, kMax3, done3);
         if (e != cudaSuccess) return (int)e;
         rc.col_blocks = col_blocks;
-        if (p->dim <= 32) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<8>, kMax1, done1[0]); launch_chained(retention_chunk_state_kernel<8>, grid, 256, smem1, s, rc); }
-        else if (p->dim <= 64) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<16>, kMax1, done1[1]); launch_chained(retention_chunk_state_kernel<16>, grid, 256, smem1, s, rc); }
-        else if (p->dim <= 128) { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<32>, kMax1, done1[2]); launch_chained(retention_chunk_state_kernel<32>, grid, 256, smem1, s, rc); }
-        else { ensure_max_dynamic_smem((const void*)retention_chunk_state_kernel<64>, kMax1, done1[3]); launch_chained(retention_chunk_state_kernel<64>, grid, 256, smem1, s, rc); }
+        auto state = [&](auto kernel, unsigned long long& done) {
+            ensure_max_dynamic_smem((const void*)kernel, kMax1, done);
+            launch_chained(kernel, grid, 256, smem1, s, rc);
+        };
+        if (p->dim < 32) state(retention_chunk_state_kernel<8, false>, done1[0]);
+        else if (p->dim == 32) state(retention_chunk_state_kernel<8, true>, done1[1]);
+        else if (p->dim < 64) state(retention_chunk_state_kernel<16, false>, done1[2]);
+        else if (p->dim == 64) state(retention_chunk_state_kernel<16, true>, done1[3]);
+        else if (p->dim < 128) state(retention_chunk_state_kernel<32, false>, done1[4]);
+        else if (p->dim == 128) state(retention_chunk_state_kernel<32, true>, done1[5]);
+        else if (p->dim < 256) state(retention_chunk_state_kernel<64, false>, done1[6]);
+        else state(retention_chunk_state_kernel<64, true>, done1[7]);
         const int per = p->dim * p->vdim;
-        launch_chained(retention_chunk_scan_kernel, dim3(p->n_entries, p->heads, (per + 255) / 256), 256, 0, s, rc);
+        if (per % 4 == 0 && ((reinterpret_cast<uintptr_t>(p->state) | reinterpret_cast<uintptr_t>(p->workspace)) & 15u) == 0)
+            launch_chained(retention_chunk_scan_kernel<float4>, dim3(p->n_entries, p->heads, (per / 4 + 255) / 256), 256, 0, s, rc);
+        else
+            launch_chained(retention_chunk_scan_kernel<float>, dim3(p->n_entries, p->heads, (per + 255) / 256), 256, 0, s, rc);
         launch_chained(retention_chunk_out_kernel, grid, 256, smem3, s, rc);
         count_launch(3);
         return (int)cudaGetLastError();
