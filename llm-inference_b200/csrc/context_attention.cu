@@ -124,7 +124,7 @@ context_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int ctx_len = hist + in_len;
     const int q_hi = min(q0 + kCtxTile, in_len);
     const int kv_end = hist + q_hi;                     // keys [0, kv_end) are visible to this tile
-    const int n_kt = (kv_end + kCtxTile - 1) / kCtxTile;
+    const int n_kt = __shfl_sync(0xffffffffu, (kv_end + kCtxTile - 1) / kCtxTile, 0);
     const int kvh = head / (p.head_num / p.kv_head_num);
 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBar);
@@ -141,7 +141,7 @@ context_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     float* alpha_s = reinterpret_cast<float*>(smem + kOffAlpha);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffSlot);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         if (smem_u32(smem) & 1023u) __trap();   // swizzled tiles need a 1024-byte aligned base
         mbar_init(q_full, 1);
@@ -165,7 +165,7 @@ context_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_launch_dependents();
 
     if (warp == 0) {
@@ -204,21 +204,21 @@ context_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // ================= MMA issuer =================
         constexpr uint32_t idesc_s = make_idesc_f16(kCtxTile, kCtxTile);       // A, B K-major
         constexpr uint32_t idesc_pv = idesc_s | (1u << 16);                    // B (= V) MN-major
-        const uint32_t q_addr = smem_u32(smem + kOffQ);
+        const uint64_t q_desc = make_kmajor_sw128_desc(smem_u32(smem + kOffQ)), k_desc = make_kmajor_sw128_desc(smem_u32(smem + kOffK)), p_desc = make_kmajor_sw128_desc(smem_u32(smem + kOffP));
+        const uint64_t v_desc = make_mnmajor_sw128_desc(smem_u32(smem + kOffV), kBoxBytes, 1024u);
+        const bool leader = elect_one();   // (descriptors from values that are uniform over the warp: see gemm_tcgen05_kernel)
         auto issue_s = [&](int j) {
             const int s = j & 1;
             const uint32_t ph = (uint32_t)(j >> 1) & 1u;
             ctx_wait(&k_full[s], ph);
             ctx_wait(&s_empty[s], ph ^ 1u);
             tc_fence_after();
-            if (lane == 0) {
-                const uint32_t k_addr = smem_u32(smem + kOffK + (uint32_t)s * kTileBytes);
+            if (leader) {
+                const uint64_t kd = k_desc + (uint64_t)(s * (int)(kTileBytes >> 4));
 #pragma unroll
                 for (int ks = 0; ks < kCtxTile / kUmmaK; ++ks) {
-                    const uint32_t off = (uint32_t)(ks >> 2) * kBoxBytes;
-                    umma_f16(tmem_base + (uint32_t)(s * kCtxTile),
-                             make_kmajor_sw128_desc(q_addr + off) + (uint64_t)(2 * (ks & 3)),
-                             make_kmajor_sw128_desc(k_addr + off) + (uint64_t)(2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
+                    const uint64_t off = (uint64_t)((ks >> 2) * (int)(kBoxBytes >> 4) + 2 * (ks & 3));
+                    umma_f16(tmem_base + (uint32_t)(s * kCtxTile), q_desc + off, kd + off, idesc_s, ks > 0 ? 1u : 0u);
                 }
                 umma_commit(&k_empty[s]);
                 umma_commit(&s_full[s]);
@@ -233,15 +233,12 @@ context_attn_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             ctx_wait(&p_full[s], ph);
             ctx_wait(&o_empty[s], ph ^ 1u);
             tc_fence_after();
-            if (lane == 0) {
-                const uint32_t p_addr = smem_u32(smem + kOffP + (uint32_t)s * kTileBytes);
-                const uint32_t v_addr = smem_u32(smem + kOffV + (uint32_t)s * kTileBytes);
+            if (leader) {
+                const uint64_t pd = p_desc + (uint64_t)(s * (int)(kTileBytes >> 4)), vd = v_desc + (uint64_t)(s * (int)(kTileBytes >> 4));
 #pragma unroll
                 for (int ks = 0; ks < kCtxTile / kUmmaK; ++ks) {
                     // 16 keys = two 8-row groups of 1024 bytes; the two 64-wide halves of d are 16 KB apart
-                    const uint64_t dv = make_mnmajor_sw128_desc(v_addr + (uint32_t)ks * 2048u, kBoxBytes, 1024u);
-                    umma_f16(tmem_base + (uint32_t)(256 + s * kCtxTile),
-                             make_kmajor_sw128_desc(p_addr + (uint32_t)(ks >> 2) * kBoxBytes) + (uint64_t)(2 * (ks & 3)), dv,
+                    umma_f16(tmem_base + (uint32_t)(256 + s * kCtxTile), pd + (uint64_t)((ks >> 2) * (int)(kBoxBytes >> 4) + 2 * (ks & 3)), vd + (uint64_t)(ks * (2048 >> 4)),
                              idesc_pv, ks > 0 ? 1u : 0u);
                 }
                 umma_commit(&v_empty[s]);

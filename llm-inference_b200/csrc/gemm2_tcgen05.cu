@@ -164,7 +164,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     uint64_t* acc_full = empty_bar + k2Stages;   // [2]
     uint64_t* acc_empty = acc_full + 2;          // [2], used in the leader only
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + k2OffSlot);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();     // 0 = leader
     if (threadIdx.x == 0) {
         if (smem_u32(smem) & 1023u) __trap();
@@ -185,7 +185,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __syncthreads();
     cluster_sync_all();   // the peer's barriers exist before anything is signalled on them
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_launch_dependents();
     pdl_wait();
 
@@ -218,6 +218,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // ================= MMA issuer (leader CTA only) =================
         if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_f16(256, 256);
+            const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(smem)), b_desc = make_kmajor_sw128_desc(smem_u32(smem) + k2ABytes);
+            const bool leader = elect_one();   // (descriptors from values that are uniform over the warp: see gemm_tcgen05_kernel)
             int stage = 0, acc = 0;
             uint32_t phase = 0, acc_phase = 0;
             for (int u = cluster_id; u < units; u += n_clusters) {
@@ -227,10 +229,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
                     mbar_wait_bounded(&full_bar[stage], phase);
                     tc_fence_after();
-                    if (lane == 0) {
-                        const uint32_t sa = smem_u32(smem + (size_t)stage * k2StageBytes);
-                        const uint64_t da = make_kmajor_sw128_desc(sa);
-                        const uint64_t db = make_kmajor_sw128_desc(sa + k2ABytes);
+                    if (leader) {
+                        const uint64_t da = a_desc + (uint64_t)(stage * (k2StageBytes >> 4)), db = b_desc + (uint64_t)(stage * (k2StageBytes >> 4));
 #pragma unroll
                         for (int k = 0; k < k2BK / kUmmaK; ++k)
                             umma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
@@ -306,7 +306,7 @@ gemm2w_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     uint64_t* acc_full = empty_bar + kwStages;   // [2]: accumulator h of the current unit is complete
     uint64_t* acc_empty = acc_full + 2;          // [2], leader only: accumulator h has been drained by both CTAs
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kwOffSlot);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();     // 0 = leader
     if (threadIdx.x == 0) {
         if (smem_u32(smem) & 1023u) __trap();
@@ -327,7 +327,7 @@ gemm2w_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     __syncthreads();
     cluster_sync_all();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_launch_dependents();
     pdl_wait();
 
@@ -374,6 +374,8 @@ gemm2w_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         // ================= MMA issuer (leader CTA only) =================
         if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_f16(256, 256);
+            const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(smem));
+            const bool leader = elect_one();   // (see gemm_tcgen05_kernel)
             int stage = 0;
             uint32_t phase = 0, acc_phase = 0;
             for (int v = cluster_id; v < items; v += n_clusters) {
@@ -381,15 +383,14 @@ gemm2w_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                 item(v, u, hsel);
                 for (int kb = 0; kb < p.k_blocks; ++kb) {
                     mbar_wait_bounded(&full_bar[stage], phase);
-                    const uint32_t sa = smem_u32(smem + (size_t)stage * kwStageBytes);
-                    const uint64_t da = make_kmajor_sw128_desc(sa);
+                    const uint64_t da = a_desc + (uint64_t)(stage * (kwStageBytes >> 4));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         // the previous unit's accumulator h must have been drained before its first MMA overwrites it
                         if (kb == 0) mbar_wait_bounded(&acc_empty[h], acc_phase ^ 1);
                         tc_fence_after();
-                        if (lane == 0 && (hsel < 0 || hsel == h)) {
-                            const uint64_t db = make_kmajor_sw128_desc(sa + k2ABytes + (uint32_t)h * k2BBytes);
+                        if (leader && (hsel < 0 || hsel == h)) {
+                            const uint64_t db = da + (uint64_t)((k2ABytes + (uint32_t)h * k2BBytes) >> 4);
 #pragma unroll
                             for (int k = 0; k < k2BK / kUmmaK; ++k)
                                 umma_f16_pair(tmem_base + (uint32_t)(h * 256), da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
@@ -397,7 +398,7 @@ gemm2w_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                         }
                         __syncwarp();
                     }
-                    if (lane == 0) {
+                    if (leader) {
                         umma_commit_pair(&empty_bar[stage], 3);                      // both producers may refill
                         if (kb == p.k_blocks - 1) {                                  // both epilogues may read
                             umma_commit_pair(&acc_full[0], 3);

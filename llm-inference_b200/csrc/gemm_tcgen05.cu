@@ -156,7 +156,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     uint64_t* acc_empty = acc_full + 2;        // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full_bar[s], 1);
@@ -174,7 +174,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_launch_dependents();
     pdl_wait();   // x (and, for PDL chains, the previous kernel's output) must be complete
 
@@ -206,7 +206,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp == 1) {
         // ================= MMA issuer =================
         // bfloat16 operands: A format (bits [7,10)) and B format (bits [10,13)) = 1
+        // (descriptors and addresses from values that are uniform over the warp, one elected lane: from lane 0's own registers the four products of a stage
+        // took 560 clocks to issue, whatever their size. 512 x 8192 -> 2048 in tiles of 128 x 64: 41 -> 25 us, 128 x 128: 43 -> 31; 128 x 256, where the operands' way
+        // into shared memory takes longer, 52 -> 50)
         const uint32_t idesc = make_idesc_f16(kBM, BN) | (p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+        const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(tiles)), b_desc = make_kmajor_sw128_desc(smem_u32(tiles) + A_BYTES);
+        const bool leader = elect_one();
         int stage = 0;
         uint32_t phase = 0;
         int acc = 0;
@@ -218,10 +223,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int kb = 0; kb < p.k_blocks; ++kb) {
                 mbar_wait(&full_bar[stage], phase);
                 tc_fence_after();
-                if (lane == 0) {
-                    const uint32_t sa = smem_u32(tiles + (size_t)stage * S::kStageBytes);
-                    const uint64_t da = make_kmajor_sw128_desc(sa);
-                    const uint64_t db = make_kmajor_sw128_desc(sa + A_BYTES);
+                if (leader) {
+                    const uint64_t da = a_desc + (uint64_t)(stage * (S::kStageBytes >> 4)), db = b_desc + (uint64_t)(stage * (S::kStageBytes >> 4));
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k)
                         umma_f16(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc,
@@ -352,7 +355,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* om = reinterpret_cast<float*>(tiles);   // [tokens][128]: this CTA's sums, once the stages have been used
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int sp = blockIdx.x % p.splits, mt = blockIdx.x / p.splits;
     const int kb0 = (int)((long long)p.k_blocks * sp / p.splits), kb1 = (int)((long long)p.k_blocks * (sp + 1) / p.splits);
     if (threadIdx.x == 0) {
@@ -371,7 +374,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_launch_dependents();
     pdl_wait();
 
@@ -395,6 +398,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
     } else if (warp == 1) {
         const uint32_t idesc = make_idesc_f16(kBM, BN) | (p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+        const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(tiles)), b_desc = make_kmajor_sw128_desc(smem_u32(tiles) + A_BYTES);
+        const bool leader = elect_one();
         auto chain_end = [&](int i) { return p.accs == 1 ? kb1 : kb0 + (kb1 - kb0) * (i + 1) / p.accs; };
         int stage = 0, at = 0, end = chain_end(0);
         bool fresh = true;   // the first products of a chain
@@ -404,9 +409,8 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             if (FOLD && fresh && at >= 2) mbar_wait_or_leave(&acc_empty[slot], (uint32_t)((at >> 1) - 1) & 1u, dead);
             mbar_wait_or_leave(&full_bar[stage], phase, dead);
             tc_fence_after();
-            if (lane == 0) {
-                const uint32_t sa = smem_u32(tiles + (size_t)stage * S::kStageBytes);
-                const uint64_t da = make_kmajor_sw128_desc(sa), db = make_kmajor_sw128_desc(sa + A_BYTES);
+            if (leader) {
+                const uint64_t da = a_desc + (uint64_t)(stage * (S::kStageBytes >> 4)), db = b_desc + (uint64_t)(stage * (S::kStageBytes >> 4));
 #pragma unroll
                 for (int k = 0; k < kBK / kUmmaK; ++k)
                     umma_f16(tmem + (uint32_t)(slot * BN), da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (!fresh || k > 0) ? 1u : 0u);
