@@ -11,6 +11,10 @@
 //   warps 2-5 epilogue (both CTAs): own 128 rows from own TMEM, then a remote arrive on the leader's
 //             accumulator-empty barrier
 // GLU: as in gemm_tcgen05.cu — the leader's B half is 128 gate rows, the peer's the matching 128 up rows.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
 #include "common.cuh"
 #include "launch_count.h"
 #include "tc_common.cuh"
@@ -36,6 +40,8 @@ struct Gemm2Params {
     int ldc, k_blocks;
     int m_tiles, n_tiles;   // tiles of 256 rows x (256 features | GLU: 128 features)
     int group_m;            // tile order: bands of group_m row tiles swept over all column tiles (0: column-major over all rows)
+    int in_bf16, out_kind, glu_act, unary;   // the families' calls (KIND 2 and 3 of the kernel), as GemmParams in gemm_tcgen05.cu
+    float glu_limit;
     int wide_full;          // wide kernel: units [0, wide_full) are 256 x 512, the rest is run as single 256 x 256 column tiles
 };
 
@@ -155,9 +161,84 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
     }
 }
 
-template <bool GLU>
+// The same for the families: bfloat16 or fp32 outputs, no bias; plain with an optional squared relu, or gated (silu, tanh-gelu, clamped) in fp32. A pass is
+// 64 output columns of bfloat16 or 32 of fp32, 128 bytes of a row in the stage.
+template <bool GLU, int ACT, bool F32>
+__device__ __forceinline__ void store_tile_warp_ex(const Gemm2Params& p, uint32_t taddr, int row0, int nt, uint32_t stg, int lane) {
+    constexpr int kOutCols = GLU ? 128 : 256, kPass = F32 ? 32 : 64;
+    const int tile_col0 = nt * kOutCols;
+    if (row0 >= p.tokens) return;
+    const bool vec_ok = (p.ldc & (F32 ? 3 : 7)) == 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < kOutCols && tile_col0 + c0 < p.n_out; c0 += kPass) {
+#pragma unroll 1
+        for (int cc = c0; cc < c0 + kPass; cc += 16) {
+            uint32_t v[16], u[16];
+            __syncwarp();   // the loads of tensor memory are warp-wide
+            tmem_ld_32x16_async(taddr + (uint32_t)cc, v);
+            if (GLU) tmem_ld_32x16_async(taddr + (uint32_t)(128 + cc), u);
+            tmem_wait_ld<16>(v);
+            if (GLU) tmem_wait_ld<16>(u);
+            float f[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float g = __uint_as_float(v[e]);
+                if (GLU) {
+                    const float w = __uint_as_float(u[e]);
+                    f[e] = ACT == 2 ? tile_glu_clamp(g, w, p.glu_limit) : (ACT == 1 ? tile_gelu_tanh(g) : tile_silu(g)) * w;
+                } else {
+                    const float r = fmaxf(g, 0.f);
+                    f[e] = p.unary == 1 ? r * r : g;
+                }
+            }
+            if (F32) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    stg_st_v4(stg + (uint32_t)lane * 128u + (uint32_t)((((cc - c0) / 4 + q) ^ (lane & 7)) << 4), __float_as_uint(f[4 * q]), __float_as_uint(f[4 * q + 1]), __float_as_uint(f[4 * q + 2]), __float_as_uint(f[4 * q + 3]));
+            } else {
+                uint32_t h[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+                    h[e] = *reinterpret_cast<const uint32_t*>(&b);
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    stg_st_v4(stg + (uint32_t)lane * 128u + (uint32_t)((((cc - c0) / 8 + q) ^ (lane & 7)) << 4), h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+            }
+        }
+        __syncwarp();
+        constexpr int kPiece = F32 ? 4 : 8;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int r = j * 4 + (lane >> 3), ch = lane & 7;
+            const uint4 val = stg_ld_v4(stg + (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4));
+            const int row = row0 + r, col = tile_col0 + c0 + ch * kPiece;
+            if (row < p.tokens && col < p.n_out) {
+                const size_t at = (size_t)row * p.ldc + col;
+                if (vec_ok && col + kPiece <= p.n_out) {
+                    if (F32) *reinterpret_cast<uint4*>(reinterpret_cast<float*>(p.C) + at) = val;
+                    else *reinterpret_cast<uint4*>(p.C + at) = val;
+                } else {
+                    const uint32_t w[4] = {val.x, val.y, val.z, val.w};
+#pragma unroll
+                    for (int e = 0; e < kPiece; ++e) {
+                        if (col + e >= p.n_out) continue;
+                        if (F32) reinterpret_cast<uint32_t*>(p.C)[at + e] = w[e];
+                        else reinterpret_cast<uint16_t*>(p.C)[at + e] = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// KIND 0: fp16, 1: fp16 gated; 2 and 3: the families' plain and gated outputs
+template <int KIND>
 __global__ void __launch_bounds__(k2Threads, 1)
 gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Gemm2Params p) {
+    constexpr bool GLU = (KIND & 1) != 0;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + k2OffBar);
     uint64_t* empty_bar = full_bar + k2Stages;
@@ -217,7 +298,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else if (warp == 1) {
         // ================= MMA issuer (leader CTA only) =================
         if (rank == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(256, 256);
+            const uint32_t idesc = make_idesc_f16(256, 256) | (KIND >= 2 && p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
             const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(smem)), b_desc = make_kmajor_sw128_desc(smem_u32(smem) + k2ABytes);
             const bool leader = elect_one();   // (descriptors from values that are uniform over the warp: see gemm_tcgen05_kernel)
             int stage = 0, acc = 0;
@@ -254,11 +335,18 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             tile_of_unit(p, p.n_tiles, u, mt, nt);
             mbar_wait_bounded(&acc_full[acc], acc_phase);
             tc_fence_after();
-            const int row = mt * 256 + (int)rank * 128 + quarter * 32 + lane;
-            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256);
-            (void)row;
-            store_tile_warp<GLU>(p, taddr, mt * 256 + (int)rank * 128 + quarter * 32, nt,
-                                 smem_u32(smem + k2OffStg + (uint32_t)(warp - 2) * kStgBytes), lane);
+            const int row0 = mt * 256 + (int)rank * 128 + quarter * 32;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256), stg = smem_u32(smem + k2OffStg + (uint32_t)(warp - 2) * kStgBytes);
+            if constexpr (KIND < 2) store_tile_warp<GLU>(p, taddr, row0, nt, stg, lane);
+            else if (p.out_kind == 2) {
+                if (!GLU || p.glu_act == 0) store_tile_warp_ex<GLU, 0, true>(p, taddr, row0, nt, stg, lane);
+                else if (p.glu_act == 1) store_tile_warp_ex<GLU, 1, true>(p, taddr, row0, nt, stg, lane);
+                else store_tile_warp_ex<GLU, 2, true>(p, taddr, row0, nt, stg, lane);
+            } else {
+                if (!GLU || p.glu_act == 0) store_tile_warp_ex<GLU, 0, false>(p, taddr, row0, nt, stg, lane);
+                else if (p.glu_act == 1) store_tile_warp_ex<GLU, 1, false>(p, taddr, row0, nt, stg, lane);
+                else store_tile_warp_ex<GLU, 2, false>(p, taddr, row0, nt, stg, lane);
+            }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[acc]), 0));
@@ -481,9 +569,9 @@ static int gemm2_launch_wide(const CUtensorMap& ma, const CUtensorMap& mb, const
     return (int)e;
 }
 
-template <bool GLU>
+template <int KIND>
 static int gemm2_launch(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm2Params& p, int grid, cudaStream_t s) {
-    auto kern = gemm2_tcgen05_kernel<GLU>;
+    auto kern = gemm2_tcgen05_kernel<KIND>;
     static unsigned long long attr_done = 0;   // per instantiation, one bit per device
     {
         cudaError_t e = ensure_max_dynamic_smem(reinterpret_cast<const void*>(kern), (int)k2Smem, attr_done);
@@ -521,9 +609,8 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
     static int mode = -1;   // B200_GEMM_PAIR=0 keeps the one-CTA kernel
     if (mode < 0) { const char* e = getenv("B200_GEMM_PAIR"); mode = (e && e[0] == '0') ? 0 : 1; }
     if (!mode) return B200_EUNSUPPORTED;
-    // below 512 token rows only the one case the caller has measured (gemm_tcgen05.cu: one row tile x >= 60 column tiles)
-    const bool one_row_tile = !glu && M > 160 && M <= 256 && (N + 255) / 256 >= 60;
-    if ((M < 512 && !one_row_tile) || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
+    // (plain products come by the rules of gemm_tcgen05.cu: plain_tile, and one row tile x >= 60 column tiles)
+    if ((glu ? M < 512 : M <= 160) || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
     if (glu && ((N & 127) || bias || residual)) return B200_EUNSUPPORTED;
     Gemm2Params p{};
     p.C = reinterpret_cast<__half*>(y);
@@ -563,7 +650,23 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
     const int units = p.m_tiles * p.n_tiles;
     int clusters = sm_count() / 2;
     if (clusters > units) clusters = units;
-    return glu ? gemm2_launch<true>(ma, mb, p, 2 * clusters, s) : gemm2_launch<false>(ma, mb, p, 2 * clusters, s);
+    return glu ? gemm2_launch<1>(ma, mb, p, 2 * clusters, s) : gemm2_launch<0>(ma, mb, p, 2 * clusters, s);
+}
+
+// The families' linears: fp16 or bfloat16 operands, outputs and epilogues as gemm_tcgen05_ex takes them (there is the rule that sends a call here); gated: W = [2 N, K], N % 128 == 0
+int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, cudaStream_t s) {
+    Gemm2Params p{};
+    p.C = reinterpret_cast<__half*>(y);
+    p.tokens = M; p.n_out = N; p.ldc = N;
+    p.k_blocks = (K + k2BK - 1) / k2BK;
+    p.m_tiles = (M + 255) / 256;
+    p.n_tiles = glu ? N / 128 : (N + 255) / 256;
+    p.group_m = 16;
+    p.in_bf16 = in_bf16; p.out_kind = out_kind; p.glu_act = glu_act; p.unary = unary; p.glu_limit = glu_limit;
+    CUtensorMap ma, mb;
+    if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, 128)) return B200_EUNSUPPORTED;
+    const int clusters = std::min(p.m_tiles * p.n_tiles, sm_count() / 2);
+    return glu ? gemm2_launch<3>(ma, mb, p, 2 * clusters, s) : gemm2_launch<2>(ma, mb, p, 2 * clusters, s);
 }
 
 }  // namespace b200

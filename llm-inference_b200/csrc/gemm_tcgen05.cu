@@ -40,6 +40,7 @@ constexpr int kGemmThreads = 192;  // producer, MMA, 4 epilogue warps
 struct GemmParams {
     void* C;            // fp16 [tokens, ldc]
     const void* bias;   // fp16 [N_out] or nullptr
+    const __half* residual;   // fp16 [tokens, ldc] or nullptr (plain fp16 outputs, tokens on the M axis): C = half(half(acc + bias) + residual)
     int rows_a;         // valid rows of the A operand (tokens in normal mode, N_out in stream mode)
     int rows_b;         // valid rows of the B operand
     int K;
@@ -99,7 +100,7 @@ __device__ __forceinline__ void store1(void* C, size_t idx, float f, int kind) {
 // intermediate of ffn.cpp:72-80 is never stored.
 // A thread's row of a gated tile, sixteen features at a time, the next sixteen on their way. KIND 0: fp16 with the rounding points of the unfused
 // sequence (products, silu of the gate, their product), 1 silu, 2 gelu in its tanh form, 3 clamped. What bounds it is the instruction cache: with
-// all units in one loop over 32 unrolled features a tile took 16 us, four times its products at K = 1024 (2048 rows, 2048 -> gated 5504: 101 -> 87 us).
+// all units in one loop over 32 unrolled features a tile took 16 us, with one unit per loop 11, of which the divisions' branches were two thirds (tile_silu).
 template <int KIND>
 __device__ __forceinline__ void store_glu_row(const GemmParams& p, uint32_t taddr, int row, int nt) {
     if (row - (int)(threadIdx.x & 31) >= p.tokens) return;   // (rows behind the tokens are zeros, which take the long way through the division: not here, and not below)
@@ -129,9 +130,9 @@ __device__ __forceinline__ void store_glu_row(const GemmParams& p, uint32_t tadd
                     gv = __half2float(__float2half_rn(gv));
                     uv = __half2float(__float2half_rn(uv));
                     f[e] = __half2float(__float2half_rn(gv / (1.f + expf(-gv)))) * uv;
-                } else if (KIND == 1) f[e] = gv / (1.f + expf(-gv)) * uv;
-                else if (KIND == 2) f[e] = gelu_tanh_f(gv) * uv;
-                else f[e] = glu_clamp_f(gv, uv, p.glu_limit);
+                } else if (KIND == 1) f[e] = tile_silu(gv) * uv;
+                else if (KIND == 2) f[e] = tile_gelu_tanh(gv) * uv;
+                else f[e] = tile_glu_clamp(gv, uv, p.glu_limit);
             }
             const size_t dst = (size_t)row * p.ldc + col0;
             store8(p.C, dst, *reinterpret_cast<const float(*)[8]>(f), p.out_kind);
@@ -288,6 +289,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 if (bias) f[e] += __half2float(bias[col0 + q * 8 + e]);
                                 f[e] = gemm_unary(f[e], p.unary);
                             }
+                            if (p.residual) {
+                                float rr[8];
+                                Unpack<__half>::get(ld16(p.residual + dst + q * 8), rr);
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e])) + rr[e];
+                            }
                             store8(C, dst + q * 8, f, ok);
                         }
                     } else {
@@ -298,6 +305,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             if (col0 + j >= p.rows_b) continue;
                             float f = __uint_as_float(v[j]);
                             if (bias) f += __half2float(bias[col0 + j]);
+                            if (p.residual) f = __half2float(__float2half_rn(f)) + __half2float(p.residual[dst + j]);
                             store1(C, dst + j, gemm_unary(f, p.unary), ok);
                         }
                     }
@@ -759,8 +767,37 @@ static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int 
     }
 }
 
+int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, cudaStream_t s);
 int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, cudaStream_t s,
                       const void* residual = nullptr);
+
+// Which tile a product with more than 256 token rows takes: 64, 128 or 256 columns by 128 rows on one CTA, or (512) 256 x 256 on a pair. What a tile costs per 64-wide
+// K step is its operands' way through shared memory (written once, read by the products): 0.19, 0.24, 0.34 and 0.28 us; a round of tiles is paid in full however
+// few there are, a tile's set-up and epilogue once, the outputs at 5 TB/s. The constants are fitted to 450 measured shapes (257 to 2048 rows, 1000 to 8192
+// features, K 1024 to 8192, both widths of outputs): the tile that it names is 1.40 times as fast as 128 x 256 in the mean, 0.4 % slower than
+// the best of the four, and nowhere more than 2 % slower than 128 x 256. us, the four in this order: 1522 x 1024 -> 1024 9.1 8.3 12.4 12.6; 512 x 8192 -> 2048 25 30 50 45; 2048 x 2048
+// -> 8192 91 69 65 54; 1024 x 1024 -> 3072 14.0 15.2 15.8 13.7.
+static int plain_tile(int M, int N, int k_blocks, bool f32, int sms) {
+    struct Tile { int rows, cols, at_once; float step, once32, once16, round; };
+    const Tile tiles[4] = {{128, 64, sms, 0.192f, 2.18f, 1.61f, 0.82f}, {128, 128, sms, 0.235f, 2.92f, 2.56f, 0.81f}, {128, 256, sms, 0.342f, 5.49f, 3.66f, 0.89f}, {256, 256, sms / 2, 0.283f, 6.29f, 5.65f, 0.81f}};
+    int best = 2;
+    float least = 0.f;
+    for (int i = 0; i < 4; ++i) {
+        const Tile& t = tiles[i];
+        if (t.cols > N && i > 0) continue;
+        const long long n = ((long long)M + t.rows - 1) / t.rows * ((N + t.cols - 1) / t.cols), rounds = (n + t.at_once - 1) / t.at_once;
+        const float cost = (float)rounds * (k_blocks * t.step + t.round) + (f32 ? t.once32 : t.once16) + (float)M * N * (f32 ? 4e-6f : 2e-6f) / 5.f;
+        if (i == 0 || cost < least) { least = cost; best = i; }
+    }
+    return best == 3 ? 512 : tiles[best].cols;
+}
+
+// a gated product of more than 128 rows: tiles of 256 rows by 128 features on a pair of CTAs, or 128 x 128 on one; costs as above (us, one CTA / pair: 512 x 1024 ->
+// 2 x 4096 11.2 12.0, 2048 x 1024 -> 2 x 4096 30.3 27.3, 257 x 2048 -> 2 x 5504 18.4 25.3, 2048 x 2048 -> 2 x 5504 69.4 62.4)
+static bool gated_pair(int M, int N, int k_blocks, int sms) {
+    const long long one = ((long long)M + 127) / 128 * (N / 128), two = ((long long)M + 255) / 256 * (N / 128);
+    return (float)((two + sms / 2 - 1) / (sms / 2)) * (k_blocks * 0.283f + 0.81f) + 5.4f < (float)((one + sms - 1) / sms) * (k_blocks * 0.342f + 0.89f) + 3.7f;
+}
 
 // fewest token rows b200_linear sends to the tcgen05 weight-streaming GEMM instead of the GEMV (B200_GEMM_MIN_TOKENS
 // overrides, for sweeps)
@@ -770,6 +807,30 @@ int gemm_min_tokens() {
     return v;
 }
 
+// more than 256 token rows, plain: tokens on the M axis
+static int gemm_many_rows(const void* x, const void* W, GemmParams p, int M, int N, int K, cudaStream_t s) {
+    const int sms = sm_count();
+    int BN = plain_tile(M, N, p.k_blocks, p.out_kind == 2, sms);
+    if (BN == 512) {
+        const int rc = p.out_kind == 0 && !p.in_bf16 ? gemm2_tcgen05_f16(x, W, p.bias, p.C, M, N, K, false, s, p.residual)
+                                                     : gemm2_tcgen05_ex(x, W, p.C, M, N, K, p.in_bf16, p.out_kind, false, 0, p.unary, 0.f, s);
+        if (rc != B200_EUNSUPPORTED) return rc;
+        BN = 256;
+    }
+    if (N < 64) BN = 32;
+    CUtensorMap ma, mb;
+    p.rows_a = M; p.rows_b = N;
+    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN;
+    if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, N, K, BN)) return B200_EUNSUPPORTED;
+    const int grid = std::min(p.m_tiles * p.n_tiles, sms);
+    switch (BN) {
+        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
+        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
+        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
+        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
+    }
+}
+
 // y[M, N] = x[M, K] * W[N, K]^T (+ bias), fp16 in / fp32 accumulate / fp16 out
 int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, cudaStream_t s) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
@@ -777,11 +838,9 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     static int disabled = -1;
     if (disabled < 0) { const char* e = getenv("B200_NO_TCGEN05"); disabled = (e && e[0] == '1') ? 1 : 0; }
     if (disabled) return B200_EUNSUPPORTED;
-    const int sms = sm_count();
     GemmParams p{};
     p.C = y; p.bias = bias; p.K = K; p.ldc = N; p.tokens = M;
     p.k_blocks = (K + kBK - 1) / kBK;
-    CUtensorMap ma, mb;
     // 161..256 token rows against a wide weight matrix (>= 60 column tiles of 256: most of the 74 cluster slots busy): one row
     // tile of the two-CTA kernel beats a weight-streaming kernel's 2 waves of 128 x 256 tiles (measured, us: 22016 x 4096 at 192 /
     // 256 rows: 60.9 / 61.4 vs 75.8 / 87.6; 12288 x 4096 at 256: 35.5 vs 44.0; narrow outputs keep streaming their weights: 4096 x 11008 at
@@ -791,23 +850,7 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
         if (rc2 != B200_EUNSUPPORTED) return rc2;
     }
     if (M <= 256) return gemm_few_rows(x, W, p, M, N, K, false, s);
-    // normal: tokens on the M axis; large shapes go to the two-CTA kernel (gemm2_tcgen05.cu)
-    {
-        const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, s);
-        if (rc2 != B200_EUNSUPPORTED) return rc2;
-    }
-    const int BN = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : 32;
-    p.rows_a = M; p.rows_b = N;
-    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN;
-    if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, N, K, BN)) return B200_EUNSUPPORTED;
-    const int units = p.m_tiles * p.n_tiles;
-    const int grid = units < sms ? units : sms;
-    switch (BN) {
-        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
-        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
-        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
-        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
-    }
+    return gemm_many_rows(x, W, p, M, N, K, s);
 }
 
 // The same single-CTA kernel for the model families of b200_serve.h: operands fp16 or bfloat16, output fp16 / bfloat16 /
@@ -833,25 +876,14 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
         if (N < 128 || (N & 127)) return B200_EUNSUPPORTED;
         // (96 rows of 28672 gated features: 110 us with the weights streaming in 1.5 waves, 107 with the tokens on the M axis; 72 rows 107 / 108)
         if (M <= 64 || (M <= 128 && N <= 128 * sms)) return gemm_few_rows(x, W, p, M, N, K, true, s);
+        if (gated_pair(M, N, p.k_blocks, sms)) return gemm2_tcgen05_ex(x, W, y, M, N, K, in_bf16, out_kind, true, p.glu_act, 0, glu_limit, s);
         p.rows_a = M; p.rows_b = N;
         p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = N / 128;
         if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * N, K, 128)) return B200_EUNSUPPORTED;
         const int units = p.m_tiles * p.n_tiles;
         return gemm_launch<256, false, true>(ma, mb, p, units < sms ? units : sms, s);
     }
-    if (M <= 256) return gemm_few_rows(x, W, p, M, N, K, false, s);
-    const int BN = N >= 256 ? 256 : N >= 128 ? 128 : N >= 64 ? 64 : 32;
-    p.rows_a = M; p.rows_b = N;
-    p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = (N + BN - 1) / BN;
-    if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, N, K, BN)) return B200_EUNSUPPORTED;
-    const int units = p.m_tiles * p.n_tiles;
-    const int grid = units < sms ? units : sms;
-    switch (BN) {
-        case 32: return gemm_launch<32, false>(ma, mb, p, grid, s);
-        case 64: return gemm_launch<64, false>(ma, mb, p, grid, s);
-        case 128: return gemm_launch<128, false>(ma, mb, p, grid, s);
-        default: return gemm_launch<256, false>(ma, mb, p, grid, s);
-    }
+    return M <= 256 ? gemm_few_rows(x, W, p, M, N, K, false, s) : gemm_many_rows(x, W, p, M, N, K, s);
 }
 // out[M, inter] = silu(x W_gate^T) * (x W_up^T), W = [2*inter, K] (gate rows, then up rows): the gate_up GEMM of
 // ffn.cpp:72 with launchAct (ffn.cpp:80) as its epilogue. Prefill shapes only (M > 256, inter % 128 == 0).
@@ -876,13 +908,17 @@ int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int 
 }
 
 // y[M, N] = residual[M, N] + half(x W^T): launchLinearGemm followed by launchAddResidual (ffn.cpp:88 +
-// context_decoder.cpp:134) in the epilogue of the two-CTA GEMM; B200_EUNSUPPORTED outside its shapes
+// context_decoder.cpp:134) in the epilogue; B200_EUNSUPPORTED below 512 rows and for narrow outputs
 int gemm_tcgen05_f16_residual(const void* x, const void* W, const void* residual, void* y, int M, int N, int K, cudaStream_t s) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     if (!al(x) || !al(W) || !al(y) || !al(residual) || (N & 7)) return B200_EUNSUPPORTED;
     const char* e = getenv("B200_NO_TCGEN05");
     if (e && e[0] == '1') return B200_EUNSUPPORTED;
-    return gemm2_tcgen05_f16(x, W, nullptr, y, M, N, K, false, s, residual);
+    if (M < 512 || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
+    GemmParams p{};
+    p.C = y; p.residual = reinterpret_cast<const __half*>(residual); p.K = K; p.ldc = N; p.tokens = M;
+    p.k_blocks = (K + kBK - 1) / kBK;
+    return gemm_many_rows(x, W, p, M, N, K, s);
 }
 
 }  // namespace b200
