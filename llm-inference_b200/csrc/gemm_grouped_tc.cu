@@ -25,7 +25,7 @@ constexpr int kGtM = 128, kGtK = 64, kGtThreads = 192;
 template <int BN>
 struct GtSmem {
     static constexpr int kStageBytes = (kGtM + BN) * kGtK * 2;
-    static constexpr int kStages = BN <= 32 ? 5 : 3, kLag = kStages - 1;   // kLag: stages of rows under way before the first is announced
+    static constexpr int kStages = BN <= 32 ? 5 : 3, kLag = kStages - 2;   // kLag: stages of rows under way when one is announced (one fewer than fit: with all of them a stage was announced only after the products of the one before)
     static constexpr int kTotal = kStages * kStageBytes + (2 * kStages + 1) * 8 + 16 + 1024;
     static_assert(BN * kGtM * 4 <= kStages * kStageBytes, "the sums take the place of the stages");
 };
@@ -158,13 +158,30 @@ __global__ void __launch_bounds__(kGtThreads, 2) gemm_grouped_tc_kernel(const __
         const int r = i / (F / 4), f0 = i % (F / 4) * 4, n = n0 + f0;
         const long long row = row0 + r;
         const float4 a = *reinterpret_cast<const float4*>(om + r * kGtM + f0);
-        float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (GLU) u = *reinterpret_cast<const float4*>(om + r * kGtM + 64 + f0);
         float v[4] = {a.x, a.y, a.z, a.w};
-        const float v2[4] = {u.x, u.y, u.z, u.w};
+        if (GLU) {   // (the units of tile epilogues: without branches, see tile_silu)
+            const float4 u4 = *reinterpret_cast<const float4*>(om + r * kGtM + 64 + f0);
+            float u[4] = {u4.x, u4.y, u4.z, u4.w};
+            if (g.row_scale) {   // the row of A was meant to be scaled: the products are linear in it
+                const float f = g.row_scale[row];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (n + e < g.N) v[e] = gg_value(g, row, n + e, v[e], v2[e], 0);
+                for (int e = 0; e < 4; ++e) { v[e] *= f; u[e] *= f; }
+            }
+            if (g.epi == B200_GG_GLU) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = tile_silu(v[e]) * u[e];
+            } else if (g.epi == B200_GG_GLU_GELU) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = tile_gelu_tanh(v[e]) * u[e];
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = tile_glu_clamp(v[e], u[e], g.epi_param);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (n + e < g.N) v[e] = gg_value(g, row, n + e, v[e], 0.f, 0);
+        }
         if (wide && n + 4 <= g.N) {
             if constexpr (sizeof(TC) == 4) *reinterpret_cast<float4*>(C + row * g.ldc + n) = make_float4(v[0], v[1], v[2], v[3]);
             else {

@@ -236,6 +236,59 @@ __global__ void __launch_bounds__(256) residual_combine_kernel(float* __restrict
     }
 }
 
+// the same for up to MOST experts per token, a thread per four columns: everything that is known in advance is loaded at once, then the experts' rows (a place
+// that names none reads x instead of waiting behind a condition). 512 rows of 2048, four experts: 13.6 us a column after another, 5.4 like this.
+template <typename T, int MOST>
+__global__ void __launch_bounds__(256) residual_combine4_kernel(float* __restrict__ x, const float* __restrict__ mix, const float* __restrict__ shared,
+                                                                const float* __restrict__ eo, const int* __restrict__ dest, const float* __restrict__ weight,
+                                                                const T* __restrict__ h, int width, int top) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (c >= width) return;
+    const size_t i = (size_t)t * width + c;
+    int d[MOST];
+    float w[MOST];
+#pragma unroll
+    for (int k = 0; k < MOST; ++k) {
+        const size_t at = (size_t)t * top + min(k, top - 1);
+        d[k] = dest[at];
+        w[k] = weight[at];
+    }
+    const float4 x4 = *reinterpret_cast<const float4*>(x + i);
+    const float4 m4 = *reinterpret_cast<const float4*>((mix ? mix : x) + i), s4 = *reinterpret_cast<const float4*>((shared ? shared : x) + i);
+    float hv[4];
+    if constexpr (sizeof(T) == 4) {
+        const float4 h4 = *reinterpret_cast<const float4*>(h + i);
+        hv[0] = h4.x; hv[1] = h4.y; hv[2] = h4.z; hv[3] = h4.w;
+    } else {
+        const uint2 h4 = *reinterpret_cast<const uint2*>(h + i);
+        const T* e = reinterpret_cast<const T*>(&h4);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) hv[q] = DT<T>::to_f(e[q]);
+    }
+    float4 v[MOST];
+#pragma unroll
+    for (int k = 0; k < MOST; ++k) v[k] = *reinterpret_cast<const float4*>(d[k] >= 0 ? eo + (size_t)d[k] * width + c : x + i);
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < MOST; ++k) {
+        const float f[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = k < top ? fmaf(w[k], d[k] >= 0 ? f[q] : hv[q], r[q]) : r[q];
+    }
+    const float xs[4] = {x4.x, x4.y, x4.z, x4.w}, ms[4] = {m4.x, m4.y, m4.z, m4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+    float o[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float y = mix ? ms[q] : 0.f;
+        y += r[q];
+        if (shared) y += ss[q];
+        o[q] = xs[q] + y;
+    }
+    *reinterpret_cast<float4*>(x + i) = make_float4(o[0], o[1], o[2], o[3]);
+}
+
 // dst[i, :] = src[rows[i], :] * scale[i] (fp32 product, rounded once)
 template <typename T>
 __global__ void __launch_bounds__(256) gather_rows_scaled_kernel(const T* __restrict__ src, const int* __restrict__ rows, const float* __restrict__ scale,
@@ -405,6 +458,16 @@ extern "C" int b200_residual_combine(float* x, const float* mix, const float* sh
     if (dest && (!weight || !h || top < 1)) return B200_EINVAL;
     if (n_tokens == 0) return B200_OK;
     cudaStream_t s = (cudaStream_t)stream;
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    if (dest && top <= 8 && width % 4 == 0 && width <= 1024 * 65535 && al16(x) && al16(mix) && al16(shared) && al16(expert_out) && al16(h) && (h_dtype == B200_BF16 || h_dtype == B200_F32)) {
+        const dim3 grid((unsigned)n_tokens, (unsigned)((width + 1023) / 1024));
+        auto go = [&](auto kernel, auto* hp) { launch_chained(kernel, grid, dim3(256), 0, s, x, mix, shared, expert_out, dest, weight, hp, width, top); };
+        using bf = __nv_bfloat16;
+        if (h_dtype == B200_BF16) top <= 4 ? go(residual_combine4_kernel<bf, 4>, (const bf*)h) : go(residual_combine4_kernel<bf, 8>, (const bf*)h);
+        else top <= 4 ? go(residual_combine4_kernel<float, 4>, (const float*)h) : go(residual_combine4_kernel<float, 8>, (const float*)h);
+        count_launch();
+        return (int)cudaGetLastError();
+    }
     if (h_dtype == B200_BF16)
         launch_chained(residual_combine_kernel<__nv_bfloat16>, n_tokens, 256, 0, s, x, mix, shared, expert_out, dest, weight,
                                                                        (const __nv_bfloat16*)h, width, top);
