@@ -7,7 +7,7 @@
 // features are stored side by side and the epilogue sees one element like the other kernels of this entry point.
 //   grid: feature tiles x groups x blocks of rows; what lies behind a group's rows leaves at once
 // Measured (before: the mma.sync tiles of gemm_grouped.cu): 512 rows, four of 16 experts each, 2048 -> gated 1024 -> 2048, with dispatch and
-// combine: 247 -> 107 us.
+// combine: 247 -> 107 us, and 106 -> 83 with the rows announced a stage earlier and the epilogue decided before its passes.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -154,46 +154,49 @@ __global__ void __launch_bounds__(kGtThreads, 2) gemm_grouped_tc_kernel(const __
     const int n0 = blockIdx.x * F;
     TC* C = reinterpret_cast<TC*>(g.C);
     const bool wide = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15u) == 0;
-    for (int i = threadIdx.x; i < rows * (F / 4); i += kGtThreads) {
-        const int r = i / (F / 4), f0 = i % (F / 4) * 4, n = n0 + f0;
-        const long long row = row0 + r;
-        const float4 a = *reinterpret_cast<const float4*>(om + r * kGtM + f0);
-        float v[4] = {a.x, a.y, a.z, a.w};
-        if (GLU) {   // (the units of tile epilogues: without branches, see tile_silu)
-            const float4 u4 = *reinterpret_cast<const float4*>(om + r * kGtM + 64 + f0);
-            float u[4] = {u4.x, u4.y, u4.z, u4.w};
-            if (g.row_scale) {   // the row of A was meant to be scaled: the products are linear in it
-                const float f = g.row_scale[row];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { v[e] *= f; u[e] *= f; }
-            }
-            if (g.epi == B200_GG_GLU) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = tile_silu(v[e]) * u[e];
-            } else if (g.epi == B200_GG_GLU_GELU) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = tile_gelu_tanh(v[e]) * u[e];
+    // four features of a row per thread and pass; what an element needs besides its sum is decided before the passes (asked for element by element it took as long
+    // as the products: 20000 clocks for 128 rows)
+    auto passes = [&](auto value) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < rows * (F / 4); i += kGtThreads) {
+            const int r = i / (F / 4), f0 = i % (F / 4) * 4, n = n0 + f0;
+            const long long row = row0 + r;
+            const float4 a = *reinterpret_cast<const float4*>(om + r * kGtM + f0);
+            float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (GLU) b = *reinterpret_cast<const float4*>(om + r * kGtM + 64 + f0);
+            float v[4] = {a.x, a.y, a.z, a.w};
+            const float u[4] = {b.x, b.y, b.z, b.w};
+            value(row, n, v, u);
+            if (wide && n + 4 <= g.N) {
+                if constexpr (sizeof(TC) == 4) *reinterpret_cast<float4*>(C + row * g.ldc + n) = make_float4(v[0], v[1], v[2], v[3]);
+                else {
+                    const __nv_bfloat162 x = __floats2bfloat162_rn(v[0], v[1]), y = __floats2bfloat162_rn(v[2], v[3]);
+                    *reinterpret_cast<uint2*>(C + row * g.ldc + n) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
+                }
             } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) v[e] = tile_glu_clamp(v[e], u[e], g.epi_param);
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < g.N) C[row * g.ldc + n + e] = DT<TC>::from_f(v[e]);
             }
-        } else {
+        }
+    };
+    if (GLU) {   // (the units of tile epilogues: without branches, see tile_silu)
+        auto scaled = [&](long long row, float (&v)[4], const float (&u)[4], auto unit) {
+            const float f = g.row_scale ? g.row_scale[row] : 1.f;   // the row of A was meant to be scaled: the products are linear in it
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = g.row_scale ? unit(v[e] * f, u[e] * f) : unit(v[e], u[e]);
+        };
+        if (g.epi == B200_GG_GLU) passes([&](long long row, int, float (&v)[4], const float (&u)[4]) { scaled(row, v, u, [](float x, float y) { return tile_silu(x) * y; }); });
+        else if (g.epi == B200_GG_GLU_GELU) passes([&](long long row, int, float (&v)[4], const float (&u)[4]) { scaled(row, v, u, [](float x, float y) { return tile_gelu_tanh(x) * y; }); });
+        else passes([&](long long row, int, float (&v)[4], const float (&u)[4]) { scaled(row, v, u, [&](float x, float y) { return tile_glu_clamp(x, y, g.epi_param); }); });
+    } else if (g.epi == B200_GG_NONE && !g.row_scale)
+        passes([](long long, int, float (&)[4], const float (&)[4]) {});
+    else
+        passes([&](long long row, int n, float (&v)[4], const float (&)[4]) {
 #pragma unroll
             for (int e = 0; e < 4; ++e)
                 if (n + e < g.N) v[e] = gg_value(g, row, n + e, v[e], 0.f, 0);
-        }
-        if (wide && n + 4 <= g.N) {
-            if constexpr (sizeof(TC) == 4) *reinterpret_cast<float4*>(C + row * g.ldc + n) = make_float4(v[0], v[1], v[2], v[3]);
-            else {
-                const __nv_bfloat162 x = __floats2bfloat162_rn(v[0], v[1]), y = __floats2bfloat162_rn(v[2], v[3]);
-                *reinterpret_cast<uint2*>(C + row * g.ldc + n) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
-            }
-        } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (n + e < g.N) C[row * g.ldc + n + e] = DT<TC>::from_f(v[e]);
-        }
-    }
+        });
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, BN);
