@@ -6,6 +6,8 @@
 // CTAs' shared memory. Against the one-CTA kernel (gemm_tcgen05.cu: 48 KB of operands per 512 tensor
 // clocks, 4 stages) a stage is 32 KB per SM for the same 512 clocks: the smem read rate per SM drops from
 // 96 to 64 B/clk and the ring holds 6 stages of look-ahead instead of 4.
+// Narrower tiles (256 x 128 .. 224, Gemm2Params::cols) are the same kernel with shorter B boxes, more stages where they fit: a K step gets shorter by less than the tile
+// (0.18 us at 128 columns against 0.30 at 256), but a width that fills the last round of 74 pairs saves the rest of that round (choose_tile in gemm_tcgen05.cu).
 //   warp 0    TMA producer (both CTAs): its own A / B boxes, completion signalled on the LEADER's full barrier
 //   warp 1    TMEM allocation (both CTAs); MMA issue (leader only); tcgen05.commit multicast to both CTAs
 //   warps 2-5 epilogue (both CTAs): own 128 rows from own TMEM, then a remote arrive on the leader's
@@ -23,10 +25,10 @@ namespace b200 {
 
 constexpr int k2Threads = 192;
 constexpr int k2BK = 64;
-constexpr int k2Stages = 6;
-constexpr uint32_t k2ABytes = 128 * k2BK * 2, k2BBytes = 128 * k2BK * 2, k2StageBytes = k2ABytes + k2BBytes;
-constexpr uint32_t k2OffBar = k2Stages * k2StageBytes;                  // full[6], empty[6], acc_full[2], acc_empty[2]
-constexpr uint32_t k2OffSlot = k2OffBar + (2 * k2Stages + 4) * 8;
+constexpr int k2MaxStages = 8;
+constexpr uint32_t k2ABytes = 128 * k2BK * 2, k2BBytes = 128 * k2BK * 2, k2RingBytes = 6 * (k2ABytes + k2BBytes);   // six stages of the full width, up to eight of a narrower tile
+constexpr uint32_t k2OffBar = k2RingBytes;                              // full[8], empty[8], acc_full[2], acc_empty[2]
+constexpr uint32_t k2OffSlot = k2OffBar + (2 * k2MaxStages + 4) * 8;
 constexpr uint32_t kStgBytes = 32 * 128;                                // epilogue staging per warp: 32 rows x 64 fp16
 constexpr uint32_t k2OffStg = (k2OffSlot + 16 + 127) & ~127u;
 constexpr uint32_t k2Smem = k2OffStg + 4 * kStgBytes;
@@ -39,6 +41,7 @@ struct Gemm2Params {
     int tokens, n_out;  // valid rows of A; valid output features (GLU: inter)
     int ldc, k_blocks;
     int m_tiles, n_tiles;   // tiles of 256 rows x (256 features | GLU: 128 features)
+    int cols, stages;       // columns of a tile's accumulator (a multiple of 32 up to 256; gated: half of them gates), stages of the ring
     int group_m;            // tile order: bands of group_m row tiles swept over all column tiles (0: column-major over all rows)
     int in_bf16, out_kind, glu_act, unary;   // the families' calls (KIND 2 and 3 of the kernel), as GemmParams in gemm_tcgen05.cu
     float glu_limit;
@@ -79,20 +82,20 @@ __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
 
 template <bool GLU>
 __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t taddr, int row0, int nt, uint32_t stg, int lane) {
-    constexpr int kOutCols = GLU ? 128 : 256;
-    const int tile_col0 = nt * kOutCols;
+    const int out_cols = GLU ? p.cols / 2 : p.cols, tile_col0 = nt * out_cols, col_end = min(p.n_out, tile_col0 + out_cols);
     const bool vec_ok = (p.ldc & 7) == 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < kOutCols; c0 += 64) {
+    for (int c0 = 0; c0 < out_cols; c0 += 64) {
 #pragma unroll
         for (int sub = 0; sub < 2; ++sub) {
-            const int cc = c0 + sub * 32;
+            const int cc = c0 + sub * 32;   // (a tile that ends in the middle of these 32 columns: what lies behind them is not stored)
+            if (cc >= out_cols) break;
             uint32_t h[16];
             __syncwarp();   // the loads of tensor memory are warp-wide: lanes that took different ways through the divisions meet first
             if (GLU) {
                 uint32_t g[32], uu[32];
                 tmem_ld_32x32(taddr + (uint32_t)cc, g);
-                tmem_ld_32x32(taddr + (uint32_t)(128 + cc), uu);
+                tmem_ld_32x32(taddr + (uint32_t)(out_cols + cc), uu);
 #pragma unroll
                 for (int e = 0; e < 32; e += 2) {
                     float o[2];
@@ -125,22 +128,30 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
                           h[4 * q + 2], h[4 * q + 3]);
         }
         __syncwarp();
+        Pack16 rr[8];   // the residual, a pass's pieces in flight together
+        if (!GLU && p.residual && vec_ok) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int row = min(row0 + j * 4 + (lane >> 3), p.tokens - 1), col = min(tile_col0 + c0 + (lane & 7) * 8, p.n_out - 8);
+                rr[j] = ld16(p.residual + (size_t)row * p.ldc + col);
+            }
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int r = j * 4 + (lane >> 3), ch = lane & 7;
             const uint4 val = stg_ld_v4(stg + (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4));
             const int row = row0 + r, col = tile_col0 + c0 + ch * 8;
-            if (row < p.tokens && col < p.n_out) {
+            if (row < p.tokens && col < col_end) {
                 __half* dst = p.C + (size_t)row * p.ldc + col;
                 Pack16 pk;
                 *reinterpret_cast<uint4*>(&pk) = val;
-                if (vec_ok && col + 8 <= p.n_out) {
+                if (vec_ok && col + 8 <= col_end) {
                     if (!GLU && p.residual) {   // the linear's output was rounded to fp16 first, as the unfused pair does
-                        float a[8], rr[8];
+                        float a[8], b[8];
                         Unpack<__half>::get(pk, a);
-                        Unpack<__half>::get(ld16(p.residual + (size_t)row * p.ldc + col), rr);
+                        Unpack<__half>::get(rr[j], b);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) a[e] += rr[e];
+                        for (int e = 0; e < 8; ++e) a[e] += b[e];
                         pk = Unpack<__half>::put(a);
                     }
                     st16(dst, pk);
@@ -149,7 +160,7 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
                     Unpack<__half>::get(pk, a);
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
-                        if (col + e >= p.n_out) continue;
+                        if (col + e >= col_end) continue;
                         float f = a[e];
                         if (!GLU && p.residual) f += __half2float(p.residual[(size_t)row * p.ldc + col + e]);
                         dst[e] = __float2half_rn(f);
@@ -165,18 +176,18 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
 // 64 output columns of bfloat16 or 32 of fp32, 128 bytes of a row in the stage.
 template <bool GLU, int ACT, bool F32>
 __device__ __forceinline__ void store_tile_warp_ex(const Gemm2Params& p, uint32_t taddr, int row0, int nt, uint32_t stg, int lane) {
-    constexpr int kOutCols = GLU ? 128 : 256, kPass = F32 ? 32 : 64;
-    const int tile_col0 = nt * kOutCols;
+    constexpr int kPass = F32 ? 32 : 64;
+    const int out_cols = GLU ? p.cols / 2 : p.cols, tile_col0 = nt * out_cols, col_end = min(p.n_out, tile_col0 + out_cols);
     if (row0 >= p.tokens) return;
     const bool vec_ok = (p.ldc & (F32 ? 3 : 7)) == 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < kOutCols && tile_col0 + c0 < p.n_out; c0 += kPass) {
+    for (int c0 = 0; tile_col0 + c0 < col_end; c0 += kPass) {
 #pragma unroll 1
-        for (int cc = c0; cc < c0 + kPass; cc += 16) {
+        for (int cc = c0; cc < min(c0 + kPass, out_cols); cc += 16) {
             uint32_t v[16], u[16];
             __syncwarp();   // the loads of tensor memory are warp-wide
             tmem_ld_32x16_async(taddr + (uint32_t)cc, v);
-            if (GLU) tmem_ld_32x16_async(taddr + (uint32_t)(128 + cc), u);
+            if (GLU) tmem_ld_32x16_async(taddr + (uint32_t)(out_cols + cc), u);
             tmem_wait_ld<16>(v);
             if (GLU) tmem_wait_ld<16>(u);
             float f[16];
@@ -214,16 +225,16 @@ __device__ __forceinline__ void store_tile_warp_ex(const Gemm2Params& p, uint32_
             const int r = j * 4 + (lane >> 3), ch = lane & 7;
             const uint4 val = stg_ld_v4(stg + (uint32_t)r * 128u + (uint32_t)((ch ^ (r & 7)) << 4));
             const int row = row0 + r, col = tile_col0 + c0 + ch * kPiece;
-            if (row < p.tokens && col < p.n_out) {
+            if (row < p.tokens && col < col_end) {
                 const size_t at = (size_t)row * p.ldc + col;
-                if (vec_ok && col + kPiece <= p.n_out) {
+                if (vec_ok && col + kPiece <= col_end) {
                     if (F32) *reinterpret_cast<uint4*>(reinterpret_cast<float*>(p.C) + at) = val;
                     else *reinterpret_cast<uint4*>(p.C + at) = val;
                 } else {
                     const uint32_t w[4] = {val.x, val.y, val.z, val.w};
 #pragma unroll
                     for (int e = 0; e < kPiece; ++e) {
-                        if (col + e >= p.n_out) continue;
+                        if (col + e >= col_end) continue;
                         if (F32) reinterpret_cast<uint32_t*>(p.C)[at + e] = w[e];
                         else reinterpret_cast<uint16_t*>(p.C)[at + e] = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
                     }
@@ -241,15 +252,15 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     constexpr bool GLU = (KIND & 1) != 0;
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + k2OffBar);
-    uint64_t* empty_bar = full_bar + k2Stages;
-    uint64_t* acc_full = empty_bar + k2Stages;   // [2]
+    uint64_t* empty_bar = full_bar + k2MaxStages;
+    uint64_t* acc_full = empty_bar + k2MaxStages;   // [2]
     uint64_t* acc_empty = acc_full + 2;          // [2], used in the leader only
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + k2OffSlot);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();     // 0 = leader
     if (threadIdx.x == 0) {
         if (smem_u32(smem) & 1023u) __trap();
-        for (int s = 0; s < k2Stages; ++s) {
+        for (int s = 0; s < k2MaxStages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -270,7 +281,8 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     pdl_launch_dependents();
     pdl_wait();
 
-    const int units = p.m_tiles * p.n_tiles;
+    const int units = p.m_tiles * p.n_tiles, stages = p.stages, half = p.cols / 2;   // half: rows of B per CTA
+    const uint32_t stage_bytes = k2ABytes + (uint32_t)half * (k2BK * 2);
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
 
     if (warp == 0) {
@@ -281,24 +293,24 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             int mt, nt;
             tile_of_unit(p, p.n_tiles, u, mt, nt);
             const int a_row = mt * 256 + (int)rank * 128;
-            const int b_row = GLU ? (rank == 0 ? nt * 128 : p.n_out + nt * 128) : nt * 256 + (int)rank * 128;
+            const int b_row = GLU ? (rank == 0 ? nt * half : p.n_out + nt * half) : (2 * nt + (int)rank) * half;
             for (int kb = 0; kb < p.k_blocks; ++kb) {
                 mbar_wait_bounded(&empty_bar[stage], phase ^ 1);
                 if (lane == 0) {
-                    unsigned char* sa = smem + (size_t)stage * k2StageBytes;
+                    unsigned char* sa = smem + (size_t)stage * stage_bytes;
                     const uint32_t leader_full = mapa_shared(smem_u32(&full_bar[stage]), 0);
-                    if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * k2StageBytes);   // both CTAs' boxes
+                    if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * stage_bytes);   // both CTAs' boxes
                     tma_load_2d_pair(sa, &map_a, kb * k2BK, a_row, leader_full);
                     tma_load_2d_pair(sa + k2ABytes, &map_b, kb * k2BK, b_row, leader_full);
                 }
                 __syncwarp();
-                if (++stage == k2Stages) { stage = 0; phase ^= 1; }
+                if (++stage == stages) { stage = 0; phase ^= 1; }
             }
         }
     } else if (warp == 1) {
         // ================= MMA issuer (leader CTA only) =================
         if (rank == 0) {
-            const uint32_t idesc = make_idesc_f16(256, 256) | (KIND >= 2 && p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+            const uint32_t idesc = make_idesc_f16(256, p.cols) | (KIND >= 2 && p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
             const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(smem)), b_desc = make_kmajor_sw128_desc(smem_u32(smem) + k2ABytes);
             const bool leader = elect_one();   // (descriptors from values that are uniform over the warp: see gemm_tcgen05_kernel)
             int stage = 0, acc = 0;
@@ -311,7 +323,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     mbar_wait_bounded(&full_bar[stage], phase);
                     tc_fence_after();
                     if (leader) {
-                        const uint64_t da = a_desc + (uint64_t)(stage * (k2StageBytes >> 4)), db = b_desc + (uint64_t)(stage * (k2StageBytes >> 4));
+                        const uint64_t da = a_desc + (uint64_t)(stage * (stage_bytes >> 4)), db = b_desc + (uint64_t)(stage * (stage_bytes >> 4));
 #pragma unroll
                         for (int k = 0; k < k2BK / kUmmaK; ++k)
                             umma_f16_pair(d_tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
@@ -319,7 +331,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                         if (kb == p.k_blocks - 1) umma_commit_pair(&acc_full[acc], 3);   // both epilogues may read
                     }
                     __syncwarp();
-                    if (++stage == k2Stages) { stage = 0; phase ^= 1; }
+                    if (++stage == stages) { stage = 0; phase ^= 1; }
                 }
                 acc ^= 1;
                 if (acc == 0) acc_phase ^= 1;
@@ -602,15 +614,23 @@ static int gemm2_launch(const CUtensorMap& ma, const CUtensorMap& mb, const Gemm
     return (int)e;
 }
 
+// the tiles of a product of N output features: `cols` accumulator columns each, a ring of as many stages as fit
+static void set_cols(Gemm2Params& p, int N, bool glu, int cols) {
+    const int out_cols = glu ? cols / 2 : cols;
+    p.cols = cols;
+    p.n_tiles = (N + out_cols - 1) / out_cols;
+    p.stages = std::min(k2MaxStages, (int)(k2RingBytes / (k2ABytes + (uint32_t)cols / 2 * (k2BK * 2))));
+}
+
 // y[M, N] = x[M, K] W[N, K]^T (+ bias) or, with glu, out[M, N] = silu(x Wg^T) * (x Wu^T) with W = [2N, K].
 // Returns B200_EUNSUPPORTED for shapes the pair kernel does not cover (the one-CTA kernel takes them).
-int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, cudaStream_t s,
+int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, int cols, cudaStream_t s,
                       const void* residual) {
     static int mode = -1;   // B200_GEMM_PAIR=0 keeps the one-CTA kernel
     if (mode < 0) { const char* e = getenv("B200_GEMM_PAIR"); mode = (e && e[0] == '0') ? 0 : 1; }
     if (!mode) return B200_EUNSUPPORTED;
-    // (plain products come by the rules of gemm_tcgen05.cu: plain_tile, and one row tile x >= 60 column tiles)
-    if ((glu ? M < 512 : M <= 160) || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
+    // (cols and whether a product comes here at all: choose_tile in gemm_tcgen05.cu, and one row tile x >= 60 column tiles of 256)
+    if ((glu ? M <= 256 : M <= 160) || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
     if (glu && ((N & 127) || bias || residual)) return B200_EUNSUPPORTED;
     Gemm2Params p{};
     p.C = reinterpret_cast<__half*>(y);
@@ -619,7 +639,7 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
     p.tokens = M; p.n_out = N; p.ldc = N;
     p.k_blocks = (K + k2BK - 1) / k2BK;
     p.m_tiles = (M + 255) / 256;
-    p.n_tiles = glu ? N / 128 : (N + 255) / 256;
+    set_cols(p, N, glu, cols);
     {   // bands of 16 row tiles (measured at 8192 x 12288 x 4096, power-capped: 1108 -> 1191 TFLOP/s sustained; 8: 1150, 32 = the
         // old column-major order). B200_GEMM2_GROUP_M overrides (0 = column-major over all row tiles).
         static int group_env = -2;
@@ -635,7 +655,8 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
     // kernels (more L2 traffic = more energy) and was removed again.
     const char* wide_s = getenv("B200_GEMM2_WIDE");
     const int wide_env = (wide_s && wide_s[0] == '1') ? 1 : 0;
-    if (wide_env && M >= 512 && (p.n_tiles & 1) == 0) {
+    if (wide_env && M >= 512 && ((glu ? N / 128 : (N + 255) / 256) & 1) == 0) {
+        set_cols(p, N, glu, 256);
         int clusters = sm_count() / 2;
         const int units_w = p.m_tiles * (p.n_tiles / 2);
         if (units_w >= clusters) {
@@ -646,7 +667,7 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
             return glu ? gemm2_launch_wide<true>(ma, mb, p, clusters, s) : gemm2_launch_wide<false>(ma, mb, p, clusters, s);
         }
     }
-    if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, 128)) return B200_EUNSUPPORTED;
+    if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, p.cols / 2)) return B200_EUNSUPPORTED;
     const int units = p.m_tiles * p.n_tiles;
     int clusters = sm_count() / 2;
     if (clusters > units) clusters = units;
@@ -654,17 +675,17 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
 }
 
 // The families' linears: fp16 or bfloat16 operands, outputs and epilogues as gemm_tcgen05_ex takes them (there is the rule that sends a call here); gated: W = [2 N, K], N % 128 == 0
-int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, cudaStream_t s) {
+int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s) {
     Gemm2Params p{};
     p.C = reinterpret_cast<__half*>(y);
     p.tokens = M; p.n_out = N; p.ldc = N;
     p.k_blocks = (K + k2BK - 1) / k2BK;
     p.m_tiles = (M + 255) / 256;
-    p.n_tiles = glu ? N / 128 : (N + 255) / 256;
+    set_cols(p, N, glu, cols);
     p.group_m = 16;
     p.in_bf16 = in_bf16; p.out_kind = out_kind; p.glu_act = glu_act; p.unary = unary; p.glu_limit = glu_limit;
     CUtensorMap ma, mb;
-    if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, 128)) return B200_EUNSUPPORTED;
+    if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, p.cols / 2)) return B200_EUNSUPPORTED;
     const int clusters = std::min(p.m_tiles * p.n_tiles, sm_count() / 2);
     return glu ? gemm2_launch<3>(ma, mb, p, 2 * clusters, s) : gemm2_launch<2>(ma, mb, p, 2 * clusters, s);
 }

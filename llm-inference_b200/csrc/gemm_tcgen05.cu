@@ -249,10 +249,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const __half* bias = reinterpret_cast<const __half*>(p.bias);
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
             const int mt = u % p.m_tiles, nt = u / p.m_tiles;
-            mbar_wait(&acc_full[acc], acc_phase);
-            tc_fence_after();
             const int row = mt * kBM + quarter * 32 + lane;   // row of the A operand / of D
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN);
+            // the residual's 32 columns of a pass are read a pass ahead, the first under the products: read where they are added, each piece was a round trip of its
+            // own (512 x 4096 -> 4096 27.3 us with a residual against 18.0 without)
+            Pack16 rr[4];
+            const bool add = !GLU && !SWAP && p.residual != nullptr && row < p.tokens && (p.ldc & 7) == 0;
+            auto load_residual = [&](int col0) {
+                if (!add || col0 + 32 > p.rows_b) return;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) rr[q] = ld16(p.residual + (size_t)row * p.ldc + col0 + q * 8);
+            };
+            load_residual(nt * BN);
+            __syncwarp();
+            mbar_wait(&acc_full[acc], acc_phase);
+            tc_fence_after();
             if (GLU) {
                 // rows_b = inter; gate in columns [0,128), up in [128,256)
                 if (ok == 0) store_glu_row<0>(p, taddr, row, nt);
@@ -290,13 +301,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 f[e] = gemm_unary(f[e], p.unary);
                             }
                             if (p.residual) {
-                                float rr[8];
-                                Unpack<__half>::get(ld16(p.residual + dst + q * 8), rr);
+                                float b[8];
+                                Unpack<__half>::get(rr[q], b);
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e])) + rr[e];
+                                for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e])) + b[e];
                             }
                             store8(C, dst + q * 8, f, ok);
                         }
+                        if (c0 + 32 < BN) load_residual(col0 + 32);
                     } else {
                         // unrolled with a predicate: a run-time index would move v[] to local memory (no L1 behind
                         // it with the 227 KB carve-out) for EVERY path of the epilogue
@@ -767,36 +779,38 @@ static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int 
     }
 }
 
-int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, cudaStream_t s);
-int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, cudaStream_t s,
-                      const void* residual = nullptr);
+int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s);
+int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, int cols, cudaStream_t s, const void* residual = nullptr);
 
-// Which tile a product with more than 256 token rows takes: 64, 128 or 256 columns by 128 rows on one CTA, or (512) 256 x 256 on a pair. What a tile costs per 64-wide
-// K step is its operands' way through shared memory (written once, read by the products): 0.19, 0.24, 0.34 and 0.28 us; a round of tiles is paid in full however
-// few there are, a tile's set-up and epilogue once, the outputs at 5 TB/s. The constants are fitted to 450 measured shapes (257 to 2048 rows, 1000 to 8192
-// features, K 1024 to 8192, both widths of outputs): the tile that it names is 1.40 times as fast as 128 x 256 in the mean, 0.4 % slower than
-// the best of the four, and nowhere more than 2 % slower than 128 x 256. us, the four in this order: 1522 x 1024 -> 1024 9.1 8.3 12.4 12.6; 512 x 8192 -> 2048 25 30 50 45; 2048 x 2048
-// -> 8192 91 69 65 54; 1024 x 1024 -> 3072 14.0 15.2 15.8 13.7.
-static int plain_tile(int M, int N, int k_blocks, bool f32, int sms) {
-    struct Tile { int rows, cols, at_once; float step, once32, once16, round; };
-    const Tile tiles[4] = {{128, 64, sms, 0.192f, 2.18f, 1.61f, 0.82f}, {128, 128, sms, 0.235f, 2.92f, 2.56f, 0.81f}, {128, 256, sms, 0.342f, 5.49f, 3.66f, 0.89f}, {256, 256, sms / 2, 0.283f, 6.29f, 5.65f, 0.81f}};
-    int best = 2;
-    float least = 0.f;
-    for (int i = 0; i < 4; ++i) {
-        const Tile& t = tiles[i];
-        if (t.cols > N && i > 0) continue;
-        const long long n = ((long long)M + t.rows - 1) / t.rows * ((N + t.cols - 1) / t.cols), rounds = (n + t.at_once - 1) / t.at_once;
-        const float cost = (float)rounds * (k_blocks * t.step + t.round) + (f32 ? t.once32 : t.once16) + (float)M * N * (f32 ? 4e-6f : 2e-6f) / 5.f;
-        if (i == 0 || cost < least) { least = cost; best = i; }
+// Which tile a product of many token rows takes: 128 rows on one CTA or 256 on a pair, by the columns of its accumulator. What a tile costs per 64-wide K step is its
+// operands' way through L2 and shared memory, a round of tiles is paid in full however few there are, a tile's set-up and epilogue once, the outputs at 5 TB/s; so the
+// width that just fills the chip's last round wins. The constants (us) are fitted to 105 plain and 28 gated shapes (200 to 2048 rows, 1000 to 12288 features, K 1024 to
+// 11008, weights from HBM), each run with every tile: the tile that the rule names is 0.7 % slower than the best in the mean (gated: 0.2 %), and against the choice
+// without pairs narrower than 256 columns 5 % (gated: 9 %) faster. us, that choice / now: 1522 x 8192 -> 2048 49.2 / 38.5 (192 columns), 1522 x 2048 -> 4096 28.9 / 23.3
+// (192), 512 x 4096 -> 12288 48.1 / 41.8 (192), 512 x 11008 -> 4096 42.8 / 39.3 (128); 1024 x 1024 -> 1024 keeps 64 columns on one CTA (6.6; pairs 9.0). A pair has to be 3 %
+// cheaper than one CTA's best: below that the fit does not tell them apart.
+struct Tile { int rows, cols; float step, round, once32, once16; };
+struct TileChoice { int cols; bool pair; };
+static constexpr Tile kPlainTiles[] = {{128, 64, 0.168f, 0.f, 4.16f, 3.43f}, {128, 128, 0.205f, 0.14f, 5.10f, 3.87f}, {128, 256, 0.334f, 0.24f, 7.01f, 4.82f},
+                                       {256, 128, 0.177f, 0.f, 5.93f, 5.14f}, {256, 160, 0.190f, 0.f, 6.63f, 5.89f}, {256, 192, 0.230f, 0.f, 6.90f, 5.61f},
+                                       {256, 224, 0.252f, 0.f, 7.68f, 6.69f}, {256, 256, 0.302f, 0.f, 7.86f, 6.27f}};
+// gated: half of the columns are gates. us, pairs of 256 columns or one CTA / now: 512 x 2048 -> 2 x 5504 26.7 / 20.2 (160), 200 x 2048 -> 2 x 5504 19.1 / 14.8 (160), 2048 x 2048 -> 2 x 5504
+// stays at 256 (62.8), 257 x 4096 -> 2 x 11008 on one CTA (64; pairs 96 and more)
+static constexpr Tile kGatedTiles[] = {{128, 256, 0.349f, 1.06f, 4.23f, 4.23f}, {256, 128, 0.169f, 1.28f, 4.04f, 4.04f}, {256, 160, 0.170f, 1.76f, 5.04f, 5.04f},
+                                       {256, 192, 0.204f, 1.50f, 5.47f, 5.47f}, {256, 224, 0.221f, 1.98f, 5.85f, 5.85f}, {256, 256, 0.258f, 1.88f, 6.06f, 6.06f}};
+template <int COUNT>
+static TileChoice choose_tile(const Tile (&tiles)[COUNT], int M, int N, int k_blocks, bool glu, bool f32, int sms, bool pairs_only = false) {
+    TileChoice best{256, true};
+    float least = -1.f;
+    for (const Tile& t : tiles) {
+        const bool pair = t.rows == 256;
+        const int out_cols = glu ? t.cols / 2 : t.cols, at_once = pair ? sms / 2 : sms;
+        if (pair ? N < 256 && !glu : (pairs_only || (t.cols > N && t.cols > 64 && !glu))) continue;
+        const long long n = ((long long)M + t.rows - 1) / t.rows * ((N + out_cols - 1) / out_cols), rounds = (n + at_once - 1) / at_once;
+        const float cost = ((float)rounds * (k_blocks * t.step + t.round) + (f32 ? t.once32 : t.once16) + (float)M * N * (f32 ? 4e-6f : 2e-6f) / 5.f) * (pair && !pairs_only ? 1.03f : 1.f);
+        if (least < 0.f || cost < least) { least = cost; best = {t.cols, pair}; }
     }
-    return best == 3 ? 512 : tiles[best].cols;
-}
-
-// a gated product of more than 128 rows: tiles of 256 rows by 128 features on a pair of CTAs, or 128 x 128 on one; costs as above (us, one CTA / pair: 512 x 1024 ->
-// 2 x 4096 11.2 12.0, 2048 x 1024 -> 2 x 4096 30.3 27.3, 257 x 2048 -> 2 x 5504 18.4 25.3, 2048 x 2048 -> 2 x 5504 69.4 62.4)
-static bool gated_pair(int M, int N, int k_blocks, int sms) {
-    const long long one = ((long long)M + 127) / 128 * (N / 128), two = ((long long)M + 255) / 256 * (N / 128);
-    return (float)((two + sms / 2 - 1) / (sms / 2)) * (k_blocks * 0.283f + 0.81f) + 5.4f < (float)((one + sms - 1) / sms) * (k_blocks * 0.342f + 0.89f) + 3.7f;
+    return best;
 }
 
 // fewest token rows b200_linear sends to the tcgen05 weight-streaming GEMM instead of the GEMV (B200_GEMM_MIN_TOKENS
@@ -810,10 +824,11 @@ int gemm_min_tokens() {
 // more than 256 token rows, plain: tokens on the M axis
 static int gemm_many_rows(const void* x, const void* W, GemmParams p, int M, int N, int K, cudaStream_t s) {
     const int sms = sm_count();
-    int BN = plain_tile(M, N, p.k_blocks, p.out_kind == 2, sms);
-    if (BN == 512) {
-        const int rc = p.out_kind == 0 && !p.in_bf16 ? gemm2_tcgen05_f16(x, W, p.bias, p.C, M, N, K, false, s, p.residual)
-                                                     : gemm2_tcgen05_ex(x, W, p.C, M, N, K, p.in_bf16, p.out_kind, false, 0, p.unary, 0.f, s);
+    const TileChoice tile = choose_tile(kPlainTiles, M, N, p.k_blocks, false, p.out_kind == 2, sms);
+    int BN = tile.cols;
+    if (tile.pair) {
+        const int rc = p.out_kind == 0 && !p.in_bf16 ? gemm2_tcgen05_f16(x, W, p.bias, p.C, M, N, K, false, BN, s, p.residual)
+                                                     : gemm2_tcgen05_ex(x, W, p.C, M, N, K, p.in_bf16, p.out_kind, false, 0, p.unary, 0.f, BN, s);
         if (rc != B200_EUNSUPPORTED) return rc;
         BN = 256;
     }
@@ -846,7 +861,7 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     // 256 rows: 60.9 / 61.4 vs 75.8 / 87.6; 12288 x 4096 at 256: 35.5 vs 44.0; narrow outputs keep streaming their weights: 4096 x 11008 at
     // 256: 38.4 vs 65.5)
     if (M > 160 && M <= 256 && (N + 255) / 256 >= 60) {
-        const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, s);
+        const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, choose_tile(kPlainTiles, M, N, p.k_blocks, false, false, sm_count(), true).cols, s);
         if (rc2 != B200_EUNSUPPORTED) return rc2;
     }
     if (M <= 256) return gemm_few_rows(x, W, p, M, N, K, false, s);
@@ -876,7 +891,8 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
         if (N < 128 || (N & 127)) return B200_EUNSUPPORTED;
         // (96 rows of 28672 gated features: 110 us with the weights streaming in 1.5 waves, 107 with the tokens on the M axis; 72 rows 107 / 108)
         if (M <= 64 || (M <= 128 && N <= 128 * sms)) return gemm_few_rows(x, W, p, M, N, K, true, s);
-        if (gated_pair(M, N, p.k_blocks, sms)) return gemm2_tcgen05_ex(x, W, y, M, N, K, in_bf16, out_kind, true, p.glu_act, 0, glu_limit, s);
+        const TileChoice tile = choose_tile(kGatedTiles, M, N, p.k_blocks, true, out_kind == 2, sms);
+        if (tile.pair) return gemm2_tcgen05_ex(x, W, y, M, N, K, in_bf16, out_kind, true, p.glu_act, 0, glu_limit, tile.cols, s);
         p.rows_a = M; p.rows_b = N;
         p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = N / 128;
         if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * N, K, 128)) return B200_EUNSUPPORTED;
@@ -892,8 +908,9 @@ int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int 
     if (M <= 256 || inter < 128 || (inter & 127) || K < 8 || (K & 7) || !al(x) || !al(W) || !al(out)) return B200_EUNSUPPORTED;
     const char* e = getenv("B200_NO_TCGEN05");
     if (e && e[0] == '1') return B200_EUNSUPPORTED;
-    {
-        const int rc2 = gemm2_tcgen05_f16(x, W, nullptr, out, M, inter, K, true, s);
+    const TileChoice tile = choose_tile(kGatedTiles, M, inter, (K + kBK - 1) / kBK, true, false, sm_count());
+    if (tile.pair) {
+        const int rc2 = gemm2_tcgen05_f16(x, W, nullptr, out, M, inter, K, true, tile.cols, s);
         if (rc2 != B200_EUNSUPPORTED) return rc2;
     }
     GemmParams p{};
