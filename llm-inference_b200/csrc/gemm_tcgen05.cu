@@ -846,6 +846,11 @@ static int gemm_many_rows(const void* x, const void* W, GemmParams p, int M, int
     }
 }
 
+// 161 to 256 fp16 rows against a wide weight matrix (>= 60 column tiles of 256: most of the 74 cluster slots busy): one row tile of the two-CTA kernel beats a
+// weight-streaming kernel's 2 waves of 128 x 256 tiles (measured, us: 22016 x 4096 at 192 / 256 rows: 60.9 / 61.4 vs 75.8 / 87.6; 12288 x 4096 at 256: 35.5 vs 44.0;
+// narrow outputs keep streaming their weights: 4096 x 11008 at 256: 38.4 vs 65.5)
+static bool one_row_of_pairs(int M, int N) { return M > 160 && M <= 256 && (N + 255) / 256 >= 60; }
+
 // y[M, N] = x[M, K] * W[N, K]^T (+ bias), fp16 in / fp32 accumulate / fp16 out
 int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, cudaStream_t s) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
@@ -856,11 +861,7 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     GemmParams p{};
     p.C = y; p.bias = bias; p.K = K; p.ldc = N; p.tokens = M;
     p.k_blocks = (K + kBK - 1) / kBK;
-    // 161..256 token rows against a wide weight matrix (>= 60 column tiles of 256: most of the 74 cluster slots busy): one row
-    // tile of the two-CTA kernel beats a weight-streaming kernel's 2 waves of 128 x 256 tiles (measured, us: 22016 x 4096 at 192 /
-    // 256 rows: 60.9 / 61.4 vs 75.8 / 87.6; 12288 x 4096 at 256: 35.5 vs 44.0; narrow outputs keep streaming their weights: 4096 x 11008 at
-    // 256: 38.4 vs 65.5)
-    if (M > 160 && M <= 256 && (N + 255) / 256 >= 60) {
+    if (one_row_of_pairs(M, N)) {
         const int rc2 = gemm2_tcgen05_f16(x, W, bias, y, M, N, K, false, choose_tile(kPlainTiles, M, N, p.k_blocks, false, false, sm_count(), true).cols, s);
         if (rc2 != B200_EUNSUPPORTED) return rc2;
     }
@@ -925,13 +926,16 @@ int gemm_tcgen05_f16_swiglu(const void* x, const void* W, void* out, int M, int 
 }
 
 // y[M, N] = residual[M, N] + half(x W^T): launchLinearGemm followed by launchAddResidual (ffn.cpp:88 +
-// context_decoder.cpp:134) in the epilogue; B200_EUNSUPPORTED below 512 rows and for narrow outputs
+// context_decoder.cpp:134) in the epilogue; B200_EUNSUPPORTED below 512 rows, but for one row of pairs, and for narrow outputs
 int gemm_tcgen05_f16_residual(const void* x, const void* W, const void* residual, void* y, int M, int N, int K, cudaStream_t s) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     if (!al(x) || !al(W) || !al(y) || !al(residual) || (N & 7)) return B200_EUNSUPPORTED;
     const char* e = getenv("B200_NO_TCGEN05");
     if (e && e[0] == '1') return B200_EUNSUPPORTED;
-    if (M < 512 || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
+    if (N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
+    if (one_row_of_pairs(M, N))
+        return gemm2_tcgen05_f16(x, W, nullptr, y, M, N, K, false, choose_tile(kPlainTiles, M, N, (K + kBK - 1) / kBK, false, false, sm_count(), true).cols, s, residual);
+    if (M < 512) return B200_EUNSUPPORTED;
     GemmParams p{};
     p.C = y; p.residual = reinterpret_cast<const __half*>(residual); p.K = K; p.ldc = N; p.tokens = M;
     p.k_blocks = (K + kBK - 1) / kBK;

@@ -169,7 +169,7 @@ extern "C" int b200_linear_swiglu(const void* x, const void* W, void* out, int n
 
 /* y[n_tokens, N] = residual + x W^T (W [N, K]): launchLinearGemm + launchAddResidual (add_residual.cu:58) in one
  * tcgen05 launch, same rounding points (linear output rounded to fp16, then the sum). y may not alias x;
- * B200_EUNSUPPORTED outside fp16 prefill shapes (n_tokens >= 512): run b200_linear + b200_add_residual then. */
+ * B200_EUNSUPPORTED outside fp16 prefill shapes (n_tokens >= 512, or 161 to 256 against N > 15104): run b200_linear + b200_add_residual then. */
 extern "C" int b200_linear_residual(const void* x, const void* W, const void* residual, void* y, int n_tokens, int N,
                                     int K, int dtype, void* stream) {
     if (!x || !W || !residual || !y || n_tokens < 1 || N < 1 || K < 1) return B200_EINVAL;
