@@ -91,7 +91,7 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
             const int cc = c0 + sub * 32;   // (a tile that ends in the middle of these 32 columns: what lies behind them is not stored)
             if (cc >= out_cols) break;
             uint32_t h[16];
-            __syncwarp();   // the loads of tensor memory are warp-wide: lanes that took different ways through the divisions meet first
+            __syncwarp();   // the loads of tensor memory are warp-wide
             if (GLU) {
                 uint32_t g[32], uu[32];
                 tmem_ld_32x32(taddr + (uint32_t)cc, g);
@@ -103,7 +103,7 @@ __device__ __forceinline__ void store_tile_warp(const Gemm2Params& p, uint32_t t
                     for (int t = 0; t < 2; ++t) {
                         const float gv = __half2float(__float2half_rn(__uint_as_float(g[e + t])));
                         const float uv = __half2float(__float2half_rn(__uint_as_float(uu[e + t])));
-                        const float sv = __half2float(__float2half_rn(gv / (1.f + expf(-gv))));
+                        const float sv = __half2float(__float2half_rn(tile_silu(gv)));
                         o[t] = sv * uv;
                     }
                     h[e >> 1] = pack_half2(o[0], o[1]);

@@ -101,6 +101,7 @@ __device__ __forceinline__ void store1(void* C, size_t idx, float f, int kind) {
 // A thread's row of a gated tile, sixteen features at a time, the next sixteen on their way. KIND 0: fp16 with the rounding points of the unfused
 // sequence (products, silu of the gate, their product), 1 silu, 2 gelu in its tanh form, 3 clamped. What bounds it is the instruction cache: with
 // all units in one loop over 32 unrolled features a tile took 16 us, with one unit per loop 11, of which the divisions' branches were two thirds (tile_silu).
+// The fp16 unit had kept them: 400 x 1024 -> gated 28672 80 us without, 134 with (and 199 on the pairs that choose_tile names), 8192 x 4096 -> gated 11008 923 and 1444.
 template <int KIND>
 __device__ __forceinline__ void store_glu_row(const GemmParams& p, uint32_t taddr, int row, int nt) {
     if (row - (int)(threadIdx.x & 31) >= p.tokens) return;   // (rows behind the tokens are zeros, which take the long way through the division: not here, and not below)
@@ -129,7 +130,7 @@ __device__ __forceinline__ void store_glu_row(const GemmParams& p, uint32_t tadd
                 if (KIND == 0) {
                     gv = __half2float(__float2half_rn(gv));
                     uv = __half2float(__float2half_rn(uv));
-                    f[e] = __half2float(__float2half_rn(gv / (1.f + expf(-gv)))) * uv;
+                    f[e] = __half2float(__float2half_rn(tile_silu(gv))) * uv;
                 } else if (KIND == 1) f[e] = tile_silu(gv) * uv;
                 else if (KIND == 2) f[e] = tile_gelu_tanh(gv) * uv;
                 else f[e] = tile_glu_clamp(gv, uv, p.glu_limit);
