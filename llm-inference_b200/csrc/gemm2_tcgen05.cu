@@ -43,7 +43,7 @@ struct Gemm2Params {
     int m_tiles, n_tiles;   // tiles of 256 rows x (256 features | GLU: 128 features)
     int cols, stages;       // columns of a tile's accumulator (a multiple of 32 up to 256; gated: half of them gates), stages of the ring
     int group_m;            // tile order: bands of group_m row tiles swept over all column tiles (0: column-major over all rows)
-    int in_bf16, out_kind, glu_act, unary;   // the families' calls (KIND 2 and 3 of the kernel), as GemmParams in gemm_tcgen05.cu
+    int out_kind, glu_act, unary;   // the families' calls (KIND 2 and 3 of the kernel, bfloat16 operands), as GemmParams in gemm_tcgen05.cu
     float glu_limit;
     int wide_full;          // wide kernel: units [0, wide_full) are 256 x 512, the rest is run as single 256 x 256 column tiles
 };
@@ -310,7 +310,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else if (warp == 1) {
         // ================= MMA issuer (leader CTA only) =================
         if (rank == 0) {
-            const uint32_t idesc = make_idesc_f16(256, p.cols) | (KIND >= 2 && p.in_bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+            const uint32_t idesc = make_idesc_f16(256, p.cols) | (KIND >= 2 ? ((1u << 7) | (1u << 10)) : 0u);
             const uint64_t a_desc = make_kmajor_sw128_desc(smem_u32(smem)), b_desc = make_kmajor_sw128_desc(smem_u32(smem) + k2ABytes);
             const bool leader = elect_one();   // (descriptors from values that are uniform over the warp: see gemm_tcgen05_kernel)
             int stage = 0, acc = 0;
@@ -674,8 +674,8 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
     return glu ? gemm2_launch<1>(ma, mb, p, 2 * clusters, s) : gemm2_launch<0>(ma, mb, p, 2 * clusters, s);
 }
 
-// The families' linears: fp16 or bfloat16 operands, outputs and epilogues as gemm_tcgen05_ex takes them (there is the rule that sends a call here); gated: W = [2 N, K], N % 128 == 0
-int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s) {
+// The families' linears: bfloat16 operands, bfloat16 (out_kind 1) or fp32 (2) outputs, epilogues as gemm_tcgen05_ex takes them (there is the rule that sends a call here); gated: W = [2 N, K], N % 128 == 0
+int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s) {
     Gemm2Params p{};
     p.C = reinterpret_cast<__half*>(y);
     p.tokens = M; p.n_out = N; p.ldc = N;
@@ -683,7 +683,7 @@ int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K,
     p.m_tiles = (M + 255) / 256;
     set_cols(p, N, glu, cols);
     p.group_m = 16;
-    p.in_bf16 = in_bf16; p.out_kind = out_kind; p.glu_act = glu_act; p.unary = unary; p.glu_limit = glu_limit;
+    p.out_kind = out_kind; p.glu_act = glu_act; p.unary = unary; p.glu_limit = glu_limit;
     CUtensorMap ma, mb;
     if (!make_tma_map_2d(&ma, x, M, K, 128) || !make_tma_map_2d(&mb, W, glu ? 2ll * N : (long long)N, K, p.cols / 2)) return B200_EUNSUPPORTED;
     const int clusters = std::min(p.m_tiles * p.n_tiles, sm_count() / 2);

@@ -346,7 +346,7 @@ static int gg_launch_mma(const GG& g, dim3 grid, bool trans_b, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, int glu, cudaStream_t s,
+int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, bool out_f32, int glu, cudaStream_t s,
                     float glu_limit = 0.f);   // gemm_tcgen05.cu (glu: 0 none, 1 silu, 2 tanh-gelu, 3 no GLU but relu squared, 4 clamped)
 
 static bool mma_enabled() {
@@ -422,7 +422,7 @@ extern "C" int b200_linear_ex2(const void* x, const void* W, void* y, int n_toke
     if (n_tokens == 0) return B200_OK;
     if (in_dtype == B200_BF16 && (out_dtype == B200_BF16 || out_dtype == B200_F32)) {
         const int glu = epi == B200_GG_GLU ? 1 : epi == B200_GG_GLU_GELU ? 2 : epi == B200_GG_RELU2 ? 3 : epi == B200_GG_GLU_CLAMP ? 4 : 0;
-        const int rc = gemm_tcgen05_ex(x, W, y, n_tokens, N, K, 1, out_dtype == B200_BF16 ? 1 : 2, glu, (cudaStream_t)stream, epi_param);
+        const int rc = gemm_tcgen05_ex(x, W, y, n_tokens, N, K, out_dtype == B200_F32, glu, (cudaStream_t)stream, epi_param);
         if (rc != B200_EUNSUPPORTED) return rc;
     }
     b200_gemm_grouped_args g{};

@@ -150,7 +150,7 @@ static cudaError_t gr_launch(const GrArgs& p, cudaStream_t s) {
     return p.M <= 8 ? launch_chained(gemm_rows_kernel<T, 1, GLU, 8>, grid, dim3(256), 0, s, p) : launch_chained(gemm_rows_kernel<T, 2, GLU, 8>, grid, dim3(256), 0, s, p);
 }
 
-// 1 <= M <= 16, K % 8 == 0, x and W on 16-byte boundaries; out_kind, act and unary as GemmParams in gemm_tcgen05.cu
+// 1 <= M <= 16, K % 8 == 0, x and W on 16-byte boundaries; out_kind, act and unary as GemmParams in gemm_tcgen05.cu; gated units take bfloat16 operands (gemm_few_rows is asked for no others)
 int gemm_rows(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool bf16, int out_kind, bool glu, int act, int unary, float limit, cudaStream_t s) {
     const GrArgs p{x, W, reinterpret_cast<const __half*>(bias), y, M, N, K, out_kind, act, unary, limit};
     const cudaError_t e = bf16 ? (glu ? gr_launch<__nv_bfloat16, true>(p, s) : gr_launch<__nv_bfloat16, false>(p, s)) : gr_launch<__half, false>(p, s);

@@ -780,7 +780,7 @@ static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int 
     }
 }
 
-int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s);
+int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s);
 int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, int cols, cudaStream_t s, const void* residual = nullptr);
 
 // Which tile a product of many token rows takes: 128 rows on one CTA or 256 on a pair, by the columns of its accumulator. What a tile costs per 64-wide K step is its
@@ -828,8 +828,7 @@ static int gemm_many_rows(const void* x, const void* W, GemmParams p, int M, int
     const TileChoice tile = choose_tile(kPlainTiles, M, N, p.k_blocks, false, p.out_kind == 2, sms);
     int BN = tile.cols;
     if (tile.pair) {
-        const int rc = p.out_kind == 0 && !p.in_bf16 ? gemm2_tcgen05_f16(x, W, p.bias, p.C, M, N, K, false, BN, s, p.residual)
-                                                     : gemm2_tcgen05_ex(x, W, p.C, M, N, K, p.in_bf16, p.out_kind, false, 0, p.unary, 0.f, BN, s);
+        const int rc = p.in_bf16 ? gemm2_tcgen05_ex(x, W, p.C, M, N, K, p.out_kind, false, 0, p.unary, 0.f, BN, s) : gemm2_tcgen05_f16(x, W, p.bias, p.C, M, N, K, false, BN, s, p.residual);
         if (rc != B200_EUNSUPPORTED) return rc;
         BN = 256;
     }
@@ -870,13 +869,11 @@ int gemm_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, in
     return gemm_many_rows(x, W, p, M, N, K, s);
 }
 
-// The same single-CTA kernel for the model families of b200_serve.h: operands fp16 or bfloat16, output fp16 / bfloat16 /
-// fp32 (out_kind as GemmParams), optionally with the GLU epilogue (glu 1 silu, 2 tanh-gelu: W = [2 N, K], gate rows then up
-// rows, N % 128 == 0; glu 4: the clamped gated unit of common.cuh with its limit) or with the square of relu on every output
+// The linears of the model families of b200_serve.h: bfloat16 operands, bfloat16 or fp32 outputs, optionally with the GLU epilogue (glu 1 silu, 2 tanh-gelu:
+// W = [2 N, K], gate rows then up rows, N % 128 == 0; glu 4: the clamped gated unit of common.cuh with its limit) or with the square of relu on every output
 // (glu 3: not a GLU, W = [N, K]).
-// Up to 256 token rows (gated units: 128) the weights stream through the M axis; above, tokens are the M axis.
-int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int in_bf16, int out_kind, int glu, cudaStream_t s,
-                    float glu_limit) {
+// Up to 256 token rows (gated units: 128) the weights stream through the M axis; above, tokens are the M axis, on one CTA or a pair.
+int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, bool out_f32, int glu, cudaStream_t s, float glu_limit) {
     auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     if (M < 1 || N < 8 || K < 8 || (K & 7) || !al(x) || !al(W) || !al(y)) return B200_EUNSUPPORTED;
     const char* env = getenv("B200_NO_TCGEN05");
@@ -885,7 +882,7 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
     GemmParams p{};
     p.C = y; p.bias = nullptr; p.K = K; p.ldc = N; p.tokens = M;
     p.k_blocks = (K + kBK - 1) / kBK;
-    p.in_bf16 = in_bf16; p.out_kind = out_kind; p.glu_act = glu == 2 ? 1 : glu == 4 ? 2 : 0; p.glu_limit = glu_limit;
+    p.in_bf16 = 1; p.out_kind = out_f32 ? 2 : 1; p.glu_act = glu == 2 ? 1 : glu == 4 ? 2 : 0; p.glu_limit = glu_limit;
     p.unary = glu == 3 ? 1 : 0;
     if (glu == 3) glu = 0;
     CUtensorMap ma, mb;
@@ -893,8 +890,8 @@ int gemm_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, 
         if (N < 128 || (N & 127)) return B200_EUNSUPPORTED;
         // (96 rows of 28672 gated features: 110 us with the weights streaming in 1.5 waves, 107 with the tokens on the M axis; 72 rows 107 / 108)
         if (M <= 64 || (M <= 128 && N <= 128 * sms)) return gemm_few_rows(x, W, p, M, N, K, true, s);
-        const TileChoice tile = choose_tile(kGatedTiles, M, N, p.k_blocks, true, out_kind == 2, sms);
-        if (tile.pair) return gemm2_tcgen05_ex(x, W, y, M, N, K, in_bf16, out_kind, true, p.glu_act, 0, glu_limit, tile.cols, s);
+        const TileChoice tile = choose_tile(kGatedTiles, M, N, p.k_blocks, true, out_f32, sms);
+        if (tile.pair) return gemm2_tcgen05_ex(x, W, y, M, N, K, p.out_kind, true, p.glu_act, 0, glu_limit, tile.cols, s);
         p.rows_a = M; p.rows_b = N;
         p.m_tiles = (M + kBM - 1) / kBM; p.n_tiles = N / 128;
         if (!make_tma_map_2d(&ma, x, M, K, kBM) || !make_tma_map_2d(&mb, W, 2ll * N, K, 128)) return B200_EUNSUPPORTED;
