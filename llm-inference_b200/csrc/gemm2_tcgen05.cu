@@ -622,13 +622,17 @@ static void set_cols(Gemm2Params& p, int N, bool glu, int cols) {
     p.stages = std::min(k2MaxStages, (int)(k2RingBytes / (k2ABytes + (uint32_t)cols / 2 * (k2BK * 2))));
 }
 
+// B200_GEMM_PAIR=0 keeps every product on the one-CTA kernels
+bool gemm_pairs_enabled() {
+    static const bool on = [] { const char* e = getenv("B200_GEMM_PAIR"); return !(e && e[0] == '0'); }();
+    return on;
+}
+
 // y[M, N] = x[M, K] W[N, K]^T (+ bias) or, with glu, out[M, N] = silu(x Wg^T) * (x Wu^T) with W = [2N, K].
 // Returns B200_EUNSUPPORTED for shapes the pair kernel does not cover (the one-CTA kernel takes them).
 int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, int cols, cudaStream_t s,
                       const void* residual) {
-    static int mode = -1;   // B200_GEMM_PAIR=0 keeps the one-CTA kernel
-    if (mode < 0) { const char* e = getenv("B200_GEMM_PAIR"); mode = (e && e[0] == '0') ? 0 : 1; }
-    if (!mode) return B200_EUNSUPPORTED;
+    if (!gemm_pairs_enabled()) return B200_EUNSUPPORTED;
     // (cols and whether a product comes here at all: choose_tile in gemm_tcgen05.cu, and one row tile x >= 60 column tiles of 256)
     if ((glu ? M <= 256 : M <= 160) || N < 256 || K < 64 || (K & 7)) return B200_EUNSUPPORTED;
     if (glu && ((N & 127) || bias || residual)) return B200_EUNSUPPORTED;

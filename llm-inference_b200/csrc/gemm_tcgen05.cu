@@ -780,6 +780,7 @@ static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int 
     }
 }
 
+bool gemm_pairs_enabled();
 int gemm2_tcgen05_ex(const void* x, const void* W, void* y, int M, int N, int K, int out_kind, bool glu, int glu_act, int unary, float glu_limit, int cols, cudaStream_t s);
 int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool glu, int cols, cudaStream_t s, const void* residual = nullptr);
 
@@ -801,17 +802,25 @@ static constexpr Tile kGatedTiles[] = {{128, 256, 0.349f, 1.06f, 4.23f, 4.23f}, 
                                        {256, 192, 0.204f, 1.50f, 5.47f, 5.47f}, {256, 224, 0.221f, 1.98f, 5.85f, 5.85f}, {256, 256, 0.258f, 1.88f, 6.06f, 6.06f}};
 template <int COUNT>
 static TileChoice choose_tile(const Tile (&tiles)[COUNT], int M, int N, int k_blocks, bool glu, bool f32, int sms, bool pairs_only = false) {
-    TileChoice best{256, true};
+    TileChoice best{256, pairs_only};
     float least = -1.f;
+    const bool pairs = pairs_only || gemm_pairs_enabled();
     for (const Tile& t : tiles) {
         const bool pair = t.rows == 256;
         const int out_cols = glu ? t.cols / 2 : t.cols, at_once = pair ? sms / 2 : sms;
-        if (pair ? N < 256 && !glu : (pairs_only || (t.cols > N && t.cols > 64 && !glu))) continue;
+        if (pair ? !pairs || (N < 256 && !glu) : (pairs_only || (t.cols > N && t.cols > 64 && !glu))) continue;
         const long long n = ((long long)M + t.rows - 1) / t.rows * ((N + out_cols - 1) / out_cols), rounds = (n + at_once - 1) / at_once;
         const float cost = ((float)rounds * (k_blocks * t.step + t.round) + (f32 ? t.once32 : t.once16) + (float)M * N * (f32 ? 4e-6f : 2e-6f) / 5.f) * (pair && !pairs_only ? 1.03f : 1.f);
         if (least < 0.f || cost < least) { least = cost; best = {t.cols, pair}; }
     }
     return best;
+}
+
+// what the rule names, for tests: columns of the accumulator, negative on a pair of CTAs
+int linear_tile(int M, int N, int K, bool gated, bool f32, int sms) {
+    const int k_blocks = (K + kBK - 1) / kBK;
+    const TileChoice t = gated ? choose_tile(kGatedTiles, M, N, k_blocks, true, f32, sms) : choose_tile(kPlainTiles, M, N, k_blocks, false, f32, sms);
+    return t.pair ? -t.cols : t.cols;
 }
 
 // fewest token rows b200_linear sends to the tcgen05 weight-streaming GEMM instead of the GEMV (B200_GEMM_MIN_TOKENS
