@@ -11,6 +11,9 @@
 // picked up, and states crossed memory for every 64 tokens. Here a unit's inputs are its x, its state and its sums; the next units' are under way
 // meanwhile. (One CTA per head that walks its chunks with the state in TMEM was built too: 110 us, everything of a chunk waits for something of the chunk before.)
 // The 64 columns of a unit lie in operands and TMEM as row r = (p % 4) * 16 + p / 4: 16-byte pieces of x go to shared memory without bank conflicts.
+// The state and out kernels, a CTA on each SM that they use, start what follows by ending, not ahead of it: launched earlier, the CTAs of the carry (of the next call's
+// prep) sat down on the SMs that happened to be free, and where 128 of 148 were busy they worked there in a heap. 2 entries, 2048 tokens, 64 heads, 128: 74.4 -> 68.5 us; 1, 2048, 16
+// heads, 64: 44.7 -> 28.9 (37.3 in chunks of 64); 1, 2048, 33 heads, 128: 59.6 -> 39.6.
 // A product dt x that is not finite is multiplied as zero and its column is NaN from its token on: the zeros above the diagonal would carry it to
 // earlier tokens.
 // Measured, us, chunks of 64 on mma.sync against these (entries, tokens, heads, n_state; 64 value columns): 2, 2048, 64, 128: 164 / 84 (floor 11; prep 9, state 18, carry 17,
@@ -251,7 +254,6 @@ __global__ void __launch_bounds__(448, 1) ssd_tc_state_kernel(const SsTc t) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const float* sums = reinterpret_cast<const float*>(smem + kSuOffSums);
     if (warp < 8) {
@@ -457,7 +459,6 @@ __global__ void __launch_bounds__(26 * 32, 1) ssd_tc_out_kernel(const SsTc t) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_launch_dependents();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0), my = (uint32_t)(quarter * 32) << 16;
     const float* sums = reinterpret_cast<const float*>(smem + kSoOffSums);
     if (warp < 8) {   // ---- lane i
