@@ -111,7 +111,7 @@ __host__ __device__ __forceinline__ int chunk_row_stride(int dim) { return ((dim
 // before it, which is what a chunk's 64 tokens spent most of their time on).
 constexpr int kChunkT = kChunk + 4;
 template <bool TRANS>
-__device__ __forceinline__ void stage_rotated(const RT& a, float* dst, int col_off, int h, int row0, int len, float mul, const float* rowmul) {
+__device__ __forceinline__ void stage_rotated_wide(const RT& a, float* dst, int col_off, int h, int row0, int len, float mul, const float* rowmul) {
     const int dim = a.dim, nf = a.rot_dims / 2, rs = chunk_row_stride(dim), lane = threadIdx.x & 31, warps = blockDim.x / 32;
     const bool halves = a.rot_layout == B200_ROPE_HALF;
     const float *cosines = nf > 0 ? a.cos : a.decay, *sines = nf > 0 ? a.sin : a.decay;   // (without rotation something that can be read)
@@ -160,10 +160,49 @@ __device__ __forceinline__ void stage_rotated(const RT& a, float* dst, int col_o
         for (int i = threadIdx.x; i < len * (rs - dim); i += blockDim.x) dst[i / (rs - dim) * rs + dim + i % (rs - dim)] = 0.f;
 }
 
+// the same for up to 32 components, where most lanes of the above would have none: a thread per number, four at a time (and the state kernel with value rows four
+// at a time, in 64 registers instead of 92, so that four CTAs share an SM: 2048 tokens, 16 heads of 4 x 4 60 -> 39 us, of 16 x 32 69 -> 46)
+template <bool TRANS>
+__device__ __forceinline__ void stage_rotated_narrow(const RT& a, float* dst, int col_off, int h, int row0, int len, float mul, const float* rowmul) {
+    const int dim = a.dim, nf = a.rot_dims / 2, rs = chunk_row_stride(dim), step = blockDim.x;
+    const bool halves = a.rot_layout == B200_ROPE_HALF;
+    const float *cosines = nf > 0 ? a.cos : a.decay, *sines = nf > 0 ? a.sin : a.decay;
+#pragma unroll 1
+    for (int i0 = threadIdx.x; i0 < len * dim; i0 += 4 * step) {
+        float u[4], v[4], cs[4], sn[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = min(i0 + k * step, len * dim - 1), j = i / dim, d = i - j * dim;
+            const bool rot = d < a.rot_dims;
+            const int f = !rot ? 0 : halves ? (d < nf ? d : d - nf) : d / 2;
+            const size_t r = (size_t)(row0 + j);
+            const float* vals = a.proj + r * a.ld_proj + col_off + h * dim;
+            u[k] = vals[!rot ? d : halves ? f : 2 * f];
+            v[k] = vals[!rot ? d : halves ? f + nf : 2 * f + 1];
+            cs[k] = __ldg(cosines + r * nf + f);
+            sn[k] = __ldg(sines + r * nf + f);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = i0 + k * step, j = i / dim, d = i - j * dim;
+            float x = (halves ? d < nf : (d & 1) == 0) ? u[k] * cs[k] - v[k] * sn[k] : v[k] * cs[k] + u[k] * sn[k];
+            if (d >= a.rot_dims) x = u[k];
+            if (i < len * dim) dst[TRANS ? d * kChunkT + j : j * rs + d] = x * mul * (rowmul ? rowmul[j] : 1.f);
+        }
+    }
+    if (!TRANS)
+        for (int i = threadIdx.x; i < len * (rs - dim); i += blockDim.x) dst[i / (rs - dim) * rs + dim + i % (rs - dim)] = 0.f;
+}
+template <bool TRANS, bool NARROW>
+__device__ __forceinline__ void stage_rotated(const RT& a, float* dst, int col_off, int h, int row0, int len, float mul, const float* rowmul) {
+    if constexpr (NARROW) stage_rotated_narrow<TRANS>(a, dst, col_off, h, row0, len, mul, rowmul);
+    else stage_rotated_wide<TRANS>(a, dst, col_off, h, row0, len, mul, rowmul);
+}
+
 // What bounds these kernels is fp32 arithmetic (two columns and NACC rows of the state per thread: NACC packed products of two per 16-byte read of Kw), once the
 // loads come in groups. 4 entries of 312 to 512 tokens, 4 heads of 128 x 256: 78 us with a load per token and column, one behind the other, now see below.
 template <int NACC, bool FULL>   // accumulators per thread (a multiple of 4): dim <= 4 * NACC, FULL: equal
-__global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc) {
+__global__ void __launch_bounds__(256, NACC == 8 ? 4 : 1) retention_chunk_state_kernel(const RC rc) {
     pdl_wait();
     pdl_launch_dependents();
     extern __shared__ __align__(16) float sm[];
@@ -178,7 +217,7 @@ __global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc)
     const float decay = a.decay[h];
     for (int j = threadIdx.x; j < len; j += blockDim.x) pw[j] = powf(decay, (float)(len - 1 - j));
     __syncthreads();
-    stage_rotated<false>(a, Kw, a.k_off, h, row0, len, a.k_scale, pw);
+    stage_rotated<false, NACC == 8>(a, Kw, a.k_off, h, row0, len, a.k_scale, pw);
     __syncthreads();
     // thread: kColsPerThread value columns, NACC consecutive rows of the state (read from shared memory four at a time)
     const int c = cb * kChunkCols + (threadIdx.x & 63), d0 = (threadIdx.x >> 6) * NACC, dpad = (dim + 3) & ~3;
@@ -189,7 +228,7 @@ __global__ void __launch_bounds__(256) retention_chunk_state_kernel(const RC rc)
         for (int k = 0; k < NACC / 2; ++k) acc[q][k] = 0ull;
     if (c < a.vdim && d0 < dim) {
         const float* vcol = a.proj + (size_t)row0 * a.ld_proj + a.v_off + h * a.vdim + c;
-        constexpr int J = 8;
+        constexpr int J = NACC == 8 ? 4 : 8;
         int off[kColsPerThread];
 #pragma unroll
         for (int q = 0; q < kColsPerThread; ++q) off[q] = c + 64 * q < a.vdim ? 64 * q : 0;
@@ -279,6 +318,7 @@ __global__ void __launch_bounds__(256) retention_chunk_scan_kernel(const RC rc) 
 }
 
 // Thread: columns c, c + 64; sixteen consecutive rows, two per packed product (q and A lie transposed: a 16-byte read is four rows of one j or component).
+template <bool NARROW>
 __global__ void __launch_bounds__(256, 2) retention_chunk_out_kernel(const RC rc) {
     pdl_wait();
     pdl_launch_dependents();
@@ -297,8 +337,8 @@ __global__ void __launch_bounds__(256, 2) retention_chunk_out_kernel(const RC rc
     for (int k = threadIdx.x; k <= kChunk; k += blockDim.x) pw[k] = powf(decay, (float)k);
     if (len < kChunk)   // rows and columns behind the entry: the tiles below read them
         for (int i = threadIdx.x; i < 2 * dim * (kChunk - len); i += blockDim.x) Qt[i / (kChunk - len) * kChunkT + len + i % (kChunk - len)] = 0.f;
-    stage_rotated<true>(a, Qt, a.q_off, h, row0, len, 1.f, nullptr);
-    stage_rotated<true>(a, Kt, a.k_off, h, row0, len, a.k_scale, nullptr);
+    stage_rotated<true, NARROW>(a, Qt, a.q_off, h, row0, len, 1.f, nullptr);
+    stage_rotated<true, NARROW>(a, Kt, a.k_off, h, row0, len, a.k_scale, nullptr);
     __syncthreads();
     {   // q . k in tiles of four rows and four columns
         const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
@@ -510,10 +550,11 @@ extern "C" int b200_retention(const b200_retention_args* p, void* stream) {
         const int rs = chunk_row_stride(p->dim);
         const size_t smem1 = ((size_t)kChunk * rs + kChunk) * sizeof(float);
         const size_t smem3 = ((size_t)2 * p->dim * kChunkT + kChunk * kChunkT + kChunk + 4) * sizeof(float);
-        static unsigned long long done1[8] = {}, done3 = 0;
+        static unsigned long long done1[8] = {}, done3[2] = {};
         // the attribute is set once per kernel: to the most any supported dim (256) needs
         constexpr int kMax1 = (kChunk * 260 + kChunk) * 4, kMax3 = (2 * 256 * kChunkT + kChunk * kChunkT + kChunk + 4) * 4;
-        cudaError_t e = ensure_max_dynamic_smem((const void*)retention_chunk_out_kernel, kMax3, done3);
+        auto out = p->dim <= 32 ? retention_chunk_out_kernel<true> : retention_chunk_out_kernel<false>;
+        cudaError_t e = ensure_max_dynamic_smem((const void*)out, kMax3, done3[p->dim <= 32]);
         if (e != cudaSuccess) return (int)e;
         rc.col_blocks = col_blocks;
         auto state = [&](auto kernel, unsigned long long& done) {
@@ -533,7 +574,7 @@ extern "C" int b200_retention(const b200_retention_args* p, void* stream) {
             launch_chained(retention_chunk_scan_kernel<float4>, dim3(p->n_entries, p->heads, (per / 4 + 255) / 256), 256, 0, s, rc);
         else
             launch_chained(retention_chunk_scan_kernel<float>, dim3(p->n_entries, p->heads, (per + 255) / 256), 256, 0, s, rc);
-        launch_chained(retention_chunk_out_kernel, grid, 256, smem3, s, rc);
+        launch_chained(out, grid, 256, smem3, s, rc);
         count_launch(3);
         return (int)cudaGetLastError();
     }
