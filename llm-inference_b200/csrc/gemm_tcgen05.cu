@@ -732,18 +732,27 @@ static int least_shares(int m_tiles, int k_blocks, int sms) {
 
 int gemm_rows(const void* x, const void* W, const void* bias, void* y, int M, int N, int K, bool bf16, int out_kind, bool glu, int act, int unary, float limit, cudaStream_t s);
 
+// Up to 16 rows against few weights, where set-up and latency count: no tensor maps, barriers or tensor memory (gemm_rows.cu). The lines lie where the time of
+// gemm_stream_kernel is reached (rows / stream in a graph, weights from HBM, at 8 and at 16 rows unless it says otherwise).
+//   K <= 2048: 13 M weights up to 8 rows (4096 x 2048 0.81, 6184 x 2048 0.96, 7000 x 2048 1.00; 12288 x 1024 1.09), 8.5 M up to 16 (4096 x 2048 0.89, 5504 x 2048 1.17),
+//   17 M gated (2 x 4224 x 2048 0.86, 0.95; 2 x 8192 x 1024 0.95, 1.01; 2 x 5504 x 2048 1.17, 1.26); and 8192 features, whatever K: a CTA has too little to do for what it
+//   sets up (16384 x 512 1.31, 1.13, gated 2 x 12288 x 512 1.00, 1.09).
+//   Longer K, as long as every CTA has an SM: eight rows up to 12288 (2048 x 9216 0.94, 1024 x 12288 0.98, 1024 x 16384 1.10), more up to 6144 (2048 x 6144 0.95, 2048 x
+//   7168 1.02, 2048 x 8192 1.07, 1024 x 16384 1.17 to 1.25); but 64 features or fewer, with few clusters to share K, at any K (64 x 16384 0.72, 0.85). Gated ones, two sums for a load of x, less far the fewer CTAs share the weights' way: 3072 (2 x 128 x 3072 0.96, 1.02), from
+//   1024 features 4608 (2 x 1024 x 4608 0.94, 1.01; 2 x 256 x 4096 1.16, 1.28), from 2048 features 5504 (2 x 2048 x 5504 0.93, 0.97; 2 x 1408 x 5504 1.06, 1.09, 2 x 1920 x 6144 1.01, 1.07).
+static bool takes_rows(int M, int N, int K, bool glu, int sms) {
+    if (M > 16) return false;
+    const long long weights = (long long)N * K * (glu ? 2 : 1);
+    if (K <= 2048) return N <= 8192 && weights <= (glu ? 17000000 : M <= 8 ? 13000000 : 8500000);
+    if (N > 16 * sms || weights > 24000000) return false;
+    if (glu) return K <= (N >= 2048 ? 5504 : N >= 1024 ? 4608 : 3072);
+    return N <= 64 || K <= (M <= 8 ? 12288 : 6144);
+}
+
 // M <= 256 token rows against W = [N, K] (GLU: M <= 128, W = [2 N, K], N % 64 == 0)
 static int gemm_few_rows(const void* x, const void* W, GemmParams p, int M, int N, int K, bool glu, cudaStream_t s) {
     const int F = glu ? 64 : kBM, sms = sm_count();
-    // Up to 16 rows against few weights, where set-up and latency count: no tensor maps, barriers or tensor memory (gemm_rows.cu). The lines lie where the time of
-    // gemm_stream_kernel is reached (us in a graph, weights from HBM, stream / rows). K <= 2048, plain, up to 8 rows: 4096 x 1024 at 8 rows 5.7 / 3.6, 4096 x 2048
-    // 6.9 / 5.5, 6184 x 2048 8.6 / 8.1, 11008 x 2048 11.3 / 11.9; 9 to 16 rows: 8192 x 1024 7.2 / 6.8, 6184 x 2048 8.8 / 9.5; gated: 2 x 4096 x 2048 9.8 / 7.9,
-    // 2 x 8192 x 2048 15.0 / 15.7. Longer K, as long as every CTA has an SM: 2048 x 5504 8.7 / 6.7, 2048 x 8192 10.7 / 8.6, gated 2 x 2048 x 5504 11.7 / 10.0,
-    // 2 x 2048 x 8192 15.0 / 15.1, 4096 x 11008 18.4 / 23.0.
-    if (M <= 16) {
-        const long long weights = (long long)N * K * (glu ? 2 : 1), most = K > 2048 ? (N <= 16 * sms ? 24000000 : 0) : glu ? 17000000 : M <= 8 ? 13000000 : 8500000;
-        if (weights <= most) return gemm_rows(x, W, p.bias, p.C, M, N, K, p.in_bf16 != 0, p.out_kind, glu, p.glu_act, p.unary, p.glu_limit, s);
-    }
+    if (takes_rows(M, N, K, glu, sms)) return gemm_rows(x, W, p.bias, p.C, M, N, K, p.in_bf16 != 0, p.out_kind, glu, p.glu_act, p.unary, p.glu_limit, s);
     const int BN = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     p.rows_a = N; p.rows_b = M;
     p.m_tiles = (N + F - 1) / F; p.n_tiles = 1;
