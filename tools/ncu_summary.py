@@ -38,7 +38,7 @@ def launches(src, dst):
         agg.setdefault(key, []).append(v)
         total += v
     with open(dst, "w") as f:
-        f.write(f"ncu --metrics gpu__time_duration.sum --clock-control none (cold-cache, serialised): {src}\n\n")
+        f.write(f"ncu --metrics gpu__time_duration.sum --clock-control none (cold-cache, serialised)\n\n")
         f.write("| kernel | grid | block | launches | avg us | min us | max us | total ms | share |\n"
                 "|---|---|---|---|---|---|---|---|---|\n")
         for (name, g, b), v in sorted(agg.items(), key=lambda kv: -sum(kv[1])):
@@ -52,7 +52,7 @@ def full(src, dst):
     rows = list(csv.reader(out.splitlines()))
     hdr, units = rows[0], rows[1]
     with open(dst, "w") as f:
-        f.write(f"ncu --set full --clock-control none: {src}\n\n")
+        f.write(f"ncu --set full --clock-control none\n\n")
         for r in rows[2:]:
             f.write(f"### `{r[hdr.index('Kernel Name')]}`\n\n| metric | value | unit |\n|---|---|---|\n")
             for k in FULL_KEYS:
