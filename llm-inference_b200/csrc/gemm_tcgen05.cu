@@ -800,6 +800,13 @@ int gemm2_tcgen05_f16(const void* x, const void* W, const void* bias, void* y, i
 // without pairs narrower than 256 columns 5 % (gated: 9 %) faster. us, that choice / now: 1522 x 8192 -> 2048 49.2 / 38.5 (192 columns), 1522 x 2048 -> 4096 28.9 / 23.3
 // (192), 512 x 4096 -> 12288 48.1 / 41.8 (192), 512 x 11008 -> 4096 42.8 / 39.3 (128); 1024 x 1024 -> 1024 keeps 64 columns on one CTA (6.6; pairs 9.0). A pair has to be 3 %
 // cheaper than one CTA's best: below that the fit does not tell them apart.
+// Beyond what it was fitted to. A product of more than 100 GFLOP runs long enough for the power limit to set the clock, and a narrow tile moves more bytes per product: the pair of
+// 256 columns stands there unless another tile is 8 % cheaper. us back to back for seconds at the clock that this leaves, the tile named without that / 256 columns: 4096 x 11008 ->
+// 4096 355 (160) / 319, 4096 x 8192 -> 2048 128 (160) / 118, 6000 x 11008 -> 4096 502 (160) / 456, 6000 x 4096 -> 4096 179 (160) / 169, 2048 x 11008 -> 4096 162 (160) / 154, 8192 x 5504 -> 2048 168 (160) /
+// 163, 4096 x 4096 -> 4096 117 (160) / 114, 4096 x 4096 -> 12288 307 (224) / 309, 8192 x 4096 -> 12288 622 (224) / 615, 8192 x 4096 -> gated 11008 1088 (224) / 1072, 3000 x 1024 -> 32000 192 (224) / 185; 256 either way:
+// 8192 x 4096 -> 4096 210, 8192 x 11008 -> 4096 578, 4096 x 4096 -> gated 11008 535; kept: 2048 x 4096 -> 12288 159 (224) / 163. Shorter ones do not tell: 4096 x 5504 -> 2048 79.7 (160) / 79.3 for seconds, 72 / 77 one
+// at a time. Above 2048 rows, outputs whose rows do not end on 64 columns: what is stored across the lines' borders is priced too (least where a pass has most columns of a
+// row; one CTA stores a row per thread): 4096 x 1032 -> 1000 fp32 21.2 (128 columns on one CTA) / 15.3 (pairs of 256), weights from HBM.
 struct Tile { int rows, cols; float step, round, once32, once16; };
 struct TileChoice { int cols; bool pair; };
 static constexpr Tile kPlainTiles[] = {{128, 64, 0.168f, 0.f, 4.16f, 3.43f}, {128, 128, 0.205f, 0.14f, 5.10f, 3.87f}, {128, 256, 0.334f, 0.24f, 7.01f, 4.82f},
@@ -812,17 +819,22 @@ static constexpr Tile kGatedTiles[] = {{128, 256, 0.349f, 1.06f, 4.23f, 4.23f}, 
 template <int COUNT>
 static TileChoice choose_tile(const Tile (&tiles)[COUNT], int M, int N, int k_blocks, bool glu, bool f32, int sms, bool pairs_only = false) {
     TileChoice best{256, pairs_only};
-    float least = -1.f;
-    const bool pairs = pairs_only || gemm_pairs_enabled();
+    float least = -1.f, full = -1.f;   // full: the pair of 256 columns
+    const float outputs = (float)M * N * 1e-6f;
+    const bool pairs = pairs_only || gemm_pairs_enabled(), ragged = M > 2048 && N % 64 != 0;
     for (const Tile& t : tiles) {
         const bool pair = t.rows == 256;
         const int out_cols = glu ? t.cols / 2 : t.cols, at_once = pair ? sms / 2 : sms;
         if (pair ? !pairs || (N < 256 && !glu) : (pairs_only || (t.cols > N && t.cols > 64 && !glu))) continue;
         const long long n = ((long long)M + t.rows - 1) / t.rows * ((N + out_cols - 1) / out_cols), rounds = (n + at_once - 1) / at_once;
-        const float cost = ((float)rounds * (k_blocks * t.step + t.round) + (f32 ? t.once32 : t.once16) + (float)M * N * (f32 ? 4e-6f : 2e-6f) / 5.f) * (pair && !pairs_only ? 1.03f : 1.f);
+        float cost = (float)rounds * (k_blocks * t.step + t.round) + (f32 ? t.once32 : t.once16) + outputs * (f32 ? 4.f : 2.f) / 5.f;
+        if (ragged) cost += outputs * (!pair ? 1.7f : t.cols < 256 ? 0.8f : 0.4f);
+        if (pair && !pairs_only) cost *= 1.03f;
         if (least < 0.f || cost < least) { least = cost; best = {t.cols, pair}; }
+        if (pair && t.cols == 256) full = cost;
     }
-    return best;
+    const bool long_call = (glu ? 4.f : 2.f) * outputs * (float)k_blocks * kBK > 1e5f;   // MFLOP
+    return long_call && full > 0.f && least > 0.92f * full ? TileChoice{256, true} : best;
 }
 
 // what the rule names, for tests: columns of the accumulator, negative on a pair of CTAs

@@ -39,3 +39,11 @@ def test_the_switch_keeps_pairs_out(tile):
             "assert all(f(*s, False, 148) > 0 for s in %r)" % (shapes,))
     lib = sys.modules["llm_inference_b200"].lib_path()
     subprocess.run([sys.executable, "-c", code, lib], check=True, env=dict(os.environ, B200_GEMM_PAIR="0"))
+
+
+@pytest.mark.parametrize("M,N,K,gated,want", [
+    (4096, 4096, 11008, False, -256), (6000, 4096, 4096, False, -256), (4096, 2048, 8192, False, -256), (2048, 4096, 11008, False, -256), (8192, 11008, 4096, True, -256),   # at the power limit
+    (2048, 12288, 4096, False, -224), (3000, 2048, 5504, False, -192), (1522, 2048, 8192, False, -192), (1024, 1024, 1024, False, 64),                                      # 8 % cheaper, or too short for it
+    (4096, 1000, 1032, False, -256), (8192, 1000, 1032, False, -256), (4096, 1024, 1024, False, 256), (3000, 264, 136, False, 64)])                                          # rows that end inside 64 columns
+def test_beyond_the_fitted_sizes(tile, M, N, K, gated, want):
+    assert tile(M, N, K, gated, False) == want
