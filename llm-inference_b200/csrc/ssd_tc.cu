@@ -16,8 +16,9 @@
 // heads, 64: 44.7 -> 28.9 (37.3 in chunks of 64); 1, 2048, 33 heads, 128: 59.6 -> 39.6.
 // A product dt x that is not finite is multiplied as zero and its column is NaN from its token on: the zeros above the diagonal would carry it to
 // earlier tokens.
-// Measured, us, chunks of 64 on mma.sync against these (entries, tokens, heads, n_state; 64 value columns): 2, 2048, 64, 128: 164 / 84 (floor 11; prep 9, state 18, carry 17,
-// out 37: the last reads x twice and the states, 5 TB/s); 1, 2048, 33, 128: 91 / 60; 1, 128, 8, 128: 31 / 20; 1, 8192, 64, 128: 572 / 355; 4, 1500, 64, 64: 81 / 64.
+// Measured in a graph, us, chunks of 64 on mma.sync against these (entries, tokens, heads, n_state; 64 value columns): 2, 2048, 64, 128: 149 / 68.5 (floor 11; the out kernel is the longest:
+// x a second time and the states, 5 TB/s); 1, 2048, 33, 128: 86 / 40; 1, 128, 8, 128: 25.7 / 18.7; 2, 2048, 64, 64: 92 / 67; 4, 1500, 64, 64: 74 / 54. Error against 64 bits 3.2e-4 of the outputs'
+// norm, 2.9e-4 of the states', in either.
 #include <limits.h>
 
 #include <algorithm>
@@ -727,27 +728,34 @@ size_t ssd_scan_tc_bytes(int n_tokens, int n_entries, int heads, int groups, int
     return places * ((size_t)groups * 3 * kStImg + (size_t)heads * kStSums + units * kStUnit) + 256;
 }
 
+// units per CTA: the rounds of CTAs, one per SM, times what a CTA takes, three units' time for what its units share (state and out: 8 us before the first
+// unit, 2 to 4 us each)
+int ssd_tc_units(int n_tokens, int n_entries, int longest_entry, int heads, int groups, int vdim, int sms) {
+    const long long places = (long long)n_tokens / kStChunk + n_entries + 1, chunks = (longest_entry + kStChunk - 1) / kStChunk;
+    const long long some_chunks = std::min<long long>(chunks * n_entries, places - 1), per_group = (long long)heads * ((vdim + kStCols - 1) / kStCols) / groups;
+    long long per = 1, best = LLONG_MAX;
+    for (long long u = 1; u <= std::min<long long>(per_group, 64); ++u) {
+        const long long cost = (some_chunks * groups * ((per_group + u - 1) / u) + sms - 1) / sms * (u + 3);
+        if (cost < best) { best = cost; per = u; }
+    }
+    return (int)per;
+}
+
 int ssd_scan_tc(const SS& s, const b200_ssd_scan_args& p, cudaStream_t stream) {
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
-    // n_state: the products' rows are padded to 128. 2048 tokens, one entry, 16 heads x 16: 45 us here, 34 in chunks of 64; 64 heads x 64: 82 and 99
+    // n_state: the products' rows are padded to 128. us here / in chunks of 64, 2 entries, 2048 tokens, 64 heads: 16 states 66 / 61, 32 states 66 / 69, 64 states 69 / 92; 8 entries of 150
+    // tokens, 8 heads of 128 columns: 27 / 22, 28 / 24, 28 / 28
     if (p.n_state > 128 || p.n_state <= 32 || p.vdim % 4 || p.ld_u % 4 || p.x_off % 4 || !al16(p.u) || !al16(p.out) || !al16(p.state) || !p.workspace) return -1;
     const long long places = (long long)p.n_tokens / kStChunk + p.n_entries + 1, col_blocks = (p.vdim + kStCols - 1) / kStCols, all_units = p.heads * col_blocks;
-    const long long chunks = (p.longest_entry + kStChunk - 1) / kStChunk, some_chunks = std::min<long long>(chunks * p.n_entries, places - 1), per_group = all_units / p.groups;
+    const long long chunks = (p.longest_entry + kStChunk - 1) / kStChunk, per_group = all_units / p.groups;
     const size_t pad = (256 - (reinterpret_cast<uintptr_t>(p.workspace) & 255u)) & 255u;
     const size_t need = ssd_scan_tc_bytes(p.n_tokens, p.n_entries, p.heads, p.groups, p.vdim, p.n_state);
     const long long jobs = p.n_entries * (8ll * p.groups + (p.heads + 3) / 4);
     if (p.workspace_bytes < need || chunks > 65535 || p.n_entries > 65535 || jobs > 0x7fffffffll) return -1;
-    // units per CTA: the rounds of CTAs, one per SM, times what a CTA takes, three units' time for what its units share (state and out: 8 us before the first
-    // unit, 2 to 4 us each)
-    const int sms = sm_count();
-    long long per = 1, best = LLONG_MAX;
-    for (long long u = 1; u <= std::min<long long>(per_group, 64); ++u) {
-        const long long cost = (some_chunks * p.groups * ((per_group + u - 1) / u) + sms - 1) / sms * (u + 3);
-        if (cost < best) { best = cost; per = u; }
-    }
     SsTc t{};
     t.s = s;
     t.s.col_blocks = (int)col_blocks;
+    const long long per = ssd_tc_units(p.n_tokens, p.n_entries, p.longest_entry, p.heads, p.groups, p.vdim, sm_count());
     const long long blocks = (long long)p.groups * ((per_group + per - 1) / per);
     t.blocks = (int)blocks;
     if (blocks * p.n_entries > 0x7fffffffll || all_units * 4 > 0x7fffffffll) return -1;

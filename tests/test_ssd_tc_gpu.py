@@ -1,5 +1,6 @@
 """The state-space recurrence in chunks of 128 tokens: ends of chunks, of their sixteen-token parts and of column blocks, odd state sizes, groups, carried states,
-values that are not finite, and a workspace of the size that the 64-token chunks need."""
+many turns of the rings, values that are not finite; and the 64-token chunks behind the same call, for leading dimensions that four does not divide and for the workspace
+that they need."""
 import ctypes as C
 
 import pytest
@@ -44,10 +45,8 @@ class Call:
         ws = torch.full((need,), 255, dtype=torch.uint8, device="cuda")
         a.workspace, a.workspace_bytes = ws.data_ptr(), need
         torch.cuda.synchronize()
-        before = S.lib().b200_launch_count()
         assert S.lib().b200_ssd_scan(C.byref(a), None) == 0
         torch.cuda.synchronize()
-        return S.lib().b200_launch_count() - before
 
     def check(self):
         v, H, G, P, N = self.u.double(), self.H, self.G, self.P, self.N
@@ -67,7 +66,34 @@ class Call:
     (5, 1, 64, 128, 0, (128,)), (6, 2, 64, 33, 2, (129, 127, 1)), (3, 1, 68, 72, 0, (257, 16, 17)), (4, 4, 128, 128, 4, (383, 2)), (2, 1, 4, 100, 0, (640, 130)),
     (64, 1, 64, 128, 0, (300, 200)), (1, 1, 192, 64, 0, (145,))])
 def test_chunks_of_128(S, H, G, P, N, pad, cnt):
+    """(129, 127, 1) with a leading dimension of 518 falls to the 64-token chunks: test_odd_states has its sizes in chunks of 128"""
     c = Call(S, H, G, P, N, pad, cnt)
+    c.run()
+    c.check()
+
+
+def in_chunks_of_128(H, G, P, N, pad, cnt):
+    """what ssd_scan_tc asks of a call besides its workspace"""
+    return 32 < N <= 128 and P % 4 == 0 and (H * P + 2 * G * N + pad) % 4 == 0 and max(cnt) >= 128
+
+
+@pytest.mark.parametrize("H,G,P,N,pad,cnt", [(6, 2, 64, 33, 0, (129, 127, 1)), (3, 1, 64, 34, 0, (200, 100)), (5, 1, 68, 127, 2, (256, 131)), (2, 1, 4, 101, 2, (140,)), (4, 4, 64, 67, 0, (385,))])
+def test_odd_states(S, H, G, P, N, pad, cnt):
+    assert in_chunks_of_128(H, G, P, N, pad, cnt) and N % 4
+    c = Call(S, H, G, P, N, pad, cnt)
+    c.run()
+    c.check()
+
+
+@pytest.mark.parametrize("H,G,P,N,cnt,most", [(64, 1, 64, 128, (1500, 1300), 11), (33, 1, 64, 128, (2400, 2300), 11), (48, 2, 128, 72, (1100, 1000), 12), (33, 1, 128, 126, (1500, 700, 300, 900), 17),
+                                              (72, 1, 72, 64, (520, 1530), 18)])
+def test_many_units_per_cta(S, pkg, H, G, P, N, cnt, most):
+    """a CTA's rings of sums (four slots), inputs, states and results (two each) go round several times, in some CTAs once more than in others"""
+    units = C.CDLL(pkg.lib_path())["_ZN4b20012ssd_tc_unitsEiiiiiii"](sum(cnt), len(cnt), max(cnt), H, G, P, torch.cuda.get_device_properties(0).multi_processor_count)
+    per_group = H * ((P + 63) // 64) // G
+    blocks = -(-per_group // units)
+    assert in_chunks_of_128(H, G, P, N, 0, cnt) and -(-per_group // blocks) == most >= 9
+    c = Call(S, H, G, P, N, 0, cnt)
     c.run()
     c.check()
 
