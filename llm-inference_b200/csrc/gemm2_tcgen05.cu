@@ -1,6 +1,6 @@
 // Two-CTA tcgen05 GEMM for the prefill linears (launchLinearGemm with many token rows, linear.cu:39-104):
-//   D[256, 256] (fp32, TMEM of two SMs) += A[256, 64] * B[256, 64]^T per K step, fp16 operands, K-major.
-// A cluster of two CTAs (one TPC) owns a 256 x 256 output tile: each CTA loads ITS 128 rows of A and ITS
+//   D[256, 256] (fp32, TMEM of two SMs) += A[256, 64] * B[256, 64]^T per K step, fp16 or bfloat16 operands, K-major.
+// A cluster of two CTAs (one TPC) owns an output tile of 256 rows and, at its widest, 256 columns: each CTA loads ITS 128 rows of A and ITS
 // 128 rows of B (half of the N extent) and keeps 128 rows x 256 columns of the accumulator in its own
 // TMEM; the leader CTA's single MMA thread issues tcgen05.mma.cta_group::2 (M = 256), which reads both
 // CTAs' shared memory. Against the one-CTA kernel (gemm_tcgen05.cu: 48 KB of operands per 512 tensor
@@ -12,7 +12,7 @@
 //   warp 1    TMEM allocation (both CTAs); MMA issue (leader only); tcgen05.commit multicast to both CTAs
 //   warps 2-5 epilogue (both CTAs): own 128 rows from own TMEM, then a remote arrive on the leader's
 //             accumulator-empty barrier
-// GLU: as in gemm_tcgen05.cu — the leader's B half is 128 gate rows, the peer's the matching 128 up rows.
+// GLU: as in gemm_tcgen05.cu — the leader's B half is cols / 2 gate rows (128 at the full width), the peer's the matching up rows.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -40,7 +40,7 @@ struct Gemm2Params {
     const __half* residual;   // [tokens, ldc] or nullptr: C = half(half(acc + bias) + residual), launchAddResidual folded in
     int tokens, n_out;  // valid rows of A; valid output features (GLU: inter)
     int ldc, k_blocks;
-    int m_tiles, n_tiles;   // tiles of 256 rows x (256 features | GLU: 128 features)
+    int m_tiles, n_tiles;   // tiles of 256 rows x (cols features | GLU: cols / 2 features)
     int cols, stages;       // columns of a tile's accumulator (a multiple of 32 up to 256; gated: half of them gates), stages of the ring
     int group_m;            // tile order: bands of group_m row tiles swept over all column tiles (0: column-major over all rows)
     int out_kind, glu_act, unary;   // the families' calls (KIND 2 and 3 of the kernel, bfloat16 operands), as GemmParams in gemm_tcgen05.cu
@@ -61,7 +61,7 @@ __device__ __forceinline__ void tile_of_unit(const Gemm2Params& p, int n_tiles, 
 }
 
 // One warp's part of an accumulator tile (32 rows x the tile's columns): TMEM (taddr: this warp's lane quarter, the tile's first column) -> fp16 -> C.
-// nt: column tile (256 features, GLU: 128 features with gate in columns [0,128) and up in [128,256) of the accumulator). Every thread owns an
+// nt: column tile (p.cols features; GLU: half as many, their gates in the first half of the accumulator, their ups in the second). Every thread owns an
 // accumulator ROW in TMEM, so storing straight from registers makes each store instruction touch 32 rows x 16 bytes - 8192
 // sixteen-byte transactions per 128 x 512 CTA tile, ~20 k clocks that the 256 x 512 kernel cannot hide. Here 64 output
 // columns of the warp's 32 rows are rounded to fp16, staged in 4 KB of shared memory (16-byte chunks XOR-swizzled by row:
@@ -381,7 +381,7 @@ gemm2_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // of both accumulators from the same A descriptors. Against the 256 x 256 tile: 24 instead of 32 KB loaded per 128 x 256 x
 // 64 MAC block (L2 -> SM and TMA smem writes -25 %), shared-memory traffic (TMA writes + MMA operand reads) 112 KB per
 // 1024 tensor clocks instead of 128 KB - the 256 x 256 kernel asks for exactly the 128 B/clk an SM's shared memory
-// delivers, which is where its 83 % tensor-pipe ceiling comes from (ncu: profiles/gemm_vs_cublas_full.md; cuBLAS'
+// delivers, which is where its 83 % tensor-pipe ceiling comes from (seen under ncu; cuBLAS'
 // kernel for this shape has the same 48 KB stages x 4). Price: both accumulators fill all 512 TMEM columns, so the
 // epilogue of a tile is not hidden behind the next tile's MMAs any more; eight epilogue warps (four per accumulator)
 // keep it short, and the first K steps of the next tile's accumulator 0 are issued as soon as ITS half is drained.

@@ -1,12 +1,12 @@
 // y[M, N] = x[M, K] W[N, K]^T for up to 16 token rows, fp16 or bfloat16 operands, fp32 sums: one CTA per 16 features (gated units: 16 gate rows and their 16 up
-// rows), its eight warps share K in pieces of 32 and meet in shared memory.
+// rows), its eight warps (sixteen above K = 2048) share K in pieces of 32 and meet in shared memory.
 //
 // What bounds it is the weights' way from HBM and, at the sizes of a decode step (a few MB, 1 to 3 us), everything around it: launch, set-up, the first
 // load's latency, the merge. So there is nothing to set up (no tensor maps, barriers, tensor memory or cluster): a lane's 16-byte loads are the fragments of
 // mma.sync m16n8k16 as they come (a K index may stand anywhere as long as weights and tokens agree: a lane holds eight consecutive k of its row where the
 // instruction thinks of two times two pairs), four pieces per warp are in flight ahead of the products, and the lines of a CTA's weights are prefetched
 // to L2 while the launch before is still running (a prefetch reads nothing: what that launch writes is seen all the same).
-// Measured in gemm_few_rows (gemm_tcgen05.cu), where the line to the tcgen05 kernels lies.
+// Measured at takes_rows (gemm_tcgen05.cu), where the lines to the tcgen05 kernels lie.
 #include <cuda_bf16.h>
 
 #include <type_traits>

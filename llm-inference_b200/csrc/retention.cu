@@ -200,7 +200,7 @@ __device__ __forceinline__ void stage_rotated(const RT& a, float* dst, int col_o
 }
 
 // What bounds these kernels is fp32 arithmetic (two columns and NACC rows of the state per thread: NACC packed products of two per 16-byte read of Kw), once the
-// loads come in groups. 4 entries of 312 to 512 tokens, 4 heads of 128 x 256: 78 us with a load per token and column, one behind the other, now see below.
+// loads come in groups. 4 entries of 312 to 512 tokens, 4 heads of 128 x 256: 68 us with a load per token and column, one behind the other, 34 now.
 template <int NACC, bool FULL>   // accumulators per thread (a multiple of 4): dim <= 4 * NACC, FULL: equal
 __global__ void __launch_bounds__(256, NACC == 8 ? 4 : 1) retention_chunk_state_kernel(const RC rc) {
     pdl_wait();

@@ -1,4 +1,4 @@
-"""Linears of more than 256 token rows: every tile that the rule can name (64, 128, 256 columns on one CTA, 256 x 256 on a pair), ragged in rows, features and K,
+"""Linears of more than 256 token rows: the tiles of one CTA (64, 128, 256 columns) and some of a pair's (test_linear_pair_widths_gpu has them all), ragged in rows, features and K,
 plain, squared relu and gated, bfloat16 and fp32 outputs; fp16 with a bias and with a residual."""
 import pytest
 
