@@ -92,3 +92,18 @@ def test_gelu_is_no_further_off_than_by_tanh(S):
     assert float((tiles - want).norm()) <= float((few - want).norm())
     at = (z.abs() < 4) & (z.abs() > 1e-3)
     assert float(((tiles - want).abs() / want.abs())[at].max()) <= 1.0625 * float(((few - want).abs() / want.abs())[at].max())
+
+
+@pytest.mark.parametrize("M,N", [(257, 128), (600, 1024), (1100, 5504)])
+def test_fp16_gives_the_bits_of_the_unfused_sequence(pkg, S, M, N):
+    """the product rounded to fp16, silu of the gate rounded, their product rounded; sums are single products"""
+    x, W = (t.clamp(-90, 90).half() for t in operands(M, N))
+    x[M // 4 + 1] = 0
+    y, capi = torch.full((M + 1, N), 7.0, dtype=torch.float16, device="cuda"), pkg.capi
+    torch.cuda.synchronize()
+    assert capi.lib().b200_linear_swiglu(x.data_ptr(), W.data_ptr(), y.data_ptr(), M, N, 8, capi.F16, None) == 0
+    torch.cuda.synchronize()
+    z = (x.float() @ W.float().T).half().float()
+    g, u = z[:, :N], z[:, N:]
+    assert same(y[:M], ((g / (1 + torch.exp(-g))).half().float() * u).half())
+    assert bool((y[M] == 7.0).all())
