@@ -16,8 +16,8 @@
 // heads, 64: 44.7 -> 28.9 (37.3 in chunks of 64); 1, 2048, 33 heads, 128: 59.6 -> 39.6.
 // A product dt x that is not finite is multiplied as zero and its column is NaN from its token on: the zeros above the diagonal would carry it to
 // earlier tokens.
-// Measured in a graph, us, chunks of 64 on mma.sync against these (entries, tokens, heads, n_state; 64 value columns): 2, 2048, 64, 128: 149 / 68.5 (floor 11; the out kernel is the longest:
-// x a second time and the states, 5 TB/s); 1, 2048, 33, 128: 86 / 40; 1, 128, 8, 128: 25.7 / 18.7; 2, 2048, 64, 64: 92 / 67; 4, 1500, 64, 64: 74 / 54. Error against 64 bits 3.2e-4 of the outputs'
+// Measured in a graph, us, chunks of 64 on mma.sync against these (entries, tokens, heads, n_state; 64 value columns): 2, 2048, 64, 128: 149 / 68.5 (floor 11; under ncu 9, 19,
+// 22 and 39 of 90: the latency of loads, DRAM a quarter and L2 a fifth to two fifths busy, the tensor pipe an eighth); 1, 2048, 33, 128: 86 / 40; 1, 128, 8, 128: 25.7 / 18.7; 2, 2048, 64, 64: 92 / 67; 4, 1500, 64, 64: 74 / 54. Error against 64 bits 3.2e-4 of the outputs'
 // norm, 2.9e-4 of the states', in either.
 #include <limits.h>
 
