@@ -237,13 +237,16 @@ __global__ void __launch_bounds__(448, 1) ssd_tc_state_kernel(const SsTc t) {
     uint64_t *sum_full = bars, *sum_empty = bars + 2, *x_full = bars + 4, *x_empty = bars + 6, *d_full = bars + 8, *d_empty = bars + 10, *b_full = bars + 12;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint64_t* drained = bars + 14;
+    volatile int* asked = reinterpret_cast<volatile int*>(bars + 15);   // sums requested so far
     const SS& a = t.s;
     const StWork w(t);
     if (w.len <= 0 || w.count <= 0) return;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, quarter = warp & 3;
     if (warp == 12) tmem_alloc(tmem_slot, 128);
     if (threadIdx.x == 0) {
-        *dead = 0;
+        *dead = *asked = 0;
+        mbar_init(drained, 1);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&sum_full[i], 1); mbar_init(&sum_empty[i], 8);
             mbar_init(&x_full[i], 8); mbar_init(&x_empty[i], 1);
@@ -344,7 +347,9 @@ __global__ void __launch_bounds__(448, 1) ssd_tc_state_kernel(const SsTc t) {
         for (int u = 0; u < w.count; ++u) {
             const int b = u & 1;
             mbar_wait_or_leave(&sum_empty[b], ((uint32_t)(u >> 1) & 1u) ^ 1u, dead);
+            if (__any_sync(0xffffffffu, *dead)) break;
             if (lane == 0) {
+                *asked = u + 1;
                 mbar_expect_tx(&sum_full[b], kStSums);
                 bulk_g2s(smem + kSuOffSums + b * kStSums, t.sums + (w.place * a.heads + w.head(u)) * (kStSums / 4), kStSums, &sum_full[b]);
             }
@@ -352,6 +357,16 @@ __global__ void __launch_bounds__(448, 1) ssd_tc_state_kernel(const SsTc t) {
         }
     }
     __syncthreads();
+    if (*dead) {   // what is under way lands first
+        if (warp == 13) {
+            mbar_wait_limited(b_full, 0u);
+            for (int u = max(0, *asked - 2); u < *asked; ++u) mbar_wait_limited(&sum_full[u & 1], (uint32_t)(u >> 1) & 1u);
+        } else if (warp == 12) {
+            if (elect_one()) umma_commit(drained);
+            mbar_wait_limited(drained, 0u);
+        }
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 12) tmem_dealloc(tmem, 128);
 }
@@ -437,13 +452,16 @@ __global__ void __launch_bounds__(26 * 32, 1) ssd_tc_out_kernel(const SsTc t) {
              *d_full = bars + 24, *d_empty = bars + 26, *c_full = bars + 28, *cb_full = bars + 29;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 30);
     volatile int* dead = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint64_t* drained = bars + 31;
+    volatile int* asked = reinterpret_cast<volatile int*>(bars + 32);   // sums, states requested so far
     const SS& a = t.s;
     const StWork w(t);
     if (w.len <= 0 || w.count <= 0) return;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, quarter = warp & 3;
     if (warp == 24) tmem_alloc(tmem_slot, 512);
     if (threadIdx.x == 0) {
-        *dead = 0;
+        *dead = asked[0] = asked[1] = 0;
+        mbar_init(drained, 1);
         for (int i = 0; i < 4; ++i) {
             mbar_init(&sum_full[i], 1); mbar_init(&sum_empty[i], 24);
             mbar_init(&m_full[i], 4 - i); mbar_init(&m_empty[i], 1);
@@ -703,14 +721,18 @@ __global__ void __launch_bounds__(26 * 32, 1) ssd_tc_out_kernel(const SsTc t) {
         for (int u = 0; u < w.count; ++u) {
             const int b = u & 1;
             mbar_wait_or_leave(&sum_empty[u & 3], ((uint32_t)(u >> 2) & 1u) ^ 1u, dead);
+            if (__any_sync(0xffffffffu, *dead)) break;
             if (lane == 0) {
+                asked[0] = u + 1;
                 mbar_expect_tx(&sum_full[u & 3], kStSums);
                 bulk_g2s(smem + kSoOffSums + (u & 3) * kStSums, t.sums + (w.place * a.heads + w.head(u)) * (kStSums / 4), kStSums, &sum_full[u & 3]);
             }
             __syncwarp();
             if (u == 0) mbar_wait_or_leave(cb_full, 0u, dead);   // B has been read
             mbar_wait_or_leave(&s_empty[b], ((uint32_t)(u >> 1) & 1u) ^ 1u, dead);
+            if (__any_sync(0xffffffffu, *dead)) break;
             if (lane == 0) {
+                asked[1] = u + 1;
                 mbar_expect_tx(&s_full[b], kStUnit);
                 bulk_g2s(smem + kSoOffS + b * kStUnit, reinterpret_cast<const unsigned char*>(t.states) + (w.place * ((size_t)a.heads * a.col_blocks) + w.unit(u)) * kStUnit, kStUnit, &s_full[b]);
             }
@@ -718,6 +740,17 @@ __global__ void __launch_bounds__(26 * 32, 1) ssd_tc_out_kernel(const SsTc t) {
         }
     }
     __syncthreads();
+    if (*dead) {   // what is under way lands first
+        if (warp == 25) {
+            mbar_wait_limited(c_full, 0u);
+            for (int u = max(0, asked[0] - 4); u < asked[0]; ++u) mbar_wait_limited(&sum_full[u & 3], (uint32_t)(u >> 2) & 1u);
+            for (int u = max(0, asked[1] - 2); u < asked[1]; ++u) mbar_wait_limited(&s_full[u & 1], (uint32_t)(u >> 1) & 1u);
+        } else if (warp == 24) {
+            if (elect_one()) umma_commit(drained);
+            mbar_wait_limited(drained, 0u);
+        }
+        __syncthreads();
+    }
     tc_fence_after();
     if (warp == 24) tmem_dealloc(tmem, 512);
 }

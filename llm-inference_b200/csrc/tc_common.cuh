@@ -212,6 +212,28 @@ __device__ __forceinline__ void mbar_wait_or_leave(uint64_t* bar, uint32_t parit
     __syncwarp();
 }
 
+// A CTA that gave up (dead) still has copies and products under way, which must not land behind its end in what is somebody else's by then: a wait for one of them that
+// takes no notice of dead and itself ends after a second.
+__device__ __forceinline__ void mbar_wait_limited(uint64_t* bar, uint32_t parity) {
+    uint64_t t0, now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (;;) {
+        uint32_t done;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        if (done || now - t0 > 1000000000ull) break;
+    }
+    __syncwarp();
+}
+
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
