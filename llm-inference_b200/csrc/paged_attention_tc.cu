@@ -467,7 +467,7 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     else if (a.dim == 128 && a.vdim == 256) rc = launch_tc_for<128, 256>(a, longest_entry, s);
     if (rc != 0) return rc;
     count_launch();
-    if (a.n_tokens != longest_entry) return paged_decode(a, longest_seen, true, s);   // the sequences that bring one token
+    if (a.n_tokens != longest_entry) return paged_decode(a, longest_seen, a.n_tokens - (longest_entry > 0 ? longest_entry : 0), 0, s);   // the sequences that bring one token
     return 0;
 }
 

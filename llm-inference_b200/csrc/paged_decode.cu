@@ -3,7 +3,7 @@
 //
 // What bounds it: the keys and values, read once (8 KB per 16 keys of 128 x 128), so the kernel has to keep enough of them on their way
 // and spend few instructions per byte. A warp walks its own run of keys, 16 at a time, out of a ring of its own in shared memory that
-// cp.async fills three steps deep (24 KB per warp, two CTAs of four warps per SM), and never waits for another warp:
+// one lane fills three steps ahead by TMA (24 KB per warp, two CTAs of four warps per SM; keys are asked for again as soon as the scores are formed), and never waits for another warp:
 //   S^T = K Q^T   mma.sync m16n8k16, keys on the M axis, the R <= 8 query heads of the key head on the N axis
 //   softmax       fp32 in registers, a running (maximum, denominator) per warp; cap, bias, temperature and masks as in the row kernel
 //   O^T = V^T P^T value dimensions on the M axis (ldmatrix.trans). The weights keep 24 bits: p = hi + mid + lo (three bfloat16, the
@@ -11,9 +11,10 @@
 //                 movmatrix turns the weights' fragments.
 // Warps merge through shared memory, CTAs through distributed shared memory (rank order, so the sum does not depend on timing). The merge
 // adds the sink.
-// Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128: 20.5 -> 7.1 us;
-// 32 sequences of up to 2048 tokens, 16 / 8 heads x 128 (190 MB), bias and sink: 384 -> 59 us (69 us with a step's keys and values in
-// registers, requested one step ahead); 128 such sequences without bias run at 5.0 TB/s.
+// Measured (before: the group kernel of capped_attention.cu with a combine launch): one sequence of 500 tokens, 8 / 4 heads x 128: 20.5 -> 6.6 us;
+// 32 sequences of up to 2048 tokens, 16 / 8 heads x 128 (190 MB), bias and sink: 384 -> 48 us. With the rows brought by cp.async (16 instructions and their addresses per lane and step) and a lookup of the bias for
+// keys beyond its table those were 6.9 and 59 us, 8 sequences of up to 2048 17.6 / 14.2, 12 of up to 1500, capped, 24.0 / 17.1. Two stages per warp and three CTAs per SM: slower (8 of 2048 18.4:
+// clusters are laid onto as few SMs as hold them).
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -23,6 +24,7 @@
 #include "common.cuh"
 #include "launch_count.h"
 #include "paged_attention.cuh"
+#include "tc_common.cuh"
 
 namespace b200 {
 namespace cg = cooperative_groups;
@@ -30,10 +32,11 @@ namespace cg = cooperative_groups;
 constexpr int kPdWarps = 4, kPdStep = 16, kPdHeads = 8, kPdMaxCluster = 8;
 
 template <int D, int VD>
-struct PdRing {   // row strides in elements (16 bytes of padding: conflict-free ldmatrix), a step's keys, then its values
-    static constexpr int kRS = D + 8, kRSV = VD + 8, kStages = VD > 128 ? 2 : 3;
-    static constexpr int kStep = kPdStep * (kRS + kRSV), kWarp = kStages * kStep;   // elements
-    static constexpr int kBytes = kPdWarps * kWarp * 2;
+struct PdRing {   // a step's keys, then its values, as TMA brings them: boxes of 16 rows x 64 columns, swizzled over 128 bytes
+    static constexpr int kStages = VD > 128 ? 2 : 3, kBox = kPdStep * 128;
+    static constexpr int kK = D / 64 * kBox, kStep = kK + VD / 64 * kBox, kWarp = kStages * kStep;
+    static constexpr int kBytes = kPdWarps * kWarp + 1024;
+    static constexpr int kPerSm = 2;
 };
 
 __device__ __forceinline__ uint32_t pd_transpose(uint32_t v) {   // 8 x 8 tile of 16-bit numbers, a pair per thread
@@ -42,40 +45,68 @@ __device__ __forceinline__ uint32_t pd_transpose(uint32_t v) {   // 8 x 8 tile o
     return r;
 }
 
+__device__ __forceinline__ void pd_ldsm_x4(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void pd_ldsm_x4_trans(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+
 // MIXED: a batch that also holds prompt portions, which other kernels take. Cluster z looks after the tokens z, z + gridDim.z, ... and serves
 // those that are their sequence's only token in the batch.
 template <int D, int VD, bool MIXED>
-__global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA a) {
+__global__ void __launch_bounds__(kPdWarps * 32, PdRing<D, VD>::kPerSm)
+paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a) {
     using bf = __nv_bfloat16;
     using L = PdRing<D, VD>;
     constexpr int KS = D / 16;        // k steps of the scores
     constexpr int MT = VD / 16;       // m tiles of the output
-    extern __shared__ __align__(16) float pd_sm[];
+    constexpr int NS = L::kStages;
+    extern __shared__ __align__(1024) unsigned char pd_raw[];
+    unsigned char* pd_sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(pd_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t pd_bars[kPdWarps * 2 * NS];
+    __shared__ int pd_dead;
+    volatile int* dead = &pd_dead;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32, gid = lane >> 2, tig = lane & 3;
+    uint64_t *k_full = pd_bars + warp * 2 * NS, *v_full = k_full + NS;   // of this warp's ring
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < 2 * NS; ++i) mbar_init(&k_full[i], 1);
+        mbar_fence_init();
+        if (warp == 0) { *dead = 0; tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
+    }
+    __syncthreads();
     if (!MIXED) {
         pdl_wait();
         pdl_launch_dependents();
     }
     const int R = a.heads / a.kv_heads, splits = gridDim.x;
-    float* om = pd_sm;                                 // once the rings have been used: [warps][R][VD], then this CTA's share in the first [R][VD]
+    float* om = reinterpret_cast<float*>(pd_sm);                                 // once the rings have been used: [warps][R][VD], then this CTA's share in the first [R][VD]
     __shared__ float ms[kPdWarps * kPdHeads], ls[kPdWarps * kPdHeads];   // [warps][R], then [R]
     const int ku = blockIdx.y, g = ku / a.maps, mp = ku % a.maps;
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane >> 2, tig = lane & 3;
-    const int k_units = a.kv_heads * a.maps, q_units = a.heads * a.maps;
-    const bf* K = reinterpret_cast<const bf*>(a.k_pool) + (size_t)ku * D;
-    const bf* V = reinterpret_cast<const bf*>(a.v_pool) + (size_t)g * VD;
-    bf* ring = reinterpret_cast<bf*>(pd_sm) + warp * L::kWarp;
-    const size_t k_row = (size_t)k_units * D, v_row = (size_t)a.kv_heads * VD;
-
+    const int q_units = a.heads * a.maps;
+    const uint32_t ring = smem_u32(pd_sm) + (uint32_t)(warp * L::kWarp);
+    // where this lane's rows of the matrix loads lie in a stage: keys row lane & 15, piece lane >> 4; values (transposed) row (lane & 7) + 8 (lane >> 4), piece
+    // (lane >> 3) & 1; two pieces per 16 columns, swizzled by the row
+    uint32_t k_at[4], v_at[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        k_at[i] = ring + (uint32_t)((lane & 15) * 128 + (((2 * i + (lane >> 4)) ^ (lane & 7)) << 4));
+        v_at[i] = ring + (uint32_t)(L::kK + ((lane & 7) + (lane >> 4) * 8) * 128 + (((2 * i + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+    }
+    uint32_t stage = 0, parity = 0;   // of the step that is worked on
     // this thread's two heads (columns of S^T and O^T)
     float sc[2], hb[2];
     const float over_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
     const float* bias[2];
+    float far[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
         const int h = min(g * R + 2 * tig + x, a.heads - 1);
         sc[x] = pa_scale(a, h);
         hb[x] = (a.sigmoid && a.head_bias) ? a.head_bias[h] : 0.f;
         bias[x] = a.dist_bias ? a.dist_bias + (size_t)h * a.dist_n : nullptr;
+        far[x] = a.dist_bias ? bias[x][a.dist_n - 1] : 0.f;
     }
     for (int base = blockIdx.z; base < a.n_tokens; base += 32 * gridDim.z) {
         uint32_t todo = 1u;
@@ -108,59 +139,70 @@ __global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA
             int j0 = first + s0 * kPdStep;
             int page_at = j0 / a.page_rows, off = j0 - page_at * a.page_rows;    // of the step that is fetched next
             int page = s0 < s1 ? plist[page_at] : 0;
-            auto fetch = [&](int s) {   // step s into its stage; keys that the token does not see arrive as zeros (their rows may hold anything)
-                bf* dst = ring + (s - s0) % L::kStages * L::kStep;
-                const size_t row0 = (size_t)page * a.page_rows + off;
-                const int j = first + s * kPdStep;
+            int row = 0;   // pool row of the step whose keys were asked for last
+            auto fetch_k = [&](uint32_t st) {   // the keys of the next step into stage st (rows that the token does not see may hold anything)
+                row = page * a.page_rows + off;
+                if (lane == 0) {
+                    mbar_expect_tx(&k_full[st], L::kK);
 #pragma unroll
-                for (int i = 0; i < kPdStep * (D / 8) / 32; ++i) {
-                    const int at = i * 32 + lane, r = at / (D / 8), c = at % (D / 8) * 8;
-                    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * L::kRS + c);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(K + (row0 + r) * k_row + c), "r"(j + r >= j_lo && j + r <= p ? 16 : 0) : "memory");
+                    for (int c = 0; c < D / 64; ++c) tma_load_2d(pd_sm + warp * L::kWarp + st * L::kStep + c * L::kBox, &map_k, ku * D + c * 64, row, &k_full[st]);
                 }
-                dst += kPdStep * L::kRS;
+                __syncwarp();
+            };
+            auto fetch_v = [&](uint32_t st, int s) {   // and its values; the page of the step after is looked up
+                if (lane == 0) {
+                    mbar_expect_tx(&v_full[st], L::kStep - L::kK);
 #pragma unroll
-                for (int i = 0; i < kPdStep * (VD / 8) / 32; ++i) {
-                    const int at = i * 32 + lane, r = at / (VD / 8), c = at % (VD / 8) * 8;
-                    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * L::kRSV + c);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(V + (row0 + r) * v_row + c), "r"(j + r >= j_lo && j + r <= p ? 16 : 0) : "memory");
+                    for (int c = 0; c < VD / 64; ++c) tma_load_2d(pd_sm + warp * L::kWarp + st * L::kStep + L::kK + c * L::kBox, &map_v, g * VD + c * 64, row, &v_full[st]);
                 }
-                off += kPdStep;   // the page of the step after is looked up now
+                __syncwarp();
+                off += kPdStep;
                 if (off == a.page_rows) { off = 0; ++page_at; if (s + 1 < s1) page = plist[page_at]; }
             };
-            auto close_group = [&]() {
-                __syncwarp();   // the lanes close their group of copies together
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            };
+            {
+                uint32_t st = stage;
 #pragma unroll
-            for (int i = 0; i < L::kStages - 1; ++i) {
-                if (s0 + i < s1) fetch(s0 + i);
-                close_group();
+                for (int i = 0; i < NS; ++i) {
+                    if (s0 + i < s1) { fetch_k(st); fetch_v(st, s0 + i); }
+                    st = st + 1 == NS ? 0 : st + 1;
+                }
             }
             for (int s = s0; s < s1; ++s, j0 += kPdStep) {
                 const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p;
-                if (s + L::kStages - 1 < s1) fetch(s + L::kStages - 1);
-                close_group();
-                asm volatile("cp.async.wait_group %0;" ::"n"(L::kStages - 1) : "memory");
-                __syncwarp();   // step s has landed for every lane
-                const bf* Ks = ring + (s - s0) % L::kStages * L::kStep;
-                const bf* Vs = Ks + kPdStep * L::kRS;
+                const uint32_t at = stage * L::kStep;
                 float bv[4] = {0.f, 0.f, 0.f, 0.f};
-                if (a.dist_bias) {   // requested before the scores are formed
+                if (a.dist_bias) {   // requested before the scores are formed; beyond the table the last number stands for all
+                    if (p - (j0 + kPdStep - 1) >= a.dist_n - 1) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) bv[e] = bias[e & 1][min(max(p - (j0 + gid + (e >> 1) * 8), 0), a.dist_n - 1)];
+                        for (int e = 0; e < 4; ++e) bv[e] = far[e & 1];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) bv[e] = bias[e & 1][min(max(p - (j0 + gid + (e >> 1) * 8), 0), a.dist_n - 1)];
+                    }
                 }
+                mbar_wait_or_leave(&k_full[stage], parity, dead);
                 float st[4] = {0.f, 0.f, 0.f, 0.f}, su[4] = {0.f, 0.f, 0.f, 0.f};   // two chains of products
 #pragma unroll
                 for (int ks = 0; ks < KS; ks += 2) {
                     uint32_t k0[4], k1[4];
-                    pa_ldsm_x4(k0, Ks + (lane & 15) * L::kRS + (lane >> 4) * 8 + ks * 16);
-                    pa_ldsm_x4(k1, Ks + (lane & 15) * L::kRS + (lane >> 4) * 8 + ks * 16 + 16);
+                    pd_ldsm_x4(k0, k_at[ks & 3] + at + (uint32_t)((ks >> 2) * L::kBox));
+                    pd_ldsm_x4(k1, k_at[(ks + 1) & 3] + at + (uint32_t)((ks >> 2) * L::kBox));
                     pa_mma(st, k0, qf[ks]);
                     pa_mma(su, k1, qf[ks + 1]);
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) st[e] = (st[e] + su[e]) * sc[e & 1];
+                __syncwarp();   // every lane has read the keys: their place may be filled again
+                if (s + NS < s1) fetch_k(stage);
+                bool seen[4] = {true, true, true, true};   // key j0 + gid (+ 8), head 2 tig (+ 1)
+                if (!whole) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int j = j0 + gid + (e >> 1) * 8;
+                        seen[e] = j >= j_lo && j <= p;
+                        if (!seen[e]) st[e] = 0.f;   // (of a key that may be anything)
+                    }
+                }
                 if (a.softcap > 0.f) {
                     // cap * tanh(v / cap): the odd series up to x^7 while every |x| is below 0.2 (its next term is below 2^-24 of x there)
                     float x[4], big = 0.f;
@@ -179,10 +221,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA
                 }
                 float pr[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {   // key j0 + gid (+ 8), head 2 tig (+ 1)
-                    const int j = j0 + gid + (e >> 1) * 8;
-                    pr[e] = whole || (j >= j_lo && j <= p) ? st[e] + bv[e] : -INFINITY;
-                }
+                for (int e = 0; e < 4; ++e) pr[e] = seen[e] ? st[e] + bv[e] : -INFINITY;
                 if (a.sigmoid) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) pr[e] = pr[e] == -INFINITY ? 0.f : 1.f / (1.f + expf(-(pr[e] + hb[e & 1])));
@@ -221,19 +260,34 @@ __global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA
                         pr[2 * hf + 1] -= f.y;
                         b[q][hf] = pd_transpose(*reinterpret_cast<const uint32_t*>(&h2));
                     }
+                mbar_wait_or_leave(&v_full[stage], parity, dead);
+                if (!whole) {   // values of keys that the token does not see: 0 * NaN must stay 0
+                    for (int i = lane; i < kPdStep * (VD / 8); i += 32) {
+                        const int r = i / (VD / 8), c = i % (VD / 8);
+                        if (j0 + r < j_lo || j0 + r > p) st_shared_v4(ring + at + (uint32_t)(L::kK + (c / 8) * L::kBox + r * 128 + (c & 7) * 16), 0u, 0u, 0u, 0u);
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                }
 #pragma unroll
                 for (int j = 0; j < MT; j += 4) {   // four tiles of 16 dimensions at a time: consecutive products feed different sums
                     uint32_t af[4][4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) pa_ldsm_x4_trans(af[e], Vs + ((lane & 7) + (lane >> 4) * 8) * L::kRSV + (j + e) * 16 + ((lane >> 3) & 1) * 8);
+                    for (int e = 0; e < 4; ++e) pd_ldsm_x4_trans(af[e], v_at[e] + at + (uint32_t)((j >> 2) * L::kBox));
 #pragma unroll
                     for (int q = 2; q >= 0; --q)
 #pragma unroll
                         for (int e = 0; e < 4; ++e) pa_mma(o[j + e], af[e], b[q]);
                 }
-                __syncwarp();   // the stage may be filled again
+                __syncwarp();   // and the values
+                if (s + NS < s1) fetch_v(stage, s + NS);
+                if (++stage == NS) { stage = 0; parity ^= 1u; }
             }
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            const bool gave_up = *dead != 0;
+            if (gave_up) {   // nothing may land behind this CTA's end, or on the sums
+#pragma unroll
+                for (int i = 0; i < 2 * NS; ++i) { mbar_wait_limited(&k_full[i], 0); mbar_wait_limited(&k_full[i], 1); }
+            }
             __syncthreads();    // the rings' place is taken by the sums
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
@@ -242,7 +296,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA
                 l[x] += __shfl_xor_sync(0xffffffffu, l[x], 16);
                 const int h = 2 * tig + x;
                 if (h < R) {
-                    if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = l[x]; }
+                    if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = gave_up ? __int_as_float(0x7fffffff) : l[x]; }
                     float* dst = om + (size_t)(warp * R + h) * VD + gid;
 #pragma unroll
                     for (int j = 0; j < MT; ++j) {
@@ -300,6 +354,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, 2) paged_decode_kernel(const PA
                     }
                 pa_store<bf>(a, ((size_t)t * q_units + (size_t)qh * a.maps + mp) * VD + i % VD, acc / L);
             }
+            fence_proxy_async_smem();   // TMA writes where the sums lay
             cluster.sync();   // nobody leaves (or starts its next token) while its shared memory is read
         }
         if (!MIXED) break;
@@ -311,6 +366,9 @@ template <int D, int VD, bool MIXED>
 static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s) {
     constexpr int smem = PdRing<D, VD>::kBytes;
     static_assert(kPdWarps * kPdHeads * VD * 4 <= smem, "the warps' sums take the rings' place");
+    CUtensorMap mk, mv;
+    constexpr long long kAnyRow = (1ll << 31) - 1;   // the pool's height is not part of the call: any row that an int can name
+    if (!make_tma_map_2d(&mk, a.k_pool, kAnyRow, a.kv_heads * a.maps * D, kPdStep) || !make_tma_map_2d(&mv, a.v_pool, kAnyRow, a.kv_heads * VD, kPdStep)) return -1;
     static unsigned long long done = 0;
     cudaError_t e = ensure_max_dynamic_smem((const void*)paged_decode_kernel<D, VD, MIXED>, smem, done);
     if (e != cudaSuccess) return (int)e;
@@ -330,7 +388,7 @@ static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, a);
+    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, mk, mv, a);
     if (e != cudaSuccess) return (int)e;
     count_launch();
     return (int)cudaGetLastError();
@@ -345,17 +403,27 @@ static int paged_decode_for(const PA& a, int splits, int rows, cudaStream_t s) {
     return -1;
 }
 
-int paged_decode(const PA& a, int longest_seen, bool mixed, cudaStream_t s) {
+int paged_decode(const PA& a, int longest_seen, int singles, long long room, cudaStream_t s) {
+    const bool mixed = singles > 0;
     if (a.heads / a.kv_heads > kPdHeads || a.page_rows % kPdStep || a.kv_heads * a.maps > 65535) return -1;
     // how many tokens of a mixed batch are single ones is only known on the device: sixteen rows of clusters share them
-    const int rows = mixed ? std::min(a.n_tokens, 16) : a.n_tokens;
+    const int rows = mixed ? std::min(singles, 16) : a.n_tokens;
     if (rows > 65535) return -1;
-    // three CTAs for every two SMs, as long as every warp of a cluster keeps a step of its own (32 sequences of up to 2048 tokens, 16 / 8
-    // heads: 256 / 512 / 1024 CTAs 49 / 51 / 63 us; 8 of up to 1024: 256 / 512 CTAs 14.5 / 20.6 us)
+    // as many shares as the two CTAs per SM that fit hold at once, as long as every warp of a cluster keeps a step of its own (16 / 8 heads x 128, us at 1 / 2 / 4 / 8
+    // shares: 32 sequences of up to 2048 tokens 42.5 / 44.5 / 52.7 / 78.0, 16 such 35.0 / 24.4 / 28.2 / 40.9, 12 of up to 1500 27.4 / 17.1 / 20.4 / 25.4, 8 of up to 2048
+    // 34.4 / 20.0 / 14.3 / 19.8, 4 such 34.3 / 19.8 / 13.5 / 10.8)
     const long long pairs = (long long)rows * a.kv_heads * a.maps;
-    const int most = mixed ? 4 : kPdMaxCluster;
     int splits = 1;
-    while (splits < most && (mixed || 2 * pairs * splits < 3ll * sm_count()) && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+    if (mixed) {
+        // on what the portions' CTAs leave free (`room` CTAs) if eight single tokens can sit there beside each other, else behind them (us at 2 / 4 / 8 shares: 8 single tokens and a portion of 512 behind
+        // 4000 57.2 / 77.7 / 83.0, 4 and 64 36.8 / 31.7 / 40.9, 12 and three of 512, which fill the GPU, 123 / 119 / 133)
+        const long long likely = (long long)std::min(singles, 8) * a.kv_heads * a.maps;
+        if (room < likely) room = 4 * likely;
+        splits = 2;
+        while (splits < (likely <= 8 ? kPdMaxCluster : 4) && likely * splits * 2 <= room) splits *= 2;
+        while (splits > 1 && longest_seen > 0 && splits / 2 * kPdWarps * kPdStep >= longest_seen) splits /= 2;
+    } else
+        while (splits < kPdMaxCluster && pairs * splits <= sm_count() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
     return mixed ? paged_decode_for<true>(a, splits, rows, s) : paged_decode_for<false>(a, splits, rows, s);
 }
 
