@@ -226,3 +226,52 @@ def test_head_temperatures_and_an_unknown_longest_entry(S, G, longest):
         want = reference(q[b] * o["temp"][None, :, None, None], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
         assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 3e-5, b
         at += new[b]
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("H,G,M,d,dv", [(4, 2, 1, 128, 128), (6, 2, 1, 64, 64), (4, 2, 2, 128, 256)])
+@pytest.mark.parametrize("before,new", [([760], [9]), ([1290], [70]), ([2110], [33]), ([2100, 0, 700, 5], [20, 40, 3, 1])])
+def test_key_tiles_of_a_portion_are_shared_by_a_cluster(S, form, H, G, M, d, dv, before, new):
+    """few rows behind long contexts: two, four and eight CTAs share the key tiles of a tile of rows; entries with fewer key tiles than CTAs, and a single token, beside them.
+    fp32 outputs: the bound of test_prompt_weights_are_the_sum_of_two_bfloat16, whose chain of additions is longer"""
+    if M > 1 and FORMS[form].get("sigmoid"):
+        pytest.skip("sigmoid weights have one map")
+    if d == 64 and form == "biased" and before == [760]:
+        pytest.skip("up to 1200 keys these go to the mma.sync tiles, whose weights are rounded to bfloat16")
+    g = torch.Generator().manual_seed(H * d + len(before))
+    o = options(form, H, d, g)
+    if o.get("chunk"):
+        o["chunk"] = 1500
+    if o.get("window"):
+        o["window"] = 1100
+    PR = 64
+    k, v, kp, vp, table = sequences(g, [a + b for a, b in zip(before, new)], G, M, d, dv, PR)
+    q = [torch.randn(n, H, M, d, generator=g).bfloat16().double() for n in new]
+    slot = [b for b in range(len(new)) for _ in range(new[b])]
+    pos = [before[b] + i for b in range(len(new)) for i in range(new[b])]
+    got = run(S, torch.cat(q).bfloat16().cuda(), kp, vp, table, PR, slot, pos, o, max(new))
+    at = 0
+    for b in range(len(new)):
+        want = reference(q[b], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
+        assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 3e-5, b
+        at += new[b]
+
+
+@pytest.mark.parametrize("form", ["plain", "capped", "biased"])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("before", [[0, 130, 700, 40], [2100, 130, 700, 40]])
+def test_more_tiles_than_the_gpu_holds_at_once(S, form, d, before):
+    """several entries whose tiles come in more than one round: short contexts on two CTAs per SM, long ones sorted by what they see. The bound is that of portions beside single tokens"""
+    g = torch.Generator().manual_seed(d + before[0])
+    H, new, PR = 20, [130, 640, 500, 1], 64
+    o = options(form, H, d, g)
+    k, v, kp, vp, table = sequences(g, [a + b for a, b in zip(before, new)], H, 1, d, d, PR)
+    q = [torch.randn(n, H, 1, d, generator=g).bfloat16().double() for n in new]
+    slot = [b for b in range(4) for _ in range(new[b])]
+    pos = [before[b] + i for b in range(4) for i in range(new[b])]
+    got = run(S, torch.cat(q).bfloat16().cuda(), kp, vp, table, PR, slot, pos, o, max(new), f32=False)
+    at = 0
+    for b in range(4):
+        want = reference(q[b], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
+        assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 5e-3, b
+        at += new[b]
