@@ -55,3 +55,9 @@ def test_groups(S, counts, M, N, K, epi, f32, gather, scaled):
             assert float((y[at:at + n].double() - z).norm() / z.norm()) < (2e-5 if f32 else 4e-3), (e, n)
         at += n
     assert bool((y[R:] == 7.0).all())
+
+
+@pytest.mark.parametrize("N,epi", [(5760, "none"), (2880, "glu"), (7680, "none"), (3840, "glu")])
+def test_blocks_of_rows_by_the_number_of_feature_tiles(S, N, epi):
+    """270 and 360 feature tiles over all groups: blocks of up to 192 rows, and three CTAs per SM; groups that end at, before and behind such a block. The bounds of test_groups"""
+    test_groups(S, [0, 191, 193, 16, 177, 400], 400, N, 136, epi, epi == "none", True, False)
