@@ -1,19 +1,21 @@
 // bfloat16 prompt portions of b200_latent_attention_ex on tcgen05 / TMEM: 128 (token, head) rows per tile, cached rows 64 at a time, 256 output
 // columns per CTA (two CTAs form the 512 columns of a row, each with scores of its own: a whole row of sums would fill TMEM alone).
 //
-// What bounds it: per 128 x 64 scores over rows of 576 the tensor pipe needs about 2000 clocks (nine chunks of 64 dimensions, then the weighted
-// sum over 256 columns), four times the softmax; so the next tile's scores run under the softmax of this one, and enough of the cached
+// What bounds it: per 128 x 64 scores over rows of 576 the tensor pipe needs 2500 clocks (nine chunks of 64 dimensions, 1470, then the weighted
+// sum over 256 columns, 1030), three times the softmax; so the next tile's scores run under the softmax of this one, and enough of the cached
 // rows has to be on its way. Shared memory is what limits that: the query rows alone are 144 KB. Four of their chunks lie in TMEM as
-// first operands instead, beside the sums (256 columns) and two score buffers, which leaves room for 128 KB of cached rows:
-//   chunks of 64 dimensions that this CTA only scores with:  a ring of eight, given back after their product
+// first operands instead, beside the sums (256 columns) and two score buffers, which leaves room for 144 KB of cached rows:
+//   chunks of 64 dimensions that this CTA only scores with:  all of a row's at once (rows of 640: half of them), a ring of two such groups, given back after their products
 //   the four chunks whose columns it also sums:              two groups, given back after the weighted sum; they are the operand of both products
 //   warp 0      TMA: chunks of 64 rows x 64 dimensions out of their page
-//   warp 1      tcgen05.mma, scores of tile j + 1 ahead of the weighted sum of tile j
+//   warp 1      tcgen05.mma: scores of a tile as soon as its rows are there and their buffer is free
 //   warps 2-5   the query rows (rounded to bfloat16, as in the mma.sync kernel), then the softmax, a thread per row, as in paged_attention_tc.cu
+//   warp 6      tcgen05.mma: the weighted sums. (One warp for both, and a barrier per chunk, spent 3550 clocks a tile on waits, products and commits; now 2970)
 // The weights go back over their scores as the sum of two bfloat16; the sums are rescaled only when a row's maximum has grown by more than 2^8. A window of
 // packed tokens that holds several sequences is walked tile by tile (latent_tc_parts CTAs share it).
-// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, this 179 us (160 with
-// weights rounded to bfloat16 alone, and 183 then with the query rows loaded a chunk at a time and the results stored from registers). A tile per CTA takes half of that: what is left is mostly the query's way in.
+// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, one warp for all products 171, this 157; 592 tokens behind 1024 62 / 57, 400 and 319
+// behind 900 with 3 single ones 73 / 67. A CTA's fixed part (its query rows 18000 clocks, results 5000) is as much as seven of its key tiles.
+// Tried and taken back: the query's rows read one after the other, 16 bytes per thread (26000 clocks: three times the address and place arithmetic, on one warp per scheduler).
 #include <cuda_bf16.h>
 
 #include "b200_serve.h"
@@ -24,13 +26,15 @@
 
 namespace b200 {
 
-constexpr int kLtRows = 128, kLtKeys = 64, kLtThreads = 192, kLtChunk = kLtKeys * 128, kLtQChunk = kLtRows * 128, kLtRing = 8, kLtV = 4;
+constexpr int kLtRows = 128, kLtKeys = 64, kLtThreads = 224, kLtChunk = kLtKeys * 128, kLtQChunk = kLtRows * 128, kLtV = 4;
 
 template <int NCH>   // chunks of a cached row
 struct LtSmem {
     static constexpr int kScoreOnly = NCH - kLtV, kInTmem = NCH >= 8 ? 4 : 0;   // chunks without sums; of these, how many of the query's lie in TMEM
-    static constexpr int kOffRing = (NCH - kInTmem) * kLtQChunk, kOffV = kOffRing + kLtRing * kLtChunk, kOffBar = kOffV + 2 * kLtV * kLtChunk;
-    static constexpr int kBars = 2 * kLtRing + 10, kOffSlot = kOffBar + kBars * 8, kTotal = kOffSlot + (kLtRows + 2 + 16) * 4 + 1024;
+    // what is only scored with comes kGroup chunks at a time, through a ring of kRing such groups
+    static constexpr int kGroup = kScoreOnly == 6 ? 3 : kScoreOnly > 1 ? kScoreOnly : 1, kGroups = kScoreOnly / kGroup, kRing = kScoreOnly > 1 ? 2 : 4;
+    static constexpr int kOffRing = (NCH - kInTmem) * kLtQChunk, kOffV = kOffRing + kRing * kGroup * kLtChunk, kOffBar = kOffV + 2 * kLtV * kLtChunk;
+    static constexpr int kBars = 2 * kRing + 8, kOffSlot = kOffBar + kBars * 8, kTotal = kOffSlot + (kLtRows + 2 + 16) * 4 + 1024;
     static_assert(kTotal <= 227 * 1024, "one CTA per SM");
 };
 
@@ -47,7 +51,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     extern __shared__ __align__(1024) unsigned char lt_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(lt_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
-    uint64_t *r_full = bars, *r_empty = bars + kLtRing, *v_full = bars + 2 * kLtRing, *v_empty = v_full + 2, *s_full = v_full + 4, *p_full = v_full + 6, *o_done = v_full + 8;
+    constexpr int RING = L::kRing, GC = L::kGroup, GN = L::kGroups;
+    uint64_t *r_full = bars, *r_empty = bars + RING, *v_full = bars + 2 * RING, *s_full = v_full + 2, *p_full = v_full + 4, *o_done = v_full + 6;
     int* slots = reinterpret_cast<int*>(smem + L::kOffSlot);
     uint32_t* masks = reinterpret_cast<uint32_t*>(slots + kLtRows + 2);
     uint32_t* tmem_slot = masks + 8;
@@ -75,9 +80,9 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     if (n_tiles <= part) return;   // nothing here for this CTA (no barrier, no TMEM yet)
     if (warp == 1) tmem_alloc(tmem_slot, 512);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kLtRing; ++i) { mbar_init(&r_full[i], 1); mbar_init(&r_empty[i], 1); }
+        for (int i = 0; i < RING; ++i) { mbar_init(&r_full[i], 1); mbar_init(&r_empty[i], 1); }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+            mbar_init(&v_full[s], 1);
             mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 4);
             mbar_init(&o_done[s], 1);
         }
@@ -109,45 +114,43 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
         const int key0 = (a.window > 0 ? max(0, pA - a.window + 1) : 0) & ~(kLtKeys - 1), n_kt = (pZ - key0) / kLtKeys + 1;
         const int* plist = a.pages + (size_t)slots[first] * a.max_pages;
 
-        if (warp >= 2) {   // ---- query rows: chunks [QT, NCH) to shared memory, chunks [0, QT) to TMEM
-            const int tid = threadIdx.x - 64, by_h = (65536 + H - 1) / H;
+        if (warp >= 2 && warp < 6) {   // ---- query rows: chunks [QT, NCH) to shared memory, chunks [0, QT) to TMEM
+            const int tid = threadIdx.x - 64;
             const uint32_t flip = a.scale < 0.f ? 0x80008000u : 0u;   // the softmax works with |scale|
             auto pack8 = [&](const float4& x, const float4& y, uint32_t (&o)[4]) {
                 const __nv_bfloat162 b0 = __floats2bfloat162_rn(x.x, x.y), b1 = __floats2bfloat162_rn(x.z, x.w), b2 = __floats2bfloat162_rn(y.x, y.y), b3 = __floats2bfloat162_rn(y.z, y.w);
                 o[0] = *reinterpret_cast<const uint32_t*>(&b0) ^ flip; o[1] = *reinterpret_cast<const uint32_t*>(&b1) ^ flip;
                 o[2] = *reinterpret_cast<const uint32_t*>(&b2) ^ flip; o[3] = *reinterpret_cast<const uint32_t*>(&b3) ^ flip;
             };
-            // chunk by chunk through shared memory, the next chunk's loads under way; the first QT chunks go on to TMEM from there
+            // Chunk by chunk through shared memory, the next two chunks' loads under way; the first QT chunks go on to TMEM from there. One warp per scheduler does this, so
+            // instructions count: the tile's rows lie side by side in memory and a thread's are 16 apart, so addresses and predicates are formed once.
             const int c = tid % 8, rb = tid / 8, quarter = warp & 3, mr = quarter * 32 + lane;
-            float4 x[8], y[8];
-            auto load = [&](int o) {
-                const float* src = a.qa + chunk_of(o) * 64 + c * 8;
+            const float* mine = a.qa + ((size_t)tA * H + rb) * a.rank + c * 8;
+            const size_t step = (size_t)16 * a.rank;
+            const uint32_t at0 = (uint32_t)(rb * 128 + ((c ^ (rb & 7)) << 4));
+            uint32_t have = 0u;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = rb + i * 16, tl = (r * by_h) >> 16, h = r - tl * H;
-                    x[i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (tl < count) {
-                        const float4* p = reinterpret_cast<const float4*>(src + ((size_t)(tA + tl) * H + h) * a.rank);
-                        x[i] = p[0];
-                        y[i] = p[1];
+            for (int i = 0; i < 8; ++i) have |= rb + i * 16 < count * H ? 1u << i : 0u;
+            struct Piece { float4 x[8], y[8]; };
+            auto load = [&](int o, Piece& q) {   // (rows that the tile does not have keep their zeros)
+                const float* src = mine + chunk_of(o) * 64;
+#pragma unroll
+                for (int i = 0; i < 8; ++i, src += step)
+                    if (have >> i & 1u) {
+                        q.x[i] = reinterpret_cast<const float4*>(src)[0];
+                        q.y[i] = reinterpret_cast<const float4*>(src)[1];
                     }
-                }
             };
-            load(0);
-#pragma unroll 1
-            for (int o = 0; o < NCH; ++o) {
+            auto place = [&](int o, Piece& q) {
                 uint32_t v[8][4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) pack8(x[i], y[i], v[i]);
-                if (o + 1 < NCH) load(o + 1);
+                for (int i = 0; i < 8; ++i) pack8(q.x[i], q.y[i], v[i]);
+                if (o + 2 < NCH) load(o + 2, q);
                 const uint32_t base = smem_u32(smem + (o < QT ? o : o - QT) * kLtQChunk);
                 __syncwarp();   // lanes without a row skipped its loads; the barriers and tensor memory stores are warp-wide
                 if (QT > 0 && o == QT) asm volatile("bar.sync 2, 128;" ::: "memory");   // those chunks have gone to TMEM
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = rb + i * 16;
-                    st_shared_v4(base + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)), v[i][0], v[i][1], v[i][2], v[i][3]);
-                }
+                for (int i = 0; i < 8; ++i) st_shared_v4(base + at0 + (uint32_t)(i * 2048), v[i][0], v[i][1], v[i][2], v[i][3]);
                 if (o < QT) {
                     asm volatile("bar.sync 2, 128;" ::: "memory");
                     uint32_t t[32];
@@ -158,12 +161,22 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
                     __syncwarp();
                     tmem_st_32x32(q_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(o * 32), t);
                 }
+            };
+            Piece q0, q1;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q0.x[i] = q0.y[i] = q1.x[i] = q1.y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            load(0, q0);
+            load(1, q1);
+#pragma unroll 1
+            for (int o = 0; o < NCH; o += 2) {
+                place(o, q0);
+                if (o + 1 < NCH) place(o + 1, q1);
             }
             tmem_wait_st();
             fence_proxy_async_smem();
             tc_fence_before();
         }
-        if (warp >= 1) asm volatile("bar.sync 1, 160;" ::: "memory");
+        if (warp >= 1 && warp < 6) asm volatile("bar.sync 1, 160;" ::: "memory");
         tc_fence_after();
 
         if (warp == 0) {
@@ -175,16 +188,17 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
             for (int j = 0; j < n_kt; ++j, row = next) {
                 const int it = it0 + j, s = it & 1;
                 next = row_of(j + 1);
-                for (int o = 0; o < NS; ++o) {
-                    const int q = it * NS + o, i = q % kLtRing;
-                    mbar_wait_or_leave(&r_empty[i], ((uint32_t)(q / kLtRing) & 1u) ^ 1u, dead);
+                for (int gi = 0; gi < GN; ++gi) {
+                    const int q = it * GN + gi, i = q % RING;
+                    mbar_wait_or_leave(&r_empty[i], ((uint32_t)(q / RING) & 1u) ^ 1u, dead);
                     if (lane == 0) {
-                        mbar_expect_tx(&r_full[i], kLtChunk);
-                        tma_load_2d(smem + L::kOffRing + i * kLtChunk, &map, chunk_of(o) * 64, row, &r_full[i]);
+                        mbar_expect_tx(&r_full[i], GC * kLtChunk);
+#pragma unroll
+                        for (int o = 0; o < GC; ++o) tma_load_2d(smem + L::kOffRing + (i * GC + o) * kLtChunk, &map, chunk_of(gi * GC + o) * 64, row, &r_full[i]);
                     }
                     __syncwarp();
                 }
-                mbar_wait_or_leave(&v_empty[s], ((uint32_t)(it >> 1) & 1u) ^ 1u, dead);
+                mbar_wait_or_leave(&o_done[s], ((uint32_t)(it >> 1) & 1u) ^ 1u, dead);   // (the weighted sum is what last reads them)
                 if (lane == 0) {
                     mbar_expect_tx(&v_full[s], kLtV * kLtChunk);
 #pragma unroll
@@ -193,32 +207,36 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
                 __syncwarp();
             }
         } else if (warp == 1) {
-            constexpr uint32_t kBf16 = (1u << 7) | (1u << 10);
-            constexpr uint32_t idesc_s = make_idesc_f16(kLtRows, kLtKeys) | kBf16, idesc_o = make_idesc_f16(kLtRows, 256) | kBf16 | (1u << 16);
+            // scores of tile i as soon as its rows are there and the weights that lay in their place have been used
+            constexpr uint32_t idesc_s = make_idesc_f16(kLtRows, kLtKeys) | (1u << 7) | (1u << 10);
             const uint64_t q_desc = make_kmajor_sw128_desc(smem_u32(smem)), r_desc = make_kmajor_sw128_desc(smem_u32(smem + L::kOffRing));
-            const uint64_t vk_desc = make_kmajor_sw128_desc(smem_u32(smem + L::kOffV)), vm_desc = make_mnmajor_sw128_desc(smem_u32(smem + L::kOffV), kLtChunk, 1024u);
-            const int n = __shfl_sync(0xffffffffu, n_kt, 0);
-            int it = __shfl_sync(0xffffffffu, it0, 0);
+            const uint64_t vk_desc = make_kmajor_sw128_desc(smem_u32(smem + L::kOffV));
+            const int n = __shfl_sync(0xffffffffu, n_kt, 0), c0 = __shfl_sync(0xffffffffu, it0, 0);
             const bool leader = elect_one();
-            auto issue_s = [&](int i) {
-                const uint32_t s = (uint32_t)i & 1u, d = s_tmem + s * kLtKeys;
+            for (int i = c0; i < c0 + n; ++i) {
+                const uint32_t s = (uint32_t)i & 1u, d = s_tmem + s * kLtKeys, ph = (uint32_t)(i >> 1) & 1u;
+                mbar_wait_or_leave(&o_done[s], ph ^ 1u, dead);
 #pragma unroll
-                for (int o = 0; o < NS; ++o) {
-                    const uint32_t q = (uint32_t)(i * NS + o), x = q % kLtRing;
-                    mbar_wait_or_leave(&r_full[x], (q / kLtRing) & 1u, dead);
+                for (int gi = 0; gi < GN; ++gi) {
+                    const uint32_t q = (uint32_t)(i * GN + gi), x = q % RING;
+                    mbar_wait_or_leave(&r_full[x], (q / RING) & 1u, dead);
                     tc_fence_after();
                     if (leader) {
-                        const uint64_t kd = r_desc + (uint64_t)(x * (kLtChunk >> 4));
+                        const uint64_t kd = r_desc + (uint64_t)(x * (GC * kLtChunk >> 4));
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            if (o < QT) umma_f16_ts(d, q_tmem + (uint32_t)(o * 32 + k * 8), kd + (uint64_t)(2 * k), idesc_s, o > 0 || k > 0 ? 1u : 0u);
-                            else umma_f16(d, q_desc + (uint64_t)((o - QT) * (kLtQChunk >> 4) + 2 * k), kd + (uint64_t)(2 * k), idesc_s, o > 0 || k > 0 ? 1u : 0u);
+                        for (int oo = 0; oo < GC; ++oo) {
+                            const int o = gi * GC + oo;
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                if (o < QT) umma_f16_ts(d, q_tmem + (uint32_t)(o * 32 + k * 8), kd + (uint64_t)(oo * (kLtChunk >> 4) + 2 * k), idesc_s, o > 0 || k > 0 ? 1u : 0u);
+                                else umma_f16(d, q_desc + (uint64_t)((o - QT) * (kLtQChunk >> 4) + 2 * k), kd + (uint64_t)(oo * (kLtChunk >> 4) + 2 * k), idesc_s, o > 0 || k > 0 ? 1u : 0u);
+                            }
                         }
                         umma_commit(&r_empty[x]);
                     }
                     __syncwarp();
                 }
-                mbar_wait_or_leave(&v_full[s], (uint32_t)(i >> 1) & 1u, dead);
+                mbar_wait_or_leave(&v_full[s], ph, dead);
                 tc_fence_after();
                 if (leader) {
                     const uint64_t kd = vk_desc + (uint64_t)(s * (kLtV * kLtChunk >> 4));
@@ -230,19 +248,21 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
                     umma_commit(&s_full[s]);
                 }
                 __syncwarp();
-            };
-            issue_s(it);
-            for (int j = 0; j < n; ++j, ++it) {
-                if (j + 1 < n) issue_s(it + 1);
-                const uint32_t s = (uint32_t)it & 1u;
-                mbar_wait_or_leave(&p_full[s], (uint32_t)(it >> 1) & 1u, dead);
+            }
+        } else if (warp == 6) {
+            constexpr uint32_t idesc_o = make_idesc_f16(kLtRows, 256) | (1u << 7) | (1u << 10) | (1u << 16);
+            const uint64_t vm_desc = make_mnmajor_sw128_desc(smem_u32(smem + L::kOffV), kLtChunk, 1024u);
+            const int n = __shfl_sync(0xffffffffu, n_kt, 0), c0 = __shfl_sync(0xffffffffu, it0, 0);
+            const bool leader = elect_one();
+            for (int j = 0; j < n; ++j) {
+                const uint32_t s = (uint32_t)(c0 + j) & 1u;
+                mbar_wait_or_leave(&p_full[s], (uint32_t)((c0 + j) >> 1) & 1u, dead);
                 tc_fence_after();
                 if (leader) {
                     const uint64_t vd = vm_desc + (uint64_t)(s * (kLtV * kLtChunk >> 4));
 #pragma unroll
                     for (int ks = 0; ks < 2 * kLtKeys / kUmmaK; ++ks)   // hi, then lo
                         umma_f16_ts(o_tmem, s_tmem + s * kLtKeys + (uint32_t)(ks * 8), vd + (uint64_t)((ks & 3) * (2048 >> 4)), idesc_o, j > 0 || ks > 0 ? 1u : 0u);
-                    umma_commit(&v_empty[s]);
                     umma_commit(&o_done[s]);
                 }
                 __syncwarp();
