@@ -123,9 +123,11 @@ class Engine:
         if not self.h:
             raise RuntimeError("[b200][ERROR] engine_create: " + self.lib.b200_engine_last_error().decode())
         self._cb = None
+        self._logits = None   # (address, tensor over it)
 
     def close(self):
         if self.h:
+            self._logits = None
             self.lib.b200_engine_destroy(self.h)
             self.h = None
 
@@ -319,8 +321,11 @@ class Engine:
 
     def logits(self):
         import torch
-        td = torch.float16 if self.dtype == capi.F16 else torch.float32
-        return self._view(self.lib.b200_engine_logits(self.h), (self.batch, self.cfg.vocab_size), td)
+        # the engine's own buffer: the tensor over it is made once (56 us, in which the GPU waits for the next step), each call returns an alias
+        at = self.lib.b200_engine_logits(self.h)
+        if self._logits is None or self._logits[0] != at:
+            self._logits = (at, self._view(at, (self.batch, self.cfg.vocab_size), torch.float16 if self.dtype == capi.F16 else torch.float32))
+        return self._logits[1].view(self.batch, self.cfg.vocab_size)
 
     def hidden(self):
         import torch

@@ -2,6 +2,7 @@
 cache, continuous-batching scheduler) and the kernels it brings. Tests and the bench call the library through this
 module; the product path is the C ABI itself and ``bin/b200_serve``."""
 import ctypes as C
+import itertools
 
 import numpy as np
 
@@ -289,11 +290,11 @@ class Model:
         """entries: list of (slot, tokens, want). Returns logits [sum want, vocab] (and greedy ids when ids=True)."""
         slots, _s = _ints([e[0] for e in entries])
         counts, _c = _ints([len(e[1]) for e in entries])
-        toks, _t = _ints([t for e in entries for t in e[1]] or [0])
+        toks, _t = _ints(np.fromiter(itertools.chain.from_iterable(e[1] for e in entries), np.int32, int(counts.sum())) if counts.sum() else [0])
         nw, _nw = _ints([len(e[2]) for e in entries])
         want, _w = _ints([w for e in entries for w in e[2]] or [0])
         total = int(nw.sum())
-        out = np.zeros((max(total, 1), self.vocab), np.float32)
+        out = (np.empty if logits and total else np.zeros)((max(total, 1), self.vocab), np.float32)   # (rows that were asked for are all written)
         picks = np.zeros(max(total, 1), np.int32)
         rc = lib().b200_model_step(self._h, len(entries), _s, _c, _t, _nw, _w,
                                    out.ctypes.data_as(_vp) if logits else None, picks.ctypes.data_as(_vp) if ids else None)
