@@ -7,15 +7,15 @@
 // first operands instead, beside the sums (256 columns) and two score buffers, which leaves room for 144 KB of cached rows:
 //   chunks of 64 dimensions that this CTA only scores with:  all of a row's at once (rows of 640: half of them), a ring of two such groups, given back after their products
 //   the four chunks whose columns it also sums:              two groups, given back after the weighted sum; they are the operand of both products
-//   warp 0      TMA: chunks of 64 rows x 64 dimensions out of their page
+//   warp 0      TMA: the query's chunks in fp32, through the places of the cached rows; then chunks of 64 rows x 64 dimensions out of their page
 //   warp 1      tcgen05.mma: scores of a tile as soon as its rows are there and their buffer is free
 //   warps 2-5   the query rows (rounded to bfloat16, as in the mma.sync kernel), then the softmax, a thread per row, as in paged_attention_tc.cu
 //   warp 6      tcgen05.mma: the weighted sums. (One warp for both, and a barrier per chunk, spent 3550 clocks a tile on waits, products and commits; now 2970)
 // The weights go back over their scores as the sum of two bfloat16; the sums are rescaled only when a row's maximum has grown by more than 2^8. A window of
 // packed tokens that holds several sequences is walked tile by tile (latent_tc_parts CTAs share it).
-// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, one warp for all products 171, this 157; 592 tokens behind 1024 62 / 57, 400 and 319
-// behind 900 with 3 single ones 73 / 67. A CTA's fixed part (its query rows 18000 clocks, results 5000) is as much as seven of its key tiles.
-// Tried and taken back: the query's rows read one after the other, 16 bytes per thread (26000 clocks: three times the address and place arithmetic, on one warp per scheduler).
+// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, one warp for all products 171, a second one 157, the
+// query by TMA too 144; 592 tokens behind 1024 62 / 57 / 53, 400 and 319 behind 900 with 3 single ones 73 / 67 / 65. A CTA's fixed part (its query rows, results 5000 clocks) is as much as five of its key tiles.
+// Tried and taken back: the query's rows read by the four warps one row after the other, 16 bytes per thread (26000 clocks: three times the address and place arithmetic, on one warp per scheduler).
 #include <cuda_bf16.h>
 
 #include "b200_serve.h"
@@ -34,7 +34,9 @@ struct LtSmem {
     // what is only scored with comes kGroup chunks at a time, through a ring of kRing such groups
     static constexpr int kGroup = kScoreOnly == 6 ? 3 : kScoreOnly > 1 ? kScoreOnly : 1, kGroups = kScoreOnly / kGroup, kRing = kScoreOnly > 1 ? 2 : 4;
     static constexpr int kOffRing = (NCH - kInTmem) * kLtQChunk, kOffV = kOffRing + kRing * kGroup * kLtChunk, kOffBar = kOffV + 2 * kLtV * kLtChunk;
-    static constexpr int kBars = 2 * kRing + 8, kOffSlot = kOffBar + kBars * 8, kTotal = kOffSlot + (kLtRows + 2 + 16) * 4 + 1024;
+    // the query's chunks come in fp32 through the cached rows' places, kSlots at a time
+    static constexpr int kSlot = 2 * kLtQChunk, kSlots = (kOffBar - kOffRing) / kSlot;
+    static constexpr int kBars = 2 * kRing + 8 + 2 * kSlots, kOffSlot = kOffBar + kBars * 8, kTotal = kOffSlot + (kLtRows + 2 + 16) * 4 + 1024;
     static_assert(kTotal <= 227 * 1024, "one CTA per SM");
 };
 
@@ -45,14 +47,14 @@ struct LtArgs {
 };
 
 template <int NCH>
-__global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const LtArgs a) {
+__global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map_q, const LtArgs a) {
     using L = LtSmem<NCH>;
     constexpr int NS = L::kScoreOnly, QT = L::kInTmem;
     extern __shared__ __align__(1024) unsigned char lt_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(lt_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
     constexpr int RING = L::kRing, GC = L::kGroup, GN = L::kGroups;
-    uint64_t *r_full = bars, *r_empty = bars + RING, *v_full = bars + 2 * RING, *s_full = v_full + 2, *p_full = v_full + 4, *o_done = v_full + 6;
+    uint64_t *r_full = bars, *r_empty = bars + RING, *v_full = bars + 2 * RING, *s_full = v_full + 2, *p_full = v_full + 4, *o_done = v_full + 6, *q_full = v_full + 8, *q_empty = q_full + L::kSlots;
     int* slots = reinterpret_cast<int*>(smem + L::kOffSlot);
     uint32_t* masks = reinterpret_cast<uint32_t*>(slots + kLtRows + 2);
     uint32_t* tmem_slot = masks + 8;
@@ -86,15 +88,17 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
             mbar_init(&s_full[s], 1); mbar_init(&p_full[s], 4);
             mbar_init(&o_done[s], 1);
         }
+        for (int i = 0; i < L::kSlots; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 4); }
         mbar_fence_init();
         tma_prefetch_desc(&map);
+        tma_prefetch_desc(&map_q);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0), o_tmem = tmem, s_tmem = tmem + 256, q_tmem = tmem + 256 + 2 * kLtKeys;
 
-    int it0 = 0, ordinal = 0;
+    int it0 = 0, q0 = 0, ordinal = 0;   // key tiles, query chunks, tiles of the window so far
     for (int first = 0; first < rows;) {
         int w = first >> 5;
         uint32_t left = w < 4 ? masks[w] & (0xffffffffu << (first & 31)) : 0u;
@@ -114,68 +118,70 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
         const int key0 = (a.window > 0 ? max(0, pA - a.window + 1) : 0) & ~(kLtKeys - 1), n_kt = (pZ - key0) / kLtKeys + 1;
         const int* plist = a.pages + (size_t)slots[first] * a.max_pages;
 
-        if (warp >= 2 && warp < 6) {   // ---- query rows: chunks [QT, NCH) to shared memory, chunks [0, QT) to TMEM
-            const int tid = threadIdx.x - 64;
+        // ---- query rows: chunks [QT, NCH) to shared memory, chunks [0, QT) to TMEM, rounded to bfloat16 on the way. TMA brings them in fp32 into the places of the cached rows,
+        // kSlots chunks under way (64 KB of loads per SM, requested by the four warps themselves, came at 16 bytes a clock, 18000 clocks in all)
+        if (warp == 0) {
+            for (int o = 0; o < NCH; ++o) {
+                const int q = q0 + o, i = q % L::kSlots;
+                mbar_wait_or_leave(&q_empty[i], ((uint32_t)(q / L::kSlots) & 1u) ^ 1u, dead);
+                if (lane == 0) {
+                    mbar_expect_tx(&q_full[i], L::kSlot);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) tma_load_2d(smem + L::kOffRing + i * L::kSlot + b * kLtQChunk, &map_q, chunk_of(o) * 128 + b * 64, tA * H, &q_full[i]);   // (in 16-bit columns)
+                }
+                __syncwarp();
+            }
+        } else if (warp >= 2 && warp < 6) {
+            const int tid = threadIdx.x - 64, c = tid % 8, rb = tid / 8, quarter = warp & 3, mr = quarter * 32 + lane;
             const uint32_t flip = a.scale < 0.f ? 0x80008000u : 0u;   // the softmax works with |scale|
-            auto pack8 = [&](const float4& x, const float4& y, uint32_t (&o)[4]) {
-                const __nv_bfloat162 b0 = __floats2bfloat162_rn(x.x, x.y), b1 = __floats2bfloat162_rn(x.z, x.w), b2 = __floats2bfloat162_rn(y.x, y.y), b3 = __floats2bfloat162_rn(y.z, y.w);
-                o[0] = *reinterpret_cast<const uint32_t*>(&b0) ^ flip; o[1] = *reinterpret_cast<const uint32_t*>(&b1) ^ flip;
-                o[2] = *reinterpret_cast<const uint32_t*>(&b2) ^ flip; o[3] = *reinterpret_cast<const uint32_t*>(&b3) ^ flip;
+            auto ld4 = [&](uint32_t at) {
+                float4 v;
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+                return v;
             };
-            // Chunk by chunk through shared memory, the next two chunks' loads under way; the first QT chunks go on to TMEM from there. One warp per scheduler does this, so
-            // instructions count: the tile's rows lie side by side in memory and a thread's are 16 apart, so addresses and predicates are formed once.
-            const int c = tid % 8, rb = tid / 8, quarter = warp & 3, mr = quarter * 32 + lane;
-            const float* mine = a.qa + ((size_t)tA * H + rb) * a.rank + c * 8;
-            const size_t step = (size_t)16 * a.rank;
-            const uint32_t at0 = (uint32_t)(rb * 128 + ((c ^ (rb & 7)) << 4));
-            uint32_t have = 0u;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) have |= rb + i * 16 < count * H ? 1u << i : 0u;
-            struct Piece { float4 x[8], y[8]; };
-            auto load = [&](int o, Piece& q) {   // (rows that the tile does not have keep their zeros)
-                const float* src = mine + chunk_of(o) * 64;
-#pragma unroll
-                for (int i = 0; i < 8; ++i, src += step)
-                    if (have >> i & 1u) {
-                        q.x[i] = reinterpret_cast<const float4*>(src)[0];
-                        q.y[i] = reinterpret_cast<const float4*>(src)[1];
-                    }
+            auto pack4 = [&](const float4& x, uint32_t* o) {
+                const __nv_bfloat162 b0 = __floats2bfloat162_rn(x.x, x.y), b1 = __floats2bfloat162_rn(x.z, x.w);
+                o[0] = *reinterpret_cast<const uint32_t*>(&b0) ^ flip;
+                o[1] = *reinterpret_cast<const uint32_t*>(&b1) ^ flip;
             };
-            auto place = [&](int o, Piece& q) {
-                uint32_t v[8][4];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) pack8(q.x[i], q.y[i], v[i]);
-                if (o + 2 < NCH) load(o + 2, q);
-                const uint32_t base = smem_u32(smem + (o < QT ? o : o - QT) * kLtQChunk);
-                __syncwarp();   // lanes without a row skipped its loads; the barriers and tensor memory stores are warp-wide
-                if (QT > 0 && o == QT) asm volatile("bar.sync 2, 128;" ::: "memory");   // those chunks have gone to TMEM
-#pragma unroll
-                for (int i = 0; i < 8; ++i) st_shared_v4(base + at0 + (uint32_t)(i * 2048), v[i][0], v[i][1], v[i][2], v[i][3]);
-                if (o < QT) {
-                    asm volatile("bar.sync 2, 128;" ::: "memory");
+#pragma unroll 1
+            for (int o = 0; o < NCH; ++o) {
+                const int q = q0 + o, i = q % L::kSlots;
+                const uint32_t src = smem_u32(smem + L::kOffRing + i * L::kSlot);
+                mbar_wait_or_leave(&q_full[i], (uint32_t)(q / L::kSlots) & 1u, dead);
+                if (o < QT) {   // a row per lane
                     uint32_t t[32];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(t[4 * e]), "=r"(t[4 * e + 1]), "=r"(t[4 * e + 2]), "=r"(t[4 * e + 3])
-                                     : "r"(base + (uint32_t)(mr * 128 + ((e ^ (mr & 7)) << 4))) : "memory");
-                    __syncwarp();
+                    for (int e = 0; e < 16; ++e) pack4(ld4(src + (uint32_t)((e >> 3) * kLtQChunk + mr * 128 + (((e & 7) ^ (mr & 7)) << 4))), t + 2 * e);
                     tmem_st_32x32(q_tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(o * 32), t);
-                }
-            };
-            Piece q0, q1;
+                } else {        // columns 8 c .. 8 c + 7 of every 16th row (the halves of the lanes begin with different pieces: no bank conflicts)
+                    const uint32_t dst = smem_u32(smem + (o - QT) * kLtQChunk), from = src + (uint32_t)((c >> 2) * kLtQChunk), swap = c >> 2;
+                    uint32_t v[8][4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) q0.x[i] = q0.y[i] = q1.x[i] = q1.y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            load(0, q0);
-            load(1, q1);
-#pragma unroll 1
-            for (int o = 0; o < NCH; o += 2) {
-                place(o, q0);
-                if (o + 1 < NCH) place(o + 1, q1);
+                    for (int k = 0; k < 8; ++k) {
+                        const int r = rb + k * 16;
+                        const uint32_t piece = (uint32_t)((c & 3) * 2) + swap;
+                        const float4 x = ld4(from + (uint32_t)(r * 128) + ((piece ^ (uint32_t)(r & 7)) << 4)), y = ld4(from + (uint32_t)(r * 128) + ((piece ^ 1u ^ (uint32_t)(r & 7)) << 4));
+                        uint32_t px[2], py[2];
+                        pack4(x, px);
+                        pack4(y, py);
+                        v[k][0] = swap ? py[0] : px[0]; v[k][1] = swap ? py[1] : px[1];
+                        v[k][2] = swap ? px[0] : py[0]; v[k][3] = swap ? px[1] : py[1];
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int r = rb + k * 16;
+                        st_shared_v4(dst + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)), v[k][0], v[k][1], v[k][2], v[k][3]);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&q_empty[i]);
             }
             tmem_wait_st();
             fence_proxy_async_smem();
             tc_fence_before();
         }
+        if (warp == 0 || (warp >= 2 && warp < 6)) asm volatile("bar.sync 3, 160;" ::: "memory");   // the cached rows may come
         if (warp >= 1 && warp < 6) asm volatile("bar.sync 1, 160;" ::: "memory");
         tc_fence_after();
 
@@ -374,6 +380,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
             tc_fence_before();
         }
         it0 += n_kt;
+        q0 += NCH;
         first = end;
         __syncthreads();   // the next tile's query rows and products come after everybody is done with this one's
         tc_fence_after();
@@ -383,9 +390,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
 
 template <int NCH>
 static int launch_lt(const b200_latent_attention_args& a, int halves, cudaStream_t s) {
-    CUtensorMap map;
+    CUtensorMap map, map_q;
     constexpr long long kAnyRow = (1ll << 31) - 1;   // the pool's height is not part of the call: any row that an int can name
-    if (!make_tma_map_2d(&map, a.pool, kAnyRow, a.rank, kLtKeys)) return -1;
+    // (the query's fp32 as pairs of 16-bit columns)
+    if (!make_tma_map_2d(&map, a.pool, kAnyRow, a.rank, kLtKeys) || !make_tma_map_2d(&map_q, a.qa, (long long)a.n_tokens * a.heads, 2 * a.rank, kLtRows)) return -1;
     static unsigned long long done = 0;
     const cudaError_t e = ensure_max_dynamic_smem((const void*)latent_attn_tc_kernel<NCH>, LtSmem<NCH>::kTotal, done);
     if (e != cudaSuccess) return (int)e;
@@ -393,7 +401,7 @@ static int launch_lt(const b200_latent_attention_args& a, int halves, cudaStream
     const long long windows = (a.n_tokens + TQ - 1) / TQ;
     if (windows * parts > 65535) return -1;
     const LtArgs la{a.qa, a.out, a.pages, a.slot, a.pos, a.sink, a.max_pages, a.page_rows, a.n_tokens, a.heads, a.rank, a.window, TQ, parts, a.scale};
-    latent_attn_tc_kernel<NCH><<<dim3((unsigned)halves, (unsigned)(windows * parts)), kLtThreads, LtSmem<NCH>::kTotal, s>>>(map, la);
+    latent_attn_tc_kernel<NCH><<<dim3((unsigned)halves, (unsigned)(windows * parts)), kLtThreads, LtSmem<NCH>::kTotal, s>>>(map, map_q, la);
     return (int)cudaGetLastError();
 }
 
