@@ -368,3 +368,22 @@ def test_glu_with_tanh_gelu_in_the_gemm_epilogue(S, M, N, K, kind):
     assert rel(out2.float(), want) < (2e-2 if kind == "bf16" else 2e-5)
     sync_ok(S.lib().b200_glu_act(gu.data_ptr(), out2.data_ptr(), M, N, S.GG_GLU, code, None))
     assert rel(out2.float(), O.silu(x.double() @ w[:N].double().T) * (x.double() @ w[N:].double().T)) < (2e-2 if kind == "bf16" else 2e-5)
+
+
+@pytest.mark.parametrize("width", [4, 516, 1000, 1024, 1028, 2048])
+@pytest.mark.parametrize("kind", ["f32", "bf16"])
+def test_layernorm_residual_of_many_rows(S, width, kind):
+    """a warp per row: rows that are no multiple of a CTA's, widths that end inside a warp's pass. The bounds of test_layernorm_residual_and_next_norm"""
+    code, g, n = code_of(S, kind), gen(width), 701
+    x, y = torch.randn(n, width, generator=g) * 2 + 3, torch.randn(n, width, generator=g) * 4 - 7
+    w, b, w2, b2 = (torch.randn(width, generator=g) for _ in range(4))
+    xd, out2 = dev(x), torch.empty(n, width, dtype=tdt(S, code), device="cuda")
+    sync_ok(S.lib().b200_layernorm_residual(xd.data_ptr(), dev(y).data_ptr(), n, width, 1e-5, 0.3, dev(w).data_ptr(), dev(b).data_ptr(),
+                                            dev(w2).data_ptr(), dev(b2).data_ptr(), out2.data_ptr(), code, None))
+    want_x = x.double() + 0.3 * O.layer_norm(y.double(), w.double(), b.double(), 1e-5)
+    assert rel(xd, want_x) < 2e-6
+    assert rel(out2.float(), O.layer_norm(want_x, w2.double(), b2.double(), 1e-5)) < (2e-2 if kind == "bf16" else 2e-5)
+    xd2 = dev(x)
+    sync_ok(S.lib().b200_layernorm_residual(xd2.data_ptr(), dev(y).data_ptr(), n, width, 1e-5, 0.3, dev(w).data_ptr(), dev(b).data_ptr(),
+                                            None, None, None, code, None))
+    assert torch.equal(xd2, xd)
