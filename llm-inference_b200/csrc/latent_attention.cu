@@ -28,6 +28,7 @@
 #include "latent_attention.cuh"
 #include "launch_count.h"
 #include "rotary.cuh"
+#include "tc_common.cuh"
 
 namespace b200 {
 namespace cg = cooperative_groups;
@@ -446,37 +447,54 @@ __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* _
 // A cluster of CTAs shares one token's cached rows; a CTA holds up to 16 heads of it, the M rows of one mma tile. What bounds it is
 // the way to the rows (a few MB per launch) and the length of the chain behind them, so the rows are requested before anything else,
 // two half tiles of 32 at once, two CTAs fit an SM, and the shares meet in distributed shared memory (rank order) in the same launch.
+// A half tile comes by TMA, a box per lane of one warp, its place in the pool looked up a step before (by cp.async, twelve copies and their addresses
+// per lane behind that lookup, a step of 32 rows took 2.6 us); pages that are no multiple of a half tile keep cp.async.
 //   scores   warp w: keys [16 (w & 1), +16) x 16 heads over a quarter (w >> 1) of the row; the four partial sums meet in shared memory
 //   softmax  warp w: heads 2w, 2w + 1, a key per lane; the weights leave as bfloat16 (as in the tile kernel)
 //   values   warp w: an eighth of the output columns, the rows read transposed by ldmatrix
 // The sink joins in the merge. Measured, 8 sequences of up to 1024 rows of 576, 16 heads, 512 columns out: the tile kernel with its
-// combine launch 53.3 us, this 16.2 us (clusters of at most 2 / 4 / 8 CTAs: 51 / 31 / 20.5 us).
+// combine launch 53.3 us, by cp.async 16.2, this 14.1 us; 32 sequences of up to 2048 rows 34 / 24, one of 2048 19.1 / 14.7.
 constexpr int kLdMaxCluster = 16;
 
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void* p) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+__device__ __forceinline__ void ldsm_x4_at(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_trans_at(uint32_t (&r)[4], uint32_t a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 
-template <int NT>   // n8 column tiles of the output per warp: out_cols <= 64 * NT
-__global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __restrict__ qa, float* __restrict__ out, const __nv_bfloat16* __restrict__ pool,
+// n8 column tiles of the output per warp: out_cols <= 64 * NT. TMA: a half tile lies in one page, and comes as boxes of 32 rows x 64 columns, swizzled over 128 bytes
+template <int NT, bool TMA>
+__global__ void __launch_bounds__(256, 2) latent_decode_kernel(const __grid_constant__ CUtensorMap map, const float* __restrict__ qa, float* __restrict__ out, const __nv_bfloat16* __restrict__ pool,
                                                                const int* __restrict__ pages, int max_pages, int page_rows, const int* __restrict__ slot,
                                                                const int* __restrict__ pos, const float* __restrict__ sink, float scale, int heads, int rank,
                                                                int window, int out_cols) {
     using bf = __nv_bfloat16;
-    extern __shared__ __align__(16) unsigned char smraw[];
+    extern __shared__ __align__(1024) unsigned char smraw0[];
+    unsigned char* smraw = TMA ? reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw0) + 1023) & ~(uintptr_t)1023) : smraw0;
+    __shared__ uint64_t full[2];
+    __shared__ int dead_s;
+    volatile int* dead = &dead_s;
+    if (TMA && threadIdx.x == 0) {
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        *dead = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&map);
+    }
     pdl_wait();
     pdl_launch_dependents();
     const int rpad = (rank + 15) & ~15, RS = rpad + 8, splits = gridDim.x;
     bf* Ks = reinterpret_cast<bf*>(smraw);                     // [2][32][RS]
-    bf* Qs = Ks + 2 * kHalfKeys * RS;                          // [16][RS]
+    const int boxes = (rank + 63) / 64, stage = boxes * kHalfKeys * 128;   // TMA: bytes of a half tile
+    bf* Qs = TMA ? reinterpret_cast<bf*>(smraw + 2 * stage) : Ks + 2 * kHalfKeys * RS;   // [16][RS]
     float* Ss = reinterpret_cast<float*>(Qs + 16 * RS);        // [4][16][36]: partial scores [head][key]
     bf* Ps = reinterpret_cast<bf*>(Ss + 4 * 16 * 36);          // [16][40]
     float* al_s = reinterpret_cast<float*>(Ps + 16 * 40);      // [16]
     float* ms = al_s + 16;                                     // [16]
     float* ls = ms + 16;                                       // [16]
     float* om = reinterpret_cast<float*>(smraw);               // [16][out_cols]: this CTA's share, once the rows have been used
-    const int t = blockIdx.z, h0 = blockIdx.y * 16, warp = threadIdx.x / 32, lane = threadIdx.x % 32, gid = lane / 4, tig = lane % 4;
+    const int t = blockIdx.z, h0 = blockIdx.y * 16, warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32, gid = lane / 4, tig = lane % 4;
     const int n = min(16, heads - h0), chunks = rpad / 8;
     // the query rows are requested first, ahead of the chain position -> page -> rows; a warp brings two heads
     constexpr int kQv = (32 * kMaxRankPerLane / 4 + 31) / 32;
@@ -516,10 +534,26 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
         __syncwarp();   // the lanes close their group of copies together
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (b0 < b1) load_half(b0);
-    close_group();
-    if (b0 + 1 < b1) load_half(b0 + 1);
-    close_group();
+    auto row_of = [&](int b) { return list[(first + b * kHalfKeys) / page_rows] * page_rows + (first + b * kHalfKeys) % page_rows; };
+    auto fetch = [&](int b, int row) {   // one warp, a box per lane
+        uint64_t* bar = &full[(b - b0) & 1];
+        if (lane == 0) mbar_expect_tx(bar, stage);
+        __syncwarp();
+        if (lane < boxes) tma_load_2d(smraw + ((b - b0) & 1) * stage + lane * (kHalfKeys * 128), &map, lane * 64, row, bar);
+        __syncwarp();
+    };
+    if (TMA) {
+        if (warp == 0) {
+            const int r0 = b0 < b1 ? row_of(b0) : 0, r1 = b0 + 1 < b1 ? row_of(b0 + 1) : 0;
+            if (b0 < b1) fetch(b0, r0);
+            if (b0 + 1 < b1) fetch(b0 + 1, r1);
+        }
+    } else {
+        if (b0 < b1) load_half(b0);
+        close_group();
+        if (b0 + 1 < b1) load_half(b0 + 1);
+        close_group();
+    }
 #pragma unroll
     for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -535,19 +569,42 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
     for (int i = 0; i < NT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
     const int steps = rpad / 16, kq = warp >> 1, ks0 = steps * kq / 4, ks1 = steps * (kq + 1) / 4;
     const int n8 = out_cols / 8, ntw = ((n8 + kTileWarps - 1) / kTileWarps + 1) & ~1, tile0 = warp * ntw;   // pairs of column tiles
+    // where this lane's rows of the matrix loads lie: keys, columns 16 ks .. (row, then which of the two pieces), and values, a pair of column tiles
+    const int k_row = (warp & 1) * 16 + (lane & 15), piece_hi = lane >> 4;
+    auto k_at = [&](int b, int ks) -> uint32_t {
+        if (TMA) return smem_u32(smraw) + (uint32_t)(((b - b0) & 1) * stage + (ks >> 2) * (kHalfKeys * 128) + k_row * 128 + ((((ks & 3) * 2 + piece_hi) ^ (k_row & 7)) << 4));
+        return smem_u32(Ks + (((b - b0) & 1) * kHalfKeys + k_row) * RS + piece_hi * 8 + ks * 16);
+    };
+    auto v_at = [&](int b, int kk, int tile) -> uint32_t {
+        const int r = kk + (lane & 15), piece = tile + piece_hi;
+        if (TMA) return smem_u32(smraw) + (uint32_t)(((b - b0) & 1) * stage + (piece >> 3) * (kHalfKeys * 128) + r * 128 + (((piece & 7) ^ (r & 7)) << 4));
+        return smem_u32(Ks + (((b - b0) & 1) * kHalfKeys + r) * RS + piece * 8);
+    };
+    if (TMA) __syncthreads();   // the barriers, and the query rows
     for (int b = b0; b < b1; ++b) {
-        const bf* Kb = Ks + ((b - b0) & 1) * kHalfKeys * RS;
         const int k0 = first + b * kHalfKeys;
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();   // half b has landed for everybody (and, the first time, the query rows)
+        int next_row = 0;
+        if (TMA) {
+            if (warp == 0 && b + 2 < b1) next_row = row_of(b + 2);   // its place is looked up a step ahead
+            mbar_wait_or_leave(&full[(b - b0) & 1], (uint32_t)((b - b0) >> 1) & 1u, dead);
+            if (k0 < lo || k0 + kHalfKeys - 1 > p) {   // rows that the token does not see may hold anything: 0 * NaN must stay 0
+                for (int kr = warp; kr < kHalfKeys; kr += kTileWarps)
+                    if (k0 + kr < lo || k0 + kr > p)
+                        for (int x = lane; x < boxes * 8; x += 32) *reinterpret_cast<uint4*>(smraw + ((b - b0) & 1) * stage + (x >> 3) * (kHalfKeys * 128) + kr * 128 + (x & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncthreads();
+            }
+        } else {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();   // half b has landed for everybody (and, the first time, the query rows)
+        }
         {
             float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            const bf* ka = Kb + ((warp & 1) * 16 + (lane & 15)) * RS + (lane >> 4) * 8;
             const bf* qb = Qs + ((lane & 7) + (lane >> 4) * 8) * RS + ((lane >> 3) & 1) * 8;
 #pragma unroll 3
             for (int ks = ks0; ks < ks1; ++ks) {
                 uint32_t a[4], q[4];
-                ldsm_x4(a, ka + ks * 16);
+                ldsm_x4_at(a, k_at(b, ks));
                 ldsm_x4(q, qb + ks * 16);
                 const uint32_t q0[2] = {q[0], q[1]}, q1[2] = {q[2], q[3]};
                 mma_bf16_16816(s[0], a, q0);
@@ -592,7 +649,7 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
                 for (int i = 0; i < NT; i += 2) {
                     if (i < ntw && tile0 + i < n8) {   // n8 is even: a pair of column tiles is inside or outside together
                         uint32_t v[4];
-                        ldsm_x4_trans(v, Kb + (kk + (lane & 15)) * RS + (tile0 + i + (lane >> 4)) * 8);
+                        ldsm_x4_trans_at(v, v_at(b, kk, tile0 + i));
                         const uint32_t v0[2] = {v[0], v[1]}, v1[2] = {v[2], v[3]};
                         mma_bf16_16816(o[i], a, v0);
                         mma_bf16_16816(o[i + 1], a, v1);
@@ -601,11 +658,19 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
             }
         }
         __syncthreads();   // nobody reads half b any more
-        if (b + 2 < b1) load_half(b + 2);
-        close_group();
+        if (TMA) {
+            if (warp == 0 && b + 2 < b1) fetch(b + 2, next_row);
+        } else {
+            if (b + 2 < b1) load_half(b + 2);
+            close_group();
+        }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (!TMA) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+    if (TMA && *dead) {   // a wait was given up: nothing may land on the sums, or behind this CTA's end
+        for (int i = 0; i < 2; ++i) { mbar_wait_limited(&full[i], 0); mbar_wait_limited(&full[i], 1); }
+        l_run[0] = l_run[1] = __int_as_float(0x7fffffff);
+    }
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
         const int c = (tile0 + i) * 8 + tig * 2;
@@ -652,20 +717,23 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const float* __re
     cluster.sync();   // nobody leaves while its share is read
 }
 
-template <int NT>
+template <int NT, bool TMA>
 static int launch_latent_decode(const b200_latent_attention_args& a, int out_cols, int splits, cudaStream_t s) {
     const int rpad = (a.rank + 15) & ~15, RS = rpad + 8;
-    const size_t smem = (size_t)(2 * kHalfKeys + 16) * RS * 2 + 4 * 16 * 36 * 4 + 16 * 40 * 2 + 3 * 16 * 4;
+    const size_t rows = TMA ? 1024 + (size_t)2 * ((a.rank + 63) / 64) * kHalfKeys * 128 : (size_t)2 * kHalfKeys * RS * 2, smem = rows + (size_t)16 * RS * 2 + 4 * 16 * 36 * 4 + 16 * 40 * 2 + 3 * 16 * 4;
     static unsigned long long done = 0, wide = 0;
-    cudaError_t e = ensure_max_dynamic_smem((const void*)latent_decode_kernel<NT>, 114 * 1024, done);
+    cudaError_t e = ensure_max_dynamic_smem((const void*)latent_decode_kernel<NT, TMA>, 114 * 1024, done);
     if (e == cudaSuccess && splits > 8) {
         const int dev = current_device();
         if (!(wide & (1ull << dev))) {
-            e = cudaFuncSetAttribute((const void*)latent_decode_kernel<NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            e = cudaFuncSetAttribute((const void*)latent_decode_kernel<NT, TMA>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e == cudaSuccess) wide |= 1ull << dev;
         }
     }
     if (e != cudaSuccess) return (int)e;
+    CUtensorMap map{};
+    constexpr long long kAnyRow = (1ll << 31) - 1;   // the pool's height is not part of the call: any row that an int can name
+    if (TMA && !make_tma_map_2d(&map, a.pool, kAnyRow, a.rank, kHalfKeys)) return launch_latent_decode<NT, false>(a, out_cols, splits, s);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)splits, (unsigned)((a.heads + 15) / 16), (unsigned)a.n_tokens);
     cfg.blockDim = dim3(256);
@@ -679,7 +747,7 @@ static int launch_latent_decode(const b200_latent_attention_args& a, int out_col
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, latent_decode_kernel<NT>, a.qa, a.out, (const __nv_bfloat16*)a.pool, a.pages, a.max_pages, a.page_rows, a.slot, a.pos,
+    e = cudaLaunchKernelEx(&cfg, latent_decode_kernel<NT, TMA>, map, a.qa, a.out, (const __nv_bfloat16*)a.pool, a.pages, a.max_pages, a.page_rows, a.slot, a.pos,
                            a.sink, a.scale, a.heads, a.rank, a.window, out_cols);
     if (e != cudaSuccess) return (int)e;
     count_launch();
@@ -696,10 +764,11 @@ static int latent_decode(const b200_latent_attention_args& a, int out_cols, int 
     int splits = 1;
     while (splits < kLdMaxCluster && ctas * splits * 2 <= (splits < 8 ? 2ll : 1ll) * sm_count() && (longest_seen <= 0 ? splits < 8 : splits * kHalfKeys < longest_seen)) splits *= 2;
     const int nt = ((out_cols / 8 + kTileWarps - 1) / kTileWarps + 1) & ~1;
-    if (nt <= 2) return launch_latent_decode<2>(a, out_cols, splits, s);
-    if (nt <= 4) return launch_latent_decode<4>(a, out_cols, splits, s);
-    if (nt <= 8) return launch_latent_decode<8>(a, out_cols, splits, s);
-    if (nt <= 10) return launch_latent_decode<10>(a, out_cols, splits, s);
+    const bool tma = a.page_rows % kHalfKeys == 0;   // a half tile never straddles two pages
+    if (nt <= 2) return tma ? launch_latent_decode<2, true>(a, out_cols, splits, s) : launch_latent_decode<2, false>(a, out_cols, splits, s);
+    if (nt <= 4) return tma ? launch_latent_decode<4, true>(a, out_cols, splits, s) : launch_latent_decode<4, false>(a, out_cols, splits, s);
+    if (nt <= 8) return tma ? launch_latent_decode<8, true>(a, out_cols, splits, s) : launch_latent_decode<8, false>(a, out_cols, splits, s);
+    if (nt <= 10) return tma ? launch_latent_decode<10, true>(a, out_cols, splits, s) : launch_latent_decode<10, false>(a, out_cols, splits, s);
     return -1;
 }
 
