@@ -8,7 +8,7 @@
 //   rows        TQ tokens x the R query heads of one key head (TQ = 128 / R), so a key tile is read once for the whole group and a
 //               causal edge wastes little. A CTA's window of TQ packed rows may hold the end of one sequence and the start of
 //               the next: they are separate tiles, walked by neighbouring CTAs (gridDim.y is doubled when there is more than one entry; most second ones
-//               find no tile and leave). Sequences that bring a single token are left to the cluster kernel of paged_decode.cu.
+//               find no tile and leave). Sequences that bring a single token are left to the cluster kernel of paged_decode.cu, launched behind this one or ahead of it.
 //   warp 0      TMA: K and V tiles of 64 rows out of their page (one list lookup per tile), a ring as long as the score buffers
 //   warp 1      tcgen05.mma: S = Q K^T (one group: the weighted sums too, the next tile's scores ahead of them)
 //   softmax     four warps per group, a thread per row: scores are read from TMEM once, P_j goes back over its own scores and is the A operand of the second
@@ -22,7 +22,7 @@
 //               memory, each CTA adds and stores its part of the rows. Costs 3 us, so shares keep some eight key tiles.
 // Two groups take an SM alone; one group leaves room for a second CTA, which hides what a CTA does before its first and after its last product (3.5 and 2 us):
 // better only where many short tiles come in several rounds. Measured, 16 / 8 heads x 128, us, one group (two CTAs per SM, no sharing) / this: 2048 tokens 36.6 / 32.4, 1024 19.9 / 17.5, 64
-// tokens behind 4000 45 / 17, 256 behind 1000 and 4 single tokens 24.5 / 18.5, three portions up to 512 and 12 single tokens behind 4000, capped 143 / 119.
+// tokens behind 4000 45 / 17, 256 behind 1000 and 4 single tokens 24.5 / 18.5, three portions up to 512 and 12 single tokens behind 4000, capped 143 / 107.
 // Tried and taken back: query rows in TMEM and three score buffers (the buffers' round trip costs more than the shared memory saves: 17.5 against 16.8 for 1024 tokens), one warp
 // for all products with three buffers (19.0), eight softmax warps per group, two threads per row (19.2: the pair has to meet at every tile), scores of 128 columns for both groups at
 // once (17.1, 33.4 for 2048: the groups run in step and wait for each other).
@@ -76,7 +76,7 @@ __device__ __forceinline__ float2 ld_cluster_v2(uint32_t addr) {
 
 template <int D, int DV, int W, int FORM, bool SHARED>
 __global__ void __launch_bounds__(TcSmem<D, DV, W>::kThreads, TcSmem<D, DV, W>::kPerSm)
-paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int TQ, int parts, int skip_singles, int sorted, int split2) {   // split2: log2 of the CTAs that share a tile's keys
+paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int TQ, int parts, int skip_singles, int sorted, int behind, int split2) {   // split2: log2 of the CTAs that share a tile's keys
     using bf = __nv_bfloat16;
     using L = TcSmem<D, DV, W>;
     constexpr int NB = L::kRing, NT = L::kThreads;
@@ -116,6 +116,8 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
     }
     const int t0 = window * TQ, rows = min(TQ, a.n_tokens - t0);
 
+    // behind the kernel of the single tokens, which runs beside this one: done only when both are, and one CTA to wait is enough
+    const bool last_out = behind && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1;
     // ---- TMEM, barriers, and the window's tiles
     if (warp == 1 && parts == 1) tmem_alloc(tmem_slot, L::kTmemCols);
     if (threadIdx.x == 0) {
@@ -146,7 +148,10 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         int n_tiles = 0;
 #pragma unroll
         for (int i = 4; i < 8; ++i) n_tiles += __popc(masks[i]);
-        if (n_tiles <= part) return;
+        if (n_tiles <= part) {
+            if (last_out) pdl_wait();
+            return;
+        }
         if (warp == 1) tmem_alloc(tmem_slot, L::kTmemCols);
         tc_fence_before();
     }
@@ -620,11 +625,12 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         __syncthreads();
     }
     if (warp == 1) tmem_dealloc(tmem, L::kTmemCols);
+    if (last_out) pdl_wait();
 }
 
 struct TcPlan {
     long long windows;
-    int parts, sorted, split2, bias;   // split2: log2 of the CTAs that share a tile's keys; bias: staged numbers
+    int parts, sorted, behind, split2, bias;   // split2: log2 of the CTAs that share a tile's keys; bias: staged numbers
     bool two_groups;
 };
 
@@ -644,15 +650,19 @@ static int launch_tc(const PA& a, const TcPlan& p, cudaStream_t s) {
     cfg.blockDim = dim3(L::kThreads);
     cfg.dynamicSmemBytes = L::kOffBias + p.bias * 4 + 1024;
     cfg.stream = s;
-    cudaLaunchAttribute at{};
+    cudaLaunchAttribute at[2]{};
+    cfg.attrs = at;
     if (SHARED) {
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = 1u << p.split2;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 1u << p.split2;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
     }
-    e = cudaLaunchKernelEx(&cfg, paged_attn_tc_kernel<D, DV, W, FORM, SHARED>, mk, mv, a, TQ, p.parts, p.parts - 1, p.sorted, p.split2);
+    if (p.behind && pdl_enabled()) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    e = cudaLaunchKernelEx(&cfg, paged_attn_tc_kernel<D, DV, W, FORM, SHARED>, mk, mv, a, TQ, p.parts, p.parts - 1, p.sorted, p.behind, p.split2);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -704,15 +714,24 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     while (p.two_groups && p.split2 < (tiles * 8 <= sms / 2 ? 3 : 2) && (tiles << (p.split2 + 1)) <= room && steps >= 12 && steps >= 8 << p.split2) ++p.split2;
     // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 90.2 / 84.3 us)
     p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && p.two_groups;
+    const int singles = a.n_tokens - std::max(longest_entry, 0);
+    const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));   // CTAs of single tokens that fit beside the tiles'
+    // Single tokens go beside the tiles where there is room for eight of them. Where the tiles fill the GPU for long they go ahead instead, two CTAs per SM on the SMs that they need, and the tiles take what they
+    // leave: behind them they waited for the first round to end (us, behind / ahead of the tiles, 16 / 8 heads x 128: 12 single tokens and three portions of up to 512 behind 4000, capped, 118 / 107, plain
+    // behind 2000 70.7 / 61.4, 8 and two of 512 88.6 / 83.0, 1 and two of 400 behind 3000 68.7 / 46.0, no single token and three of 512 82.9 / 83.8)
+    p.behind = several && p.two_groups && steps > 32 && (p.sorted || free < 2ll * std::min(singles, 8) * units);
+    if (p.behind) {
+        const int rc = paged_decode(a, longest_seen, singles, 0, true, s);
+        if (rc != 0) return rc;
+    }
     int rc = -1;
     if (a.dim == 128 && a.vdim == 128) rc = launch_tc_for<128, 128>(a, p, s);
     else if (a.dim == 64 && a.vdim == 64) rc = launch_tc_for<64, 64>(a, p, s);
     else if (a.dim == 128 && a.vdim == 256) rc = launch_tc_for<128, 256>(a, p, s);
     if (rc != 0) return rc;
     count_launch();
-    if (several) {   // the sequences that bring one token, on what the tiles leave free
-        const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));
-        return paged_decode(a, longest_seen, a.n_tokens - std::max(longest_entry, 0), free, s);
+    if (several && !p.behind) {   // the sequences that bring one token, on what the tiles leave free
+        return paged_decode(a, longest_seen, singles, free, false, s);
     }
     return 0;
 }

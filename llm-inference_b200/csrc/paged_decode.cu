@@ -56,7 +56,7 @@ __device__ __forceinline__ void pd_ldsm_x4_trans(uint32_t (&r)[4], uint32_t a) {
 // those that are their sequence's only token in the batch.
 template <int D, int VD, bool MIXED>
 __global__ void __launch_bounds__(kPdWarps * 32, PdRing<D, VD>::kPerSm)
-paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a) {
+paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int ahead) {
     using bf = __nv_bfloat16;
     using L = PdRing<D, VD>;
     constexpr int KS = D / 16;        // k steps of the scores
@@ -76,7 +76,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         if (warp == 0) { *dead = 0; tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
     }
     __syncthreads();
-    if (!MIXED) {
+    if (!MIXED || ahead) {
         pdl_wait();
         pdl_launch_dependents();
     }
@@ -359,11 +359,11 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
         if (!MIXED) break;
     }
-    if (MIXED) pdl_wait();   // the prompt portions' kernel runs beside this one: done only when both are
+    if (MIXED && !ahead) pdl_wait();   // the prompt portions' kernel runs beside this one: done only when both are (ahead of it: it waits)
 }
 
 template <int D, int VD, bool MIXED>
-static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s) {
+static int launch_paged_decode(const PA& a, int splits, int rows, bool ahead, cudaStream_t s) {
     constexpr int smem = PdRing<D, VD>::kBytes;
     static_assert(kPdWarps * kPdHeads * VD * 4 <= smem, "the warps' sums take the rings' place");
     CUtensorMap mk, mv;
@@ -388,22 +388,22 @@ static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, mk, mv, a);
+    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, mk, mv, a, ahead ? 1 : 0);
     if (e != cudaSuccess) return (int)e;
     count_launch();
     return (int)cudaGetLastError();
 }
 
 template <bool MIXED>
-static int paged_decode_for(const PA& a, int splits, int rows, cudaStream_t s) {
-    if (a.dim == 128 && a.vdim == 128) return launch_paged_decode<128, 128, MIXED>(a, splits, rows, s);
-    if (a.dim == 64 && a.vdim == 64) return launch_paged_decode<64, 64, MIXED>(a, splits, rows, s);
-    if (a.dim == 128 && a.vdim == 256) return launch_paged_decode<128, 256, MIXED>(a, splits, rows, s);
-    if (a.dim == 64 && a.vdim == 128) return launch_paged_decode<64, 128, MIXED>(a, splits, rows, s);
+static int paged_decode_for(const PA& a, int splits, int rows, bool ahead, cudaStream_t s) {
+    if (a.dim == 128 && a.vdim == 128) return launch_paged_decode<128, 128, MIXED>(a, splits, rows, ahead, s);
+    if (a.dim == 64 && a.vdim == 64) return launch_paged_decode<64, 64, MIXED>(a, splits, rows, ahead, s);
+    if (a.dim == 128 && a.vdim == 256) return launch_paged_decode<128, 256, MIXED>(a, splits, rows, ahead, s);
+    if (a.dim == 64 && a.vdim == 128) return launch_paged_decode<64, 128, MIXED>(a, splits, rows, ahead, s);
     return -1;
 }
 
-int paged_decode(const PA& a, int longest_seen, int singles, long long room, cudaStream_t s) {
+int paged_decode(const PA& a, int longest_seen, int singles, long long room, bool ahead, cudaStream_t s) {
     const bool mixed = singles > 0;
     if (a.heads / a.kv_heads > kPdHeads || a.page_rows % kPdStep || a.kv_heads * a.maps > 65535) return -1;
     // how many tokens of a mixed batch are single ones is only known on the device: sixteen rows of clusters share them
@@ -414,7 +414,9 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, cud
     // 34.4 / 20.0 / 14.3 / 19.8, 4 such 34.3 / 19.8 / 13.5 / 10.8)
     const long long pairs = (long long)rows * a.kv_heads * a.maps;
     int splits = 1;
-    if (mixed) {
+    if (ahead) {   // the portions' CTAs start when the last of these has: one round
+        while (splits < kPdMaxCluster && pairs * splits <= sm_count() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+    } else if (mixed) {
         // on what the portions' CTAs leave free (`room` CTAs) if eight single tokens can sit there beside each other, else behind them (us at 2 / 4 / 8 shares: 8 single tokens and a portion of 512 behind
         // 4000 57.2 / 77.7 / 83.0, 4 and 64 36.8 / 31.7 / 40.9, 12 and three of 512, which fill the GPU, 123 / 119 / 133)
         const long long likely = (long long)std::min(singles, 8) * a.kv_heads * a.maps;
@@ -424,7 +426,7 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, cud
         while (splits > 1 && longest_seen > 0 && splits / 2 * kPdWarps * kPdStep >= longest_seen) splits /= 2;
     } else
         while (splits < kPdMaxCluster && pairs * splits <= sm_count() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
-    return mixed ? paged_decode_for<true>(a, splits, rows, s) : paged_decode_for<false>(a, splits, rows, s);
+    return mixed ? paged_decode_for<true>(a, splits, rows, ahead, s) : paged_decode_for<false>(a, splits, rows, false, s);
 }
 
 }  // namespace b200
