@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     // the order in which a row's chunks are taken: those without sums first
     auto chunk_of = [&](int o) { return o >= NS ? half * kLtV + o - NS : o < half * kLtV ? o : o + kLtV; };
 
+    pdl_wait();
     // ---- the window's tiles (paged_attention_tc.cu): rows that begin a sequence
     if (threadIdx.x < TQ) slots[threadIdx.x] = (int)threadIdx.x < rows ? a.slot[t0 + threadIdx.x] : -1;
     if (threadIdx.x == 0) *dead = 0;
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_launch_dependents();   // (behind the allocation: a product kernel that moved in ahead of it would wait for this one while holding tensor memory)
     const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0), o_tmem = tmem, s_tmem = tmem + 256, q_tmem = tmem + 256 + 2 * kLtKeys;
 
     int it0 = 0, q0 = 0, ordinal = 0;   // key tiles, query chunks, tiles of the window so far
@@ -401,7 +403,8 @@ static int launch_lt(const b200_latent_attention_args& a, int halves, cudaStream
     const long long windows = (a.n_tokens + TQ - 1) / TQ;
     if (windows * parts > 65535) return -1;
     const LtArgs la{a.qa, a.out, a.pages, a.slot, a.pos, a.sink, a.max_pages, a.page_rows, a.n_tokens, a.heads, a.rank, a.window, TQ, parts, a.scale};
-    latent_attn_tc_kernel<NCH><<<dim3((unsigned)halves, (unsigned)(windows * parts)), kLtThreads, LtSmem<NCH>::kTotal, s>>>(map, map_q, la);
+    const cudaError_t le = launch_chained(latent_attn_tc_kernel<NCH>, dim3((unsigned)halves, (unsigned)(windows * parts)), dim3(kLtThreads), (size_t)LtSmem<NCH>::kTotal, s, map, map_q, la);
+    if (le != cudaSuccess) return (int)le;
     return (int)cudaGetLastError();
 }
 

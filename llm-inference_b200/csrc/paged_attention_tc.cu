@@ -7,7 +7,7 @@
 // key tile on waits, products and commits): about 1150 clocks per key tile, 1620 with one group alone on an SM. Long contexts of few rows are shared out over a cluster.
 //   rows        TQ tokens x the R query heads of one key head (TQ = 128 / R), so a key tile is read once for the whole group and a
 //               causal edge wastes little. A CTA's window of TQ packed rows may hold the end of one sequence and the start of
-//               the next: they are separate tiles, walked by neighbouring CTAs (gridDim.y is doubled when there is more than one entry; most second ones
+//               the next: they are separate tiles, walked by neighbouring CTAs (gridDim.y is doubled, or for small batches made four times as large, when there is more than one entry; most of the others
 //               find no tile and leave). Sequences that bring a single token are left to the cluster kernel of paged_decode.cu, launched behind this one or ahead of it.
 //   warp 0      TMA: K and V tiles of 64 rows out of their page (one list lookup per tile), a ring as long as the score buffers
 //   warp 1      tcgen05.mma: S = Q K^T (one group: the weighted sums too, the next tile's scores ahead of them)
@@ -54,7 +54,7 @@ struct TcSmem {
     static constexpr int kThreads = 64 + 128 * W + (W > 1 ? 32 : 0), kPvWarp = 2 + 4 * W;   // warps: TMA, products, softmax; two groups: scores and weighted sums have a warp each
     static constexpr int kQ = kTcRows * D * 2, kK = kTcKeys * D * 2, kV = kTcKeys * DV * 2;   // the query rows; a stage's bytes
     static constexpr int kOffK = kQ, kOffV = kOffK + kRing * kK, kOffBar = kOffV + kRing * kV, kOffSlot = kOffBar + 5 * kRing * 8;
-    static constexpr int kOffMl = (kOffSlot + (2 * (kTcRows + 2) + 10) * 4 + 7) & ~7;   // (reference, sum) of every row and group
+    static constexpr int kOffMl = (kOffSlot + (2 * (kTcRows + 2) + 12) * 4 + 7) & ~7;   // (reference, sum) of every row and group
     static constexpr int kOffBias = kOffMl + W * kTcRows * 8;
     static constexpr int kOffSums = kRing * kTcKeys;           // tensor memory: score buffers, then the groups' sums
     static constexpr int kTmemCols = kOffSums + W * DV <= 256 ? 256 : 512, kPerSm = kTmemCols == 256 ? 2 : 1;
@@ -94,6 +94,21 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform as the compiler sees it)
     const int split = 1 << split2, rank = SHARED ? (int)blockIdx.x & (split - 1) : 0, ku = SHARED ? (int)blockIdx.x >> split2 : (int)blockIdx.x, g = ku / a.maps, mp = ku % a.maps, R = a.heads / a.kv_heads, q_units = a.heads * a.maps;
+    // behind the kernel of the single tokens, which runs beside this one: done only when both are, and one CTA to wait is enough
+    const bool last_out = behind && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1;
+    // ---- TMEM and barriers, while the kernel before this one ends (the single tokens' kernel has waited for what this one reads)
+    const bool early = parts != 2;   // every CTA has a tile, or all start at once
+    if (warp == 1 && early) tmem_alloc(tmem_slot, L::kTmemCols);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) { mbar_init(&k_full[b], 1); mbar_init(&v_full[b], 1); mbar_init(&s_full[b], 1); mbar_init(&p_full[b], 4); mbar_init(&o_done[b], 1); }
+        mbar_fence_init();
+        tma_prefetch_desc(&map_k);
+        tma_prefetch_desc(&map_v);
+        *dead = 0;
+    }
+    if (!behind) pdl_wait();
+
     // the windows that see the most keys come first: of one prompt the last rows, of several entries by what their first and last rows see
     const int yy = gridDim.y - 1 - blockIdx.y, part = yy % parts;
     int window = yy / parts;
@@ -108,26 +123,15 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
             const int mine = slots[threadIdx.x];
             int before = 0;
             for (int i = 0; i < n; ++i) before += slots[i] > mine || (slots[i] == mine && i < (int)threadIdx.x) ? 1 : 0;
-            if (before == n - 1 - window) *tmem_slot = threadIdx.x;
+            if (before == n - 1 - window) masks[10] = threadIdx.x;
         }
         __syncthreads();
-        window = (int)*tmem_slot;
+        window = (int)masks[10];
         __syncthreads();
     }
     const int t0 = window * TQ, rows = min(TQ, a.n_tokens - t0);
 
-    // behind the kernel of the single tokens, which runs beside this one: done only when both are, and one CTA to wait is enough
-    const bool last_out = behind && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1;
-    // ---- TMEM, barriers, and the window's tiles
-    if (warp == 1 && parts == 1) tmem_alloc(tmem_slot, L::kTmemCols);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) { mbar_init(&k_full[b], 1); mbar_init(&v_full[b], 1); mbar_init(&s_full[b], 1); mbar_init(&p_full[b], 4); mbar_init(&o_done[b], 1); }
-        mbar_fence_init();
-        tma_prefetch_desc(&map_k);
-        tma_prefetch_desc(&map_v);
-        *dead = 0;
-    }
+    // ---- the window's tiles
     for (int i = (int)threadIdx.x - 64; i >= 0 && i < TQ + 2; i += NT - 64) {
         const int t = t0 - 1 + i;
         slots[i] = t >= 0 && t < a.n_tokens ? a.slot[t] : -1;
@@ -149,10 +153,11 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 #pragma unroll
         for (int i = 4; i < 8; ++i) n_tiles += __popc(masks[i]);
         if (n_tiles <= part) {
+            if (warp == 1 && early) tmem_dealloc(__shfl_sync(0xffffffffu, *tmem_slot, 0), L::kTmemCols);
             if (last_out) pdl_wait();
             return;
         }
-        if (warp == 1) tmem_alloc(tmem_slot, L::kTmemCols);
+        if (warp == 1 && !early) tmem_alloc(tmem_slot, L::kTmemCols);
         tc_fence_before();
     }
     int tn = 0;   // staged distances per head: those that a row of the window can have
@@ -658,7 +663,7 @@ static int launch_tc(const PA& a, const TcPlan& p, cudaStream_t s) {
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
     }
-    if (p.behind && pdl_enabled()) {
+    if (pdl_enabled()) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
@@ -712,6 +717,8 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     // 512 and 8 single ones behind 4000 57.2 / 62.1 / 77.0 / 115)
     const long long room = several ? 2 * sms / 3 : sms;
     while (p.two_groups && p.split2 < (tiles * 8 <= sms / 2 ? 3 : 2) && (tiles << (p.split2 + 1)) <= room && steps >= 12 && steps >= 8 << p.split2) ++p.split2;
+    // CTAs that share a window's tiles: four where they all start at once (portions of 53, 45 and 33 tokens lie in one window and a bit: 16 heads x 128, capped, 12.6 / 9.9 us)
+    if (several && p.split2 == 0 && tiles * 4 <= sms) p.parts = 4;
     // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 90.2 / 84.3 us)
     p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && p.two_groups;
     const int singles = a.n_tokens - std::max(longest_entry, 0);

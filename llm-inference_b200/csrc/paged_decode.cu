@@ -76,10 +76,8 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         if (warp == 0) { *dead = 0; tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
     }
     __syncthreads();
-    if (!MIXED || ahead) {
-        pdl_wait();
-        pdl_launch_dependents();
-    }
+    if (!MIXED || ahead) pdl_wait();
+    pdl_launch_dependents();
     const int R = a.heads / a.kv_heads, splits = gridDim.x;
     float* om = reinterpret_cast<float*>(pd_sm);                                 // once the rings have been used: [warps][R][VD], then this CTA's share in the first [R][VD]
     __shared__ float ms[kPdWarps * kPdHeads], ls[kPdWarps * kPdHeads];   // [warps][R], then [R]
