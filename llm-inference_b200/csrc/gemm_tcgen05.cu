@@ -598,10 +598,16 @@ bool make_tma_map_2d(CUtensorMap* out, const void* ptr, long long rows, int K, i
     };
     static std::unordered_map<Key, CUtensorMap, Hash> cache;
     static std::mutex mu;
-    std::lock_guard<std::mutex> g(mu);
     const Key key{ptr, rows, K, box_rows};
+    // the thread's own look first (a map follows from its key alone): no lock and no search for what a program calls again and again
+    struct Seen { Key key; CUtensorMap map; };
+    static thread_local Seen seen[64];
+    const size_t h = Hash()(key);
+    Seen& mine = seen[(h ^ h >> 9 ^ h >> 17) & 63];
+    if (mine.key.p && mine.key == key) { *out = mine.map; return true; }
+    std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(key);
-    if (it != cache.end()) { *out = it->second; return true; }
+    if (it != cache.end()) { *out = it->second; mine = Seen{key, it->second}; return true; }
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
@@ -615,6 +621,7 @@ bool make_tma_map_2d(CUtensorMap* out, const void* ptr, long long rows, int K, i
     if (r != CUDA_SUCCESS) return false;
     if (cache.size() > 4096) cache.clear();
     cache.emplace(key, m);
+    mine = Seen{key, m};
     *out = m;
     return true;
 }

@@ -761,8 +761,9 @@ static int latent_decode(const b200_latent_attention_args& a, int out_cols, int 
     // as many shares as two CTAs per SM hold at once (clusters of sixteen: one), as long as every CTA keeps a half tile of its own (us at 4 / 8 / 16 shares, 16 heads, rows of 576: 32 sequences of up to 2048
     // 49.1 / 33.8 / 51.1, of up to 700 21.5 / 17.4 / 33.5, 24 of up to 1000 26.3 / 20.0 / 27.9, 16 such 26.3 / 18.9 / 23.3, 8 of up to 1024 28.6 / 19.0 / 16.6)
     const long long ctas = (long long)a.n_tokens * ((a.heads + 15) / 16);
+    const long long sms = sm_count();
     int splits = 1;
-    while (splits < kLdMaxCluster && ctas * splits * 2 <= (splits < 8 ? 2ll : 1ll) * sm_count() && (longest_seen <= 0 ? splits < 8 : splits * kHalfKeys < longest_seen)) splits *= 2;
+    while (splits < kLdMaxCluster && ctas * splits * 2 <= (splits < 8 ? 2 * sms : sms) && (longest_seen <= 0 ? splits < 8 : splits * kHalfKeys < longest_seen)) splits *= 2;
     const int nt = ((out_cols / 8 + kTileWarps - 1) / kTileWarps + 1) & ~1;
     const bool tma = a.page_rows % kHalfKeys == 0;   // a half tile never straddles two pages
     if (nt <= 2) return tma ? launch_latent_decode<2, true>(a, out_cols, splits, s) : launch_latent_decode<2, false>(a, out_cols, splits, s);

@@ -411,9 +411,10 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, boo
     // shares: 32 sequences of up to 2048 tokens 42.5 / 44.5 / 52.7 / 78.0, 16 such 35.0 / 24.4 / 28.2 / 40.9, 12 of up to 1500 27.4 / 17.1 / 20.4 / 25.4, 8 of up to 2048
     // 34.4 / 20.0 / 14.3 / 19.8, 4 such 34.3 / 19.8 / 13.5 / 10.8)
     const long long pairs = (long long)rows * a.kv_heads * a.maps;
+    const int sms = sm_count();
     int splits = 1;
     if (ahead) {   // the portions' CTAs start when the last of these has: one round
-        while (splits < kPdMaxCluster && pairs * splits <= sm_count() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+        while (splits < kPdMaxCluster && pairs * splits <= sms && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
     } else if (mixed) {
         // on what the portions' CTAs leave free (`room` CTAs) if eight single tokens can sit there beside each other, else behind them (us at 2 / 4 / 8 shares: 8 single tokens and a portion of 512 behind
         // 4000 57.2 / 77.7 / 83.0, 4 and 64 36.8 / 31.7 / 40.9, 12 and three of 512, which fill the GPU, 123 / 119 / 133)
@@ -423,7 +424,7 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, boo
         while (splits < (likely <= 8 ? kPdMaxCluster : 4) && likely * splits * 2 <= room) splits *= 2;
         while (splits > 1 && longest_seen > 0 && splits / 2 * kPdWarps * kPdStep >= longest_seen) splits /= 2;
     } else
-        while (splits < kPdMaxCluster && pairs * splits <= sm_count() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+        while (splits < kPdMaxCluster && pairs * splits <= sms && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
     return mixed ? paged_decode_for<true>(a, splits, rows, ahead, s) : paged_decode_for<false>(a, splits, rows, false, s);
 }
 
