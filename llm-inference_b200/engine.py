@@ -324,7 +324,8 @@ class Engine:
         # the engine's own buffer: the tensor over it is made once (56 us, in which the GPU waits for the next step), each call returns an alias
         at = self.lib.b200_engine_logits(self.h)
         if self._logits is None or self._logits[0] != at:
-            self._logits = (at, self._view(at, (self.batch, self.cfg.vocab_size), torch.float16 if self.dtype == capi.F16 else torch.float32))
+            with torch.inference_mode(False):   # (an ordinary tensor, whoever asks first)
+                self._logits = (at, self._view(at, (self.batch, self.cfg.vocab_size), torch.float16 if self.dtype == capi.F16 else torch.float32))
         return self._logits[1].view(self.batch, self.cfg.vocab_size)
 
     def hidden(self):
