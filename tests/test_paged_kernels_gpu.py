@@ -275,3 +275,18 @@ def test_more_tiles_than_the_gpu_holds_at_once(S, form, d, before):
         want = reference(q[b], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
         assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 5e-3, b
         at += new[b]
+
+
+@pytest.mark.parametrize("T", [1, 60, 80])
+def test_precision_of_single_tokens_does_not_hang_on_the_shares(S, T):
+    """fp32 outputs of 1500 keys in eight shares, two and one. A warp adds up to 24 steps in fp32, each rounded to 2^-24 of a sum that grows to 1: 24^0.5 / 3 * 2^-24 = 1.0e-7, and as
+    much from a step's products and the exponentials; 4e-7 is twice both. Sums left to the tensor core are cut off three times a step: 24 * 3 * 2^-24 / 6 = 7e-7 for one share"""
+    g = torch.Generator().manual_seed(T)
+    H, d, n, PR = 2, 128, 1500, 64
+    o = dict(options("sigmoid", H, d, g), window=0)
+    k, v, kp, vp, table = sequences(g, [n], H, 1, d, d, PR)
+    q = torch.randn(T, H, 1, d, generator=g).bfloat16().double()
+    pos = [n - 1 - i for i in range(T)]
+    got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * T, pos, o, 1)
+    want = reference(q, k[0], v[0], pos, o)
+    assert float((got - want).norm() / want.norm()) < 4e-7
