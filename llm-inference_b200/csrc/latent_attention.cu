@@ -450,10 +450,11 @@ __global__ void __launch_bounds__(128) latent_attn_combine_kernel(const float* _
 // A half tile comes by TMA, a box per lane of one warp, its place in the pool looked up a step before (by cp.async, twelve copies and their addresses
 // per lane behind that lookup, a step of 32 rows took 2.6 us); pages that are no multiple of a half tile keep cp.async.
 //   scores   warp w: keys [16 (w & 1), +16) x 16 heads over a quarter (w >> 1) of the row; the four partial sums meet in shared memory
-//   softmax  warp w: heads 2w, 2w + 1, a key per lane; the weights leave as bfloat16 (as in the tile kernel)
+//   softmax  warp w: heads 2w, 2w + 1, a key per lane; the weights leave as the sum of two bfloat16: rounded to one, they lose the more the fewer
+//            shares there are (a share's largest is 1, which is exact): 1.84e-3 of the result's norm for 32 sequences in 512 shares, 1.86e-3 in 256; 1.54e-3 now, the queries' rounding
 //   values   warp w: an eighth of the output columns, the rows read transposed by ldmatrix
 // The sink joins in the merge. Measured, 8 sequences of up to 1024 rows of 576, 16 heads, 512 columns out: the tile kernel with its
-// combine launch 53.3 us, by cp.async 16.2, this 14.1 us; 32 sequences of up to 2048 rows 34 / 24, one of 2048 19.1 / 14.7.
+// combine launch 53.3 us, by cp.async 16.2, this 14.6 us (weights of one bfloat16: 14.0); 32 sequences of up to 2048 rows 34 / 26, one of 2048 19.1 / 16.1.
 constexpr int kLdMaxCluster = 16;
 
 __device__ __forceinline__ void ldsm_x4_at(uint32_t (&r)[4], uint32_t a) {
@@ -489,7 +490,8 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const __grid_cons
     const int boxes = (rank + 63) / 64, stage = boxes * kHalfKeys * 128;   // TMA: bytes of a half tile
     bf* Qs = TMA ? reinterpret_cast<bf*>(smraw + 2 * stage) : Ks + 2 * kHalfKeys * RS;   // [16][RS]
     float* Ss = reinterpret_cast<float*>(Qs + 16 * RS);        // [4][16][36]: partial scores [head][key]
-    bf* Ps = reinterpret_cast<bf*>(Ss + 4 * 16 * 36);          // [16][40]
+    bf* Ps = reinterpret_cast<bf*>(Ss + 4 * 16 * 36);          // [16][40]: the weights, rounded
+    bf* Pl = reinterpret_cast<bf*>(Ss);                        // [16][72]: what that left, over a row's own scores
     float* al_s = reinterpret_cast<float*>(Ps + 16 * 40);      // [16]
     float* ms = al_s + 16;                                     // [16]
     float* ls = ms + 16;                                       // [16]
@@ -633,7 +635,9 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const __grid_cons
             for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
             l_run[x] = l_run[x] * al + sum;
             m_run[x] = mn;
-            Ps[r * 40 + lane] = __float2bfloat16_rn(pv);
+            const bf hi = __float2bfloat16_rn(pv);
+            Ps[r * 40 + lane] = hi;
+            Pl[r * 72 + lane] = __float2bfloat16_rn(pv - __bfloat162float(hi));   // after every lane has read its scores (the shuffles above)
             if (lane == 0) al_s[r] = al;
         }
         __syncthreads();
@@ -643,14 +647,17 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const __grid_cons
             for (int i = 0; i < NT; ++i) { o[i][0] *= a0; o[i][1] *= a0; o[i][2] *= a1; o[i][3] *= a1; }
 #pragma unroll
             for (int kk = 0; kk < kHalfKeys; kk += 16) {
-                uint32_t a[4];
+                uint32_t a[4], al[4];
                 ldsm_x4(a, Ps + (lane & 15) * 40 + kk + (lane >> 4) * 8);
+                ldsm_x4(al, Pl + (lane & 15) * 72 + kk + (lane >> 4) * 8);
 #pragma unroll
                 for (int i = 0; i < NT; i += 2) {
                     if (i < ntw && tile0 + i < n8) {   // n8 is even: a pair of column tiles is inside or outside together
                         uint32_t v[4];
                         ldsm_x4_trans_at(v, v_at(b, kk, tile0 + i));
                         const uint32_t v0[2] = {v[0], v[1]}, v1[2] = {v[2], v[3]};
+                        mma_bf16_16816(o[i], al, v0);
+                        mma_bf16_16816(o[i + 1], al, v1);
                         mma_bf16_16816(o[i], a, v0);
                         mma_bf16_16816(o[i + 1], a, v1);
                     }

@@ -53,3 +53,31 @@ def test_single_tokens_share_their_rows_in_a_cluster(S, heads, W, cols, PR, wind
             w = e / (e.sum(1, keepdim=True) + (torch.exp(sk.double()[:, None] - top) if sink else 0.0))
             want = w @ kv[:, :cols]
             assert float((got[b, :, :cols] - want).norm() / want.norm()) < 8e-3, (b, n)
+
+
+@pytest.mark.parametrize("T", [1, 20, 80, 160])
+@pytest.mark.parametrize("PR", [64, 48])
+def test_weights_of_single_tokens_are_the_sum_of_two_bfloat16(S, T, PR):
+    """queries that bfloat16 holds, so what is left is a weight's rounding, 2^-18 of it, and the scores' fp32 sums, 2^-24 * 36 steps of a few units: 1e-5 together, the bound is three
+    times that. A weight rounded to one bfloat16 is off by up to 2^-9. Sixteen shares of a context to one"""
+    g = torch.Generator().manual_seed(T + PR)
+    heads, W, cols, n = 16, 576, 512, 1400
+    rows = torch.randn(n, W, generator=g).bfloat16()
+    pool = torch.full(((n + PR - 1) // PR * PR, W), float("nan"), dtype=torch.bfloat16)
+    pool[:n] = rows
+    qa, scale = torch.randn(T, heads, W, generator=g).bfloat16().float(), W ** -0.5
+    pos = [n - 1 - i for i in range(T)]
+    dev = [qa.cuda(), pool.cuda(), torch.arange(pool.shape[0] // PR, dtype=torch.int32).cuda(), torch.zeros(T, dtype=torch.int32).cuda(), torch.tensor(pos, dtype=torch.int32).cuda()]
+    out = torch.empty(T, heads, W, device="cuda")
+    a = S.LatentAttentionArgs()
+    a.qa, a.out, a.pool, a.pages, a.max_pages, a.page_rows = dev[0].data_ptr(), out.data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), dev[2].numel(), PR
+    a.slot, a.pos, a.scale = dev[3].data_ptr(), dev[4].data_ptr(), scale
+    a.n_tokens, a.heads, a.rank, a.dtype, a.longest_entry, a.longest_context, a.out_cols = T, heads, W, S.BF16, 1, n, cols
+    torch.cuda.synchronize()
+    assert S.lib().b200_latent_attention_ex(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    kv = rows.double()
+    s = qa.double() @ kv.T * scale
+    s = s.masked_fill(torch.arange(n)[None, None, :] > torch.tensor(pos)[:, None, None], float("-inf"))
+    want = torch.softmax(s, -1) @ kv[:, :cols]
+    assert float((out.double().cpu()[:, :, :cols] - want).norm() / want.norm()) < 3e-5
