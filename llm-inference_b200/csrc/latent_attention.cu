@@ -766,7 +766,8 @@ static int latent_decode(const b200_latent_attention_args& a, int out_cols, int 
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     if ((a.rank & 7) || (out_cols & 15) || a.n_tokens > 65535 || !al16(a.qa) || !al16(a.out) || !al16(a.pool)) return -1;
     // as many shares as two CTAs per SM hold at once (clusters of sixteen: one), as long as every CTA keeps a half tile of its own (us at 4 / 8 / 16 shares, 16 heads, rows of 576: 32 sequences of up to 2048
-    // 49.1 / 33.8 / 51.1, of up to 700 21.5 / 17.4 / 33.5, 24 of up to 1000 26.3 / 20.0 / 27.9, 16 such 26.3 / 18.9 / 23.3, 8 of up to 1024 28.6 / 19.0 / 16.6)
+    // 49.1 / 33.8 / 51.1, of up to 700 21.5 / 17.4 / 33.5, 24 of up to 1000 26.3 / 20.0 / 27.9, 16 such 26.3 / 18.9 / 23.3, 8 of up to 1024 28.6 / 19.0 / 16.6, measured with
+    // rows by cp.async and weights of one bfloat16; by TMA, in two, this rule's choices take 26.5, 15.2, 16.8, 15.4 and 14.1)
     const long long ctas = (long long)a.n_tokens * ((a.heads + 15) / 16);
     const long long sms = sm_count();
     int splits = 1;
