@@ -328,7 +328,7 @@ int b200_conv_state_update(const float* proj, long long ld_proj, float* conv_sta
  * sequence's rows j <= pos[t]; p_j = exp(s_j) / (denom_bias + sum_j exp(s_j)) (denom_bias 1: a sink of score 0 without
  * a value; 0: plain softmax); out[t, h, :] = sum_j p_j v_j. q [n_tokens, heads*dim], out [n_tokens, heads*vdim], pools
  * [n_pages*page_rows, kv_heads, dim | vdim], all of `dtype`; scores, softmax and sums in fp32.
- * longest_entry (0 = unknown): most tokens one sequence brings in this batch. In bfloat16 prompt portions run on tensor-core tiles
+ * longest_entry (0, or more than n_tokens: unknown): most tokens one sequence brings in this batch. In bfloat16 prompt portions run on tensor-core tiles
  * and single tokens on clusters of CTAs that share a context (head sizes 64 / 64, 64 / 128, 128 / 128 and 128 / 256, up to eight query heads
  * per key head; neither needs the workspace). fp32, other head sizes and unaligned operands run on the row kernel; with a workspace and
  * longest_context given, it splits the contexts of few rows over up to 16 CTAs and merges the shares in a second launch. */

@@ -689,6 +689,7 @@ static int launch_tc_for(const PA& a, const TcPlan& p, cudaStream_t s) {
 }
 
 int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStream_t s) {
+    if (longest_entry < 0 || longest_entry > a.n_tokens) longest_entry = 0;   // a limit instead of the batch's own number: unknown
     const int R = a.heads / a.kv_heads;
     // a cap beside a sink or a bias keeps the row kernel, whose weights stay in 32 bits
     if (R > 8 || a.page_rows % kTcKeys || (a.softcap > 0.f && (a.dist_bias || a.sink)) || a.kv_heads * a.maps > 65535) return -1;
@@ -721,7 +722,7 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     if (several && p.split2 == 0 && tiles * 4 <= sms) p.parts = 4;
     // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 90.2 / 84.3 us)
     p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && p.two_groups;
-    const int singles = a.n_tokens - std::max(longest_entry, 0);
+    const int singles = a.n_tokens - longest_entry;   // at most; with several entries at least one
     const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));   // CTAs of single tokens that fit beside the tiles'
     // Single tokens go beside the tiles where there is room for eight of them. Where the tiles fill the GPU for long they go ahead instead, two CTAs per SM on the SMs that they need, and the tiles take what they
     // leave: behind them they waited for the first round to end (us, behind / ahead of the tiles, 16 / 8 heads x 128: 12 single tokens and three portions of up to 512 behind 4000, capped, 118 / 107, plain

@@ -290,3 +290,23 @@ def test_precision_of_single_tokens_does_not_hang_on_the_shares(S, T):
     got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * T, pos, o, 1)
     want = reference(q, k[0], v[0], pos, o)
     assert float((got - want).norm() / want.norm()) < 4e-7
+
+
+@pytest.mark.parametrize("H,before,new", [(4, [250, 63, 10, 0], [1, 65, 1, 90]), (20, [2100, 130, 700, 40], [130, 640, 500, 1])])
+@pytest.mark.parametrize("beyond", [1, 4000])
+def test_a_limit_given_as_the_longest_entry(S, H, before, new, beyond):
+    """a number that no entry can have is as good as none: the same kernels, so the same bits, single tokens behind the portions' tiles and ahead of them"""
+    g = torch.Generator().manual_seed(H + beyond)
+    d, PR = 128, 64
+    o = options("plain", H, d, g)
+    k, v, kp, vp, table = sequences(g, [a + b for a, b in zip(before, new)], H, 1, d, d, PR)
+    q = torch.cat([torch.randn(n, H, 1, d, generator=g).bfloat16() for n in new])
+    slot = [b for b in range(len(new)) for _ in range(new[b])]
+    pos = [before[b] + i for b in range(len(new)) for i in range(new[b])]
+    unknown, limit = (run(S, q.cuda(), kp, vp, table, PR, slot, pos, o, longest) for longest in (0, len(pos) + beyond))
+    assert torch.equal(unknown, limit)
+    at = 0
+    for b in range(len(new)):
+        want = reference(q[at:at + new[b]].double(), k[b], v[b], list(range(before[b], before[b] + new[b])), o)
+        assert float((limit[at:at + new[b]] - want).norm() / want.norm()) < 3e-5, b   # (the bound of fp32 outputs of portions)
+        at += new[b]
