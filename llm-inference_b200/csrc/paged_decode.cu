@@ -3,7 +3,8 @@
 //
 // What bounds it: the keys and values, read once (8 KB per 16 keys of 128 x 128), so the kernel has to keep enough of them on their way
 // and spend few instructions per byte. A warp walks its own run of keys, 16 at a time, out of a ring of its own in shared memory that
-// one lane fills three steps ahead by TMA (24 KB per warp, two CTAs of four warps per SM; keys are asked for again as soon as the scores are formed), and never waits for another warp:
+// one lane fills three steps ahead by TMA (24 KB per warp, two CTAs of four warps per SM; keys are asked for again as soon as the scores are formed; heads of 64 / 64: four CTAs, by
+// cp.async), and never waits for another warp:
 //   S^T = K Q^T   mma.sync m16n8k16, keys on the M axis, the R <= 8 query heads of the key head on the N axis
 //   softmax       fp32 in registers, a running (maximum, denominator) per warp; cap, bias, temperature and masks as in the row kernel
 //   O^T = V^T P^T value dimensions on the M axis (ldmatrix.trans). The weights keep 24 bits: p = hi + mid + lo (three bfloat16, the
@@ -33,11 +34,14 @@ namespace cg = cooperative_groups;
 constexpr int kPdWarps = 4, kPdStep = 16, kPdHeads = 8, kPdMaxCluster = 8;
 
 template <int D, int VD>
-struct PdRing {   // a step's keys, then its values, as TMA brings them: boxes of 16 rows x 64 columns, swizzled over 128 bytes
+struct PdRing {   // a step's keys, then its values: boxes of 16 rows x 64 columns, swizzled over 128 bytes as TMA does
     static constexpr int kStages = VD > 128 ? 2 : 3, kBox = kPdStep * 128;
     static constexpr int kK = D / 64 * kBox, kStep = kK + VD / 64 * kBox, kWarp = kStages * kStep;
     static constexpr int kBytes = kPdWarps * kWarp + 1024;
-    static constexpr int kPerSm = 2;
+    static constexpr int kPerSm = D + VD <= 128 ? 4 : 2;
+    // Heads of 64 / 64 leave room for four CTAs per SM. With more than two there, boxes by TMA come at less than half the rate of copies by cp.async (16 query / 8 key heads, us by
+    // TMA / by cp.async: 22 sequences of up to 2000 keys 38 / 20.6, 40 53 / 34, 64 76 / 42, two shares each; at one share with 100 KB of shared memory, so that two fit, 40 take 46), so those keep cp.async
+    static constexpr bool kTma = D + VD > 128;
 };
 
 __device__ __forceinline__ uint32_t pd_transpose(uint32_t v) {   // 8 x 8 tile of 16-bit numbers, a pair per thread
@@ -70,13 +74,15 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     volatile int* dead = &pd_dead;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32, gid = lane >> 2, tig = lane & 3;
     uint64_t *k_full = pd_bars + warp * 2 * NS, *v_full = k_full + NS;   // of this warp's ring
-    if (lane == 0) {
+    if (L::kTma) {
+        if (lane == 0) {
 #pragma unroll
-        for (int i = 0; i < 2 * NS; ++i) mbar_init(&k_full[i], 1);
-        mbar_fence_init();
-        if (warp == 0) { *dead = 0; tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
+            for (int i = 0; i < 2 * NS; ++i) mbar_init(&k_full[i], 1);
+            mbar_fence_init();
+            if (warp == 0) { *dead = 0; tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v); }
+        }
+        __syncthreads();
     }
-    __syncthreads();
     if (!MIXED || ahead) pdl_wait();
     pdl_launch_dependents();
     const int R = a.heads / a.kv_heads, splits = gridDim.x;
@@ -94,6 +100,20 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         v_at[i] = ring + (uint32_t)(L::kK + ((lane & 7) + (lane >> 4) * 8) * 128 + (((2 * i + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
     }
     uint32_t stage = 0, parity = 0;   // of the step that is worked on
+    // by cp.async: this lane brings 16 bytes of rows lane / 8, lane / 8 + 4, ... of a step
+    auto copy_rows = [&](uint32_t to, const void* pool, size_t row, size_t row_width, int column) {
+        const int c = lane & 7;
+        const bf* from = reinterpret_cast<const bf*>(pool) + row * row_width + column + c * 8;
+#pragma unroll
+        for (int i = 0; i < kPdStep / 4; ++i) {
+            const int r = 4 * i + (lane >> 3);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4))), "l"(from + r * row_width) : "memory");
+        }
+    };
+    auto close_group = [&]() {
+        __syncwarp();   // the lanes close their group of copies together
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     // this thread's two heads (columns of S^T and O^T)
     float sc[2], hb[2];
     const float over_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
@@ -141,7 +161,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             int row = 0;   // pool row of the step whose keys were asked for last
             auto fetch_k = [&](uint32_t st) {   // the keys of the next step into stage st (rows that the token does not see may hold anything)
                 row = page * a.page_rows + off;
-                if (lane == 0) {
+                if (!L::kTma) {
+                    copy_rows(ring + st * L::kStep, a.k_pool, row, (size_t)a.kv_heads * a.maps * D, ku * D);
+                } else if (lane == 0) {
                     mbar_expect_tx(&k_full[st], L::kK);
 #pragma unroll
                     for (int c = 0; c < D / 64; ++c) tma_load_2d(pd_sm + warp * L::kWarp + st * L::kStep + c * L::kBox, &map_k, ku * D + c * 64, row, &k_full[st]);
@@ -149,7 +171,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 __syncwarp();
             };
             auto fetch_v = [&](uint32_t st, int s) {   // and its values; the page of the step after is looked up
-                if (lane == 0) {
+                if (!L::kTma) {
+                    copy_rows(ring + st * L::kStep + L::kK, a.v_pool, row, (size_t)a.kv_heads * VD, g * VD);
+                } else if (lane == 0) {
                     mbar_expect_tx(&v_full[st], L::kStep - L::kK);
 #pragma unroll
                     for (int c = 0; c < VD / 64; ++c) tma_load_2d(pd_sm + warp * L::kWarp + st * L::kStep + L::kK + c * L::kBox, &map_v, g * VD + c * 64, row, &v_full[st]);
@@ -162,10 +186,20 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 uint32_t st = stage;
 #pragma unroll
                 for (int i = 0; i < NS; ++i) {
-                    if (s0 + i < s1) { fetch_k(st); fetch_v(st, s0 + i); }
+                    if (s0 + i < s1) fetch_k(st);
+                    if (!L::kTma) close_group();
+                    if (s0 + i < s1) fetch_v(st, s0 + i);
+                    if (!L::kTma) close_group();
                     st = st + 1 == NS ? 0 : st + 1;
                 }
             }
+            auto arrived = [&](uint64_t* bar) {   // by cp.async: a group of keys and one of values per step, the rest of the ring behind them
+                if (L::kTma) mbar_wait_or_leave(bar, parity, dead);
+                else {
+                    asm volatile("cp.async.wait_group %0;" ::"n"(2 * NS - 1) : "memory");
+                    __syncwarp();   // for every lane
+                }
+            };
             for (int s = s0; s < s1; ++s, j0 += kPdStep) {
                 const bool whole = j0 >= j_lo && j0 + kPdStep - 1 <= p;
                 const uint32_t at = stage * L::kStep;
@@ -179,7 +213,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                         for (int e = 0; e < 4; ++e) bv[e] = bias[e & 1][min(max(p - (j0 + gid + (e >> 1) * 8), 0), a.dist_n - 1)];
                     }
                 }
-                mbar_wait_or_leave(&k_full[stage], parity, dead);
+                arrived(&k_full[stage]);
                 float st[4] = {0.f, 0.f, 0.f, 0.f}, su[4] = {0.f, 0.f, 0.f, 0.f};   // two chains of products
 #pragma unroll
                 for (int ks = 0; ks < KS; ks += 2) {
@@ -193,6 +227,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 for (int e = 0; e < 4; ++e) st[e] = (st[e] + su[e]) * sc[e & 1];
                 __syncwarp();   // every lane has read the keys: their place may be filled again
                 if (s + NS < s1) fetch_k(stage);
+                if (!L::kTma) close_group();
                 bool seen[4] = {true, true, true, true};   // key j0 + gid (+ 8), head 2 tig (+ 1)
                 if (!whole) {
 #pragma unroll
@@ -259,13 +294,13 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                         pr[2 * hf + 1] -= f.y;
                         b[q][hf] = pd_transpose(*reinterpret_cast<const uint32_t*>(&h2));
                     }
-                mbar_wait_or_leave(&v_full[stage], parity, dead);
+                arrived(&v_full[stage]);
                 if (!whole) {   // values of keys that the token does not see: 0 * NaN must stay 0
                     for (int i = lane; i < kPdStep * (VD / 8); i += 32) {
                         const int r = i / (VD / 8), c = i % (VD / 8);
                         if (j0 + r < j_lo || j0 + r > p) st_shared_v4(ring + at + (uint32_t)(L::kK + (c / 8) * L::kBox + r * 128 + (c & 7) * 16), 0u, 0u, 0u, 0u);
                     }
-                    fence_proxy_async_smem();
+                    if (L::kTma) fence_proxy_async_smem();
                     __syncwarp();
                 }
 #pragma unroll
@@ -285,9 +320,11 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 }
                 __syncwarp();   // and the values
                 if (s + NS < s1) fetch_v(stage, s + NS);
+                if (!L::kTma) close_group();
                 if (++stage == NS) { stage = 0; parity ^= 1u; }
             }
-            const bool gave_up = *dead != 0;
+            if (!L::kTma) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            const bool gave_up = L::kTma && *dead != 0;
             if (gave_up) {   // nothing may land behind this CTA's end, or on the sums
 #pragma unroll
                 for (int i = 0; i < 2 * NS; ++i) { mbar_wait_limited(&k_full[i], 0); mbar_wait_limited(&k_full[i], 1); }
@@ -358,7 +395,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                     }
                 pa_store<bf>(a, ((size_t)t * q_units + (size_t)qh * a.maps + mp) * VD + i % VD, acc / L);
             }
-            fence_proxy_async_smem();   // TMA writes where the sums lay
+            if (L::kTma) fence_proxy_async_smem();   // TMA writes where the sums lay
             cluster.sync();   // nobody leaves (or starts its next token) while its shared memory is read
         }
         if (!MIXED) break;
@@ -370,9 +407,9 @@ template <int D, int VD, bool MIXED>
 static int launch_paged_decode(const PA& a, int splits, int rows, bool ahead, cudaStream_t s) {
     constexpr int smem = PdRing<D, VD>::kBytes;
     static_assert(kPdWarps * kPdHeads * VD * 4 <= smem, "the warps' sums take the rings' place");
-    CUtensorMap mk, mv;
+    CUtensorMap mk{}, mv{};
     constexpr long long kAnyRow = (1ll << 31) - 1;   // the pool's height is not part of the call: any row that an int can name
-    if (!make_tma_map_2d(&mk, a.k_pool, kAnyRow, a.kv_heads * a.maps * D, kPdStep) || !make_tma_map_2d(&mv, a.v_pool, kAnyRow, a.kv_heads * VD, kPdStep)) return -1;
+    if (PdRing<D, VD>::kTma && (!make_tma_map_2d(&mk, a.k_pool, kAnyRow, a.kv_heads * a.maps * D, kPdStep) || !make_tma_map_2d(&mv, a.v_pool, kAnyRow, a.kv_heads * VD, kPdStep))) return -1;
     static unsigned long long done = 0;
     cudaError_t e = ensure_max_dynamic_smem((const void*)paged_decode_kernel<D, VD, MIXED>, smem, done);
     if (e != cudaSuccess) return (int)e;
@@ -429,8 +466,13 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, boo
         splits = 2;
         while (splits < (likely <= 8 ? kPdMaxCluster : 4) && likely * splits * 2 <= room) splits *= 2;
         while (splits > 1 && longest_seen > 0 && splits / 2 * kPdWarps * kPdStep >= longest_seen) splits /= 2;
-    } else
-        while (splits < kPdMaxCluster && pairs * splits <= sms && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+    } else {
+        // heads of 64 / 64, four CTAs per SM: three CTAs for every two SMs (us at 1 / 2 / 4 / 8 shares: 8 sequences of up to 2000 keys 25.3 / 15.1 / 11.7 / 10.6, 12 25.3 / 16.6 / 13.7 / 17.6,
+        // 19 28.1 / 19.8 / 20.7 / 25.3, 28 28.5 / 21.5 / 24.3 / 33.4, 40 38.3 / 34.3 / 35.8 / 46.5, 64 43.2 / 42.0 / 49.1 / 69.4; all of 2000: 40 40.7 / 47.1 / 43.2 / 52.2)
+        const bool narrow = a.dim == 64 && a.vdim == 64;
+        auto room_for_twice = [&] { return narrow ? 2 * pairs * splits < 3ll * sms : pairs * splits <= sms; };
+        while (splits < kPdMaxCluster && room_for_twice() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+    }
     return mixed ? paged_decode_for<true>(a, splits, rows, ahead, s) : paged_decode_for<false>(a, splits, rows, false, s);
 }
 

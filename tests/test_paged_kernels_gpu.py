@@ -310,3 +310,19 @@ def test_a_limit_given_as_the_longest_entry(S, H, before, new, beyond):
         want = reference(q[at:at + new[b]].double(), k[b], v[b], list(range(before[b], before[b] + new[b])), o)
         assert float((limit[at:at + new[b]] - want).norm() / want.norm()) < 3e-5, b   # (the bound of fp32 outputs of portions)
         at += new[b]
+
+
+@pytest.mark.parametrize("form", ["plain", "biased", "sigmoid"])
+@pytest.mark.parametrize("T,PR", [(1, 16), (9, 80), (25, 64), (40, 16)])
+def test_single_tokens_of_narrow_heads(S, form, T, PR):
+    """heads of 64 / 64, whose rows come by copies of 16 bytes: eight shares of a context to one, runs of steps shorter and longer than the ring, up to four CTAs per SM, contexts that begin
+    and end inside a step. The bound of test_single_tokens_share_their_context_in_a_cluster"""
+    g = torch.Generator().manual_seed(T + PR)
+    H, d, n = 8, 64, 1101
+    o = options(form, H, d, g)
+    k, v, kp, vp, table = sequences(g, [n], H, 1, d, d, PR)
+    q = torch.randn(T, H, 1, d, generator=g).bfloat16().double()
+    pos = [n - 1 - 27 * i for i in range(T)]
+    got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * T, pos, o, 1)
+    want = reference(q, k[0], v[0], pos, o)
+    assert float((got - want).norm() / want.norm()) < 2e-5
