@@ -400,7 +400,10 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
         if (!MIXED) break;
     }
-    if (MIXED && !ahead) pdl_wait();   // the prompt portions' kernel runs beside this one: done only when both are (ahead of it: it waits)
+    // the prompt portions' kernel runs beside this one: done only when both are (ahead of it: it waits). One CTA to wait is enough: clusters without a token, which are most of them,
+    // make room for those behind them (us with all of them waiting / with one, 8 / 4 heads x 128 and blocks of 1024: two portions
+    // of up to 66 behind up to 3319 and 6 single tokens 20.4 / 12.3; 16 / 8: three of up to 40 alone 8.5 / 8.1, one of 512 behind 4000 and 8 single tokens 75 / 56)
+    if (MIXED && !ahead && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
 }
 
 template <int D, int VD, bool MIXED>
