@@ -68,7 +68,7 @@ __device__ __forceinline__ uint32_t pa_pack(float lo, float hi) {
 int biased_tile(const PA& a, cudaStream_t s);
 // bfloat16 single tokens, a cluster per (token, key head) (paged_decode.cu); -1: not built for these sizes
 // singles: 0, every token is; else only the tokens that are their sequence's only one in the batch, which are not more than this
-int paged_decode(const PA& a, int longest_seen, int singles, long long room, bool ahead, cudaStream_t s);
+int paged_decode(const PA& a, int longest_seen, int singles, long long room, cudaStream_t s);
 // bfloat16 prompt portions on tcgen05 tiles (paged_attention_tc.cu); -1: not built for these sizes
 int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStream_t s);
 // b200_paged_attention with weights mixed across heads (mixed_attention.cu); a.head_mix is set

@@ -8,7 +8,7 @@
 //   rows        TQ tokens x the R query heads of one key head (TQ = 128 / R), so a key tile is read once for the whole group and a
 //               causal edge wastes little. A CTA's window of TQ packed rows may hold the end of one sequence and the start of
 //               the next: they are separate tiles, walked by neighbouring CTAs (gridDim.y is doubled, or for small batches made four times as large, when there is more than one entry; most of the others
-//               find no tile and leave). Sequences that bring a single token are left to the cluster kernel of paged_decode.cu, launched behind this one or ahead of it.
+//               find no tile and leave). Sequences that bring a single token are left to the cluster kernel of paged_decode.cu, launched behind this one.
 //   warp 0      TMA: K and V tiles of 64 rows out of their page (one list lookup per tile), a ring as long as the score buffers
 //   warp 1      tcgen05.mma: S = Q K^T (one group: the weighted sums too, the next tile's scores ahead of them)
 //   softmax     four warps per group, a thread per row: scores are read from TMEM once, P_j goes back over its own scores and is the A operand of the second
@@ -76,7 +76,7 @@ __device__ __forceinline__ float2 ld_cluster_v2(uint32_t addr) {
 
 template <int D, int DV, int W, int FORM, bool SHARED>
 __global__ void __launch_bounds__(TcSmem<D, DV, W>::kThreads, TcSmem<D, DV, W>::kPerSm)
-paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int TQ, int parts, int skip_singles, int sorted, int behind, int split2) {   // split2: log2 of the CTAs that share a tile's keys
+paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int TQ, int parts, int skip_singles, int sorted, int split2) {   // split2: log2 of the CTAs that share a tile's keys
     using bf = __nv_bfloat16;
     using L = TcSmem<D, DV, W>;
     constexpr int NB = L::kRing, NT = L::kThreads;
@@ -94,9 +94,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform as the compiler sees it)
     const int split = 1 << split2, rank = SHARED ? (int)blockIdx.x & (split - 1) : 0, ku = SHARED ? (int)blockIdx.x >> split2 : (int)blockIdx.x, g = ku / a.maps, mp = ku % a.maps, R = a.heads / a.kv_heads, q_units = a.heads * a.maps;
-    // behind the kernel of the single tokens, which runs beside this one: done only when both are, and one CTA to wait is enough
-    const bool last_out = behind && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1;
-    // ---- TMEM and barriers, while the kernel before this one ends (the single tokens' kernel has waited for what this one reads)
+    // ---- TMEM and barriers, while the kernel before this one ends
     const bool early = parts != 2;   // every CTA has a tile, or all start at once
     if (warp == 1 && early) tmem_alloc(tmem_slot, L::kTmemCols);
     if (threadIdx.x == 0) {
@@ -107,7 +105,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         tma_prefetch_desc(&map_v);
         *dead = 0;
     }
-    if (!behind) pdl_wait();
+    pdl_wait();
 
     // the windows that see the most keys come first: of one prompt the last rows, of several entries by what their first and last rows see
     const int yy = gridDim.y - 1 - blockIdx.y, part = yy % parts;
@@ -154,7 +152,6 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         for (int i = 4; i < 8; ++i) n_tiles += __popc(masks[i]);
         if (n_tiles <= part) {
             if (warp == 1 && early) tmem_dealloc(__shfl_sync(0xffffffffu, *tmem_slot, 0), L::kTmemCols);
-            if (last_out) pdl_wait();
             return;
         }
         if (warp == 1 && !early) tmem_alloc(tmem_slot, L::kTmemCols);
@@ -630,12 +627,11 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         __syncthreads();
     }
     if (warp == 1) tmem_dealloc(tmem, L::kTmemCols);
-    if (last_out) pdl_wait();
 }
 
 struct TcPlan {
     long long windows;
-    int parts, sorted, behind, split2, bias;   // split2: log2 of the CTAs that share a tile's keys; bias: staged numbers
+    int parts, sorted, split2, bias;   // split2: log2 of the CTAs that share a tile's keys; bias: staged numbers
     bool two_groups;
 };
 
@@ -667,7 +663,7 @@ static int launch_tc(const PA& a, const TcPlan& p, cudaStream_t s) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    e = cudaLaunchKernelEx(&cfg, paged_attn_tc_kernel<D, DV, W, FORM, SHARED>, mk, mv, a, TQ, p.parts, p.parts - 1, p.sorted, p.behind, p.split2);
+    e = cudaLaunchKernelEx(&cfg, paged_attn_tc_kernel<D, DV, W, FORM, SHARED>, mk, mv, a, TQ, p.parts, p.parts - 1, p.sorted, p.split2);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -724,23 +720,13 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && p.two_groups;
     const int singles = a.n_tokens - longest_entry;   // at most; with several entries at least one
     const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));   // CTAs of single tokens that fit beside the tiles'
-    // Single tokens go beside the tiles where there is room for eight of them. Where the tiles fill the GPU for long they go ahead instead, two CTAs per SM on the SMs that they need, and the tiles take what they
-    // leave: behind them they waited for the first round to end (us, behind / ahead of the tiles, 16 / 8 heads x 128: 12 single tokens and three portions of up to 512 behind 4000, capped, 118 / 107, plain
-    // behind 2000 70.7 / 61.4, 8 and two of 512 88.6 / 83.0, 1 and two of 400 behind 3000 68.7 / 46.0, no single token and three of 512 82.9 / 83.8)
-    p.behind = several && p.two_groups && steps > 32 && (p.sorted || free < 2ll * std::min(singles, 8) * units);
-    if (p.behind) {
-        const int rc = paged_decode(a, longest_seen, singles, 0, true, s);
-        if (rc != 0) return rc;
-    }
     int rc = -1;
     if (a.dim == 128 && a.vdim == 128) rc = launch_tc_for<128, 128>(a, p, s);
     else if (a.dim == 64 && a.vdim == 64) rc = launch_tc_for<64, 64>(a, p, s);
     else if (a.dim == 128 && a.vdim == 256) rc = launch_tc_for<128, 256>(a, p, s);
     if (rc != 0) return rc;
     count_launch();
-    if (several && !p.behind) {   // the sequences that bring one token, on what the tiles leave free
-        return paged_decode(a, longest_seen, singles, free, false, s);
-    }
+    if (several) return paged_decode(a, longest_seen, singles, free, s);   // the sequences that bring one token, on what the tiles leave free
     return 0;
 }
 

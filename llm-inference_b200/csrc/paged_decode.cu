@@ -61,7 +61,7 @@ __device__ __forceinline__ void pd_ldsm_x4_trans(uint32_t (&r)[4], uint32_t a) {
 // those that are their sequence's only token in the batch.
 template <int D, int VD, bool MIXED>
 __global__ void __launch_bounds__(kPdWarps * 32, PdRing<D, VD>::kPerSm)
-paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a, int ahead) {
+paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PA a) {
     using bf = __nv_bfloat16;
     using L = PdRing<D, VD>;
     constexpr int KS = D / 16;        // k steps of the scores
@@ -83,7 +83,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
         __syncthreads();
     }
-    if (!MIXED || ahead) pdl_wait();
+    if (!MIXED) pdl_wait();
     pdl_launch_dependents();
     const int R = a.heads / a.kv_heads, splits = gridDim.x;
     float* om = reinterpret_cast<float*>(pd_sm);                                 // once the rings have been used: [warps][R][VD], then this CTA's share in the first [R][VD]
@@ -400,14 +400,14 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
         }
         if (!MIXED) break;
     }
-    // the prompt portions' kernel runs beside this one: done only when both are (ahead of it: it waits). One CTA to wait is enough: clusters without a token, which are most of them,
+    // the prompt portions' kernel runs beside this one: done only when both are. One CTA to wait is enough: clusters without a token, which are most of them,
     // make room for those behind them (us with all of them waiting / with one, 8 / 4 heads x 128 and blocks of 1024: two portions
     // of up to 66 behind up to 3319 and 6 single tokens 20.4 / 12.3; 16 / 8: three of up to 40 alone 8.5 / 8.1, one of 512 behind 4000 and 8 single tokens 75 / 56)
-    if (MIXED && !ahead && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
+    if (MIXED && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
 }
 
 template <int D, int VD, bool MIXED>
-static int launch_paged_decode(const PA& a, int splits, int rows, bool ahead, cudaStream_t s) {
+static int launch_paged_decode(const PA& a, int splits, int rows, cudaStream_t s) {
     constexpr int smem = PdRing<D, VD>::kBytes;
     static_assert(kPdWarps * kPdHeads * VD * 4 <= smem, "the warps' sums take the rings' place");
     CUtensorMap mk{}, mv{};
@@ -432,22 +432,22 @@ static int launch_paged_decode(const PA& a, int splits, int rows, bool ahead, cu
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;
     }
-    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, mk, mv, a, ahead ? 1 : 0);
+    e = cudaLaunchKernelEx(&cfg, paged_decode_kernel<D, VD, MIXED>, mk, mv, a);
     if (e != cudaSuccess) return (int)e;
     count_launch();
     return (int)cudaGetLastError();
 }
 
 template <bool MIXED>
-static int paged_decode_for(const PA& a, int splits, int rows, bool ahead, cudaStream_t s) {
-    if (a.dim == 128 && a.vdim == 128) return launch_paged_decode<128, 128, MIXED>(a, splits, rows, ahead, s);
-    if (a.dim == 64 && a.vdim == 64) return launch_paged_decode<64, 64, MIXED>(a, splits, rows, ahead, s);
-    if (a.dim == 128 && a.vdim == 256) return launch_paged_decode<128, 256, MIXED>(a, splits, rows, ahead, s);
-    if (a.dim == 64 && a.vdim == 128) return launch_paged_decode<64, 128, MIXED>(a, splits, rows, ahead, s);
+static int paged_decode_for(const PA& a, int splits, int rows, cudaStream_t s) {
+    if (a.dim == 128 && a.vdim == 128) return launch_paged_decode<128, 128, MIXED>(a, splits, rows, s);
+    if (a.dim == 64 && a.vdim == 64) return launch_paged_decode<64, 64, MIXED>(a, splits, rows, s);
+    if (a.dim == 128 && a.vdim == 256) return launch_paged_decode<128, 256, MIXED>(a, splits, rows, s);
+    if (a.dim == 64 && a.vdim == 128) return launch_paged_decode<64, 128, MIXED>(a, splits, rows, s);
     return -1;
 }
 
-int paged_decode(const PA& a, int longest_seen, int singles, long long room, bool ahead, cudaStream_t s) {
+int paged_decode(const PA& a, int longest_seen, int singles, long long room, cudaStream_t s) {
     const bool mixed = singles > 0;
     if (a.heads / a.kv_heads > kPdHeads || a.page_rows % kPdStep || a.kv_heads * a.maps > 65535) return -1;
     // how many tokens of a mixed batch are single ones is only known on the device: sixteen rows of clusters share them
@@ -459,9 +459,7 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, boo
     const long long pairs = (long long)rows * a.kv_heads * a.maps;
     const int sms = sm_count();
     int splits = 1;
-    if (ahead) {   // the portions' CTAs start when the last of these has: one round
-        while (splits < kPdMaxCluster && pairs * splits <= sms && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
-    } else if (mixed) {
+    if (mixed) {
         // on what the portions' CTAs leave free (`room` CTAs) if eight single tokens can sit there beside each other, else behind them (us at 2 / 4 / 8 shares: 8 single tokens and a portion of 512 behind
         // 4000 57.2 / 77.7 / 83.0, 4 and 64 36.8 / 31.7 / 40.9, 12 and three of 512, which fill the GPU, 123 / 119 / 133)
         const long long likely = (long long)std::min(singles, 8) * a.kv_heads * a.maps;
@@ -476,7 +474,7 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, boo
         auto room_for_twice = [&] { return narrow ? 2 * pairs * splits < 3ll * sms : pairs * splits <= sms; };
         while (splits < kPdMaxCluster && room_for_twice() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
     }
-    return mixed ? paged_decode_for<true>(a, splits, rows, ahead, s) : paged_decode_for<false>(a, splits, rows, false, s);
+    return mixed ? paged_decode_for<true>(a, splits, rows, s) : paged_decode_for<false>(a, splits, rows, s);
 }
 
 }  // namespace b200
