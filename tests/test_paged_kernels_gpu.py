@@ -326,3 +326,40 @@ def test_single_tokens_of_narrow_heads(S, form, T, PR):
     got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * T, pos, o, 1)
     want = reference(q, k[0], v[0], pos, o)
     assert float((got - want).norm() / want.norm()) < 2e-5
+
+
+@pytest.mark.parametrize("H,before,new", [(4, [250, 63, 10, 0], [1, 65, 1, 90]), (16, [2100, 130, 700, 40, 1900], [130, 400, 1, 1, 1]), (8, [700, 2000, 40], [1, 1, 1]), (8, [300], [500])])
+def test_inputs_rewritten_by_the_kernels_ahead(S, H, before, new):
+    """queries and keys are rewritten by the library's own kernels, launched programmatically directly ahead of each call, several times in one stream: the bits of the same calls with the
+    GPU waited for in between. A kernel that read ahead of what it depends on, or lines that it still held, would show"""
+    g = torch.Generator().manual_seed(H + len(new))
+    d, PR, rounds = 128, 64, 6
+    lib, T = S.lib(), sum(new)
+    k, v, kp, vp, table = sequences(g, [a + b for a, b in zip(before, new)], H, 1, d, d, PR)
+    vp.nan_to_num_(0.0)
+    slot = torch.tensor([b for b in range(len(new)) for _ in range(new[b])], dtype=torch.int32).cuda()
+    pos = torch.tensor([before[b] + i for b in range(len(new)) for i in range(new[b])], dtype=torch.int32).cuda()
+    W, rows, q = H * d, kp.shape[0], torch.empty(T, H * d, dtype=torch.bfloat16, device="cuda")
+    one, zero = torch.ones(W, device="cuda"), torch.zeros(W, device="cuda")
+    src = [[torch.randn(n, W, generator=g).cuda() for n in (T, rows)] for _ in range(rounds)]
+    outs = [[torch.zeros(T, W, dtype=torch.float32, device="cuda") for _ in range(rounds)] for _ in range(2)]
+    a = S.PagedAttentionArgs()
+    a.q, a.k_pool, a.v_pool, a.pages, a.max_pages, a.page_rows = q.data_ptr(), kp.data_ptr(), vp.data_ptr(), table.data_ptr(), table.shape[1], PR
+    a.slot, a.pos, a.n_tokens, a.heads, a.kv_heads, a.dim, a.vdim, a.scale = slot.data_ptr(), pos.data_ptr(), T, H, H, d, d, d ** -0.5
+    a.dtype, a.longest_entry, a.longest_context, a.out_f32 = S.BF16, max(new), max(x + y for x, y in zip(before, new)), 1
+    for waited in (0, 1):
+        work = [[t.clone() for t in s] for s in src]   # (the norm adds to its input in place)
+        torch.cuda.synchronize()
+        for i in range(rounds):
+            for x, n, to in ((work[i][0], T, q), (work[i][1], rows, kp)):
+                assert lib.b200_layernorm_residual(x.data_ptr(), src[i][0 if n == T else 1].data_ptr(), n, W, 1e-5, 0.5, one.data_ptr(), zero.data_ptr(), one.data_ptr(), zero.data_ptr(), to.data_ptr(), S.BF16, None) == 0
+                if waited:
+                    torch.cuda.synchronize()
+            a.out = outs[waited][i].data_ptr()
+            assert lib.b200_paged_attention(C.byref(a), None) == 0
+            if waited:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+    for i in range(rounds):
+        assert torch.equal(outs[0][i], outs[1][i]), i
+        assert bool(outs[0][i].isfinite().all()) and (i == 0 or not torch.equal(outs[0][i], outs[0][i - 1])), i
