@@ -476,6 +476,10 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, cud
         const bool narrow = a.dim == 64 && a.vdim == 64;
         auto room_for_twice = [&] { return narrow ? 2 * pairs * splits < 3ll * sms : pairs * splits <= sms; };
         while (splits < kPdMaxCluster && room_for_twice() && (longest_seen <= 0 || splits * kPdWarps * kPdStep < longest_seen)) splits *= 2;
+        // just beyond one CTA per SM one share leaves nearly half of the places empty: long contexts in three, a round and a half (16 heads x 128, up to 2000 keys, us at 1 / 2 / 3 shares: 38 sequences and
+        // 4 key heads 37.9 / 29.2 / 33.2, 19 and 8 37.6 / 34.1 / 32.7, 22 37.2 / 35.7 / 34.0, 10 and 16 36.5 / 31.5 / 30.4; all of 2000 39.8 / 47.1 / 40.9, 39.0 / 43.9 / 39.1, 40.4 / 48.6 / 41.2, 38.4 / 44.6 / 38.8;
+        // 23 and 8 36.6 / 35.7 / 34.4, all of 2000 39.5 / 49.3 / 42.5; all of 1200 26.4 / 28.5 / 26.3 at 19, 27.0 / 32.8 / 29.6 at 22)
+        if (!narrow && splits == 1 && pairs > sms && 4 * pairs <= 5 * sms && longest_seen > 1000) splits = 3;
     }
     return mixed ? paged_decode_for<true>(a, splits, rows, s) : paged_decode_for<false>(a, splits, rows, s);
 }

@@ -363,3 +363,18 @@ def test_inputs_rewritten_by_the_kernels_ahead(S, H, before, new):
     for i in range(rounds):
         assert torch.equal(outs[0][i], outs[1][i]), i
         assert bool(outs[0][i].isfinite().all()) and (i == 0 or not torch.equal(outs[0][i], outs[0][i - 1])), i
+
+
+@pytest.mark.parametrize("H,d,dv", [(8, 128, 128), (8, 64, 128), (8, 128, 256)])
+def test_three_shares_of_a_context(S, H, d, dv):
+    """just more (token, key head) pairs than SMs behind more than 1200 keys: clusters of three, whose parts of the outputs do not come out even. The bound of
+    test_single_tokens_share_their_context_in_a_cluster"""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator().manual_seed(d + dv)
+    T, n, PR, o = sms // H + 1, 1301, 64, options("plain", H, d, g)
+    k, v, kp, vp, table = sequences(g, [n], H, 1, d, dv, PR)
+    q = torch.randn(T, H, 1, d, generator=g).bfloat16().double()
+    pos = [n - 1 - 61 * i for i in range(T)]
+    got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * T, pos, o, 1)
+    want = reference(q, k[0], v[0], pos, o)
+    assert float((got - want).norm() / want.norm()) < 2e-5
