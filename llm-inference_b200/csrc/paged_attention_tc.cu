@@ -632,7 +632,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
 struct TcPlan {
     long long windows;
     int parts, sorted, split2, bias;   // split2: log2 of the CTAs that share a tile's keys; bias: staged numbers
-    bool two_groups;
+    bool two_groups;   // else one, and two CTAs per SM
 };
 
 template <int D, int DV, int W, int FORM, bool SHARED>
@@ -708,7 +708,9 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     const int steps = longest_seen > 0 ? (longest_seen + kTcKeys - 1) / kTcKeys : 0;
     // tiles of several entries that come in more than one round: up to 32 key tiles each, two CTAs per SM that hide each other's start and end are faster (16 / 8 heads x 128, us, one group / two: three
     // portions of up to 680 21.0 / 28.4, of up to 512 behind 300 26.8 / 33.3, behind 1000 43.1 / 48.2), beyond that the shorter chain (behind 2000 69.6 / 70.4, behind 4000, capped, 143 / 119)
-    p.two_groups = !(several && tiles > sms && steps <= 32);
+    // (values of 256 columns: one group, whose sums take an SM alone all the same)
+    const bool short_tiles = several && tiles > sms && steps <= 32;
+    p.two_groups = a.vdim > 128 || !short_tiles;
     // shared key tiles: while the clusters fit beside each other (clusters of four and eight do not fill every group of SMs), leave room for single tokens if there may be some, and keep eight key tiles or more
     // per CTA (us at 1 / 2 / 4 / 8 CTAs: 100 tokens behind 3000 38.6 / 26.6 / 19.0 / 28.8, 300 40.8 / 28.1 / 37.1 / 45.2, 64 and 4 single ones behind 1000 19.2 / 16.9 / 14.5 / 16.5, behind 300 11.9 / 13.0 / 12.7 / 14.7,
     // 512 and 8 single ones behind 4000 57.2 / 62.1 / 77.0 / 115)
@@ -717,7 +719,7 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     // CTAs that share a window's tiles: four where they all start at once (portions of 53, 45 and 33 tokens lie in one window and a bit: 16 heads x 128, capped, 12.6 / 9.9 us)
     if (several && p.split2 == 0 && tiles * 4 <= sms) p.parts = 4;
     // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 90.2 / 84.3 us)
-    p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && p.two_groups;
+    p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && !short_tiles;
     const int singles = a.n_tokens - longest_entry;   // at most; with several entries at least one
     const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));   // CTAs of single tokens that fit beside the tiles'
     int rc = -1;

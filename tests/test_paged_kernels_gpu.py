@@ -378,3 +378,21 @@ def test_three_shares_of_a_context(S, H, d, dv):
     got = run(S, q.bfloat16().cuda(), kp, vp, table, PR, [0] * T, pos, o, 1)
     want = reference(q, k[0], v[0], pos, o)
     assert float((got - want).norm() / want.norm()) < 2e-5
+
+
+@pytest.mark.parametrize("before", [[0, 130, 700, 40], [2100, 130, 700, 40]])
+def test_more_tiles_of_wide_values_than_the_gpu_holds_at_once(S, before):
+    """values of 256 columns, whose tiles take an SM alone: the bound of test_more_tiles_than_the_gpu_holds_at_once"""
+    g = torch.Generator().manual_seed(before[0] + 256)
+    H, d, new, PR = 20, 128, [130, 640, 500, 1], 64
+    o = options("capped", H, d, g)
+    k, v, kp, vp, table = sequences(g, [a + b for a, b in zip(before, new)], H, 1, d, 256, PR)
+    q = [torch.randn(n, H, 1, d, generator=g).bfloat16().double() for n in new]
+    slot = [b for b in range(4) for _ in range(new[b])]
+    pos = [before[b] + i for b in range(4) for i in range(new[b])]
+    got = run(S, torch.cat(q).bfloat16().cuda(), kp, vp, table, PR, slot, pos, o, max(new), f32=False)
+    at = 0
+    for b in range(4):
+        want = reference(q[b], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
+        assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 5e-3, b
+        at += new[b]
