@@ -28,7 +28,9 @@ constexpr int kGtM = 128, kGtK = 64, kGtThreads = 192;
 template <int BN, int PER_SM>   // rows of a block at most, CTAs per SM
 struct GtSmem {
     // The ring takes as many stages as the group's rows leave room for: the weights' 16 KB and 128 bytes per row (in sixteens) each
-    static constexpr int kMaxStages = 6, kTmemCols = BN > 128 ? 256 : BN;
+    // Blocks of 192 rows are for nearly two CTAs on every SM: more than 128 KB on their way to an SM are slower again (routed layers of 2048 -> 1024, 16 experts, four per row, us at up to 3 / 4 / 6 stages: 64
+    // rows 42.7 / 41.9 / 43.1, 100 44.9 / 44.4 / 45.9; 200, 50 rows a group, 48.2 / 48.9 / 49.2). Where fewer CTAs share an SM more stages pay (1024 -> 1536, two per row, 33 rows 30.0 / 28.6 / 28.1)
+    static constexpr int kMaxStages = BN > 128 ? 4 : 6, kTmemCols = BN > 128 ? 256 : BN;
     static constexpr int kRing = PER_SM == 3 ? 72 * 1024 : BN > 128 ? 108 * 1024 : 100 * 1024;
     static constexpr int kTotal = kRing + (2 * kMaxStages + 1) * 8 + 16 + 1024;
     static_assert(BN * kGtM * 4 <= kRing && kRing >= 2 * (kGtM + BN) * kGtK * 2, "the sums take the place of the stages; two stages at least");
@@ -53,7 +55,7 @@ __global__ void __launch_bounds__(kGtThreads, PER_SM) gemm_grouped_tc_kernel(con
     pdl_wait();
     const int z = blockIdx.y, row0 = g.group_off[z] + (int)blockIdx.z * BN, rows = min(BN, g.group_off[z + 1] - row0);
     if (rows <= 0) return;
-    const int stage_bytes = (int)A_BYTES + (rows + 15) / 16 * 16 * 128, stages = min(S::kMaxStages, S::kRing / stage_bytes);
+    const int stage_bytes = (int)A_BYTES + (rows + 15) / 16 * 16 * 128, stages = min(BN > 128 && rows > 48 ? 3 : S::kMaxStages, S::kRing / stage_bytes);
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
             mbar_init(&full_bar[s], 1 + 4);   // the weights, and the four warps that bring the rows
