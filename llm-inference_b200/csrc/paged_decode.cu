@@ -340,7 +340,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
                 l[x] += __shfl_xor_sync(0xffffffffu, l[x], 16);
                 const int h = 2 * tig + x;
                 if (h < R) {
-                    if (gid == 0) { ms[warp * R + h] = m[x]; ls[warp * R + h] = gave_up ? __int_as_float(0x7fffffff) : l[x]; }
+                    if (gid == 0) { ms[warp * R + h] = gave_up ? 0.f : m[x]; ls[warp * R + h] = gave_up ? __int_as_float(0x7fffffff) : l[x]; }   // (NaN at a finite reference: every merge takes it in)
                     float* dst = om + (size_t)(warp * R + h) * VD + gid;
 #pragma unroll
                     for (int j = 0; j < MT; ++j) {
