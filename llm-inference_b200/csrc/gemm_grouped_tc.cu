@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(kGtThreads, PER_SM) gemm_grouped_tc_kernel(con
         const int quarter = warp & 3;
         mbar_wait_or_leave(acc_full, 0, dead);
         const bool gone = *dead != 0;
+        if (gone) linger();   // a wait was given up: no late weights on the sums, or behind this CTA's end
         tc_fence_after();
         const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1

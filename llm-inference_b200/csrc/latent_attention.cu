@@ -675,7 +675,8 @@ __global__ void __launch_bounds__(256, 2) latent_decode_kernel(const __grid_cons
     if (!TMA) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     if (TMA && *dead) {   // a wait was given up: nothing may land on the sums, or behind this CTA's end
-        for (int i = 0; i < 2; ++i) { mbar_wait_limited(&full[i], 0); mbar_wait_limited(&full[i], 1); }
+        linger();
+        __syncthreads();
         l_run[0] = l_run[1] = __int_as_float(0x7fffffff);
     }
 #pragma unroll

@@ -387,6 +387,10 @@ __global__ void __launch_bounds__(kLtThreads, 1) latent_attn_tc_kernel(const __g
         __syncthreads();   // the next tile's query rows and products come after everybody is done with this one's
         tc_fence_after();
     }
+    if (*dead) {   // a wait was given up: what is still under way must not land behind this CTA's end
+        linger();
+        __syncthreads();
+    }
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 

@@ -621,9 +621,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         tc_fence_after();
     }
     if (*dead) {   // a wait was given up: what is still under way must not land behind this CTA's end
-        if (warp == 0)
-            for (int i = 0; i < 5 * NB; ++i)
-                if (i / NB != 3) { mbar_wait_limited(&bars[i], 0); mbar_wait_limited(&bars[i], 1); }   // (weights are not copies)
+        linger();
         __syncthreads();
     }
     if (warp == 1) tmem_dealloc(tmem, L::kTmemCols);

@@ -328,10 +328,7 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
             }
             if (!L::kTma) asm volatile("cp.async.wait_group 0;" ::: "memory");
             const bool gave_up = L::kTma && *dead != 0;
-            if (gave_up) {   // nothing may land behind this CTA's end, or on the sums
-#pragma unroll
-                for (int i = 0; i < 2 * NS; ++i) { mbar_wait_limited(&k_full[i], 0); mbar_wait_limited(&k_full[i], 1); }
-            }
+            if (gave_up) linger();   // nothing may land behind this CTA's end, or on the sums
             __syncthreads();    // the rings' place is taken by the sums
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
