@@ -277,3 +277,30 @@ def test_persistent_step_kernel_70b_geometry(pkg):
         eng.close()
         if comm:
             lib.b200_p2p_destroy(comm)
+
+
+def test_logits_are_aliases_of_one_tensor_over_the_engines_buffer(pkg):
+    """the tensor over the engine's logits is made once: an ordinary one, also when it is first asked for under inference mode; what a caller does to the shape of an alias stays there,
+    and closing the engine drops it (nothing reads the buffer after that)"""
+    E = pkg.engine
+    eng = E.Engine(2, 32, dtype=pkg.F16, **SMALL)
+    eng.init_random(seed=4, std=0.05)
+    eng.decode_step_host(np.array([1, 2], np.int32))
+    with torch.inference_mode():
+        first = eng.logits()
+    second = eng.logits()
+    shape = (2, SMALL["vocab_size"])
+    assert not first.is_inference() and tuple(first.shape) == tuple(second.shape) == shape and first.dtype == torch.float16
+    assert first is not second and first.data_ptr() == second.data_ptr()
+    w = torch.ones(shape, dtype=torch.float16, device="cuda", requires_grad=True)
+    (w * first).sum().backward()
+    torch.cuda.synchronize()
+    before = first.clone()
+    assert torch.equal(w.grad, before)
+    second.unsqueeze_(0)
+    eng.decode_step_host(None)
+    torch.cuda.synchronize()
+    third = eng.logits()
+    assert tuple(third.shape) == shape and torch.equal(first, third) and torch.equal(second[0], third) and not torch.equal(before, third)
+    eng.close()
+    assert eng._logits is None and eng.h is None
