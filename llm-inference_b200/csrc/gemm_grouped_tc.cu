@@ -4,7 +4,7 @@
 // (gated units: 64 gate rows and the 64 up rows of the same features) per CTA, and a group's rows ride along as the N extent, up to 128 or 192 of
 // them, in an instruction just wide enough. Weights come by TMA; the rows, which lie anywhere, by cp.async into the same swizzled layout
 // (warps 2-5, 16 bytes at a time, a few stages ahead). A stage takes the weights' 16 KB and what the block's rows need, so few rows get more stages. Two or three CTAs share an SM:
-// while one round of them holds all tiles the weights stream at the copy rate (a stage in 1270 clocks of two CTAs), and a second round of few blocks cost half as much again. The sums leave TMEM through shared memory,
+// a second round of few blocks, which read their weights again, cost half as much again as one round that holds all tiles (there the weights come at some 0.55 of the copy rate). The sums leave TMEM through shared memory,
 // so that a token's features are stored side by side and the epilogue sees one element like the other kernels of this entry point.
 //   grid: feature tiles x groups x blocks of rows; what lies behind a group's rows leaves at once
 // Measured (before: the mma.sync tiles of gemm_grouped.cu): 512 rows, four of 16 experts each, 2048 -> gated 1024 -> 2048, with dispatch and

@@ -1,8 +1,8 @@
 // bfloat16 prompt portions of b200_latent_attention_ex on tcgen05 / TMEM: 128 (token, head) rows per tile, cached rows 64 at a time, 256 output
 // columns per CTA (two CTAs form the 512 columns of a row, each with scores of its own: a whole row of sums would fill TMEM alone).
 //
-// What bounds it: per 128 x 64 scores over rows of 576 the tensor pipe needs 2500 clocks (nine chunks of 64 dimensions, 1470, then the weighted
-// sum over 256 columns, 1030), three times the softmax; so the next tile's scores run under the softmax of this one, and enough of the cached
+// What bounds it: per 128 x 64 scores over rows of 576 the tensor pipe is active for 2176 clocks (nine chunks of 64 dimensions, 1152, then the weighted
+// sum over 256 columns, 1024; with what lies between products 2500), three times the softmax; so the next tile's scores run under the softmax of this one, and enough of the cached
 // rows has to be on its way. Shared memory is what limits that: the query rows alone are 144 KB. Four of their chunks lie in TMEM as
 // first operands instead, beside the sums (256 columns) and two score buffers, which leaves room for 144 KB of cached rows:
 //   chunks of 64 dimensions that this CTA only scores with:  all of a row's at once (rows of 640: half of them), a ring of two such groups, given back after their products
@@ -13,8 +13,9 @@
 //   warp 6      tcgen05.mma: the weighted sums. (One warp for both, and a barrier per chunk, spent 3550 clocks a tile on waits, products and commits; now 2970)
 // The weights go back over their scores as the sum of two bfloat16; the sums are rescaled only when a row's maximum has grown by more than 2^8. A window of
 // packed tokens that holds several sequences is walked tile by tile (latent_tc_parts CTAs share it).
-// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us, one warp for all products 171, a second one 157, the
-// query by TMA too 144; 592 tokens behind 1024 62 / 57 / 53, 400 and 319 behind 900 with 3 single ones 73 / 67 / 65. A CTA's fixed part (its query rows, results 5000 clocks) is as much as five of its key tiles.
+// Measured, 2048 tokens, rows of 576, 16 heads, 512 columns out (floor 44 us): the mma.sync tiles of latent_attention.cu 856 us; launches of the same call one behind the other: one warp for all products
+// 171, a second one 157, the query by TMA too 144 (with new inputs, whose query rows come from memory, 177 before and 158 now); 592 tokens behind 1024 62 / 57 / 53, 400 and 319 behind 900 with 3 single
+// ones 73 / 67 / 65. A CTA's fixed part (its query rows, results 5000 clocks) is as much as five of its key tiles.
 // Tried and taken back: the query's rows read by the four warps one row after the other, 16 bytes per thread (26000 clocks: three times the address and place arithmetic, on one warp per scheduler).
 #include <cuda_bf16.h>
 

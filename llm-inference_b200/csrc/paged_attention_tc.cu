@@ -1,7 +1,7 @@
 // bfloat16 prompt portions of b200_paged_attention on tcgen05 / TMEM: 128 (token, query head) rows per tile, keys 64 at a time.
 //
-// What bounds it: the chain of a tile's key tiles. Per 128 x 64 scores of 128-wide heads the tensor pipe needs some 900 clocks (8 products of 64 columns from shared
-// memory at 49, 8 of 128 columns with weights from tensor memory at 65), the special-function unit 512; but a key tile's way from its scores through softmax (1000 clocks from
+// What bounds it: the chain of a tile's key tiles. Per 128 x 64 scores of 128-wide heads the tensor pipe is active for 768 clocks (8 products of 64 columns at 32, 8 of 128
+// columns at 64; issued one behind the other they take some 900), the special-function unit 512; but a key tile's way from its scores through softmax (1000 clocks from
 // one product's end to the other's start) and weighted sum back to a free score buffer takes 3400. So two groups of softmax warps take the key tiles in turn, each with
 // sums of its own, over four score buffers, and scores and weighted sums are issued by a warp each (one warp that issues both spends 1400 clocks per
 // key tile on waits, products and commits): about 1150 clocks per key tile, 1620 with one group alone on an SM. Long contexts of few rows are shared out over a cluster.
@@ -21,8 +21,9 @@
 //   cluster     up to eight CTAs walk consecutive shares of a tile's key tiles; sums, references and denominators go through distributed shared
 //               memory, each CTA adds and stores its part of the rows. Costs 3 us, so shares keep some eight key tiles.
 // Two groups take an SM alone; one group leaves room for a second CTA, which hides what a CTA does before its first and after its last product (3.5 and 2 us):
-// better only where many short tiles come in several rounds. Measured, 16 / 8 heads x 128, us, one group (two CTAs per SM, no sharing) / this: 2048 tokens 36.6 / 32.4, 1024 19.9 / 17.5, 64
-// tokens behind 4000 45 / 17, 256 behind 1000 and 4 single tokens 24.5 / 18.5, three portions up to 512 and 12 single tokens behind 4000, capped 143 / 107.
+// better only where many short tiles come in several rounds. Measured, launches of the same call one behind the other (with new inputs 0.5 to 6 more), 16 / 8 heads x 128, us, one group (two CTAs per SM, no
+// sharing) / this: 2048 tokens 40.1 / 32.3, 1024 19.3 / 17.0, 64 tokens behind 4000 54 / 16, 256 behind 1000 and 4 single tokens 23.1 / 18.5, three portions up to 512 and 12 single tokens behind 4000, capped
+// 119 / 107.
 // Tried and taken back: query rows in TMEM and three score buffers (the buffers' round trip costs more than the shared memory saves: 17.5 against 16.8 for 1024 tokens), one warp
 // for all products with three buffers (19.0), eight softmax warps per group, two threads per row (19.2: the pair has to meet at every tile), scores of 128 columns for both groups at
 // once (17.1, 33.4 for 2048: the groups run in step and wait for each other).
@@ -705,18 +706,18 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     const long long tiles = p.windows * units;
     const int steps = longest_seen > 0 ? (longest_seen + kTcKeys - 1) / kTcKeys : 0;
     // tiles of several entries that come in more than one round: up to 32 key tiles each, two CTAs per SM that hide each other's start and end are faster (16 / 8 heads x 128, us, one group / two: three
-    // portions of up to 680 21.0 / 28.4, of up to 512 behind 300 26.8 / 33.3, behind 1000 43.1 / 48.2), beyond that the shorter chain (behind 2000 69.6 / 70.4, behind 4000, capped, 143 / 119)
+    // portions of up to 680 20.7 / 25.7, of up to 512 behind 300 23.1 / 26.7, behind 1000 39.4 / 45.2), beyond that the shorter chain (behind 2000 63.7 / 65.9, behind 4000, capped, 119 / 107)
     // (values of 256 columns: one group, whose sums take an SM alone all the same)
     const bool short_tiles = several && tiles > sms && steps <= 32;
     p.two_groups = a.vdim > 128 || !short_tiles;
     // shared key tiles: while the clusters fit beside each other (clusters of four and eight do not fill every group of SMs), leave room for single tokens if there may be some, and keep eight key tiles or more
-    // per CTA (us at 1 / 2 / 4 / 8 CTAs: 100 tokens behind 3000 38.6 / 26.6 / 19.0 / 28.8, 300 40.8 / 28.1 / 37.1 / 45.2, 64 and 4 single ones behind 1000 19.2 / 16.9 / 14.5 / 16.5, behind 300 11.9 / 13.0 / 12.7 / 14.7,
-    // 512 and 8 single ones behind 4000 57.2 / 62.1 / 77.0 / 115)
+    // per CTA (us at 1 / 2 / 4 / 8 CTAs: 100 tokens behind 3000 38.5 / 26.1 / 18.5 / 28.2, 300 40.5 / 27.6 / 36.6 / 45.0, 64 and 4 single ones behind 1000 19.0 / 16.6 / 14.5 / 17.6, behind 300 11.8 / 12.8 / 12.4 / 14.6,
+    // 512 and 8 single ones behind 4000 57.0 / 61.5 / 77.5 / 115)
     const long long room = several ? 2 * sms / 3 : sms;
     while (p.two_groups && p.split2 < (tiles * 8 <= sms / 2 ? 3 : 2) && (tiles << (p.split2 + 1)) <= room && steps >= 12 && steps >= 8 << p.split2) ++p.split2;
-    // CTAs that share a window's tiles: four where they all start at once (portions of 53, 45 and 33 tokens lie in one window and a bit: 16 heads x 128, capped, 12.6 / 9.9 us)
+    // CTAs that share a window's tiles: four where they all start at once (portions of 53, 45 and 33 tokens lie in one window and a bit: 16 heads x 128, capped, two / four 13.6 / 9.1 us)
     if (several && p.split2 == 0 && tiles * 4 <= sms) p.parts = 4;
-    // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 90.2 / 84.3 us)
+    // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 88.4 / 83.0 us)
     p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && !short_tiles;
     const int singles = a.n_tokens - longest_entry;   // at most; with several entries at least one
     const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));   // CTAs of single tokens that fit beside the tiles'

@@ -461,7 +461,7 @@ int paged_decode(const PA& a, int longest_seen, int singles, long long room, cud
     int splits = 1;
     if (mixed) {
         // on what the portions' CTAs leave free (`room` CTAs) if eight single tokens can sit there beside each other, else behind them (us at 2 / 4 / 8 shares: 8 single tokens and a portion of 512 behind
-        // 4000 57.2 / 77.7 / 83.0, 4 and 64 36.8 / 31.7 / 40.9, 12 and three of 512, which fill the GPU, 123 / 119 / 133)
+        // 4000 56.7 / 60.4 / 70.4, 4 and 64 35.9 / 23.8 / 23.9, 12 and three of 512, which fill the GPU, capped, 105 / 106 / 119, 1 and three 90.3 / 83.3 / 83.1, 3 and three behind 2200, biased, 64.1 / 62.2 / 63.7)
         const long long likely = (long long)std::min(singles, 8) * a.kv_heads * a.maps;
         // (values of 256 columns, 16 / 8 heads, us at 2 / 4: 8 single tokens and three of 512 behind 300 31.8 / 36.0, behind 1800 69.8 / 73.0, 12 and two of 500 behind 1500, two maps, 87.0 / 96.1)
         if (room < likely) room = (a.vdim > 128 ? 2 : 4) * likely;
