@@ -632,6 +632,7 @@ struct TcPlan {
     long long windows;
     int parts, sorted, split2, bias;   // split2: log2 of the CTAs that share a tile's keys; bias: staged numbers
     bool two_groups;   // else one, and two CTAs per SM
+    bool chained;      // launched programmatically
 };
 
 template <int D, int DV, int W, int FORM, bool SHARED>
@@ -658,7 +659,7 @@ static int launch_tc(const PA& a, const TcPlan& p, cudaStream_t s) {
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
     }
-    if (pdl_enabled()) {
+    if (p.chained && pdl_enabled()) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
@@ -719,6 +720,10 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     if (several && p.split2 == 0 && tiles * 4 <= sms) p.parts = 4;
     // several rounds: the longest tiles first (three portions of up to 512 behind 4000: 88.4 / 83.0 us)
     p.sorted = several && p.windows > 1 && p.windows <= kTcSorted && (tiles << p.split2) > sms && !short_tiles;
+    // Tiles that start before the kernel ahead has ended sit down where room comes first: two to an SM where each should have one, or, in several rounds, out of their order (us behind a residual norm, programmatically / not,
+    // 16 / 8 heads x 128: one group, 600 tokens 16.2 / 14.3, 1500, window of 1024, 34.3 / 28.4, three portions of 512 and 4 single tokens behind 300 24.3 / 23.5; sorted, behind 4000, capped, 112 / 110; but two groups, 100
+    // tokens 7.0 / 7.7, 2048 31.5 / 32.7)
+    p.chained = p.two_groups && !p.sorted;
     const int singles = a.n_tokens - longest_entry;   // at most; with several entries at least one
     const long long free = (p.two_groups ? 2 : 1) * std::max(0ll, (p.two_groups ? sms : 2 * sms) - (tiles << p.split2));   // CTAs of single tokens that fit beside the tiles'
     int rc = -1;
