@@ -381,7 +381,7 @@ extern "C" int b200_paged_attention(const b200_paged_attention_args* p, void* st
     int longest_seen = p->chunk > 0 ? std::min(p->longest_context, p->chunk) : p->longest_context;
     if (p->window > 0) longest_seen = std::min(longest_seen, p->window);
     if (p->dtype == B200_BF16 && p->longest_entry != 1 && al16(p->q) && al16(p->out) && al16(p->k_pool) && al16(p->v_pool) && !(env && env[0] == '1')) {
-        const int rc = paged_attention_tc(a, p->longest_entry, longest_seen, s);
+        const int rc = paged_attention_tc(a, p->longest_entry, longest_seen, p->longest_context, s);
         if (rc >= 0) return rc;
     }
     if (p->dtype == B200_BF16 && p->longest_entry != 1 && (p->sink || p->dist_bias) && !(p->softcap > 0.f) && p->dim % 8 == 0 && p->vdim % 8 == 0 && al16(p->q) && al16(p->out) &&

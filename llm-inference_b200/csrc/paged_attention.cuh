@@ -70,7 +70,8 @@ int biased_tile(const PA& a, cudaStream_t s);
 // singles: 0, every token is; else only the tokens that are their sequence's only one in the batch, which are not more than this
 int paged_decode(const PA& a, int longest_seen, int singles, long long room, cudaStream_t s);
 // bfloat16 prompt portions on tcgen05 tiles (paged_attention_tc.cu); -1: not built for these sizes
-int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStream_t s);
+// longest_seen: longest_context, cut to the window or block
+int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, int longest_context, cudaStream_t s);
 // b200_paged_attention with weights mixed across heads (mixed_attention.cu); a.head_mix is set
 int mixed_attention(const PA& a, int dtype, int longest_entry, int longest_context, void* workspace, size_t workspace_bytes, cudaStream_t s);
 

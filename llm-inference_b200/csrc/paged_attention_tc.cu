@@ -43,7 +43,7 @@ namespace b200 {
 enum { kTcPlain = 0, kTcCapped = 1, kTcBiased = 2, kTcSigmoid = 3 };
 constexpr int kTcRows = 128, kTcKeys = 64;
 constexpr int kTcBox = kTcKeys * 128;         // bytes of 64 rows x 64 columns
-constexpr int kTcBiasFront = kTcKeys, kTcBiasPad = kTcBiasFront + 2 * kTcRows;   // distances in front of, and around, a head's staged table
+constexpr int kTcBiasFront = kTcKeys;          // distances in front of a head's staged table; behind it kTcRows + TQ: as far as a tile's last row sees where its first row sees the table's end
 constexpr int kTcSorted = 192;                // windows that a CTA puts in order, at most (their keys take the place of the rows' slots and positions)
 constexpr int kTcSplit = 8;                   // CTAs that share a tile's keys, at most
 constexpr int kTcBiasFloats = 12288;          // at most this many staged bias numbers per CTA
@@ -56,7 +56,7 @@ struct TcSmem {
     static constexpr int kQ = kTcRows * D * 2, kK = kTcKeys * D * 2, kV = kTcKeys * DV * 2;   // the query rows; a stage's bytes
     static constexpr int kOffK = kQ, kOffV = kOffK + kRing * kK, kOffBar = kOffV + kRing * kV, kOffSlot = kOffBar + 5 * kRing * 8;
     static constexpr int kOffMl = (kOffSlot + (2 * (kTcRows + 2) + 12) * 4 + 7) & ~7;   // (reference, sum) of every row and group
-    static constexpr int kOffBias = kOffMl + W * kTcRows * 8;
+    static constexpr int kOffBias = kOffMl + (W > 1 || DV > 128 ? W * kTcRows * 8 : 0);   // (one group that shares no tile with other CTAs has no use for them)
     static constexpr int kOffSums = kRing * kTcKeys;           // tensor memory: score buffers, then the groups' sums
     static constexpr int kTmemCols = kOffSums + W * DV <= 256 ? 256 : 512, kPerSm = kTmemCols == 256 ? 2 : 1;
     static_assert(kOffSums + W * DV <= 512, "tensor memory");
@@ -158,6 +158,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         if (warp == 1 && !early) tmem_alloc(tmem_slot, L::kTmemCols);
         tc_fence_before();
     }
+    const int bias_pad = kTcBiasFront + kTcRows + TQ;
     int tn = 0;   // staged distances per head: those that a row of the window can have
     if (FORM == kTcBiased && a.dist_bias) {
         // per head: entry kTcBiasFront + distance; distances below 0 (masked keys) and beyond the table repeat its ends, so that no index needs a clamp
@@ -166,7 +167,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
         for (int x = 0; x < R; ++x) {
             const float* src = a.dist_bias + (size_t)(g * R + x) * a.dist_n;
 #pragma unroll 4
-            for (int i = threadIdx.x; i < tn + kTcBiasPad; i += NT) bias_s[x * (tn + kTcBiasPad) + i] = src[min(max(i - kTcBiasFront, 0), tn - 1)] * 1.4426950408889634f;
+            for (int i = threadIdx.x; i < tn + bias_pad; i += NT) bias_s[x * (tn + bias_pad) + i] = src[min(max(i - kTcBiasFront, 0), tn - 1)] * 1.4426950408889634f;
         }
     }
     __syncthreads();
@@ -341,7 +342,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
             const float* brow = nullptr;
             float far_bias = 0.f;
             if (FORM == kTcBiased && a.dist_bias) {
-                brow = bias_s + hr * (tn + kTcBiasPad) + kTcBiasFront;
+                brow = bias_s + hr * (tn + bias_pad) + kTcBiasFront;
                 far_bias = a.dist_bias[(size_t)h * a.dist_n + a.dist_n - 1] * kLog2E;
             }
             float m = -1e30f, l = 0.f;   // m: what the exponents are taken against (the scores of FORM plain unscaled)
@@ -397,7 +398,7 @@ paged_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
                     }
                 } else if (FORM == kTcBiased) {
                     if (brow && !__all_sync(0xffffffffu, p - (k0 + kTcKeys - 1) >= a.dist_n - 1)) {
-                        const int most = tn - 1 + 2 * kTcRows - kTcKeys;
+                        const int most = tn - 1 + kTcRows + TQ - kTcKeys;
                         const float* b = brow + max(min(p - k0, most), 0);
                         if (__all_sync(0xffffffffu, p - k0 <= most)) {
 #pragma unroll
@@ -684,7 +685,7 @@ static int launch_tc_for(const PA& a, const TcPlan& p, cudaStream_t s) {
     return launch_tc_groups<D, DV, kTcPlain>(a, p, s);
 }
 
-int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStream_t s) {
+int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, int longest_context, cudaStream_t s) {
     if (longest_entry < 0 || longest_entry > a.n_tokens) longest_entry = 0;   // a limit instead of the batch's own number: unknown
     const int R = a.heads / a.kv_heads;
     // a cap beside a sink or a bias keeps the row kernel, whose weights stay in 32 bits
@@ -701,16 +702,24 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, cudaStr
     if (p.windows * 2 > 65535) return -1;
     if (a.dist_bias && !a.sigmoid && !(a.softcap > 0.f)) {
         if (a.dist_n > kTcBiasFloats) return -1;
-        p.bias = R * (a.dist_n + kTcBiasPad);
+        p.bias = R * (a.dist_n + kTcBiasFront + kTcRows + TQ);
         if (p.bias > kTcBiasFloats) return -1;
     }
     const long long tiles = p.windows * units;
     const int steps = longest_seen > 0 ? (longest_seen + kTcKeys - 1) / kTcKeys : 0;
     // tiles of several entries that come in more than one round: up to 32 key tiles each, two CTAs per SM that hide each other's start and end are faster (16 / 8 heads x 128, us, one group / two: three
     // portions of up to 680 20.7 / 25.7, of up to 512 behind 300 23.1 / 26.7, behind 1000 39.4 / 45.2), beyond that the shorter chain (behind 2000 63.7 / 65.9, behind 4000, capped, 119 / 107)
+    // One entry: the shorter chain as long as it decides. Beyond one round the tiles of rank sms and sms + 1 share an SM: keys that they see together against a tenth more than the longest tile sees; beyond two rounds of
+    // tiles two CTAs per SM, unless a cap lengthens the chain of long tiles or staged bias numbers leave room for one CTA only (us, one group / two, 16 / 8 heads x 128: 2048 tokens 37.1 / 32.0, 2400 42.6 / 45.3, 3000 53.1 / 61.8, capped
+    // 2400 54.5 / 51.1, 4000 112 / 108; window of 1024 1300 27.6 / 21.9, 1700 29.9 / 30.3, 2048 34.1 / 37.9, 4000 61.8 / 71.0; 32 / 16 heads, 600 behind 3000 64.2 / 78.8; 16 / 4, biased, 3000 95 / 76)
     // (values of 256 columns: one group, whose sums take an SM alone all the same)
-    const bool short_tiles = several && tiles > sms && steps <= 32;
-    p.two_groups = a.vdim > 128 || !short_tiles;
+    auto fits_twice = [&](int bytes) { return bytes + p.bias * 4 + 1024 + 1024 <= 228 * 1024 / 2; };   // (what the driver keeps per CTA)
+    const bool twice = a.dim == 64 ? fits_twice(TcSmem<64, 64, 1>::kOffBias) : fits_twice(TcSmem<128, 128, 1>::kOffBias);
+    const double before = std::max(0, longest_context - a.n_tokens), shared_by = before + a.n_tokens * std::max(0.0, 1.0 - (double)sms / tiles);
+    // (a portion of up to a block that begins inside one has its longest tiles at either end)
+    const bool uneven = a.chunk > 0 ? before > 0 && a.n_tokens <= a.chunk : 2 * std::min<double>(shared_by, longest_seen) > 1.1 * longest_seen;
+    const bool short_tiles = several && tiles > sms && steps <= 32, many_tiles = !several && tiles > sms && steps > 0 && (tiles > 2 * sms ? !(a.softcap > 0.f) || steps <= 32 : uneven) && twice;
+    p.two_groups = a.vdim > 128 || !(short_tiles || many_tiles);
     // shared key tiles: while the clusters fit beside each other (clusters of four and eight do not fill every group of SMs), leave room for single tokens if there may be some, and keep eight key tiles or more
     // per CTA (us at 1 / 2 / 4 / 8 CTAs: 100 tokens behind 3000 38.5 / 26.1 / 18.5 / 28.2, 300 40.5 / 27.6 / 36.6 / 45.0, 64 and 4 single ones behind 1000 19.0 / 16.6 / 14.5 / 17.6, behind 300 11.8 / 12.8 / 12.4 / 14.6,
     // 512 and 8 single ones behind 4000 57.0 / 61.5 / 77.5 / 115)

@@ -396,3 +396,20 @@ def test_more_tiles_of_wide_values_than_the_gpu_holds_at_once(S, before):
         want = reference(q[b], k[b], v[b], list(range(before[b], before[b] + new[b])), o)
         assert float((got[at:at + new[b]] - want).norm() / want.norm()) < 5e-3, b
         at += new[b]
+
+
+@pytest.mark.parametrize("form,before,n", [("plain", 0, 1300), ("plain", 1500, 500), ("blocks", 0, 1300), ("sigmoid", 0, 1300), ("biased", 0, 1300), ("capped", 0, 1300)])
+@pytest.mark.parametrize("H,G,d", [(32, 16, 128), (32, 8, 64)])
+def test_one_prompt_of_more_tiles_than_two_rounds(S, form, before, n, H, G, d):
+    """one entry whose tiles come in more than two rounds, or behind more than it brings in more than one: one group of softmax warps and two CTAs per SM, where staged bias numbers leave room for
+    them. The bound of test_prompt_portions_beside_single_tokens"""
+    g = torch.Generator().manual_seed(H + before + d)
+    o = options(form, H, d, g)
+    if o.get("window"):
+        o["window"] = 500
+    k, v, kp, vp, table = sequences(g, [before + n], G, 1, d, d, 64)
+    q = torch.randn(n, H, 1, d, generator=g).bfloat16().double()
+    pos = list(range(before, before + n))
+    got = run(S, q.bfloat16().cuda(), kp, vp, table, 64, [0] * n, pos, o, n, f32=False)
+    want = reference(q, k[0], v[0], pos, o)
+    assert float((got - want).norm() / want.norm()) < 5e-3
