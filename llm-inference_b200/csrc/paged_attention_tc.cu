@@ -710,15 +710,16 @@ int paged_attention_tc(const PA& a, int longest_entry, int longest_seen, int lon
     // tiles of several entries that come in more than one round: up to 32 key tiles each, two CTAs per SM that hide each other's start and end are faster (16 / 8 heads x 128, us, one group / two: three
     // portions of up to 680 20.7 / 25.7, of up to 512 behind 300 23.1 / 26.7, behind 1000 39.4 / 45.2), beyond that the shorter chain (behind 2000 63.7 / 65.9, behind 4000, capped, 119 / 107)
     // One entry: the shorter chain as long as it decides. Beyond one round the tiles of rank sms and sms + 1 share an SM: keys that they see together against a tenth more than the longest tile sees; beyond two rounds of
-    // tiles two CTAs per SM, unless a cap lengthens the chain of long tiles or staged bias numbers leave room for one CTA only (us, one group / two, 16 / 8 heads x 128: 2048 tokens 37.1 / 32.0, 2400 42.6 / 45.3, 3000 53.1 / 61.8, capped
-    // 2400 54.5 / 51.1, 4000 112 / 108; window of 1024 1300 27.6 / 21.9, 1700 29.9 / 30.3, 2048 34.1 / 37.9, 4000 61.8 / 71.0; 32 / 16 heads, 600 behind 3000 64.2 / 78.8; 16 / 4, biased, 3000 95 / 76)
+    // tiles two CTAs per SM, a cap, which lengthens the chain, aside (one group for short tiles beyond two rounds), and unless staged bias numbers leave room for one CTA only (us, one group / two, 16 / 8 heads x 128: 2048 tokens 37.1 / 32.0, 2400 42.6 / 45.3, 3000 53.1 / 61.8, capped
+    // 2400 54.5 / 51.1, 4000 112 / 108; window of 1024, fp32 outputs, 1300 27.6 / 21.9, 1700 29.9 / 30.3, 2048 34.1 / 37.9, 4000 61.8 / 71.0; 32 / 16 heads, 600 behind 3000 64.2 / 78.8; 16 / 4, biased, 3000 95 / 76)
+    // fp32 outputs keep two groups, whose chains of sums are half as long: 5.1e-6 of the result's norm for 2048 tokens behind a window of 1024, 5.5e-6 in one group (34.1 against 37.9 us).
     // (values of 256 columns: one group, whose sums take an SM alone all the same)
     auto fits_twice = [&](int bytes) { return bytes + p.bias * 4 + 1024 + 1024 <= 228 * 1024 / 2; };   // (what the driver keeps per CTA)
     const bool twice = a.dim == 64 ? fits_twice(TcSmem<64, 64, 1>::kOffBias) : fits_twice(TcSmem<128, 128, 1>::kOffBias);
     const double before = std::max(0, longest_context - a.n_tokens), shared_by = before + a.n_tokens * std::max(0.0, 1.0 - (double)sms / tiles);
     // (a portion of up to a block that begins inside one has its longest tiles at either end)
     const bool uneven = a.chunk > 0 ? before > 0 && a.n_tokens <= a.chunk : 2 * std::min<double>(shared_by, longest_seen) > 1.1 * longest_seen;
-    const bool short_tiles = several && tiles > sms && steps <= 32, many_tiles = !several && tiles > sms && steps > 0 && (tiles > 2 * sms ? !(a.softcap > 0.f) || steps <= 32 : uneven) && twice;
+    const bool short_tiles = several && tiles > sms && steps <= 32, many_tiles = !several && !a.out_f32 && tiles > sms && steps > 0 && (a.softcap > 0.f ? tiles > 2 * sms && steps <= 32 : tiles > 2 * sms || uneven) && twice;
     p.two_groups = a.vdim > 128 || !(short_tiles || many_tiles);
     // shared key tiles: while the clusters fit beside each other (clusters of four and eight do not fill every group of SMs), leave room for single tokens if there may be some, and keep eight key tiles or more
     // per CTA (us at 1 / 2 / 4 / 8 CTAs: 100 tokens behind 3000 38.5 / 26.1 / 18.5 / 28.2, 300 40.5 / 27.6 / 36.6 / 45.0, 64 and 4 single ones behind 1000 19.0 / 16.6 / 14.5 / 17.6, behind 300 11.8 / 12.8 / 12.4 / 14.6,
